@@ -26,7 +26,8 @@ def ref_src():
     if "REF_SRC" in os.environ:
         return os.environ["REF_SRC"] if os.path.isdir(os.environ["REF_SRC"]) else None
     root = ref_root()
-    return os.path.join(root, "src") if root else None
+    src = os.path.join(root, "src") if root else None
+    return src if src and os.path.isdir(src) else None  # an empty checkout counts as absent
 
 
 def ref_file(*parts):
