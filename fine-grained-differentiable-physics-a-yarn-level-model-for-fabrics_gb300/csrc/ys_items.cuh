@@ -15,7 +15,7 @@ namespace ys {
 // direction (slot = k * ntot + anchor), faces one per cell (top-left node),
 // shear segments four per crossing (slot = type * ntot + crossing).
 struct Records {
-  double* edge;   // [kEdgeFields][2][ntot]
+  double* edge;   // [kEdgeFields][2][ntot] (kE_* offsets)
   double* bend;   // [kBendFields][2][ntot]
   double* face;   // [6][ntot]
   double* shear;  // [kShearFields][4][ntot]
@@ -82,7 +82,8 @@ YS_HD void gather_elements(const View& v, const Records& R, int n) {
         const int anc = a == 0 ? n : n - step;
         auto E = [&](int f) { return recT<T>(R.edge, R.dedge, f, 2, k, nt, anc); };
         const int p = 3 * a;  // block (a, a)
-        const T cI = E(kE_llI + p), cP = E(kE_llP + p);
+        const double end = a == 0 ? 1.0 : -1.0;
+        const T cI = E(kE_llI + p), cP = E(kE_lP), cl = E(kE_cl), cle = E(kE_cle);
         const T d[3] = {E(kE_d), E(kE_d + 1), E(kE_d + 2)};
         for (int r = 0; r < 3; ++r)
           for (int c = 0; c < 3; ++c) LL[3 * r + c] += (r == c ? cI : 0.0) + cP * ((r == c ? 1.0 : 0.0) - d[r] * d[c]);
@@ -90,14 +91,14 @@ YS_HD void gather_elements(const View& v, const Records& R, int n) {
           LE[2 * r + k] += E(kE_le + 3 * p + r);
           EL[3 * k + r] += E(kE_el + 3 * p + r);
           B[r] += E(kE_b + 4 * a + r);
-          CL[r] += E(kE_cl + 3 * a + r);
-          CLE[3 * k + r] += E(kE_cle + 3 * a + r);
+          CL[r] += end * (cl * d[r]);
+          if (in) CLE[3 * k + r] += cle * d[r];
         }
         EE[k] += E(kE_ee + p);
         B[3 + k] += E(kE_b + 4 * a + 3);
-        FE[k] += E(kE_fkd + 3 * a);
-        KEE[k] += E(kE_fkd + 3 * a + 1);
-        DEE[k] += E(kE_fkd + 3 * a + 2);
+        FE[k] += E(kE_fe + a);
+        KEE[k] += E(kE_kee + a);
+        DEE[k] += E(kE_dee + a);
       }
       // bend segments along k with middle m: this node is n2 (m = n + step),
       // n0 (m = n) or n1 (m = n - step)
@@ -219,7 +220,7 @@ YS_HD void gather_elements(const View& v, const Records& R, int n) {
       const int anc = dir > 0 ? n : nb;
       auto E = [&](int f) { return recT<T>(R.edge, R.dedge, f, 2, k, nt, anc); };
       const int p = 2 * a + o;
-      const T cI = E(kE_llI + p), cP = E(kE_llP + p);
+      const T cI = E(kE_llI + p), cP = -E(kE_lP);
       const T d[3] = {E(kE_d), E(kE_d + 1), E(kE_d + 2)};
       for (int r = 0; r < 3; ++r)
         for (int c = 0; c < 3; ++c) LL[3 * r + c] += (r == c ? cI : 0.0) + cP * ((r == c ? 1.0 : 0.0) - d[r] * d[c]);

@@ -57,6 +57,20 @@ YS_HD void matmul3(const T A[3][3], const T B[3][3], T O[3][3]) {
   for (int i = 0; i < 3; ++i)
     for (int j = 0; j < 3; ++j) O[i][j] = A[i][0] * B[0][j] + A[i][1] * B[1][j] + A[i][2] * B[2][j];
 }
+// 1 / sqrt(x): one device instruction sequence instead of a square root and a
+// division (1 ulp)
+YS_HD double rsqrt_(double x) {
+#if defined(__CUDA_ARCH__)
+  return ::rsqrt(x);
+#else
+  return 1.0 / ::sqrt(x);
+#endif
+}
+template <int K>
+YS_HD Dual<K> rsqrt_(const Dual<K>& a) {
+  const double r = rsqrt_(a.v);
+  return chain(a, r, -0.5 * r * (r * r));
+}
 YS_HD double ld(const double* p, int comp, int ntot, int node) { return p[(int64_t)comp * ntot + node]; }
 YS_HD double& st(double* p, int comp, int ntot, int node) { return p[(int64_t)comp * ntot + node]; }
 
@@ -115,453 +129,245 @@ YS_HD T cloth_mu(const View& v, int c) { return ldpT<T>(&v.cp[c].mu, v.dmu ? v.d
 
 // ------------------------------------------------------------ edge element
 // Local DOFs of an edge: x0 (0..2), e0 (3), x1 (4..6), e1 (7), where e is the
-// Eulerian coordinate along the edge's yarn (u for warp, v for weft).
-// Every node-node 3x3 block an edge produces is a I + b P with P = I - d d^T
-// (mass, inertia and dM/dt blocks are multiples of I, stretch adds P), so an
-// edge's contribution to A is held as 4 (a, b) pairs plus the Eulerian
-// couplings; block index p = 2*(row node) + (column node).
+// Eulerian coordinate along the edge's yarn (u for warp, v for weft); blocks
+// are indexed p = 2 * (row node) + (column node). Every node-node block is
+// iso I + s lP (I - d d^T) with s = +1 on the diagonal and -1 across (mass,
+// inertia and dM/dt blocks are multiples of I, stretch adds the projector).
+//
+// The record of an edge: what the gathers read of it.
+constexpr int kE_llI = 0;   // [4]     iso of A[x(n_a)][x(n_b)]
+constexpr int kE_lP = 4;    //         -h^2 ks / l
+constexpr int kE_d = 5;     // [3]     edge direction
+constexpr int kE_le = 8;    // [4][3]  A[x(n_a)][e(n_b)]
+constexpr int kE_el = 20;   // [4][3]  A[e(n_a)][x(n_b)]
+constexpr int kE_ee = 32;   // [4]     A[e(n_a)][e(n_b)]
+constexpr int kE_b = 36;    // [8]     contribution to b
+constexpr int kE_fe = 44;   // [2]     F_E before friction
+constexpr int kE_kee = 46;  // [2]     dF_E/dE, position
+constexpr int kE_dee = 48;  // [2]     dF_E/dE, velocity
+constexpr int kE_cl = 50;   //         crimp compression: +cl d at n0, -cl d at n1
+constexpr int kE_cle = 51;  //         its Eulerian derivative: cle d at the interior ends
+constexpr int kEdgeFields = 52;
+
 template <class T>
 struct EdgeOut {
-  T llI[4], llP[4];  // A[x(n_a)][x(n_b)] = llI I + llP P
-  T d[3];            // edge direction (defines P)
-  T le[4][3];        // A[x(n_a)][e(n_b)]
-  T el[4][3];        // A[e(n_a)][x(n_b)]
-  T ee[4];           // A[e(n_a)][e(n_b)]
-  T b[8];            // contribution to b
-  T fe[2], kee[2], dee[2];  // F_E, dF_E/dE (position, velocity) before friction
-  T cl[2][3], cle[2][3];    // crimp-compression accumulators
-  T V[8];            // the step's velocity vector restricted to the edge (not stored)
-  double h, h2;
-  bool in[2];
-  bool trunc;        // tangents of b through F and v only (M and D held constant)
+  T f[kEdgeFields];
 };
-constexpr int kEdgeFields = 65;
 
-enum Mat { kM = 0, kK = 1, kD = 2 };
-
-template <class T>
-YS_HD double wt(const EdgeOut<T>& o, int X) { return X == kM ? 1.0 : X == kK ? -o.h2 : -o.h; }
-// a matrix coefficient as it enters b = h F + (M - h D^T) v: detached when
-// the tangents follow the reference's autograd, where M and D are built
-// without a graph (src/MatrixMp.cpp:40-99)
-template <class T>
-YS_HD T mcoef(const EdgeOut<T>& o, const T& x) { return o.trunc ? detach(x) : x; }
-
-// block (a, b) += val I of matrix X; b receives M V and -h D^T V
-// (src/TrainHelper.cpp:19-20). LL blocks of X_LL[find_index(f, d, "LL")] are
-// written transposed by To_Sparse_Mat (src/MatrixMp.cpp:54-65); a I + b P is
-// symmetric, so the transpose changes nothing here.
-template <class T>
-YS_HD void acc_LLi(EdgeOut<T>& o, int X, int a, int b, const T& val) {
-  o.llI[2 * a + b] += wt(o, X) * val;
-  if (X == kM) {
-    const T m = mcoef(o, val);
-    for (int r = 0; r < 3; ++r) o.b[4 * a + r] += m * o.V[4 * b + r];
-  } else if (X == kD) {
-    const T m = mcoef(o, val);
-    for (int r = 0; r < 3; ++r) o.b[4 * b + r] -= o.h * m * o.V[4 * a + r];
-  }
-}
-template <class T>
-YS_HD void acc_LLp(EdgeOut<T>& o, int a, int b, const T& val) { o.llP[2 * a + b] += -o.h2 * val; }  // stiffness only
-// A[x(n_a)][e(n_b)] (X_LE[find_index(n_a, n_b, "EL") + k])
-template <class T>
-YS_HD void acc_LE(EdgeOut<T>& o, int X, int a, int b, const T* vec) {
-  const double w = wt(o, X);
-  T s = 0.0;
-  for (int r = 0; r < 3; ++r) {
-    o.le[2 * a + b][r] += w * vec[r];
-    if (X == kM) o.b[4 * a + r] += mcoef(o, vec[r]) * o.V[4 * b + 3];
-    if (X == kD) s += mcoef(o, vec[r]) * o.V[4 * a + r];
-  }
-  if (X == kD) o.b[4 * b + 3] -= o.h * s;
-}
-// A[e(n_a)][x(n_b)] (X_EL[find_index(n_b, n_a, "EL") + k])
-template <class T>
-YS_HD void acc_EL(EdgeOut<T>& o, int X, int a, int b, const T* vec) {
-  const double w = wt(o, X);
-  T s = 0.0;
-  for (int c = 0; c < 3; ++c) {
-    o.el[2 * a + b][c] += w * vec[c];
-    if (X == kM) s += mcoef(o, vec[c]) * o.V[4 * b + c];
-    if (X == kD) o.b[4 * b + c] -= o.h * mcoef(o, vec[c]) * o.V[4 * a + 3];
-  }
-  if (X == kM) o.b[4 * a + 3] += s;
-}
-template <class T>
-YS_HD void acc_EE(EdgeOut<T>& o, int X, int a, int b, const T& val) {
-  o.ee[2 * a + b] += wt(o, X) * val;
-  if (X == kM) o.b[4 * a + 3] += mcoef(o, val) * o.V[4 * b + 3];
-  else if (X == kD) o.b[4 * b + 3] -= o.h * mcoef(o, val) * o.V[4 * a + 3];
-  if (a == b) {
-    if (X == kK) o.kee[a] += val;
-    else if (X == kD) o.dee[a] += val;
-  }
-}
-template <class T>
-YS_HD void acc_F(EdgeOut<T>& o, int dof, const T& f) {
-  o.b[dof] += o.h * f;
-  if ((dof & 3) == 3) o.fe[dof >> 2] += f;
-}
-
-// One node-pair block p = 2a + b of an edge Jacobian written with the
-// pattern shared by Inertia_D_Pos, Inertia_D_Vel, MDotVDot_D_Pos and
-// MDotVDot_D_Vel (src/PhysicsCloth.cpp:1544-1600, 1848-1900, 2226-2308,
-// 2505-2577): C(i, j) = d(force DOF i)/d(DOF j) in edge-local order, given as
-// the isotropic node-node factor iso, the (x, e) column lec[r] = C(4a+r,
-// 4b+3), the (e, x) row elr[c] = C(4a+3, 4b+c) and eev = C(4a+3, 4b+3), added
-// with sign s under the reference's interior tests. Each section adds a
-// block as soon as it is formed, so no section holds all four blocks.
-template <class T>
-YS_HD void acc_jac_p(EdgeOut<T>& o, int X, double s, int p, const T& iso, const T* lec, const T* elr, const T& eev) {
-  const int a = p >> 1, b = p & 1;
-  acc_LLi(o, X, a, b, s * iso);
-  const bool ok = (a == b) ? o.in[a] : (o.in[0] && o.in[1]);
-  if (!ok) return;
-  T t[3];
-  for (int r = 0; r < 3; ++r) t[r] = s * lec[r];
-  acc_LE(o, X, a, b, t);
-  for (int c = 0; c < 3; ++c) t[c] = s * elr[c];
-  acc_EL(o, X, a, b, t);
-  acc_EE(o, X, a, b, s * eev);
-}
-
-template <class T>
-YS_HD void edge_store_groups(const View& v, double* buf, double* dbuf, int n0, int k, const EdgeOut<T>& o,
-                             bool early, bool late);
-
-// All terms of one edge (src/PhysicsCloth.cpp:64-80): Mass, Gravity, Stretch,
-// Inertia, MDotVDot, ParaColli; forces and both Jacobians. With ebuf given,
-// the fields that are final once ParaColli is done (the stretch projector's
-// factors and direction, the crimp accumulators) are stored to the record
-// there, so they hold no registers through the kinetic-energy terms; the
-// caller then stores the rest with edge_store_groups(..., false, true).
-template <class T>
-YS_HD void edge_element(const View& v, int n0, int n1, int k, EdgeOut<T>& o, double* ebuf = nullptr,
-                        double* edbuf = nullptr) {
+// All terms of one edge (src/PhysicsCloth.cpp:64-80): Mass (250-338), Gravity
+// (340-425), Stretch (427-577), ParaColli (989-1069), Inertia (1071-1901) and
+// MDotVDot (1903-2577), forces and both Jacobians, as they enter
+// A = M - h^2 K - h D and b = h F + (M - h D^T) V; put(field, value) receives
+// each field of the record once.
+//
+// With w = dx / du, m0 = 2 a0 + a1, m1 = a0 + 2 a1 (mu0, mu1 the same of the
+// Eulerian velocities), S = a0 mu0 + a1 mu1, D = a1 - a0 and delta = e1 - e0,
+// the reference's expressions collapse: both mixed sums of its quadratic form
+// equal S; Inertia's forces are r6 (S - See w) and r6 (w.w See - a.Ma) / 2;
+// B_M m and B_dot m of MDotVDot combine to r_b = r6 (delta m_b - mu_b D); the
+// node-node part of MDotVDot_D_Pos cancels; the two velocity Jacobians add to
+// multiples of m, D and mu w. Every block is then a few multiples of S, w, D,
+// m and G. Its quirks are kept: the sign-asymmetric mixed block of
+// Inertia_D_Pos (1357-1361; the +1 / -3 below), MDotVDot_D_Pos added and with
+// the squared r6 of "- rho / 6 r" (2154-2234), ParaColli_D proportional to the
+// overlap itself. Term by term as the reference writes them, an edge took
+// 1,690 FP64 operations; this form takes about 400.
+template <class T, class Put>
+YS_HD void edge_terms(const View& v, int n0, int n1, int k, Put&& put) {
   const int nt = v.ntot;
   const ClothParams& P = v.cp[v.node_cloth[n0]];
   const uint8_t f0 = v.flags[n0], f1 = v.flags[n1];
-  o.in[0] = (f0 & YS_INTERIOR) != 0;
-  o.in[1] = (f1 & YS_INTERIOR) != 0;
+  const bool in[2] = {(f0 & YS_INTERIOR) != 0, (f1 & YS_INTERIOR) != 0};
+  const bool both = in[0] && in[1];
   const int line = (k == 0) ? P.warp_line_off + v.node_v[n0] : P.weft_line_off + v.node_u[n0];
   const T rho = ldpT<T>(v.line_rho, v.dline_rho, line, v.nlines), ks = ldpT<T>(v.line_ks, v.dline_ks, line, v.nlines);
-  o.h = v.h;
-  o.h2 = v.h * v.h;
-  o.trunc = v.trunc != 0;
-  for (int p = 0; p < 4; ++p) {
-    o.llI[p] = o.llP[p] = o.ee[p] = 0.0;
-    for (int r = 0; r < 3; ++r) o.le[p][r] = o.el[p][r] = 0.0;
-  }
-  for (int i = 0; i < 8; ++i) o.b[i] = 0.0;
-  for (int t = 0; t < 2; ++t) {
-    o.fe[t] = o.kee[t] = o.dee[t] = 0.0;
-    for (int i = 0; i < 3; ++i) o.cl[t][i] = o.cle[t][i] = 0.0;
-  }
-  // geometry (src/ClothUnit.h:134-154)
-  T x0[3], x1[3], a0[3], a1[3], dx[3], w[3], d[3];
+  const double h = v.h, mh2 = -(v.h * v.h);
+  T a[2][3], e[2], dx[3], gx = 0.0;
   for (int i = 0; i < 3; ++i) {
-    x0[i] = ldT<T>(v.X, v.dX, i, nt, n0); x1[i] = ldT<T>(v.X, v.dX, i, nt, n1);
-    a0[i] = ldT<T>(v.V, v.dV, i, nt, n0); a1[i] = ldT<T>(v.V, v.dV, i, nt, n1);
+    const T x0 = ldT<T>(v.X, v.dX, i, nt, n0), x1 = ldT<T>(v.X, v.dX, i, nt, n1);
+    dx[i] = x1 - x0;
+    gx += P.G[i] * (x0 + x1);
+    a[0][i] = ldT<T>(v.V, v.dV, i, nt, n0);
+    a[1][i] = ldT<T>(v.V, v.dV, i, nt, n1);
   }
   const T du = ldT<T>(v.UV, v.dUV, k, nt, n1) - ldT<T>(v.UV, v.dUV, k, nt, n0);
-  const T e0 = ldT<T>(v.UVD, v.dUVD, k, nt, n0), e1 = ldT<T>(v.UVD, v.dUVD, k, nt, n1);
-  // reciprocals of the Eulerian length and of the length: one division each,
-  // the terms below multiply by them
-  const T idu = 1.0 / du, idu2 = idu * idu, idu3 = idu2 * idu;
-  for (int i = 0; i < 3; ++i) { dx[i] = x1[i] - x0[i]; w[i] = dx[i] * idu; }
-  const T l = norm3(dx);
-  const T il = 1.0 / l;
-  for (int i = 0; i < 3; ++i) { d[i] = dx[i] * il; o.d[i] = d[i]; }
-  for (int i = 0; i < 3; ++i) { o.V[i] = a0[i]; o.V[4 + i] = a1[i]; }
-  o.V[3] = o.in[0] ? e0 : 0.0;
-  o.V[7] = o.in[1] ? e1 : 0.0;
-  const T wTw = dot3(w, w);
-  const T nw = norm3(w);
-  T t3[3];
-
-  // ---- Mass (src/PhysicsCloth.cpp:250-338)
-  {
-    const T coeff = (1.0 / 6.0) * rho * du;
-    acc_LLi(o, kM, 0, 0, 2.0 * coeff);
-    acc_LLi(o, kM, 1, 0, coeff);
-    acc_LLi(o, kM, 0, 1, coeff);
-    acc_LLi(o, kM, 1, 1, 2.0 * coeff);
-    T LE2[3], LE1[3];
-    for (int r = 0; r < 3; ++r) { LE2[r] = -2.0 * coeff * w[r]; LE1[r] = -1.0 * coeff * w[r]; }
-    const T EE2 = 2.0 * coeff * wTw, EE1 = 0.5 * EE2;
-    if (o.in[0]) { acc_LE(o, kM, 0, 0, LE2); acc_EL(o, kM, 0, 0, LE2); acc_EE(o, kM, 0, 0, EE2); }
-    if (o.in[1]) { acc_LE(o, kM, 1, 1, LE2); acc_EL(o, kM, 1, 1, LE2); acc_EE(o, kM, 1, 1, EE2); }
-    if (o.in[0] && o.in[1]) {
-      acc_LE(o, kM, 1, 0, LE1);
-      acc_LE(o, kM, 0, 1, LE1);
-      acc_EL(o, kM, 0, 1, LE1);  // M_EL[find_index(n1, n0)] = E0L1
-      acc_EL(o, kM, 1, 0, LE1);  // M_EL[find_index(n0, n1)] = E1L0
-      acc_EE(o, kM, 0, 1, EE1);
-      acc_EE(o, kM, 1, 0, EE1);
-    }
-  }
-  // ---- Gravity_F / Gravity_D (src/PhysicsCloth.cpp:340-425)
-  {
-    for (int i = 0; i < 3; ++i) {
-      const T g = 0.5 * rho * P.G[i] * du;
-      acc_F(o, i, -g);
-      acc_F(o, 4 + i, -g);
-    }
-    T sx[3] = {x0[0] + x1[0], x0[1] + x1[1], x0[2] + x1[2]};
-    const T gx = P.G[0] * sx[0] + P.G[1] * sx[1] + P.G[2] * sx[2];
-    if (o.in[0]) acc_F(o, 3, -((-0.5) * rho * gx));
-    if (o.in[1]) acc_F(o, 7, -(0.5 * rho * gx));
-    T g0[3], g1[3];
-    for (int r = 0; r < 3; ++r) { g0[r] = 0.5 * rho * P.G[r]; g1[r] = -g0[r]; }
-    if (o.in[0]) { acc_EL(o, kK, 0, 0, g0); acc_LE(o, kK, 0, 0, g0); }
-    if (o.in[1]) { acc_EL(o, kK, 1, 1, g1); acc_LE(o, kK, 1, 1, g1); }
-    if (o.in[0] && o.in[1]) {
-      acc_LE(o, kK, 1, 0, g0);  // L1E0
-      acc_LE(o, kK, 0, 1, g1);  // L0E1
-      acc_EL(o, kK, 0, 1, g0);  // E0L1
-      acc_EL(o, kK, 1, 0, g1);  // E1L0
-    }
-  }
-  // ---- Stretch_F / Stretch_D (src/PhysicsCloth.cpp:427-577)
+  e[0] = ldT<T>(v.UVD, v.dUVD, k, nt, n0);
+  e[1] = ldT<T>(v.UVD, v.dUVD, k, nt, n1);
+  const T idu = 1.0 / du, aidu = fabs(idu);
+  const T il = rsqrt_(dot3(dx, dx));
+  T w[3], d[3];
+  for (int i = 0; i < 3; ++i) { w[i] = dx[i] * idu; d[i] = dx[i] * il; }
+  const T ww = dot3(w, w);
+  const T nw = (dot3(dx, dx) * il) * aidu;  // |w|
+  const T r6 = (1.0 / 6.0) * rho, q = r6 * du;
+  const T zero = T(0.0);
+  // ---- stretch scalars; the crimp accumulators
+  const T strf = ks * (nw - 1.0), ksw = ks * aidu, ksi = ks * idu;
   {
     const double sgn = (k == 0) ? 1.0 : -1.0;
-    for (int i = 0; i < 3; ++i) {
-      const T f = ks * (nw - 1) * d[i];
-      acc_F(o, i, f);
-      acc_F(o, 4 + i, -f);
-      o.cl[0][i] += sgn * f;
-      o.cl[1][i] -= sgn * f;
-    }
-    const T fe = 0.5 * ks * (nw * nw - 1);
-    if (o.in[0]) acc_F(o, 3, -fe);
-    if (o.in[1]) acc_F(o, 7, fe);
-    // LL = (ks / l) P - (ks / du) I, +LL on (0,0), (1,1) and -LL across
-    const T cP = ks * il, cI = -(ks * idu);
-    acc_LLp(o, 0, 0, cP); acc_LLp(o, 1, 0, -cP); acc_LLp(o, 0, 1, -cP); acc_LLp(o, 1, 1, cP);
-    acc_LLi(o, kK, 0, 0, cI); acc_LLi(o, kK, 1, 0, -cI); acc_LLi(o, kK, 0, 1, -cI); acc_LLi(o, kK, 1, 1, cI);
-    const T EE = -ks * ((nw * nw) * idu);
-    T LE[3], EL[3], nLE[3], nEL[3];
-    for (int r = 0; r < 3; ++r) {
-      LE[r] = ks * (nw * idu) * d[r];
-      EL[r] = ks * idu * w[r];
-      nLE[r] = -LE[r];
-      nEL[r] = -EL[r];
-    }
-    if (o.in[0]) {
-      acc_LE(o, kK, 0, 0, LE); acc_EL(o, kK, 0, 0, EL); acc_EE(o, kK, 0, 0, EE);
-      for (int i = 0; i < 3; ++i) o.cle[0][i] += sgn * LE[i];
-    }
-    if (o.in[1]) {
-      acc_LE(o, kK, 1, 1, LE); acc_EL(o, kK, 1, 1, EL); acc_EE(o, kK, 1, 1, EE);
-      for (int i = 0; i < 3; ++i) o.cle[1][i] += sgn * LE[i];
-    }
-    if (o.in[0] && o.in[1]) {
-      acc_LE(o, kK, 1, 0, nLE); acc_LE(o, kK, 0, 1, nLE);
-      acc_EL(o, kK, 0, 1, nEL); acc_EL(o, kK, 1, 0, nEL);
-      acc_EE(o, kK, 0, 1, -EE); acc_EE(o, kK, 1, 0, -EE);
-    }
+    put(kE_cl, sgn * strf);
+    put(kE_cle, sgn * (ksw * nw));
+    put(kE_lP, mh2 * (ks * il));
+    for (int i = 0; i < 3; ++i) put(kE_d + i, d[i]);
   }
-  // ---- ParaColli_F / ParaColli_D (src/PhysicsCloth.cpp:989-1069)
+  // ---- shared kinetic sums
+  T m[2][3], mu[2], D[3];
+  for (int i = 0; i < 3; ++i) {
+    m[0][i] = 2.0 * a[0][i] + a[1][i];
+    m[1][i] = a[0][i] + 2.0 * a[1][i];
+    D[i] = a[1][i] - a[0][i];
+  }
+  mu[0] = 2.0 * e[0] + e[1];
+  mu[1] = e[0] + 2.0 * e[1];
+  const T dl = e[1] - e[0], See = e[0] * mu[0] + e[1] * mu[1];
+  const T wD = dot3(w, D), r6i = r6 * idu, dlww = dl * ww;
+  const T swe = r6i * See;  // r6 See / du
+  T S[3];
+  for (int i = 0; i < 3; ++i) S[i] = a[0][i] * mu[0] + a[1][i] * mu[1];
+  // ---- F, and b = h F + ...
+  T bx[2][3], be[2], re[2], Dm[2];
+  for (int b = 0; b < 2; ++b) {
+    Dm[b] = dot3(D, m[b]);
+    re[b] = r6 * (2.0 * wD * mu[b] - dlww * mu[b] - Dm[b]);
+  }
   {
-    const T dd = (((f0 & YS_FLIP) != 0) != ((f1 & YS_FLIP) != 0)) ? 4.0 * P.R : 2.0 * P.R;
-    T rl = dd - du;
+    T rl = ((((f0 & YS_FLIP) != 0) != ((f1 & YS_FLIP) != 0)) ? 4.0 * P.R : 2.0 * P.R) - du;
     if (rl < 0) rl = 0.0;
-    const T fu0 = P.kc * P.L * rl;
-    if (o.in[0]) acc_F(o, 3, fu0);
-    if (o.in[1]) acc_F(o, 7, -fu0);
-    const T ee = -P.kc * P.L * rl;
-    if (o.in[0]) acc_EE(o, kK, 0, 0, ee);
-    if (o.in[1]) acc_EE(o, kK, 1, 1, ee);
-    if (o.in[0] && o.in[1]) { acc_EE(o, kK, 0, 1, ee); acc_EE(o, kK, 1, 0, ee); }
-  }
-  if (ebuf) edge_store_groups(v, ebuf, edbuf, n0, k, o, true, false);
-
-  // ---- kinetic-energy terms: shared sums
-  T m0a[3], m1a[3];
-  for (int i = 0; i < 3; ++i) { m0a[i] = 2.0 * a0[i] + a1[i]; m1a[i] = a0[i] + 2.0 * a1[i]; }
-  const T m0e = 2.0 * e0 + e1, m1e = e0 + 2.0 * e1;
-  const T Saa = dot3(a0, m0a) + dot3(a1, m1a);
-  T Sae[3], Sea[3];
-  for (int i = 0; i < 3; ++i) { Sae[i] = a0[i] * m0e + a1[i] * m1e; Sea[i] = e0 * m0a[i] + e1 * m1a[i]; }
-  const T See = e0 * m0e + e1 * m1e;
-  const T r6 = (1.0 / 6.0) * rho;
-  const T sc = 1.0 / 6.0 * rho * du;
-  const T wSae = dot3(w, Sae), wSea = dot3(w, Sea);
-  const T pj = -(-idu);  // (-w_x0)_j for the active component j
-
-  // ---- Inertia_F (src/PhysicsCloth.cpp:1071-1186)
-  {
-    for (int j = 0; j < 3; ++j) {
-      const T sj = (-2.0 * idu2 * dx[j]);
-      const T T0 = 0.5 * (sc * (pj * Sae[j] + pj * Sea[j] + sj * See));
-      acc_F(o, j, T0);
-      acc_F(o, 4 + j, -T0);
+    const T crowd = P.kc * P.L * rl;
+    const T Saa = dot3(a[0], m[0]) + dot3(a[1], m[1]);
+    // stretch, gravity, contact and inertia act oppositely on the two ends
+    const T Fe = 0.5 * (rho * gx - ks * (ww - 1.0) + r6 * (ww * See - Saa)) + crowd;
+    const T F0 = Fe - re[0], F1 = -Fe - re[1];
+    put(kE_fe + 0, in[0] ? F0 : zero);
+    put(kE_fe + 1, in[1] ? F1 : zero);
+    be[0] = h * F0;
+    be[1] = h * F1;
+    const T hr = 0.5 * (rho * du);
+    for (int i = 0; i < 3; ++i) {
+      const T t = strf * d[i] + r6 * (S[i] - See * w[i]), g = hr * P.G[i];
+      bx[0][i] = h * (t - g - r6 * (dl * m[0][i] - mu[0] * D[i]));
+      bx[1][i] = h * (-t - g - r6 * (dl * m[1][i] - mu[1] * D[i]));
     }
-    const T QM = Saa - wSae - wSea + wTw * See;
-    const T Quv = (-idu) * wSae + (-idu) * wSea + (2.0 * idu) * wTw * See;
-    const T Tuv0 = 0.5 * (-(1.0 / 6.0) * rho * QM + (1.0 / 6.0) * rho * du * Quv);
-    if (o.in[0]) acc_F(o, 3, Tuv0);
-    if (o.in[1]) acc_F(o, 7, -Tuv0);
-  }
-  // ---- Inertia_D_Pos (src/PhysicsCloth.cpp:1188-1601)
-  {
-    const T T00 = 0.5 * (r6 * ((2.0 * idu2) * See));
-    T Tx0uv0[3], Tuv0x0[3];
-    for (int j = 0; j < 3; ++j) {
-      const T Qx0 = pj * Sae[j] + pj * Sea[j] + (-2.0 * idu2 * dx[j]) * See;
-      const T c2 = idu2;
-      // the sign-asymmetric mixed block of src/PhysicsCloth.cpp:1357-1361
-      const T Qx0uv0 = (-c2) * Sae[j] + (-(-c2)) * Sea[j] + ((-4.0 * idu2) * w[j]) * See;
-      Tx0uv0[j] = 0.5 * ((-1.0 / 6.0) * rho * Qx0 + (1.0 / 6.0) * rho * du * Qx0uv0);
-      Tuv0x0[j] = 0.5 * ((-1.0 / 6.0) * rho * Qx0 + (1.0 / 6.0) * rho * du * (-Qx0uv0));
-    }
-    const T Quv0 = (-idu) * wSae + (-idu) * wSea + (2.0 * idu) * wTw * See;
-    const T c6 = 2.0 * idu2;
-    const T Quvuv = (-c6) * wSae + (-c6) * wSea + (6.0 * idu2) * wTw * See;
-    const T Tuu = 0.5 * ((-1.0 / 6.0) * rho * Quv0 - (1.0 / 6.0) * rho * Quv0 + (1.0 / 6.0) * rho * du * Quvuv);
+    // the Eulerian diagonal blocks: K_ee and D_ee
+    const T Kee = ksi * ww;  // stretch: s (-ks ww / du)
+    T kk[2][2], dd[2][2];
     for (int p = 0; p < 4; ++p) {
-      const double sgn = ((p >> 1) == (p & 1)) ? 1.0 : -1.0;
-      T lec[3], elr[3];
-      for (int r = 0; r < 3; ++r) { lec[r] = sgn * Tx0uv0[r]; elr[r] = sgn * Tuv0x0[r]; }
-      acc_jac_p(o, kK, 1.0, p, sgn * T00, lec, elr, sgn * Tuu);
+      const int ra = p >> 1, cb = p & 1;
+      const T kin = r6i * (Dm[ra] - 3.0 * (dl * dot3(w, m[ra])) + 8.0 * (dlww * mu[ra]));
+      const T base = ra == cb ? swe * ww - Kee : Kee - swe * ww;
+      kk[ra][cb] = base - crowd + (cb == 0 ? -kin : kin) - r6 * re[ra];
+    }
+    dd[0][0] = dd[1][1] = (2.0 * r6) * (dlww - 2.0 * wD);
+    dd[0][1] = (2.0 * r6) * (ww * mu[1] - wD);
+    dd[1][0] = (-2.0 * r6) * (ww * mu[0] + wD);
+    const T qw = q * ww;
+    for (int p = 0; p < 4; ++p) {
+      const int ra = p >> 1, cb = p & 1;
+      const bool ok = ra == cb ? in[ra] : both;
+      const T ee = (ra == cb ? 2.0 : 1.0) * qw + mh2 * kk[ra][cb] - h * dd[ra][cb];
+      put(kE_ee + p, ok ? ee : zero);
+      if (ra == cb) {
+        put(kE_kee + ra, ok ? kk[ra][ra] : zero);
+        put(kE_dee + ra, ok ? dd[ra][ra] : zero);
+      }
     }
   }
-  // ---- Inertia_D_Vel (src/PhysicsCloth.cpp:1602-1901): row x_j of C = M_xj qdot
+  // ---- iso blocks
   {
-    const T me_[2] = {m0e, m1e};
-    const T* ma_[2] = {m0a, m1a};
-    for (int b = 0; b < 2; ++b) {
-      const T iso = sc * (pj * me_[b]);
-      T lec[3], elr[3];
-      const T wm = dot3(w, ma_[b]);
-      for (int r = 0; r < 3; ++r) {
-        lec[r] = sc * (pj * ma_[b][r] + (-2.0 * idu2 * dx[r]) * me_[b]);
-        elr[r] = -(1.0 / 6.0) * rho * (ma_[b][r] - w[r] * me_[b]) + (1.0 / 6.0) * rho * du * ((-idu) * w[r] * me_[b]);
-      }
-      const T eev = -(1.0 / 6.0) * rho * (-wm + wTw * me_[b]) +
-                         (1.0 / 6.0) * rho * du * ((-idu) * wm + (2.0 * idu) * wTw * me_[b]);
-      for (int a = 0; a < 2; ++a) {
-        const double sgn = a == 0 ? 1.0 : -1.0;  // rows of x1 / uv1 are the negated rows of x0 / uv0
-        T lp[3], ep[3];
-        for (int r = 0; r < 3; ++r) { lp[r] = sgn * lec[r]; ep[r] = sgn * elr[r]; }
-        acc_jac_p(o, kD, 1.0, 2 * a + b, sgn * iso, lp, ep, sgn * eev);
-      }
-    }
+    const T kI = mh2 * (swe * idu - ksi), hr6 = 2.0 * h * r6;
+    put(kE_llI + 0, 2.0 * q + kI + hr6 * dl);
+    put(kE_llI + 1, q - kI - hr6 * mu[0]);
+    put(kE_llI + 2, q - kI + hr6 * mu[1]);
+    put(kE_llI + 3, 2.0 * q + kI + hr6 * dl);
   }
-  // ---- MDotVDot (src/PhysicsCloth.cpp:1903-2577)
+  // ---- (M - h D^T) V, V = (a0, E0, a1, E1) with the interior velocities only.
+  // M and D enter b without a graph in the reference (src/MatrixMp.cpp:40-99),
+  // so the reference-mode tangents hold their factors constant.
   {
-    const T dud = e1 - e0;
-    T wd[3];
-    for (int i = 0; i < 3; ++i) wd[i] = ((a1[i] - a0[i]) * du - dx[i] * dud) * idu2;
-    const T wTwd = dot3(w, wd) + dot3(wd, w);
-    // B_M m and B_dot m for m = m0, m1 (4-vectors); M_dot qdot = r6 dud (B_M m) + r6 du (B_dot m)
-    T BMm[2][4], Bdm[2][4], r[8];
-    for (int b = 0; b < 2; ++b) {
-      const T* ma = b == 0 ? m0a : m1a;
-      const T me = b == 0 ? m0e : m1e;
-      for (int i = 0; i < 3; ++i) { BMm[b][i] = ma[i] + (-w[i]) * me; Bdm[b][i] = (-wd[i]) * me; }
-      BMm[b][3] = (-w[0]) * ma[0] + (-w[1]) * ma[1] + (-w[2]) * ma[2] + wTw * me;
-      Bdm[b][3] = (-wd[0]) * ma[0] + (-wd[1]) * ma[1] + (-wd[2]) * ma[2] + wTwd * me;
-      for (int i = 0; i < 4; ++i) r[4 * b + i] = r6 * dud * BMm[b][i] + r6 * du * Bdm[b][i];
+    auto cst = [&](const T& x) { return v.trunc ? detach(x) : x; };
+    const T cq = cst(q), ce0 = cst(e[0]), ce1 = cst(e[1]), c2 = cst(-2.0 * h * r6);
+    const T cm0 = 2.0 * ce0 + ce1, cm1 = ce0 + 2.0 * ce1, cdl = ce1 - ce0;
+    T ca[2][3], cw[3], cD[3];
+    for (int i = 0; i < 3; ++i) {
+      ca[0][i] = cst(a[0][i]);
+      ca[1][i] = cst(a[1][i]);
+      cw[i] = cst(w[i]);
+      cD[i] = ca[1][i] - ca[0][i];
     }
-    // MDotVDot_F: F -= M_dot qdot
-    for (int i = 0; i < 3; ++i) { acc_F(o, i, -r[i]); acc_F(o, 4 + i, -r[4 + i]); }
-    if (o.in[0]) acc_F(o, 3, -r[3]);
-    if (o.in[1]) acc_F(o, 7, -r[7]);
-    // MDotVDot_D_Pos, added (src/PhysicsCloth.cpp:2154-2234)
-    for (int t = 0; t < 2; ++t) {
-      const double sw = t == 0 ? -1.0 : 1.0;
-      const T wxj = sw * idu;
-      const T P1 = -wxj;
-      const T wdxj = t == 0 ? (dud * idu2) : -(dud * idu2);
-      const T P2 = -wdxj;
-      T wuv[3], wduv[3];
-      for (int i = 0; i < 3; ++i) wuv[i] = (sw * w[i]) * idu;
-      const T wTwuv = sw * (2.0 * idu) * wTw;
-      for (int i = 0; i < 3; ++i) {
-        wduv[i] = (a1[i] - a0[i]) * idu2 - (4 * dx[i] * dud) * idu3;
-        if (t == 1) wduv[i] = -wduv[i];
-      }
-      const T wTwduv = 2 * dot3(wuv, wd) + 2 * dot3(wduv, w);
-      for (int b = 0; b < 2; ++b) {
-        const T* ma = b == 0 ? m0a : m1a;
-        const T me = b == 0 ? m0e : m1e;
-        const T iso = r6 * dud * (P1 * me) + r6 * du * (P2 * me);
-        T elr[3], lec[3];
-        for (int j = 0; j < 3; ++j) {
-          const T S1 = (sw * 2.0 * idu2 * dx[j]);
-          const T S2 = 2 * (wxj * wd[j]) + 2 * (w[j] * wdxj);
-          elr[j] = r6 * dud * (P1 * ma[j] + S1 * me) + r6 * du * (P2 * ma[j] + S2 * me);
-          lec[j] = r6 * dud * (wuv[j] * me) - r6 * r[4 * b + j] + r6 * du * (-wduv[j] * me);
-        }
-        const T eev = r6 * dud * (dot3(wuv, ma) + wTwuv * me) - r6 * r[4 * b + 3] +
-                      r6 * du * (-dot3(wduv, ma) + wTwduv * me);
-        acc_jac_p(o, kK, 1.0, 2 * b + t, iso, lec, elr, eev);
-      }
+    const T E0 = in[0] ? e[0] : zero, E1 = in[1] ? e[1] : zero;
+    const T B0 = both ? e[0] : zero, B1 = both ? e[1] : zero;
+    // x rows: M, then -h D^T (c2 = -2 h r6)
+    const T k0 = c2 * (E0 * cm0 + B1 * cm1) - cq * (2.0 * E0 + B1);
+    const T k1 = -(c2 * (B0 * cm0 + E1 * cm1)) - cq * (2.0 * E1 + B0);
+    const T x00 = 2.0 * cq - c2 * cdl, x01 = cq - c2 * cm1, x10 = cq + c2 * cm0;
+    for (int i = 0; i < 3; ++i) {
+      bx[0][i] += x00 * a[0][i] + x01 * a[1][i] + k0 * cw[i] - (3.0 * c2) * (E0 * ca[0][i]);
+      bx[1][i] += x10 * a[0][i] + x00 * a[1][i] + k1 * cw[i] + (3.0 * c2) * (E1 * ca[1][i]);
     }
-    // MDotVDot_D_Vel, subtracted (src/PhysicsCloth.cpp:2342-2577)
-    for (int t = 0; t < 2; ++t) {
-      const double sw = t == 0 ? -1.0 : 1.0;
-      const T wdj = sw * idu;
-      const T P1 = -wdj;
-      T wdv[3];
-      for (int i = 0; i < 3; ++i) wdv[i] = (t == 0 ? idu : -idu) * w[i];
-      const T wtwd = 2 * dot3(w, wdv);
-      const T cm = (t == 0 ? -1.0 : 1.0) * (1.0 / 6.0) * rho;
-      for (int b = 0; b < 2; ++b) {
-        const T* ma = b == 0 ? m0a : m1a;
-        const T me = b == 0 ? m0e : m1e;
-        const double f = (b == t) ? 2.0 : 1.0;  // [[2B, B], [B, 2B]] block factor of M_dot
-        const T iso = (1.0 / 6.0) * rho * du * (P1 * me) + (r6 * dud * (f * 1.0) + r6 * du * (f * 0.0));
-        T elr[3], lec[3];
-        for (int j = 0; j < 3; ++j) {
-          const T S1 = 2 * (w[j] * wdj);
-          elr[j] = (1.0 / 6.0) * rho * du * (P1 * ma[j] + S1 * me) +
-                   (r6 * dud * (f * -w[j]) + r6 * du * (f * -wd[j]));
-          lec[j] = cm * BMm[b][j] + (1.0 / 6.0) * rho * du * (-wdv[j] * me) +
-                   (r6 * dud * (f * -w[j]) + r6 * du * (f * -wd[j]));
-        }
-        const T eev = cm * BMm[b][3] + (1.0 / 6.0) * rho * du * (-dot3(wdv, ma) + wtwd * me) +
-                      (r6 * dud * (f * wTw) + r6 * du * (f * wTwd));
-        acc_jac_p(o, kD, -1.0, 2 * b + t, iso, lec, elr, eev);
-      }
+    // e rows
+    const T wa0 = dot3(cw, a[0]), wa1 = dot3(cw, a[1]);
+    const T cww = dot3(cw, cw), cwD = dot3(cw, cD);
+    const T Da0 = dot3(cD, a[0]), Da1 = dot3(cD, a[1]);
+    const T aa0 = dot3(ca[0], a[0]) + 2.0 * dot3(ca[1], a[0]), aa1 = 2.0 * dot3(ca[0], a[1]) + dot3(ca[1], a[1]);
+    const T dia = cdl * cww - 2.0 * cwD;
+    T r0 = c2 * (aa0 - cm0 * wa0 + dia * E0) - cq * (2.0 * wa0 - 2.0 * cww * E0);
+    T r1 = c2 * (cm1 * wa1 - aa1 + dia * E1) - cq * (2.0 * wa1 - 2.0 * cww * E1);
+    const T s0 = c2 * (Da1 + cm0 * wa1 - (cww * cm0 + cwD) * e[1]) - cq * (wa1 - cww * e[1]);
+    const T s1 = c2 * (Da0 - cm1 * wa0 + (cww * cm1 - cwD) * e[0]) - cq * (wa0 - cww * e[0]);
+    if (both) { r0 += s0; r1 += s1; }
+    be[0] += r0;
+    be[1] += r1;
+    for (int i = 0; i < 3; ++i) { put(kE_b + i, bx[0][i]); put(kE_b + 4 + i, bx[1][i]); }
+    put(kE_b + 3, in[0] ? be[0] : zero);
+    put(kE_b + 7, in[1] ? be[1] : zero);
+  }
+  // ---- the mixed blocks, component by component
+  {
+    const T hr6 = -2.0 * h * r6;             // -h D's common factor
+    const T p0 = mh2 * (r6i * mu[0]), p1 = mh2 * (r6i * mu[1]);
+    const T kS = mh2 * r6i, kr = mh2 * (r6 * r6);
+    const T uE = mh2 * (ksw - swe), uL = mh2 * (ksi + 3.0 * swe);
+    const T q2 = -2.0 * q, hm0 = hr6 * mu[0], hm1 = hr6 * mu[1];
+    for (int i = 0; i < 3; ++i) {
+      const T g = (0.5 * mh2 * P.G[i]) * rho;
+      const T sS = kS * S[i];
+      const T U = uE * w[i] - sS, UL = uL * w[i] - sS;
+      const T dw = dl * w[i];
+      const T Y = D[i] - 3.0 * dw, Z = 2.0 * (D[i] - dw);
+      const T R0 = kr * (dl * m[0][i] - mu[0] * D[i]), R1 = kr * (dl * m[1][i] - mu[1] * D[i]);
+      const T y0 = p0 * Y - g, y1 = p1 * Y - g;
+      // A[x(n_a)][e(n_c)] = -f q w - h^2 (s U + sw_c (mu_a Y - g) - r6 r_a) - h D
+      const T le00 = (q2 - hm0) * w[i] + hr6 * m[1][i] + U - y0 - R0;
+      const T le01 = (-q - hm1) * w[i] + hr6 * D[i] - U + y0 - R0;
+      const T le10 = (hm0 - q) * w[i] + hr6 * D[i] - U - y1 - R1;
+      const T le11 = (q2 + hm1) * w[i] - hr6 * m[0][i] + U + y1 - R1;
+      // A[e(n_a)][x(n_c)] = -f q w - h^2 (s UL - sw_a g + sw_c mu_a Z) - h D
+      const T z0 = p0 * Z, z1 = p1 * Z;
+      const T el00 = (q2 + hm0) * w[i] - (3.0 * hr6) * a[0][i] + UL + g - z0;
+      const T el01 = (-q - hm0) * w[i] - UL + g + z0;
+      const T el10 = (hm1 - q) * w[i] - UL - g - z1;
+      const T el11 = (q2 - hm1) * w[i] + (3.0 * hr6) * a[1][i] + UL - g + z1;
+      put(kE_le + i, in[0] ? le00 : zero);
+      put(kE_le + 3 + i, both ? le01 : zero);
+      put(kE_le + 6 + i, both ? le10 : zero);
+      put(kE_le + 9 + i, in[1] ? le11 : zero);
+      put(kE_el + i, in[0] ? el00 : zero);
+      put(kE_el + 3 + i, both ? el01 : zero);
+      put(kE_el + 6 + i, both ? el10 : zero);
+      put(kE_el + 9 + i, in[1] ? el11 : zero);
     }
   }
-  (void)t3;
 }
-
-// record layout of an edge in the per-element buffer (field-major over the
-// 2 * ntot edge slots: slot = k * ntot + n0; tangents in dbuf)
-// `early`: llP, d, cl, cle (final after the stretch and contact terms);
-// `late`: every other field
 template <class T>
-YS_HD void edge_store_groups(const View& v, double* buf, double* dbuf, int n0, int k, const EdgeOut<T>& o,
-                             bool early, bool late) {
-  const int nt = v.ntot;
-  int f = 0;
-  auto put = [&](const T& x, bool g) {
-    if (g) stT(buf, dbuf, 2 * f + k, nt, n0, x);
-    ++f;
-  };
-  for (int p = 0; p < 4; ++p) put(o.llI[p], late);
-  for (int p = 0; p < 4; ++p) put(o.llP[p], early);
-  for (int i = 0; i < 3; ++i) put(o.d[i], early);
-  for (int p = 0; p < 4; ++p) for (int r = 0; r < 3; ++r) put(o.le[p][r], late);
-  for (int p = 0; p < 4; ++p) for (int r = 0; r < 3; ++r) put(o.el[p][r], late);
-  for (int p = 0; p < 4; ++p) put(o.ee[p], late);
-  for (int i = 0; i < 8; ++i) put(o.b[i], late);
-  for (int t = 0; t < 2; ++t) { put(o.fe[t], late); put(o.kee[t], late); put(o.dee[t], late); }
-  for (int t = 0; t < 2; ++t) for (int i = 0; i < 3; ++i) put(o.cl[t][i], early);
-  for (int t = 0; t < 2; ++t) for (int i = 0; i < 3; ++i) put(o.cle[t][i], early);
+YS_HD void edge_element(const View& v, int n0, int n1, int k, EdgeOut<T>& o) {
+  edge_terms<T>(v, n0, n1, k, [&](int f, const T& x) { o.f[f] = x; });
 }
+// the record in the per-element buffer: field-major over the 2 * ntot edge
+// slots (slot = k * ntot + n0), tangents in dbuf
 template <class T>
 YS_HD void edge_store(const View& v, double* buf, double* dbuf, int n0, int k, const EdgeOut<T>& o) {
-  edge_store_groups(v, buf, dbuf, n0, k, o, true, true);
+  for (int f = 0; f < kEdgeFields; ++f) stT(buf, dbuf, 2 * f + k, v.ntot, n0, o.f[f]);
 }
-// field offsets of the layout above
-constexpr int kE_llI = 0, kE_llP = 4, kE_d = 8, kE_le = 11, kE_el = 23, kE_ee = 35, kE_b = 39, kE_fkd = 47,
-              kE_cl = 53, kE_cle = 59;
 
 // ------------------------------------------------------------ bend element
 template <class T>
