@@ -109,60 +109,52 @@ YS_HD void gather_elements(const View& v, const Records& R, int n) {
         if (mid < 1 || mid > len - 2) continue;
         const int anc = role == 0 ? n + step : role == 1 ? n : n - step;
         auto Bf = [&](int f) { return recT<T>(R.bend, R.dbend, f, 2, k, nt, anc); };
-        T blk[9];
-        if (role == 0) {
-          for (int i = 0; i < 9; ++i) blk[i] = Bf(kB_L22 + i);
-        } else if (role == 2) {
-          for (int i = 0; i < 9; ++i) blk[i] = Bf(kB_L11 + i);
-        } else {  // L00 = -(L10 + L20) (src/PhysicsCloth.cpp:709)
-          for (int i = 0; i < 9; ++i) {
-            const T L10 = -(Bf(kB_L11 + i) + Bf(kB_L12 + i)), L20 = -(Bf(kB_L21 + i) + Bf(kB_L22 + i));
-            blk[i] = -(L10 + L20);
+        if (role != 1) {
+          const int f = role == 0 ? kB_L22 : kB_L11;
+          T blk[6];
+          for (int i = 0; i < 6; ++i) blk[i] = Bf(f + i);
+          for (int r = 0; r < 3; ++r)
+            for (int c = 0; c < 3; ++c) LL[3 * r + c] += blk[sym3(r, c)];
+        } else {  // L00 = L11 + L12 + L21 + L22 (src/PhysicsCloth.cpp:709), symmetric
+          T blk[6], x12[9];
+          for (int i = 0; i < 6; ++i) blk[i] = Bf(kB_L11 + i) + Bf(kB_L22 + i);
+          for (int i = 0; i < 9; ++i) x12[i] = Bf(kB_L12 + i);
+          for (int r = 0; r < 3; ++r)
+            for (int c = r; c < 3; ++c) {
+              const T t = blk[sym3(r, c)] + (x12[3 * r + c] + x12[3 * c + r]);
+              LL[3 * r + c] += t;
+              if (c != r) LL[3 * c + r] += t;
+            }
+        }
+        if (role == 1) {  // n0: F_x0 = -(F_x1 + F_x2), F_u0 = 0
+          for (int r = 0; r < 3; ++r) {
+            B[r] -= h * (Bf(kB_F1 + r) + Bf(kB_F2 + r));
+            CL[r] -= sgn * (Bf(kB_cF1 + r) + Bf(kB_cF2 + r));
+          }
+          continue;
+        }
+        // n2 (src/PhysicsCloth.cpp:737-753) or n1 (755-772): its force F, and
+        // end / du times it in the Eulerian couplings (+ at n2, - at n1)
+        const int f0 = role == 0 ? kB_F2 : kB_F1, g0 = role == 0 ? kB_cF2 : kB_cF1;
+        const double end = role == 0 ? 1.0 : -1.0;
+        const T idu = end * Bf(kB_idu), cidu = (end * sgn) * Bf(kB_cidu);
+        for (int r = 0; r < 3; ++r) {
+          const T F = Bf(f0 + r), cF = Bf(g0 + r);
+          B[r] += h * F;
+          CL[r] += sgn * cF;
+          if (in) {
+            const T t = mh2 * (idu * F);
+            LE[2 * r + k] += t;
+            EL[3 * k + r] += t;
+            CLE[3 * k + r] += cidu * cF;
           }
         }
-        for (int r = 0; r < 3; ++r)
-          for (int c = 0; c < 3; ++c) LL[3 * r + c] += mh2 * blk[3 * c + r];
-        if (role == 0) {  // n2 (src/PhysicsCloth.cpp:737-753)
-          for (int r = 0; r < 3; ++r) {
-            B[r] += h * Bf(kB_Fx2 + r);
-            CL[r] += sgn * Bf(kB_cFx2 + r);
-          }
-          if (in) {
-            const T e11 = Bf(kB_E1E1), fu2 = Bf(kB_Fu2);
-            for (int r = 0; r < 3; ++r) {
-              const T l2e2 = -Bf(kB_L2E1 + r);
-              LE[2 * r + k] += mh2 * l2e2;
-              EL[3 * k + r] += mh2 * l2e2;  // E2L2 = -E1L2 carries the values of -L2E1
-              CLE[3 * k + r] += sgn * (-Bf(kB_cL2E1 + r));
-            }
-            EE[k] += mh2 * e11;
-            KEE[k] += e11;
-            B[3 + k] += h * fu2;
-            FE[k] += fu2;
-          }
-        } else if (role == 2) {  // n1 (src/PhysicsCloth.cpp:755-772)
-          for (int r = 0; r < 3; ++r) {
-            B[r] += h * Bf(kB_Fx1 + r);
-            CL[r] += sgn * Bf(kB_cFx1 + r);
-          }
-          if (in) {
-            const T e11 = Bf(kB_E1E1), fu1 = -1 * Bf(kB_Fu2);
-            for (int r = 0; r < 3; ++r) {
-              const T l1e1 = Bf(kB_L1E1 + r);
-              LE[2 * r + k] += mh2 * l1e1;
-              EL[3 * k + r] += mh2 * l1e1;
-              CLE[3 * k + r] += sgn * Bf(kB_cL1E1 + r);
-            }
-            EE[k] += mh2 * e11;
-            KEE[k] += e11;
-            B[3 + k] += h * fu1;
-            FE[k] += fu1;
-          }
-        } else {  // n0: F_x0 = -(F_x1 + F_x2), F_u0 = 0
-          for (int r = 0; r < 3; ++r) {
-            B[r] += h * (-(Bf(kB_Fx1 + r) + Bf(kB_Fx2 + r)));
-            CL[r] += sgn * (-(Bf(kB_cFx1 + r) + Bf(kB_cFx2 + r)));
-          }
+        if (in) {
+          const T e11 = Bf(kB_E1E1), fu = end * Bf(kB_Fu2);
+          EE[k] += mh2 * e11;
+          KEE[k] += e11;
+          B[3 + k] += h * fu;
+          FE[k] += fu;
         }
       }
     }
@@ -237,18 +229,20 @@ YS_HD void gather_elements(const View& v, const Records& R, int n) {
         if (mid < 1 || mid > len - 2) continue;
         const int ancb = which == 0 ? n : nb;
         auto Bf = [&](int f) { return recT<T>(R.bend, R.dbend, f, 2, k, nt, ancb); };
-        T blk[9];
-        for (int i = 0; i < 9; ++i) {
-          const T L11 = Bf(kB_L11 + i), L12 = Bf(kB_L12 + i), L21 = Bf(kB_L21 + i), L22 = Bf(kB_L22 + i);
-          if (which == 0) blk[i] = dir > 0 ? -(L11 + L21) : -(L12 + L22);  // L01 or L02
-          else blk[i] = dir > 0 ? -(L21 + L22) : -(L11 + L12);             // L20 or L10
-        }
+        // L01 = -(L11 + L21), L10 = -(L11 + L12), L02 = -(L12 + L22),
+        // L20 = -(L21 + L22), written transposed: L21 = L12^T, so L12
+        // enters as it is towards the next crossing and transposed towards the last
+        const int fs = (which == 0) == (dir > 0) ? kB_L11 : kB_L22;
+        T blk[6], x12[9];
+        for (int i = 0; i < 6; ++i) blk[i] = Bf(fs + i);
+        for (int i = 0; i < 9; ++i) x12[i] = Bf(kB_L12 + i);
         for (int r = 0; r < 3; ++r)
-          for (int c = 0; c < 3; ++c) LL[3 * r + c] += mh2 * blk[3 * c + r];
+          for (int c = 0; c < 3; ++c) LL[3 * r + c] -= blk[sym3(r, c)] + (dir < 0 ? x12[3 * c + r] : x12[3 * r + c]);
         // Eulerian couplings of Bending_D (src/PhysicsCloth.cpp:774-822):
         // q = L1E1 + L2E1 = L0E2 = E2L0 = -L0E1 = -E1L0
         T q[3];
-        for (int r = 0; r < 3; ++r) q[r] = Bf(kB_L1E1 + r) + Bf(kB_L2E1 + r);
+        const T idu = -Bf(kB_idu);
+        for (int r = 0; r < 3; ++r) q[r] = idu * (Bf(kB_F1 + r) + Bf(kB_F2 + r));
         if (which == 0 && in && inb) {
           if (dir < 0)  // row n0 = n, column e / x of n2 = nb
             for (int r = 0; r < 3; ++r) { LE[r] += mh2 * q[r]; EL[r] += mh2 * q[r]; }
@@ -277,9 +271,9 @@ YS_HD void gather_elements(const View& v, const Records& R, int n) {
     const bool ok = mid >= 1 && mid <= len - 2;
     const int anc = n + dir * step;
     for (int r = 0; r < 3; ++r)
-      for (int c = 0; c < 3; ++c)  // n is n2 (dir +1): L21; n is n1 (dir -1): L12
+      for (int c = 0; c < 3; ++c)  // transposed L21 = L12^T where n is n2 (dir +1), transposed L12 where n is n1
         putA(YS_SLOT_LL + 9 * s + 3 * r + c, n,
-            ok ? T(mh2 * recT<T>(R.bend, R.dbend, (dir > 0 ? kB_L21 : kB_L12) + 3 * c + r, 2, k, nt, anc)) : T(0.0));
+            ok ? recT<T>(R.bend, R.dbend, kB_L12 + (dir > 0 ? 3 * r + c : 3 * c + r), 2, k, nt, anc) : T(0.0));
   }
   // diagonal neighbours: shear only (gather_shear_finalize)
   for (int s = 9; s < 13; ++s)

@@ -71,6 +71,20 @@ YS_HD Dual<K> rsqrt_(const Dual<K>& a) {
   const double r = rsqrt_(a.v);
   return chain(a, r, -0.5 * r * (r * r));
 }
+// x / l from l and il = 1 / l, correctly rounded but for rare ties: the
+// product and its residual, two operations more than the bare product. An
+// axis-aligned x gives exactly +-1 (x = l), as a division does.
+YS_HD double quot(double x, double l, double il) {
+  const double q = x * il;
+  return fma(fma(-q, l, x), il, q);
+}
+template <int K>
+YS_HD Dual<K> quot(const Dual<K>& x, const Dual<K>& l, const Dual<K>& il) {
+  Dual<K> r;
+  r.v = quot(x.v, l.v, il.v);
+  for (int k = 0; k < K; ++k) r.d[k] = (x.d[k] - r.v * l.d[k]) * il.v;
+  return r;
+}
 YS_HD double ld(const double* p, int comp, int ntot, int node) { return p[(int64_t)comp * ntot + node]; }
 YS_HD double& st(double* p, int comp, int ntot, int node) { return p[(int64_t)comp * ntot + node]; }
 
@@ -370,106 +384,76 @@ YS_HD void edge_store(const View& v, double* buf, double* dbuf, int n0, int k, c
 }
 
 // ------------------------------------------------------------ bend element
+// Geometry of a bend segment x2 - x0 - x1 and the factors of its terms
+// (src/ClothUnit.h:197-210): unit directions d1, d2, a = P1 d2 and b = P2 d1
+// (the directions projected across each other), the angle th of cosine
+// c = -d1.d2 and 1 / sin(th). active is false for an exactly straight
+// segment (sin = 0), where the reference switches bending off.
 template <class T>
 struct BendGeom {
-  T du, l1, l2, d1[3], d2[3], P1[3][3], P2[3][3], theta;
-  T c;  // cos(theta), the clamped argument of the acos
-};
-// src/ClothUnit.h:197-210; the theta clamp uses EPS = DBL_MIN
-// (src/Constants.h:25) and so never changes a finite value.
-template <class T>
-YS_HD void bend_geom(const T* x2, const T* x0, const T* x1, T du, BendGeom<T>& g) {
-  T a1[3], a2[3];
-  for (int i = 0; i < 3; ++i) { a1[i] = x1[i] - x0[i]; a2[i] = x2[i] - x0[i]; }
-  g.du = du;
-  g.l1 = norm3(a1);
-  g.l2 = norm3(a2);
-  for (int i = 0; i < 3; ++i) { g.d1[i] = a1[i] / g.l1; g.d2[i] = a2[i] / g.l2; }
-  proj3(g.d1, g.P1);
-  proj3(g.d2, g.P2);
-  T c = -dot3(g.d1, g.d2);
-  const double lo = -1.0 + 2.2250738585072014e-308, hi = 1.0 - 2.2250738585072014e-308;
-  if (c < lo) c = lo;
-  if (c > hi) c = hi;
-  g.c = c;
-  g.theta = acos(c);
-}
-
-// Bending force and Hessian blocks shared by Bending_* and Crimp_Bending_*
-// (src/PhysicsCloth.cpp:579-822, 824-987).
-template <class T>
-struct BendTerms {
-  T Fx1[3], Fx2[3];
-  T L11[3][3], L12[3][3], L21[3][3], L22[3][3];
-  T L1E1[3], L2E1[3];
+  T il1, il2, d1[3], d2[3], a[3], b[3], th, c, is;
   bool active;
 };
 template <class T>
-YS_HD void bend_terms(const BendGeom<T>& g, const T& kb, BendTerms<T>& t) {
-  for (int i = 0; i < 3; ++i) {
-    t.Fx1[i] = t.Fx2[i] = t.L1E1[i] = t.L2E1[i] = 0.0;
-    for (int j = 0; j < 3; ++j) t.L11[i][j] = t.L12[i][j] = t.L21[i][j] = t.L22[i][j] = 0.0;
-  }
-  // sin and cos of theta = acos(c) from c itself: sin = sqrt((1 - c)(1 + c))
-  // (zero exactly where sin(acos(c)) is: c = +-1), cos = c
-  const T th = g.theta, s = sqrt((1.0 - g.c) * (1.0 + g.c));
-  t.active = (s != 0.0);
-  if (!t.active) return;
-  const T co = g.c, du = g.du;
-  T a[3], b[3];
-  matvec3(g.P1, g.d2, a);
-  matvec3(g.P2, g.d1, b);
-  const T il1 = 1.0 / g.l1, il2 = 1.0 / g.l2, idu = 1.0 / du, is = 1.0 / s;  // one division each
-  const T c1 = (-2 * kb * th) * (il1 * idu * is), c2 = (-2 * kb * th) * (il2 * idu * is);
-  for (int i = 0; i < 3; ++i) { t.Fx1[i] = c1 * a[i]; t.Fx2[i] = c2 * b[i]; }
-  const T k11 = (2 * kb) * ((il1 * il1) * idu * is), k12 = (-2 * kb) * (il1 * il2 * idu * is);
-  const T k22 = (2 * kb) * ((il2 * il2) * idu * is);
-  const T cs2 = co * (is * is);
-  T Tm[3][3];
-  for (int i = 0; i < 3; ++i)
-    for (int j = 0; j < 3; ++j) {
-      const T ad1 = a[i] * g.d1[j], aa = a[i] * a[j], d1a = g.d1[i] * a[j];
-      const T bd2 = b[i] * g.d2[j], bb = b[i] * b[j], d2b = g.d2[i] * b[j];
-      t.L11[i][j] = k11 * (th * (ad1 + cs2 * aa + co * g.P1[i][j] + d1a) - is * aa);
-      t.L22[i][j] = k22 * (th * (bd2 + cs2 * bb + co * g.P2[i][j] + d2b) - is * bb);
-      Tm[i][j] = th * (g.P1[i][j] - cs2 * ad1) + is * ad1;
-    }
-  matmul3(Tm, g.P2, t.L12);
-  for (int i = 0; i < 3; ++i)
-    for (int j = 0; j < 3; ++j) t.L12[i][j] *= k12;
-  for (int i = 0; i < 3; ++i)
-    for (int j = 0; j < 3; ++j) {
-      const T bd2 = b[i] * g.d2[j];
-      Tm[i][j] = th * (g.P2[i][j] - cs2 * bd2) + is * bd2;
-    }
-  matmul3(Tm, g.P1, t.L21);
-  for (int i = 0; i < 3; ++i)
-    for (int j = 0; j < 3; ++j) t.L21[i][j] *= k12;
-  const T e1 = (2 * kb * th) * (il1 * (idu * idu) * is), e2 = (2 * kb * th) * (il2 * (idu * idu) * is);
-  for (int i = 0; i < 3; ++i) { t.L1E1[i] = e1 * a[i]; t.L2E1[i] = e2 * b[i]; }
+YS_HD void bend_geom(const T* x2, const T* x0, const T* x1, BendGeom<T>& g) {
+  for (int i = 0; i < 3; ++i) { g.d1[i] = x1[i] - x0[i]; g.d2[i] = x2[i] - x0[i]; }
+  const T l1 = norm3(g.d1), l2 = norm3(g.d2);
+  g.il1 = 1.0 / l1;
+  g.il2 = 1.0 / l2;
+  // rounded as divisions: a straight yarn along an axis has c = 1 exactly,
+  // and with it no bending, where the reference has none
+  for (int i = 0; i < 3; ++i) { g.d1[i] = quot(g.d1[i], l1, g.il1); g.d2[i] = quot(g.d2[i], l2, g.il2); }
+  const T dd = dot3(g.d1, g.d2);
+  for (int i = 0; i < 3; ++i) { g.a[i] = g.d2[i] - dd * g.d1[i]; g.b[i] = g.d1[i] - dd * g.d2[i]; }
+  // the reference's clamp (EPS = DBL_MIN, src/Constants.h:25) acts only where
+  // rounding has carried the cosine past +-1
+  T c = -dd;
+  if (c < -1.0) c = -1.0;
+  if (c > 1.0) c = 1.0;
+  g.c = c;
+  g.th = acos(c);
+  const T ss = (1.0 - c) * (1.0 + c);  // sin^2(th); zero exactly at c = +-1
+  // a NaN counts as active, as sin(th) != 0 does
+  g.active = !(ss == 0.0);
+  g.is = g.active ? rsqrt_(ss) : T(0.0);
 }
 
-// Bend segment record (one per middle node and yarn direction): the four
-// independent Hessian blocks of Bending_D and its Eulerian couplings, the
-// forces of Bending_F, and the crimp-bending forces / couplings that feed the
-// compression estimate (Crimp_Bending_F/D). The other blocks follow from
-// these as in src/PhysicsCloth.cpp:705-727 and are formed by the gather.
-constexpr int kBendFields = 62;
-constexpr int kB_L11 = 0, kB_L12 = 9, kB_L21 = 18, kB_L22 = 27, kB_L1E1 = 36, kB_L2E1 = 39, kB_E1E1 = 42,
-              kB_Fx1 = 43, kB_Fx2 = 46, kB_Fu2 = 49, kB_cFx1 = 50, kB_cFx2 = 53, kB_cL1E1 = 56, kB_cL2E1 = 59;
+// Bend segment record (one per middle node and yarn direction), as it enters
+// the system: the independent Hessian blocks scaled by -h^2 -- L11 and L22
+// symmetric (xx, xy, xz, yy, yz, zz), L12 full, L21 its transpose (P1 P2 =
+// (P2 P1)^T, and the rank-1 parts of src/PhysicsCloth.cpp:700-703 mirror each
+// other) -- the forces F1, F2 of Bending_F, and those of the crimp segment
+// that feed the compression estimate. The Eulerian couplings are
+// L1E1 = -F1 / du, L2E1 = -F2 / du; the other blocks follow as in
+// src/PhysicsCloth.cpp:705-727 and are formed by the gather. 37 fields for the
+// 62 that hold every block: on 255,292 nodes the producer (FP64 bound) takes
+// 0.33 ms for 0.63, the gather that reads the records 0.53 for 0.70.
+constexpr int kB_L11 = 0, kB_L22 = 6, kB_L12 = 12, kB_F1 = 21, kB_F2 = 24, kB_idu = 27, kB_E1E1 = 28, kB_Fu2 = 29,
+              kB_cF1 = 30, kB_cF2 = 33, kB_cidu = 36;
+constexpr int kBendFields = 37;
+YS_HD int sym3(int i, int j) { return i <= j ? i * (5 - i) / 2 + j : j * (5 - j) / 2 + i; }
+
+// a diagonal block k (th (v d^T + cs2 v v^T + c (I - d d^T) + d v^T) - is v v^T)
+template <class T, class Put>
+YS_HD void bend_diag(const T& k, const T& th, const T& c, const T& kA, const T* vv, const T* d, int f, Put&& put) {
+  const T kS = k * th, kP = kS * c;
+  for (int i = 0; i < 3; ++i) {
+    const T al = kA * vv[i] + kS * d[i], be = kS * vv[i] - kP * d[i];
+    for (int j = i; j < 3; ++j) {
+      const T x = al * vv[j] + be * d[j];
+      put(f + sym3(i, j), i == j ? x + kP : x);
+    }
+  }
+}
 
 // Bending_F / Bending_D on the real nodes (src/PhysicsCloth.cpp:579-822) and
 // Crimp_Bending_F / Crimp_Bending_D on the crimp-offset centre lines
 // (src/PhysicsCloth.cpp:824-987) for the segment n2 - n0 - n1 along yarn
-// direction k; written to the bend buffer at slot k * ntot + n0.
-template <class T>
-YS_HD void bend_element(const View& v, double* buf, double* dbuf, int n2, int n0, int n1, int k, int line) {
+// direction k; put(field, value) receives each field of the record once.
+template <class T, class Put>
+YS_HD void bend_terms(const View& v, int n2, int n0, int n1, int k, int line, Put&& put) {
   const int nt = v.ntot;
-  const int64_t stride = 2LL * nt, base = (int64_t)k * nt + n0;
-  (void)stride;
-  (void)base;
   const T kb = ldpT<T>(v.line_kb, v.dline_kb, line, v.nlines);
-  auto put = [&](int f, const T& x) { stT(buf, dbuf, 2 * f + k, nt, n0, x); };
   {
     T x2[3], x0[3], x1[3];
     for (int i = 0; i < 3; ++i) {
@@ -477,50 +461,56 @@ YS_HD void bend_element(const View& v, double* buf, double* dbuf, int n2, int n0
       x0[i] = ldT<T>(v.X, v.dX, i, nt, n0);
       x1[i] = ldT<T>(v.X, v.dX, i, nt, n1);
     }
+    const T idu = 1.0 / (ldT<T>(v.UV, v.dUV, k, nt, n1) - ldT<T>(v.UV, v.dUV, k, nt, n2));
     BendGeom<T> g;
-    bend_geom(x2, x0, x1, ldT<T>(v.UV, v.dUV, k, nt, n1) - ldT<T>(v.UV, v.dUV, k, nt, n2), g);
-    BendTerms<T> t;
-    bend_terms(g, kb, t);
-    for (int i = 0; i < 3; ++i)
-      for (int j = 0; j < 3; ++j) {
-        put(kB_L11 + 3 * i + j, t.L11[i][j]);
-        put(kB_L12 + 3 * i + j, t.L12[i][j]);
-        put(kB_L21 + 3 * i + j, t.L21[i][j]);
-        put(kB_L22 + 3 * i + j, t.L22[i][j]);
+    bend_geom(x2, x0, x1, g);
+    const T kt = kb * g.th * idu;
+    put(kB_idu, idu);
+    put(kB_Fu2, -kt * idu);
+    put(kB_E1E1, (-2.0 * kt * g.th) * (idu * idu));
+    const T on = g.active ? kb : T(0.0);
+    const T f = -2.0 * (on * g.th) * (idu * g.is), f1 = f * g.il1, f2 = f * g.il2;
+    for (int i = 0; i < 3; ++i) { put(kB_F1 + i, f1 * g.a[i]); put(kB_F2 + i, f2 * g.b[i]); }
+    const T K = (-2.0 * v.h * v.h) * on * (idu * g.is);  // 2 kb / (du sin), scaled by -h^2
+    const T k11 = K * (g.il1 * g.il1), k22 = K * (g.il2 * g.il2), k12 = -K * (g.il1 * g.il2);
+    const T tc = g.th * (g.c * (g.is * g.is)) - g.is;
+    bend_diag(k11, g.th, g.c, k11 * tc, g.a, g.d1, kB_L11, put);
+    bend_diag(k22, g.th, g.c, k22 * tc, g.b, g.d2, kB_L22, put);
+    // L12 = k12 (th P1 P2 - tc a b^T), P1 P2 = I - d1 d1^T - a d2^T
+    const T kt12 = k12 * g.th, kab = -k12 * tc;
+    for (int j = 0; j < 3; ++j) {
+      const T pa = kab * g.b[j] - kt12 * g.d2[j], pd = -kt12 * g.d1[j];
+      for (int i = 0; i < 3; ++i) {
+        const T x = pa * g.a[i] + pd * g.d1[i];
+        put(kB_L12 + 3 * i + j, i == j ? x + kt12 : x);
       }
-    for (int i = 0; i < 3; ++i) {
-      put(kB_L1E1 + i, t.L1E1[i]);
-      put(kB_L2E1 + i, t.L2E1[i]);
-      put(kB_Fx1 + i, t.Fx1[i]);
-      put(kB_Fx2 + i, t.Fx2[i]);
     }
-    const T th = g.theta, idu = 1.0 / g.du;
-    put(kB_E1E1, (-2 * kb * (th * th)) * (idu * idu * idu));
-    put(kB_Fu2, (-kb * th) * (idu * idu));
   }
   {
     const double R = v.cp[v.node_cloth[n0]].R;
-    const double sg = k == 0 ? -1.0 : 1.0;  // warp: x - R n, weft: x + R n
+    const double sg = k == 0 ? -R : R;  // warp: x - R n, weft: x + R n
     T x[3][3];
     const int nd[3] = {n2, n0, n1};
     for (int m = 0; m < 3; ++m) {
       const bool in = (v.flags[nd[m]] & YS_INTERIOR) != 0;
-      for (int i = 0; i < 3; ++i)
-        x[m][i] = in ? ldT<T>(v.X, v.dX, i, nt, nd[m]) + sg * (R * ldT<T>(v.NRM, v.dNRM, i, nt, nd[m]))
-                     : ldT<T>(v.X, v.dX, i, nt, nd[m]);
+      for (int i = 0; i < 3; ++i) {
+        x[m][i] = ldT<T>(v.X, v.dX, i, nt, nd[m]);
+        if (in) x[m][i] += sg * ldT<T>(v.NRM, v.dNRM, i, nt, nd[m]);
+      }
     }
-    // crimp segments keep the EPos of the build (src/Cloth.cpp:107)
     BendGeom<T> g;
-    bend_geom(x[0], x[1], x[2], T(ld(v.UV0, k, nt, n1) - ld(v.UV0, k, nt, n2)), g);
-    BendTerms<T> t;
-    bend_terms(g, kb, t);
-    for (int i = 0; i < 3; ++i) {
-      put(kB_cFx1 + i, t.Fx1[i]);
-      put(kB_cFx2 + i, t.Fx2[i]);
-      put(kB_cL1E1 + i, t.L1E1[i]);
-      put(kB_cL2E1 + i, t.L2E1[i]);
-    }
+    bend_geom(x[0], x[1], x[2], g);
+    // crimp segments keep the EPos of the build (src/Cloth.cpp:107)
+    const double cidu = 1.0 / (ld(v.UV0, k, nt, n1) - ld(v.UV0, k, nt, n2));
+    const T f = g.active ? T((-2.0 * cidu) * (kb * g.th) * g.is) : T(0.0), f1 = f * g.il1, f2 = f * g.il2;
+    put(kB_cidu, T(cidu));
+    for (int i = 0; i < 3; ++i) { put(kB_cF1 + i, f1 * g.a[i]); put(kB_cF2 + i, f2 * g.b[i]); }
   }
+}
+// the record in the bend buffer at slot k * ntot + n0
+template <class T>
+YS_HD void bend_element(const View& v, double* buf, double* dbuf, int n2, int n0, int n1, int k, int line) {
+  bend_terms<T>(v, n2, n0, n1, k, line, [&](int f, const T& x) { stT(buf, dbuf, 2 * f + k, v.ntot, n0, x); });
 }
 
 // ------------------------------------------------------------ wind (faces)
