@@ -295,11 +295,11 @@ YS_HD bool gather_shear_finalize(const View& v, const Records& R, int n, double*
   const ClothParams& P = v.cp[v.node_cloth[n]];
   const int W = P.W, H = P.H, u = v.node_u[n], w = v.node_v[n];
   const uint8_t fl = v.flags[n];
-  const double h = v.h, mh2 = -(v.h * v.h);
+  const double h = v.h;
   auto interior = [&](int uu, int vv) { return uu >= 1 && uu <= W - 2 && vv >= 1 && vv <= H - 2; };
   auto S = [&](int f, int seg, int anc) { return recT<T>(R.shear, R.dshear, f, 4, seg, nt, anc); };
   bool finf = true;  // every slot value this routine writes is finite
-  auto addLL = [&](int du, int dv, const T* blk) {  // A[x(n)][x(n + (du, dv))] += -h^2 blk^T
+  auto addLL = [&](int du, int dv, const T* blk) {  // A[x(n)][x(n + (du, dv))] += blk
     const int s = stencil_index(du, dv);
     if (s < 0) return;
     // the block's nine slots are loaded together, then updated: a load per
@@ -313,7 +313,7 @@ YS_HD bool gather_shear_finalize(const View& v, const Records& R, int n, double*
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         T& x = a[3 * r + c];
-        x += mh2 * blk[3 * c + r];
+        x += blk[3 * r + c];
         finf = finf && isfinite(val(x));
       }
 #pragma unroll
@@ -348,7 +348,7 @@ YS_HD bool gather_shear_finalize(const View& v, const Records& R, int n, double*
             xa[ix][i] += -(a11 + a31);                   // J01, towards n1 = n + (du, 0)
             ya[iy][i] += -(a13 + a33);                   // J03, towards n3 = n + (0, dv)
           }
-          for (int r = 0; r < 3; ++r) Bx[r] += h * (-1 * (S(kS_F1 + r, seg, n) + S(kS_F3 + r, seg, n)));
+          for (int r = 0; r < 3; ++r) Bx[r] -= S(kS_F1 + r, seg, n) + S(kS_F3 + r, seg, n);
         }
         if (interior(u - du, w)) {  // as the warp neighbour n1 of the crossing n - (du, 0)
           const int anc = n - du;
@@ -358,7 +358,7 @@ YS_HD bool gather_shear_finalize(const View& v, const Records& R, int n, double*
             self[i] += b11;
             xa[1 - ix][i] += -(b11 + b13);  // J10, towards n0 = n + (-du, 0)
           }
-          for (int r = 0; r < 3; ++r) Bx[r] += h * S(kS_F1 + r, seg, anc);
+          for (int r = 0; r < 3; ++r) Bx[r] += S(kS_F1 + r, seg, anc);
         }
         if (interior(u, w - dv)) {  // as the weft neighbour n3 of the crossing n - (0, dv)
           const int anc = n - dv * W;
@@ -368,7 +368,7 @@ YS_HD bool gather_shear_finalize(const View& v, const Records& R, int n, double*
             self[i] += c33;
             ya[1 - iy][i] += -(c31 + c33);  // J30, towards n0 = n + (0, -dv)
           }
-          for (int r = 0; r < 3; ++r) Bx[r] += h * S(kS_F3 + r, seg, anc);
+          for (int r = 0; r < 3; ++r) Bx[r] += S(kS_F3 + r, seg, anc);
         }
       }
       addLL(0, 0, self);
@@ -415,7 +415,7 @@ YS_HD bool gather_shear_finalize(const View& v, const Records& R, int n, double*
         addLL(shear_du(seg), 0, J);
         for (int i = 0; i < 9; ++i) J[i] = -(S(kS_J13 + i, seg, n) + S(kS_J33 + i, seg, n));  // J03
         addLL(0, shear_dv(seg), J);
-        for (int r = 0; r < 3; ++r) Bx[r] += h * (-1 * (S(kS_F1 + r, seg, n) + S(kS_F3 + r, seg, n)));
+        for (int r = 0; r < 3; ++r) Bx[r] -= S(kS_F1 + r, seg, n) + S(kS_F3 + r, seg, n);
       }
     }
     // as the warp neighbour n1 = n0 + (du, 0)
@@ -429,7 +429,7 @@ YS_HD bool gather_shear_finalize(const View& v, const Records& R, int n, double*
       addLL(-du, 0, J);
       for (int i = 0; i < 9; ++i) J[i] = S(kS_J13 + i, seg, anc);  // towards n3 = n + (-du, dv)
       addLL(-du, dv, J);
-      for (int r = 0; r < 3; ++r) Bx[r] += h * S(kS_F1 + r, seg, anc);
+      for (int r = 0; r < 3; ++r) Bx[r] += S(kS_F1 + r, seg, anc);
     }
     // as the weft neighbour n3 = n0 + (0, dv)
     for (int seg = 0; seg < 4; ++seg) {
@@ -442,7 +442,7 @@ YS_HD bool gather_shear_finalize(const View& v, const Records& R, int n, double*
       addLL(0, -dv, J);
       for (int i = 0; i < 9; ++i) J[i] = S(kS_J31 + i, seg, anc);  // towards n1 = n + (du, -dv)
       addLL(du, -dv, J);
-      for (int r = 0; r < 3; ++r) Bx[r] += h * S(kS_F3 + r, seg, anc);
+      for (int r = 0; r < 3; ++r) Bx[r] += S(kS_F3 + r, seg, anc);
     }
   }
   for (int r = 0; r < 3; ++r) addB(r, Bx[r]);

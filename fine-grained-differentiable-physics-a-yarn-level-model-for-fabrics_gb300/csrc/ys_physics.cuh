@@ -782,74 +782,88 @@ YS_HD void friction_node(const View& v, int n, const T* fe, const T* kee, const 
 
 // ------------------------------------------------------------ shear
 // Shear segment record (one per crossing and segment type): the forces on the
-// warp and weft neighbours and the four independent Hessian blocks; the
-// crossing's own force and blocks follow from them (src/PhysicsCloth.cpp:2710,
-// 3033-3037) and are formed by the gather.
+// warp and weft neighbours scaled by h, and the four independent Hessian
+// blocks as they enter A, scaled by -h^2 and transposed (To_Sparse_Mat,
+// src/MatrixMp.cpp:54-65); the crossing's own force and blocks follow from
+// them (src/PhysicsCloth.cpp:2710, 3033-3037) and are formed by the gather.
 constexpr int kShearFields = 42;
 constexpr int kS_F1 = 0, kS_F3 = 3, kS_J11 = 6, kS_J13 = 15, kS_J31 = 24, kS_J33 = 33;
 // segment types in the order of src/Cloth.cpp:178-181: (warp, weft) offsets
 YS_HD int shear_du(int seg) { return seg < 2 ? -1 : 1; }
 YS_HD int shear_dv(int seg) { return (seg & 1) ? -1 : 1; }
 
+// kA v v^T + kS (v d^T + d v^T - co d d^T) + kS co I, plus one + g v in row r
+template <class T, class Put>
+YS_HD void shear_diag(const T& kA, const T& kS, const T& co, const T* vv, const T* d, bool lock, const T& one,
+                      const T& g, int f, Put&& put) {
+  const T kP = kS * co;
+  for (int i = 0; i < 3; ++i) {
+    const T al = kA * vv[i] + kS * d[i], be = kS * vv[i] - kP * d[i];
+    for (int j = i; j < 3; ++j) {
+      T x = al * vv[j] + be * d[j];
+      if (i == j) x += kP;
+      if (lock) {
+        put(f + 3 * i + j, x + (one + g * vv[i]));
+        if (i != j) put(f + 3 * j + i, x + (one + g * vv[j]));
+      } else {
+        put(f + 3 * i + j, x);
+        if (i != j) put(f + 3 * j + i, x);
+      }
+    }
+  }
+}
+
 // Shear_F / Shear_D (src/PhysicsCloth.cpp:2643-3089) for crossing n0 with warp
-// neighbour n1 = n0 + (shear_du, 0) and weft neighbour n3 = n0 + (0, shear_dv),
-// written to the shear buffer at slot seg * ntot + n0.
-template <class T>
-YS_HD void shear_element(const View& v, double* buf, double* dbuf, int n0, int seg) {
+// neighbour n1 = n0 + (shear_du, 0) and weft neighbour n3 = n0 + (0, shear_dv);
+// put(field, value) receives each field of the record once.
+// FP64-pipe bound: projections as d - (d.d') d', one reciprocal each for the
+// lengths and for the lock's denominator, and the vanishing P3 d3 block left
+// out took the producer from 1.23 to 0.95 ms on 255,292 nodes (0.97 M segments).
+template <class T, class Put>
+YS_HD void shear_terms(const View& v, int n0, int seg, Put&& put) {
   const ClothParams& P = v.cp[v.node_cloth[n0]];
   const int n1 = n0 + shear_du(seg), n3 = n0 + shear_dv(seg) * P.W;
   const int nt = v.ntot;
-  const double Lc = P.L, R = P.R;
-  const T S = cloth_S<T>(v, v.node_cloth[n0]);
-  const T comp = ldT<T>(v.COMP, v.dCOMP, 0, nt, n0);
-  T a1v[3], a3v[3], d1[3], d3[3], P1[3][3], P3[3][3];
+  const double Lc = P.L, R = P.R, h = v.h, mh2 = -(v.h * v.h);
+  const T SR = (ldT<T>(v.COMP, v.dCOMP, 0, nt, n0) + 1.0) * (cloth_S<T>(v, v.node_cloth[n0]) * (R * R));
+  T d1[3], d3[3], a3[3], a1[3];
   for (int i = 0; i < 3; ++i) {
     const T x0 = ldT<T>(v.X, v.dX, i, nt, n0);
-    a1v[i] = ldT<T>(v.X, v.dX, i, nt, n1) - x0;
-    a3v[i] = ldT<T>(v.X, v.dX, i, nt, n3) - x0;
+    d1[i] = ldT<T>(v.X, v.dX, i, nt, n1) - x0;
+    d3[i] = ldT<T>(v.X, v.dX, i, nt, n3) - x0;
   }
-  const T l1 = norm3(a1v), l3 = norm3(a3v);
-  const T il1 = 1.0 / l1, il3 = 1.0 / l3;  // reciprocals, one division each
-  for (int i = 0; i < 3; ++i) { d1[i] = a1v[i] * il1; d3[i] = a3v[i] * il3; }
-  proj3(d1, P1);
-  proj3(d3, P3);
-  // the crossing angle, and its sine and cosine from its cosine c:
-  // sin = sqrt((1 - c)(1 + c)), cos = c (phi in [0, pi])
-  const T cph = dot3(d1, d3);
-  const T phi = acos(cph);
-  const T s = sqrt((1.0 - cph) * (1.0 + cph)), co = cph;
-  T a3[3], a1[3];  // a3 = P1 d3, a1 = P3 d1
-  matvec3(P1, d3, a3);
-  matvec3(P3, d1, a1);
+  const T il1 = rsqrt_(dot3(d1, d1)), il3 = rsqrt_(dot3(d3, d3));
+  for (int i = 0; i < 3; ++i) { d1[i] *= il1; d3[i] *= il3; }
+  // the crossing angle phi in [0, pi] and 1 / sin(phi) from its cosine co;
+  // a3 = P1 d3, a1 = P3 d1, P = I - d d^T
+  const T co = dot3(d1, d3);
+  for (int i = 0; i < 3; ++i) { a3[i] = d3[i] - co * d1[i]; a1[i] = d1[i] - co * d3[i]; }
+  const T phi = acos(co);
+  const T is = rsqrt_((1.0 - co) * (1.0 + co)), is2 = is * is, cs2 = co * is2;
+  const T i11 = il1 * il1, i33 = il3 * il3, i13 = il1 * il3;
   const uint8_t f0 = v.flags[n0], f1 = v.flags[n1], f3 = v.flags[n3];
   const bool jam = (((f0 & YS_FLIP) != 0) != ((f1 & YS_FLIP) != 0)) && (((f0 & YS_FLIP) != 0) != ((f3 & YS_FLIP) != 0));
-  T Fx1[3], Fx3[3], J11[3][3], J13[3][3], J31[3][3], J33[3][3];
-  const T is = 1.0 / s, cs2 = co * (is * is);
   if (!jam) {
-    const T kx = (comp + 1.0) * S * R * R * kPi;
+    const T kL = SR * (kPi * Lc) * is;
     const T ph = phi - kPi / 2;
     // Shear_F takes phi.item() in (phi - PI/2) (src/PhysicsCloth.cpp:2720-2721):
     // that factor carries no derivative along the reference's gradient path
     const T phf = v.trunc ? detach(phi) - kPi / 2 : ph;
-    const T cf1 = (kx * Lc * phf) * (il1 * is), cf3 = (kx * Lc * phf) * (il3 * is);
-    for (int i = 0; i < 3; ++i) { Fx1[i] = cf1 * a3[i]; Fx3[i] = cf3 * a1[i]; }
-    const T k11 = (kx * Lc) * ((il1 * il1) * is), k33 = (kx * Lc) * ((il3 * il3) * is);
-    const T k13 = (kx * Lc) * (il3 * il1 * is), k31 = (kx * Lc) * (il1 * il3 * is);
+    const T cf = h * (kL * phf), cf1 = cf * il1, cf3 = cf * il3;
+    for (int i = 0; i < 3; ++i) { put(kS_F1 + i, cf1 * a3[i]); put(kS_F3 + i, cf3 * a1[i]); }
     // src/PhysicsCloth.cpp:2715-2751 per block:
     //   J11 = k11 (ph (-a3 d1^T + cs2 a3 a3^T - co P1 - d1 a3^T) - a3 a3^T / s)
     //   J13 = k13 ph (cs2 - 1/s) (a3 d1^T) P3 = k13 ph (cs2 - 1/s) a3 a1^T, as a1 = P3 d1
     // (J33, J31 likewise with 1 <-> 3)
-    const T kA1 = k11 * (ph * cs2 - is), kS1 = -k11 * ph, kP1 = kS1 * co;
-    const T kA3 = k33 * (ph * cs2 - is), kS3 = -k33 * ph, kP3 = kS3 * co;
-    const T kx13 = k13 * ph * (cs2 - is), kx31 = k31 * ph * (cs2 - is);
+    const T k = mh2 * kL, kA = k * (ph * cs2 - is), kS = -k * ph, kx = i13 * (k * ph) * (cs2 - is);
+    shear_diag(kA * i11, kS * i11, co, a3, d1, false, kA, kA, kS_J11, put);
+    shear_diag(kA * i33, kS * i33, co, a1, d3, false, kA, kA, kS_J33, put);
     for (int i = 0; i < 3; ++i) {
-      const T al1 = kA1 * a3[i] + kS1 * d1[i], be1 = kS1 * a3[i];
-      const T al3 = kA3 * a1[i] + kS3 * d3[i], be3 = kS3 * a1[i];
+      const T x = kx * a3[i];
       for (int j = 0; j < 3; ++j) {
-        J11[i][j] = al1 * a3[j] + be1 * d1[j] + kP1 * P1[i][j];
-        J33[i][j] = al3 * a1[j] + be3 * d3[j] + kP3 * P3[i][j];
-        J13[i][j] = kx13 * (a3[i] * a1[j]);
-        J31[i][j] = kx31 * (a1[i] * a3[j]);
+        const T y = x * a1[j];  // J13[i][j] = J31[j][i]
+        put(kS_J13 + 3 * j + i, y);
+        put(kS_J31 + 3 * i + j, y);
       }
     }
   } else {
@@ -860,36 +874,30 @@ YS_HD void shear_element(const View& v, double* buf, double* dbuf, int n0, int s
     // broadcasts a scalar 1 and so equals beta0 (1,1,1) + beta1 phi_x. With
     // the scalars below each Hessian entry is a short combination of rank-1
     // products; the arithmetic is the reference's, regrouped.
-    const double pb = kPi / 2, pl = P.jam, sig = 0.6;
-    const double cc = 3.0;
-    const double LR = Lc / R;
-    const T rl1s = il1 * is, rl3s = il3 * is;
-    T px1[3], px3[3];
-    for (int i = 0; i < 3; ++i) { px1[i] = -a3[i] * rl1s; px3[i] = -a1[i] * rl3s; }
-    // half-angle sine and cosine: sqrt((1 -+ c) / 2), both >= 0 for phi in [0, pi]
-    const T sh = sqrt(0.5 * (1.0 - cph)), ch = sqrt(0.5 * (1.0 + cph));
-    const T gamma = (Lc * sqrt(2.0) - 2 * Lc * sh) / R;
-    const T kap = -LR * ch;                       // gamma_x = kap * phi_x
-    const T Aq = phi - pl, Bq = phi - pb;
-    const T phs = phi * Aq * Bq;
-    const T sgm = Aq * Bq + phi * Bq + phi * Aq;  // phi_s_x = sgm * phi_x
-    const T omg = 2.0 * (Aq + Bq + phi);
+    const double pb = kPi / 2, sig = 0.6, LR = Lc / R;
     const double pb5 = P.pb5, pb4 = P.pb4;
+    // half-angle sine and cosine: sqrt((1 -+ c) / 2), both >= 0 for phi in [0, pi]
+    const T sh = sqrt(0.5 * (1.0 - co)), ch = sqrt(0.5 * (1.0 + co));
+    const T gamma = LR * (sqrt(2.0) - 2.0 * sh);
+    const T kap = -LR * ch;                       // gamma_x = kap * phi_x
+    const T Aq = phi - P.jam, Bq = phi - pb;
+    const T AB = Aq * Bq, phs = phi * AB;
+    const T sgm = AB + phi * (Aq + Bq);           // phi_s_x = sgm * phi_x
+    const T omg = 2.0 * (Aq + Bq + phi);
     const T num = pb5 * Aq, den = phs * phs + pb4 * sig * sig;
-    const T cf = tanh(num / den);
-    const T den2 = den * den, rden2 = 1.0 / den2, rden22 = rden2 * rden2;
-    const T tau = pb5 * den - num * (2 * phs * sgm);  // con_func_x_x numerator / phi_x
-    const T muc = tau * rden2;                         // con_func_x_x = muc * phi_x
-    const T g3 = gamma * gamma * gamma, g2 = gamma * gamma;
-    const T base = 0.5 * (comp + 1.0) * S * kPi * (R * R);
-    const T kx = base * ((1 + g3) + (1 - g3) * cf);
-    const T beta0 = base * (1 - g3);
-    const T beta1 = base * (cc * g2 * kap * (1 - cf) - (1 - g3) * cf * cf * muc);
-    const T Bq2 = Bq * Bq;
-    const T cf1 = (kx * Lc * Bq) * rl1s, cf3 = (kx * Lc * Bq) * rl3s;
-    for (int i = 0; i < 3; ++i) {
-      Fx1[i] = -0.5 * (beta0 + beta1 * px1[i]) * Lc * Bq2 + cf1 * a3[i];
-      Fx3[i] = -0.5 * (beta0 + beta1 * px3[i]) * Lc * Bq2 + cf3 * a1[i];
+    const T rden = 1.0 / den, rden2 = rden * rden;
+    const T cf = tanh(num * rden);
+    const T ps2 = 2.0 * (phs * sgm);
+    const T muc = (pb5 * den - num * ps2) * rden2;  // con_func_x_x = muc * phi_x
+    const T g2 = gamma * gamma, g3 = g2 * gamma, g3c = 1.0 - g3, cf1m = 1.0 - cf, cf2 = cf * cf, eX = 1.0 - cf2;
+    const T base2 = 0.5 * SR;
+    const T kL = (kPi * Lc) * base2 * ((1.0 + g3) + g3c * cf);
+    const T beta0 = kPi * base2 * g3c;
+    const T beta1 = kPi * base2 * (3.0 * g2 * kap * cf1m - g3c * cf2 * muc);
+    const T LBq = Lc * Bq, hLB2 = 0.5 * LBq * Bq;
+    {
+      const T u = -h * hLB2 * beta0, t = h * (hLB2 * beta1 + kL * Bq) * is, t1 = t * il1, t3 = t * il3;
+      for (int i = 0; i < 3; ++i) { put(kS_F1 + i, u + t1 * a3[i]); put(kS_F3 + i, u + t3 * a1[i]); }
     }
     // The Hessian entries of src/PhysicsCloth.cpp:2753-3031 are, for each
     // block, one fixed linear map (scalars below) applied to a few per-entry
@@ -899,97 +907,71 @@ YS_HD void shear_element(const View& v, double* buf, double* dbuf, int n0, int s
     // rows/columns. Those quantities are in turn combinations of a handful of
     // rank-1 matrices (a3 a3^T, a3 d1^T + d1 a3^T, P1, ...), so each block is
     // J = sum_k c_k B_k with c_k computed once per block.
-    T P1P3[3][3], e3[3];
-    matmul3(P1, P3, P1P3);  // P3 P1 is its transpose (both projectors symmetric)
-    matvec3(P3, d3, e3);    // P3 d3: src/PhysicsCloth.cpp:2775-2777 multiplies outer(P3 d1, d3) by P3
-    const T cfq = -2 * cf * (1 - cf * cf);
-    const T c1 = cc * (cc - 1) * gamma, c2 = cc * g2;
-    const T base2 = 0.5 * (comp + 1.0) * S * (R * R);
-    const T kO = c1 * kap * kap * (1 - cf) - 2 * c2 * kap * (1 - cf * cf) * muc;
-    const T kG = c2 * (1 - cf);
-    const T cfqm2 = cfq * muc * muc;
-    const T X4 = 4 * tau * den * phs * sgm;
-    const T tns2 = 2 * num * sgm * sgm, tnp = 2 * num * phs, pb5den = pb5 * den;
-    const T cross = 2 * phs * pb5 * sgm;
-    const T hLB2 = 0.5 * Lc * Bq2, LB = Lc * Bq;
-    const T kL = kx * Lc;
-    const T r11 = (il1 * il1) * is, r33 = (il3 * il3) * is, r13 = il1 * il3 * is;
-    const T qR11 = 0.5 * LR * sh * (rl1s * rl1s), qR33 = 0.5 * LR * sh * (rl3s * rl3s);
-    const T qR13 = 0.5 * LR * sh * (il1 * il3 * (is * is));
-    const T rho1 = rl1s * rl1s, rho3 = rl3s * rl3s, rho13 = rl1s * rl3s;
     // J = cP*pxx + cO*O + cOb*Ob + cR*Rg + fo (+ cOne*1 + row/column terms)
-    const T hb = hLB2 * base2, g3c = 1 - g3;
-    const T cR = -hb * kG;
-    const T cnx_p = pb5den - tnp * sgm;  // nx = cnx_p pxx + ...
-    // x1x1 and x3x3: psx = sgm pxx + omg O, cfdd = cfqm2 O + 1 - cf^2 cfx
-    const T eD = -cf * cf;
-    const T cPd = -hb * (kG * kap + g3c * eD * rden2 * cnx_p);
-    const T cOd = -hb * (kO + g3c * (eD * (rden2 * (-tns2 - tnp * omg) - rden22 * X4) + cfqm2)) - 2 * LB * beta1;
-    const T cOne = -hb * g3c;
-    // x1x3 (psx = sgm pxx + omg (O + Ob) / 2) and x3x1 (psx = sgm pxx + omg O);
-    // both: nx += cross (O - Ob), cfdd = cfqm2 Ob + (1 - cf^2) cfx
-    const T eX = 1 - cf * cf;
-    const T cPx = -hb * (kG * kap + g3c * eX * rden2 * cnx_p);
-    const T cO13 = -hb * (kO + g3c * eX * (rden2 * (-tns2 - tnp * 0.5 * omg + cross) - rden22 * X4)) -
-                        2 * LB * beta1;
-    const T cOb13 = -hb * g3c * (eX * rden2 * (-tnp * 0.5 * omg - cross) + cfqm2);
-    const T cO31 = -hb * (kO + g3c * eX * (rden2 * (-tns2 - tnp * omg + cross) - rden22 * X4)) - 2 * LB * beta1;
-    const T cOb31 = -hb * g3c * (eX * rden2 * (-cross) + cfqm2);
-    const T kq = Bq * cs2 - is;
+    const T kG = 3.0 * g2 * cf1m, kO = kap * (6.0 * gamma * kap * cf1m - 6.0 * g2 * eX * muc);
+    const T cfqm2 = -2.0 * cf * eX * (muc * muc);
+    const T X4 = 2.0 * muc * ps2 * rden;
+    const T tnp = 2.0 * (num * phs) * rden2, tns2 = 2.0 * (num * (sgm * sgm)) * rden2, cross = ps2 * pb5 * rden2;
+    const T cnx_p = pb5 * rden - tnp * sgm, tom = tnp * omg;
+    const T H = (h * h) * hLB2 * base2;  // -h^2 times -(L Bq^2 / 2) base
+    const T Hg = H * g3c, Hx = Hg * eX, HG = H * kG * kap;
+    const T LB2 = 2.0 * mh2 * LBq, kLs = mh2 * kL;
+    const T hk = H * kO - LB2 * beta1;
+    const T hR = 0.5 * LR * (H * kG) * sh;
+    const T kq = kLs * (Bq * cs2 - is), kB = kLs * Bq;
+    // x1x1 and x3x3: psx = sgm pxx + omg O, cfdd = cfqm2 O + 1 - cf^2 cfx;
     // x1x1: pxx = r11 (S - cs2 A + co P1), O = Ob = rho1 A, Rg = qR11 A,
-    //       fo = kL r11 (-Bq S + kq A - Bq co P1); A = a3 a3^T, S = a3 d1^T + d1 a3^T
+    //       fo = kL r11 (-Bq S + kq A - Bq co P1); A = a3 a3^T, S = a3 d1^T + d1 a3^T;
+    // x3x3: the same with (a1, d3, P3)
     {
-      const T kA = cPd * (-cs2 * r11) + cOd * rho1 + cR * qR11 + kL * r11 * kq;
-      const T kS = (cPd - kL * Bq) * r11;
-      const T kP = (cPd - kL * Bq) * r11 * co;
-      for (int i = 0; i < 3; ++i) {
-        const T al = kA * a3[i] + kS * d1[i], be = kS * a3[i];
-        for (int j = 0; j < 3; ++j)
-          J11[i][j] = al * a3[j] + be * d1[j] + kP * P1[i][j] + (cOne - 2 * LB * beta0 * px1[j]);
-      }
+      const T cP = HG - Hg * cf2 * cnx_p;
+      const T cO = hk + Hg * (cf2 * (tns2 + tom + X4) + cfqm2);
+      const T kA = is * (kq - cP * cs2) + is2 * (cO + hR), kS = (cP - kB) * is;
+      const T g = LB2 * beta0 * is;
+      shear_diag(kA * i11, kS * i11, co, a3, d1, true, Hg, g * il1, kS_J11, put);
+      shear_diag(kA * i33, kS * i33, co, a1, d3, true, Hg, g * il3, kS_J33, put);
     }
-    // x3x3: the same with (a1, d3, P3, r33, qR33, rho3, px3)
-    {
-      const T kA = cPd * (-cs2 * r33) + cOd * rho3 + cR * qR33 + kL * r33 * kq;
-      const T kS = (cPd - kL * Bq) * r33;
-      const T kP = (cPd - kL * Bq) * r33 * co;
-      for (int i = 0; i < 3; ++i) {
-        const T al = kA * a1[i] + kS * d3[i], be = kS * a1[i];
-        for (int j = 0; j < 3; ++j)
-          J33[i][j] = al * a1[j] + be * d3[j] + kP * P3[i][j] + (cOne - 2 * LB * beta0 * px3[j]);
-      }
-    }
+    // x1x3 (psx = sgm pxx + omg (O + Ob) / 2) and x3x1 (psx = sgm pxx + omg O);
+    // both: nx += cross (O - Ob), cfdd = cfqm2 Ob + (1 - cf^2) cfx.
     // x1x3: pxx = -r13 (cs2 A + M), O = rho13 A, Ob = rho13 B, Rg = qR13 A,
     //       fo = kL r13 (kq A + Bq M); A = a3 a1^T, B = a1 a3^T, M = P1 P3
+    // x3x1: pxx = -r13 M^T (its outer(P3 d1, d3) P3, src/PhysicsCloth.cpp:2775-2777,
+    //       is zero: P3 d3 = 0), O = rho13 A, Ob = rho13 B, Rg = qR13 A,
+    //       fo = kL r13 (kq A + Bq M^T); A = a1 a3^T, B = a3 a1^T
     {
-      const T kA = -cPx * r13 * cs2 + cO13 * rho13 + cR * qR13 + kL * r13 * kq;
-      const T kB = cOb13 * rho13;
-      const T kM = (-cPx + kL * Bq) * r13;
-      for (int i = 0; i < 3; ++i)
-        for (int j = 0; j < 3; ++j)
-          J13[i][j] = kA * (a3[i] * a1[j]) + kB * (a1[i] * a3[j]) + kM * P1P3[i][j] - LB * beta0 * (px3[j] + px1[i]);
-    }
-    // x3x1: pxx = -r13 (cs2 E + M^T), O = rho13 A, Ob = rho13 B, Rg = qR13 A,
-    //       fo = kL r13 (kq A + Bq M^T); A = a1 a3^T, B = a3 a1^T, E = a1 e3^T
-    {
-      const T kA = cO31 * rho13 + cR * qR13 + kL * r13 * kq;
-      const T kB = cOb31 * rho13;
-      const T kE = -cPx * r13 * cs2;
-      const T kM = (-cPx + kL * Bq) * r13;
-      for (int i = 0; i < 3; ++i)
-        for (int j = 0; j < 3; ++j)
-          J31[i][j] = kA * (a1[i] * a3[j]) + kB * (a3[i] * a1[j]) + kE * (a1[i] * e3[j]) + kM * P1P3[j][i] -
-                      LB * beta0 * (px1[j] + px3[i]);
+      const T cP = HG + Hx * cnx_p, ik = i13 * is, ik2 = i13 * is2;
+      const T com = hk + hR + Hx * (cross - tns2 - X4);
+      const T kM = (kB - cP) * ik;
+      const T g = 0.5 * LB2 * beta0 * is, g1 = g * il1, g3_ = g * il3;
+      {  // M = I - d1 d1^T - a3 d3^T
+        const T kA = ik * (kq - cP * cs2) + ik2 * (com - 0.5 * Hx * tom);
+        const T kb = ik2 * (Hg * cfqm2 - Hx * (0.5 * tom + cross));
+        for (int j = 0; j < 3; ++j) {
+          const T pa3 = kA * a1[j] - kM * d3[j] + g1, pa1 = kb * a3[j], pd = -kM * d1[j], p0 = g3_ * a1[j];
+          for (int i = 0; i < 3; ++i) {
+            const T x = pa3 * a3[i] + pa1 * a1[i] + pd * d1[i] + p0;
+            put(kS_J13 + 3 * j + i, i == j ? x + kM : x);
+          }
+        }
+      }
+      {  // M^T = I - d3 d3^T - a1 d1^T
+        const T kA = ik * kq + ik2 * (com - Hx * tom);
+        const T kb = ik2 * (Hg * cfqm2 - Hx * cross);
+        for (int j = 0; j < 3; ++j) {
+          const T pa1 = kA * a3[j] - kM * d1[j] + g3_, pa3 = kb * a1[j], pd = -kM * d3[j], p0 = g1 * a3[j];
+          for (int i = 0; i < 3; ++i) {
+            const T x = pa1 * a1[i] + pa3 * a3[i] + pd * d3[i] + p0;
+            put(kS_J31 + 3 * j + i, i == j ? x + kM : x);
+          }
+        }
+      }
     }
   }
-  int f = 0;
-  auto put = [&](const T& x) { stT(buf, dbuf, 4 * (f++) + seg, nt, n0, x); };
-  for (int i = 0; i < 3; ++i) put(Fx1[i]);
-  for (int i = 0; i < 3; ++i) put(Fx3[i]);
-  for (int i = 0; i < 3; ++i) for (int j = 0; j < 3; ++j) put(J11[i][j]);
-  for (int i = 0; i < 3; ++i) for (int j = 0; j < 3; ++j) put(J13[i][j]);
-  for (int i = 0; i < 3; ++i) for (int j = 0; j < 3; ++j) put(J31[i][j]);
-  for (int i = 0; i < 3; ++i) for (int j = 0; j < 3; ++j) put(J33[i][j]);
+}
+// the record in the shear buffer at slot seg * ntot + n0
+template <class T>
+YS_HD void shear_element(const View& v, double* buf, double* dbuf, int n0, int seg) {
+  shear_terms<T>(v, n0, seg, [&](int f, const T& x) { stT(buf, dbuf, 4 * f + seg, v.ntot, n0, x); });
 }
 
 }  // namespace ys
