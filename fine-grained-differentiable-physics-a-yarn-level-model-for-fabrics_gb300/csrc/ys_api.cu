@@ -200,7 +200,7 @@ struct ys_batch {
     int max_nodes = 0;
   } plan;
   std::vector<ys_schedule> tuned;  // every schedule the last ys_autotune timed
-  int producer_threads = ys::kBlock;  // block size of the record producers and the gather
+  int producer_threads = ys::kBlock;  // block size of the record producers
   bool has_system = false;  // v.A / v.B hold an assembled system (kept after the update)
   // learned preconditioner (ys_set_preconditioner); buffers allocated on first use
   struct Learn {
@@ -497,7 +497,6 @@ ys_status ys_batch_create(int32_t n_cloths, const ys_cloth_desc* descs, int32_t 
   A(&v.A, (size_t)ys::YS_NUM_SLOTS * nt); A(&v.B, 5 * nt);
   A(&b->rec.edge, (size_t)ys::kEdgeFields * 2 * nt); A(&b->rec.bend, (size_t)ys::kBendFields * 2 * nt);
   A(&b->rec.face, 6 * nt); A(&b->rec.shear, (size_t)ys::kShearFields * 4 * nt);
-  A(&b->rec.nonfinite, nt);
   A(&b->vecs, 25 * nt);
   if (b->vecs) {
     b->so.x = b->vecs; b->so.r = b->vecs + 5 * nt; b->so.p = b->vecs + 10 * nt;
@@ -760,11 +759,11 @@ ys_status ys_assemble(ys_batch* b, double h, const double* ext_force, int32_t fl
   b->run(YS_PROF_EDGES, 1, [&] { ys::launch_edge_records(v, R, s, pt); });
   b->run(YS_PROF_BENDS, 1, [&] { ys::launch_bend_records(v, R, s, pt); });
   b->run(YS_PROF_FACES, 1, [&] { ys::launch_face_records(v, R, s, pt); });
-  // row blocks + ConSlideFriction (needs every edge and bend term; shear
-  // needs its compression, src/PhysicsCloth.cpp:97-131)
-  b->run(YS_PROF_GATHER, 1, [&] { ys::launch_gather(v, R, s, pt); });
+  // ConSlideFriction (needs every edge and bend term; shear needs its
+  // compression, src/PhysicsCloth.cpp:97-131), then the row blocks
+  b->run(YS_PROF_GATHER, 1, [&] { ys::launch_cross(v, R, s); });
   b->run(YS_PROF_SHEAR, 1, [&] { ys::launch_shear_records(v, R, s, pt); });
-  b->run(YS_PROF_FINALIZE, 1, [&] { ys::launch_finalize(v, R, b->blk, b->so, s); });
+  b->run(YS_PROF_FINALIZE, 1, [&] { ys::launch_rows(v, R, b->so, s); });
   YS_CUDA(cudaGetLastError());
   b->assembled = true;
   b->has_system = true;
@@ -1618,9 +1617,9 @@ void capture_assembly(ys_batch* b, cudaStream_t cs, int override_max) {
     cudaEventRecord(G.join[k], G.side[k]);
     cudaStreamWaitEvent(cs, G.join[k], 0);
   }
-  ys::launch_gather(v, R, cs, b->producer_threads);
+  ys::launch_cross(v, R, cs);
   ys::launch_shear_records(v, R, cs, b->producer_threads);
-  ys::launch_finalize(v, R, b->blk, b->so, cs);
+  ys::launch_rows(v, R, b->so, cs);
   k_reset_pc<<<(b->ncloth + 127) / 128, 128, 0, cs>>>(b->so.pc, b->maxiter_dev, b->ncloth, override_max);
 }
 

@@ -1,4 +1,4 @@
-// ys_elem_kernels.cuh -- the element-record and gather kernels of one step,
+// ys_elem_kernels.cuh -- the element-record kernels of one step,
 // templates over the scalar type (double for the step, Dual<kTangents> for
 // its forward-mode sensitivities); instantiated in ys_kernels.cu and
 // ys_tangent.cu.
@@ -9,8 +9,8 @@
 
 namespace ys {
 
-// The record producers and the gather: one thread per element (or node),
-// nothing shared between threads, so any block size gives the same bits; the
+// The record producers: one thread per element, nothing shared between
+// threads, so any block size gives the same bits; the
 // block size is a schedule choice (up to kMaxProducerBlock threads; up to
 // kBlock for the edges, whose 254 registers spill when compiled for 256-thread
 // blocks).
@@ -52,13 +52,6 @@ __global__ void __launch_bounds__(kMaxProducerBlock) k_face_rec(View v, Records 
   const ClothParams& P = v.cp[v.node_cloth[n]];
   if (v.node_u[n] >= P.W - 1 || v.node_v[n] >= P.H - 1) return;
   cell_faces<T>(v, R.face, R.dface, n);
-}
-
-// row blocks from edge / bend / face records, plus sliding friction
-template <class T>
-__global__ void __launch_bounds__(kMaxProducerBlock) k_gather(View v, Records R) {
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n < v.ntot) gather_elements<T>(v, R, n);
 }
 
 // one thread per (segment type, crossing)

@@ -24,9 +24,6 @@ struct Records {
   double* dbend;
   double* dface;
   double* dshear;
-  // per node: 1 if a coefficient or right-hand side the gather wrote is not
-  // finite (null: the finalize checks every slot itself)
-  uint8_t* nonfinite;
 };
 
 YS_HD double rec(const double* buf, int field, int nslot, int slot_, int ntot, int node) {
@@ -43,451 +40,375 @@ YS_HD void stA(const View& v, int s, int n, const T& x) { stT(v.A, v.dA, s, v.nt
 template <class T>
 YS_HD T ldA(const View& v, int s, int n) { return ldT<T>(v.A, v.dA, s, v.ntot, n); }
 
-// Gathers, for row block n, every contribution of the edges, bend segments
-// and faces that touch it, runs ConSlideFriction on the gathered no-slide
-// quantities, and writes all 159 coefficient slots and b (the diagonal
-// blocks, which only shear segments fill, are set to 0 here). Node-node
-// blocks of X_LL are written transposed into the dense matrix
-// (src/MatrixMp.cpp:54-65), hence the blk[3 * c + r] reads.
-template <class T>
-YS_HD void gather_elements(const View& v, const Records& R, int n) {
-  bool fin = true;  // every value written below is finite
-  auto putA = [&](int s_, int n_, const T& x) {
-    fin = fin && isfinite(val(x));
-    stA(v, s_, n_, x);
-  };
-  const int nt = v.ntot;
-  const ClothParams& P = v.cp[v.node_cloth[n]];
-  const int W = P.W, H = P.H, u = v.node_u[n], w = v.node_v[n];
-  const bool in = (v.flags[n] & YS_INTERIOR) != 0;
-  const double h = v.h, mh2 = -(v.h * v.h);
-  // ------------------------------------------------------------ self block
-  {
-    T LL[9], LE[6], EL[6], EE[2], B[5], FE[2], KEE[2], DEE[2], CL[3], CLE[6];
-    for (int i = 0; i < 9; ++i) LL[i] = 0.0;
-    for (int i = 0; i < 6; ++i) LE[i] = EL[i] = CLE[i] = 0.0;
-    for (int i = 0; i < 2; ++i) EE[i] = FE[i] = KEE[i] = DEE[i] = 0.0;
-    for (int i = 0; i < 5; ++i) B[i] = 0.0;
-    for (int i = 0; i < 3; ++i) CL[i] = 0.0;
-    // unrolled: the accumulators are indexed by k, and a rolled loop would
-    // put them in local memory
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      // edges along k: this node as n0 (anchor n) and as n1 (anchor n - step)
-      const int step = k == 0 ? 1 : W;
-      const bool has0 = k == 0 ? (u < W - 1) : (w < H - 1);
-      const bool has1 = k == 0 ? (u > 0) : (w > 0);
-      for (int a = 0; a < 2; ++a) {
-        if (!(a == 0 ? has0 : has1)) continue;
-        const int anc = a == 0 ? n : n - step;
-        auto E = [&](int f) { return recT<T>(R.edge, R.dedge, f, 2, k, nt, anc); };
-        const int p = 3 * a;  // block (a, a)
-        const double end = a == 0 ? 1.0 : -1.0;
-        const T cI = E(kE_llI + p), cP = E(kE_lP), cl = E(kE_cl), cle = E(kE_cle);
-        const T d[3] = {E(kE_d), E(kE_d + 1), E(kE_d + 2)};
-        for (int r = 0; r < 3; ++r)
-          for (int c = 0; c < 3; ++c) LL[3 * r + c] += (r == c ? cI : 0.0) + cP * ((r == c ? 1.0 : 0.0) - d[r] * d[c]);
-        for (int r = 0; r < 3; ++r) {
-          LE[2 * r + k] += E(kE_le + 3 * p + r);
-          EL[3 * k + r] += E(kE_el + 3 * p + r);
-          B[r] += E(kE_b + 4 * a + r);
-          CL[r] += end * (cl * d[r]);
-          if (in) CLE[3 * k + r] += cle * d[r];
-        }
-        EE[k] += E(kE_ee + p);
-        B[3 + k] += E(kE_b + 4 * a + 3);
-        FE[k] += E(kE_fe + a);
-        KEE[k] += E(kE_kee + a);
-        DEE[k] += E(kE_dee + a);
-      }
-      // bend segments along k with middle m: this node is n2 (m = n + step),
-      // n0 (m = n) or n1 (m = n - step)
-      const int pos = k == 0 ? u : w, len = k == 0 ? W : H;
-      const double sgn = (k == 0) ? 1.0 : -1.0;
-      for (int role = 0; role < 3; ++role) {
-        const int mid = role == 0 ? pos + 1 : role == 1 ? pos : pos - 1;
-        if (mid < 1 || mid > len - 2) continue;
-        const int anc = role == 0 ? n + step : role == 1 ? n : n - step;
-        auto Bf = [&](int f) { return recT<T>(R.bend, R.dbend, f, 2, k, nt, anc); };
-        if (role != 1) {
-          const int f = role == 0 ? kB_L22 : kB_L11;
-          T blk[6];
-          for (int i = 0; i < 6; ++i) blk[i] = Bf(f + i);
-          for (int r = 0; r < 3; ++r)
-            for (int c = 0; c < 3; ++c) LL[3 * r + c] += blk[sym3(r, c)];
-        } else {  // L00 = L11 + L12 + L21 + L22 (src/PhysicsCloth.cpp:709), symmetric
-          T blk[6], x12[9];
-          for (int i = 0; i < 6; ++i) blk[i] = Bf(kB_L11 + i) + Bf(kB_L22 + i);
-          for (int i = 0; i < 9; ++i) x12[i] = Bf(kB_L12 + i);
-          for (int r = 0; r < 3; ++r)
-            for (int c = r; c < 3; ++c) {
-              const T t = blk[sym3(r, c)] + (x12[3 * r + c] + x12[3 * c + r]);
-              LL[3 * r + c] += t;
-              if (c != r) LL[3 * c + r] += t;
-            }
-        }
-        if (role == 1) {  // n0: F_x0 = -(F_x1 + F_x2), F_u0 = 0
-          for (int r = 0; r < 3; ++r) {
-            B[r] -= h * (Bf(kB_F1 + r) + Bf(kB_F2 + r));
-            CL[r] -= sgn * (Bf(kB_cF1 + r) + Bf(kB_cF2 + r));
-          }
-          continue;
-        }
-        // n2 (src/PhysicsCloth.cpp:737-753) or n1 (755-772): its force F, and
-        // end / du times it in the Eulerian couplings (+ at n2, - at n1)
-        const int f0 = role == 0 ? kB_F2 : kB_F1, g0 = role == 0 ? kB_cF2 : kB_cF1;
-        const double end = role == 0 ? 1.0 : -1.0;
-        const T idu = end * Bf(kB_idu), cidu = (end * sgn) * Bf(kB_cidu);
-        for (int r = 0; r < 3; ++r) {
-          const T F = Bf(f0 + r), cF = Bf(g0 + r);
-          B[r] += h * F;
-          CL[r] += sgn * cF;
-          if (in) {
-            const T t = mh2 * (idu * F);
-            LE[2 * r + k] += t;
-            EL[3 * k + r] += t;
-            CLE[3 * k + r] += cidu * cF;
-          }
-        }
-        if (in) {
-          const T e11 = Bf(kB_E1E1), fu = end * Bf(kB_Fu2);
-          EE[k] += mh2 * e11;
-          KEE[k] += e11;
-          B[3 + k] += h * fu;
-          FE[k] += fu;
-        }
-      }
-    }
-    // faces of the (up to) four cells around the node (src/Cloth.cpp:271-287)
-    for (int cj = w - 1; cj <= w; ++cj)
-      for (int ci = u - 1; ci <= u; ++ci) {
-        if (ci < 0 || ci >= W - 1 || cj < 0 || cj >= H - 1) continue;
-        const int tl = n + (ci - u) + (cj - w) * W;
-        const bool right = ci != u, below = cj != w;  // node is tr / bl / br of that cell
-        const bool even = ((ci + cj) & 1) == 0;
-        bool inA, inB;
-        if (!right && !below) { inA = true; inB = even; }       // tl
-        else if (right && !below) { inA = true; inB = !even; }  // tr
-        else if (!right && below) { inA = !even; inB = true; }  // bl
-        else { inA = even; inB = true; }                        // br
-        for (int r = 0; r < 3; ++r) {
-          if (inA) B[r] += h * ldT<T>(R.face, R.dface, r, nt, tl);
-          if (inB) B[r] += h * ldT<T>(R.face, R.dface, 3 + r, nt, tl);
-        }
-      }
-    if (in) {
-      T aEE[2], bE[2];
-      friction_node(v, n, FE, KEE, DEE, CL, CLE, aEE, bE);
-      for (int k = 0; k < 2; ++k) {
-        EE[k] += aEE[k];
-        B[3 + k] += bE[k];
-      }
-    }
-    for (int i = 0; i < 9; ++i) putA(YS_SLOT_LL + i, n, LL[i]);
-    for (int i = 0; i < 6; ++i) {
-      putA(YS_SLOT_LE_SELF + i, n, LE[i]);
-      putA(YS_SLOT_EL_SELF + i, n, EL[i]);
-    }
-    for (int k = 0; k < 2; ++k) putA(YS_SLOT_EE_SELF + k, n, EE[k]);
-    for (int i = 0; i < 5; ++i) {
-      fin = fin && isfinite(val(B[i]));
-      stT(v.B, v.dB, i, nt, n, B[i]);
-    }
-  }
-  // ------------------------------------------------ yarn neighbours (+-1)
-  for (int m = 0; m < 4; ++m) {
-    const int k = m < 2 ? 0 : 1;
-    const int dir = (m & 1) ? 1 : -1;  // -1: previous, +1: next along the yarn
-    const int step = k == 0 ? 1 : W;
-    const int pos = k == 0 ? u : w, len = k == 0 ? W : H;
-    const int s = stencil_index(k == 0 ? dir : 0, k == 1 ? dir : 0);
-    T LL[9], LE[3], EL[3], EE = 0.0;
-    for (int i = 0; i < 9; ++i) LL[i] = 0.0;
-    for (int i = 0; i < 3; ++i) LE[i] = EL[i] = 0.0;
-    if (pos + dir >= 0 && pos + dir < len) {
-      const int nb = n + dir * step;
-      const bool inb = (v.flags[nb] & YS_INTERIOR) != 0;
-      // the edge between n and nb: n is its n0 when dir = +1
-      const int a = dir > 0 ? 0 : 1, o = 1 - a;
-      const int anc = dir > 0 ? n : nb;
-      auto E = [&](int f) { return recT<T>(R.edge, R.dedge, f, 2, k, nt, anc); };
-      const int p = 2 * a + o;
-      const T cI = E(kE_llI + p), cP = -E(kE_lP);
-      const T d[3] = {E(kE_d), E(kE_d + 1), E(kE_d + 2)};
-      for (int r = 0; r < 3; ++r)
-        for (int c = 0; c < 3; ++c) LL[3 * r + c] += (r == c ? cI : 0.0) + cP * ((r == c ? 1.0 : 0.0) - d[r] * d[c]);
-      for (int r = 0; r < 3; ++r) {
-        LE[r] += E(kE_le + 3 * p + r);
-        EL[r] += E(kE_el + 3 * p + r);
-      }
-      EE += E(kE_ee + p);
-      // bend segments containing both n and nb
-      for (int which = 0; which < 2; ++which) {
-        // which 0: middle = n (nb is n1 if dir = +1, n2 if dir = -1)
-        // which 1: middle = nb (n is n2 if dir = +1, n1 if dir = -1)
-        const int mid = which == 0 ? pos : pos + dir;
-        if (mid < 1 || mid > len - 2) continue;
-        const int ancb = which == 0 ? n : nb;
-        auto Bf = [&](int f) { return recT<T>(R.bend, R.dbend, f, 2, k, nt, ancb); };
-        // L01 = -(L11 + L21), L10 = -(L11 + L12), L02 = -(L12 + L22),
-        // L20 = -(L21 + L22), written transposed: L21 = L12^T, so L12
-        // enters as it is towards the next crossing and transposed towards the last
-        const int fs = (which == 0) == (dir > 0) ? kB_L11 : kB_L22;
-        T blk[6], x12[9];
-        for (int i = 0; i < 6; ++i) blk[i] = Bf(fs + i);
-        for (int i = 0; i < 9; ++i) x12[i] = Bf(kB_L12 + i);
-        for (int r = 0; r < 3; ++r)
-          for (int c = 0; c < 3; ++c) LL[3 * r + c] -= blk[sym3(r, c)] + (dir < 0 ? x12[3 * c + r] : x12[3 * r + c]);
-        // Eulerian couplings of Bending_D (src/PhysicsCloth.cpp:774-822):
-        // q = L1E1 + L2E1 = L0E2 = E2L0 = -L0E1 = -E1L0
-        T q[3];
-        const T idu = -Bf(kB_idu);
-        for (int r = 0; r < 3; ++r) q[r] = idu * (Bf(kB_F1 + r) + Bf(kB_F2 + r));
-        if (which == 0 && in && inb) {
-          if (dir < 0)  // row n0 = n, column e / x of n2 = nb
-            for (int r = 0; r < 3; ++r) { LE[r] += mh2 * q[r]; EL[r] += mh2 * q[r]; }
-          else  // row n0 = n, column e of n1 = nb
-            for (int r = 0; r < 3; ++r) LE[r] += mh2 * (-q[r]);
-        }
-        if (which == 1 && dir < 0 && in && inb)  // row n1 = n, column x of n0 = nb
-          for (int r = 0; r < 3; ++r) EL[r] += mh2 * (-q[r]);
-      }
-    }
-    for (int i = 0; i < 9; ++i) putA(YS_SLOT_LL + 9 * s + i, n, LL[i]);
-    for (int r = 0; r < 3; ++r) {
-      putA(YS_SLOT_LE_NBR + 3 * m + r, n, LE[r]);
-      putA(YS_SLOT_EL_NBR + 3 * m + r, n, EL[r]);
-    }
-    putA(YS_SLOT_EE_NBR + m, n, EE);
-  }
-  // ------------------------------------------- second neighbours (+-2)
-  for (int m = 0; m < 4; ++m) {
-    const int k = m < 2 ? 0 : 1;
-    const int dir = (m & 1) ? 1 : -1;
-    const int step = k == 0 ? 1 : W;
-    const int pos = k == 0 ? u : w, len = k == 0 ? W : H;
-    const int s = stencil_index(k == 0 ? 2 * dir : 0, k == 1 ? 2 * dir : 0);
-    const int mid = pos + dir;
-    const bool ok = mid >= 1 && mid <= len - 2;
-    const int anc = n + dir * step;
-    for (int r = 0; r < 3; ++r)
-      for (int c = 0; c < 3; ++c)  // transposed L21 = L12^T where n is n2 (dir +1), transposed L12 where n is n1
-        putA(YS_SLOT_LL + 9 * s + 3 * r + c, n,
-            ok ? recT<T>(R.bend, R.dbend, kB_L12 + (dir > 0 ? 3 * r + c : 3 * c + r), 2, k, nt, anc) : T(0.0));
-  }
-  // diagonal neighbours: shear only (gather_shear_finalize)
-  for (int s = 9; s < 13; ++s)
-    for (int i = 0; i < 9; ++i) putA(YS_SLOT_LL + 9 * s + i, n, T(0.0));
-  if (R.nonfinite) R.nonfinite[n] = fin ? 0 : 1;
+// every bit pattern but infinities and NaN; an integer test, as a compare would
+// take the FP64 pipe the producers and gathers wait for
+YS_HD bool finite_(double x) {
+#if defined(__CUDA_ARCH__)
+  return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000;
+#else
+  return isfinite(x);
+#endif
 }
 
-// Adds the shear segments touching row block n (as crossing n0, as warp
-// neighbour n1 or as weft neighbour n3; src/PhysicsCloth.cpp:2643-3089), then
-// the handle springs (Constraint_F / Constraint_D, src/PhysicsCloth.cpp:232-248),
-// the external force of SimStep(..., ext_force) (src/TrainHelper.cpp:63),
-// identity rows for the Eulerian DOFs boundary nodes do not have, and the
-// Jacobi preconditioner (zero diagonal -> 1, as Eigen's
-// DiagonalPreconditioner). Returns false if the row block holds a non-finite
-// value (SimStep's DetectNaN / DetectInf, src/TrainHelper.cpp:22-37).
+// The two gathers split a node's work into four parts, one per yarn neighbour
+// m = 0..3: (-1, 0), (1, 0), (0, -1), (0, 1). Part m sums what the elements
+// towards that neighbour give to the node's own block, and owns the blocks
+// towards the neighbour, towards the next crossing beyond it and towards one
+// diagonal neighbour. No record is read by two parts except a bend segment's
+// L12 and forces (by the two parts along its yarn). On the device four lanes
+// of a warp (lanes i, i + 8, i + 16, i + 24 for node i of eight) run the parts
+// of a node and combine the sums by shuffles, so a small cloth has four times
+// the threads and a quarter of the chain; combined in the same order on the
+// host and for the tangents.
+YS_HD int part_k(int m) { return m >> 1; }
+YS_HD int part_dir(int m) { return (m & 1) ? 1 : -1; }
+
+struct NodeAt {
+  int n, u, w, W, H;
+  bool in;
+  YS_HD NodeAt(const View& v, int n_) : n(n_) {
+    const ClothParams& P = v.cp[v.node_cloth[n]];
+    W = P.W;
+    H = P.H;
+    u = v.node_u[n];
+    w = v.node_v[n];
+    in = (v.flags[n] & YS_INTERIOR) != 0;
+  }
+  YS_HD int step(int k) const { return k == 0 ? 1 : W; }
+  YS_HD int pos(int k) const { return k == 0 ? u : w; }
+  YS_HD int len(int k) const { return k == 0 ? W : H; }
+  YS_HD bool interior(int uu, int vv) const { return uu >= 1 && uu <= W - 2 && vv >= 1 && vv <= H - 2; }
+};
+
+// ---- the crossing pass: ConSlideFriction's inputs (src/PhysicsCloth.cpp:97-131)
+template <class T>
+struct CrossPart {
+  T CL[3];             // crimp compression, summed over the four parts
+  T FE, KEE, DEE;      // no-slide force and stiffness along yarn k, over its two parts
+  T CLE[3];
+};
+template <class T>
+YS_HD void cross_part(const View& v, const Records& R, const NodeAt& N, int m, CrossPart<T>& c) {
+  const int nt = v.ntot, n = N.n, k = part_k(m), dir = part_dir(m), step = N.step(k), pos = N.pos(k), len = N.len(k);
+  for (int r = 0; r < 3; ++r) c.CL[r] = c.CLE[r] = 0.0;
+  c.FE = c.KEE = c.DEE = 0.0;
+  const double sgn = k == 0 ? 1.0 : -1.0;
+  if (pos + dir >= 0 && pos + dir < len) {  // the edge: n is its n0 when dir = +1
+    const int a = dir > 0 ? 0 : 1, anc = dir > 0 ? n : n - step;
+    auto E = [&](int f) { return recT<T>(R.edge, R.dedge, f, 2, k, nt, anc); };
+    const T cl = E(kE_cl), cle = E(kE_cle);
+    for (int r = 0; r < 3; ++r) {
+      const T d = E(kE_d + r);
+      c.CL[r] += dir > 0 ? cl * d : -(cl * d);
+      c.CLE[r] += cle * d;
+    }
+    c.FE += E(kE_fe + a);
+    c.KEE += E(kE_kee + a);
+    c.DEE += E(kE_dee + a);
+  }
+  const int mid = pos + dir;
+  if (mid >= 1 && mid <= len - 2) {  // the segment centred on the neighbour: n is its n2 (dir = +1) or n1
+    auto Bf = [&](int f) { return recT<T>(R.bend, R.dbend, f, 2, k, nt, n + dir * step); };
+    const double end = dir;
+    const T cidu = (end * sgn) * Bf(kB_cidu);
+    for (int r = 0; r < 3; ++r) {
+      const T cF = Bf((dir > 0 ? kB_cF2 : kB_cF1) + r);
+      c.CL[r] += sgn * cF;
+      c.CLE[r] += cidu * cF;
+    }
+    c.KEE += Bf(kB_E1E1);
+    c.FE += end * Bf(kB_Fu2);
+  }
+  if (dir > 0 && pos >= 1 && pos <= len - 2) {  // the segment centred on n
+    auto Bf = [&](int f) { return recT<T>(R.bend, R.dbend, f, 2, k, nt, n); };
+    for (int r = 0; r < 3; ++r) c.CL[r] -= sgn * (Bf(kB_cF1 + r) + Bf(kB_cF2 + r));
+  }
+}
+
+// the crossing pass of node n: stores COMP and SLIDE, and leaves friction's
+// share of the Eulerian rows in their diagonal slots and in b
+template <class T>
+YS_HD void gather_elements(const View& v, const Records& R, int n) {
+  const NodeAt N(v, n);
+  if (!N.in) return;
+  CrossPart<T> c[4];
+  for (int m = 0; m < 4; ++m) cross_part(v, R, N, m, c[m]);
+  T CL[3];
+  for (int r = 0; r < 3; ++r) CL[r] = (c[0].CL[r] + c[1].CL[r]) + (c[2].CL[r] + c[3].CL[r]);
+  const T comp = crossing_comp(v, n, CL);
+  stT(v.COMP, v.dCOMP, 0, v.ntot, n, comp);
+  for (int k = 0; k < 2; ++k) {
+    const CrossPart<T>&a = c[2 * k], &b = c[2 * k + 1];
+    const T CLE[3] = {a.CLE[0] + b.CLE[0], a.CLE[1] + b.CLE[1], a.CLE[2] + b.CLE[2]};
+    T aEE, bE;
+    friction_node(v, n, k, comp, a.FE + b.FE, a.KEE + b.KEE, a.DEE + b.DEE, CLE, aEE, bE);
+    stA(v, YS_SLOT_EE_SELF + k, n, aEE);
+    stT(v.B, v.dB, 3 + k, v.ntot, n, bE);
+  }
+}
+
+// ---- the row pass
+// what part m gives to the node's own block: LL and b of the x rows (summed
+// over the four parts), and the Eulerian couplings of yarn k (over its two)
+template <class T>
+struct RowPart {
+  T LL[9], B[3], LE[3], EL[3], EE, Be;
+};
+// The diagonal neighbour (dx, dy) gets J13 from part (u, dx) and J31 from
+// part (v, dy). Part 0 owns (-1, -1), part 1 (1, 1), part 2 (1, -1), part 3
+// (-1, 1); each sends one share and receives one:
+YS_HD int diag_from(int m) { return m == 0 ? 2 : m == 1 ? 3 : m == 2 ? 1 : 0; }
+YS_HD int diag_slot(int m) { return m == 0 ? 9 : m == 1 ? 12 : m == 2 ? 10 : 11; }
+
+// Part m of row block n: writes the blocks towards the yarn neighbour and the
+// crossing beyond it, fills the sums of `o`, and hands its entries i of the
+// diagonal blocks to share(mine, i, value): mine, of the one it owns, else of
+// the one it sends. Node-node blocks are in the
+// orientation of the dense matrix (src/MatrixMp.cpp:54-65). Clears fin if a
+// value written is not finite.
+template <class T, class Share>
+YS_HD void row_part(const View& v, const Records& R, const NodeAt& N, int m, RowPart<T>& o, bool& fin, Share&& share) {
+  const int nt = v.ntot, n = N.n, k = part_k(m), dir = part_dir(m), step = N.step(k), pos = N.pos(k), len = N.len(k);
+  const double h = v.h, mh2 = -(v.h * v.h);
+  T nLL[9], nLE[3], nEL[3], nEE = 0.0;
+  for (int i = 0; i < 9; ++i) o.LL[i] = nLL[i] = 0.0;
+  for (int i = 0; i < 3; ++i) o.B[i] = o.LE[i] = o.EL[i] = nLE[i] = nEL[i] = 0.0;
+  o.EE = o.Be = 0.0;
+  const bool has = pos + dir >= 0 && pos + dir < len;
+  const int nb = has ? n + dir * step : n;
+  const bool inb = has && (v.flags[nb] & YS_INTERIOR) != 0;
+  if (has) {  // the edge between n and nb
+    const int a = dir > 0 ? 0 : 1, p = 3 * a, q = a + 1, anc = dir > 0 ? n : nb;
+    auto E = [&](int f) { return recT<T>(R.edge, R.dedge, f, 2, k, nt, anc); };
+    const T cP = E(kE_lP), cI = E(kE_llI + p), cJ = E(kE_llI + q);
+    const T d[3] = {E(kE_d), E(kE_d + 1), E(kE_d + 2)};
+    for (int r = 0; r < 3; ++r) {
+      const T pd = cP * d[r];
+      for (int c = 0; c < 3; ++c) {
+        const T x = (r == c ? cP : T(0.0)) - pd * d[c];
+        o.LL[3 * r + c] = r == c ? x + cI : x;
+        nLL[3 * r + c] = r == c ? cJ - x : -x;
+      }
+      o.B[r] = E(kE_b + 4 * a + r);
+      o.LE[r] = E(kE_le + 3 * p + r);
+      o.EL[r] = E(kE_el + 3 * p + r);
+      nLE[r] = E(kE_le + 3 * q + r);
+      nEL[r] = E(kE_el + 3 * q + r);
+    }
+    o.EE = E(kE_ee + p);
+    nEE = E(kE_ee + q);
+    o.Be = E(kE_b + 4 * a + 3);
+  }
+  if (has && pos >= 1 && pos <= len - 2) {  // the bend segment centred on n (nb is its n1 if dir = +1, else n2)
+    auto Bf = [&](int f) { return recT<T>(R.bend, R.dbend, f, 2, k, nt, n); };
+    // L01 = -(L11 + L21), L02 = -(L12 + L22), written transposed; L21 = L12^T
+    T own[6], x12[9], F[3];
+    for (int i = 0; i < 6; ++i) own[i] = Bf((dir > 0 ? kB_L11 : kB_L22) + i);
+    for (int i = 0; i < 9; ++i) x12[i] = Bf(kB_L12 + i);
+    for (int r = 0; r < 3; ++r)
+      for (int c = 0; c < 3; ++c) nLL[3 * r + c] -= own[sym3(r, c)] + (dir > 0 ? x12[3 * r + c] : x12[3 * c + r]);
+    for (int r = 0; r < 3; ++r) F[r] = Bf(kB_F1 + r) + Bf(kB_F2 + r);
+    if (dir > 0) {  // the middle's own block L00 = L11 + L12 + L21 + L22 (src/PhysicsCloth.cpp:709); F_x0 = -(F_x1 + F_x2)
+      for (int r = 0; r < 3; ++r) {
+        for (int c = r; c < 3; ++c) {
+          const T t = (own[sym3(r, c)] + Bf(kB_L22 + sym3(r, c))) + (x12[3 * r + c] + x12[3 * c + r]);
+          o.LL[3 * r + c] += t;
+          if (c != r) o.LL[3 * c + r] += t;
+        }
+        o.B[r] -= h * F[r];
+      }
+    }
+    // Eulerian couplings of Bending_D (src/PhysicsCloth.cpp:774-822):
+    // q = L1E1 + L2E1 = L0E2 = E2L0 = -L0E1 = -E1L0
+    if (N.in && inb) {
+      const T t = -mh2 * Bf(kB_idu);
+      for (int r = 0; r < 3; ++r) {
+        const T q = t * F[r];
+        if (dir < 0) { nLE[r] += q; nEL[r] += q; }  // row n0, column e / x of n2
+        else nLE[r] -= q;                           // row n0, column e of n1
+      }
+    }
+  }
+  const int mid = pos + dir;
+  const bool beyond = mid >= 1 && mid <= len - 2;
+  if (beyond) {  // the segment centred on nb: n is its n2 (dir = +1) or its n1
+    auto Bf = [&](int f) { return recT<T>(R.bend, R.dbend, f, 2, k, nt, nb); };
+    T own[6], x12[9], F[3], G[3];
+    for (int i = 0; i < 6; ++i) own[i] = Bf((dir > 0 ? kB_L22 : kB_L11) + i);
+    for (int i = 0; i < 9; ++i) x12[i] = Bf(kB_L12 + i);
+    const int s2 = stencil_index(k == 0 ? 2 * dir : 0, k == 1 ? 2 * dir : 0);
+    for (int r = 0; r < 3; ++r)
+      for (int c = 0; c < 3; ++c) {
+        // L20 = -(L21 + L22) or L10 = -(L11 + L12), and L21 or L12, transposed
+        const T x = dir > 0 ? x12[3 * r + c] : x12[3 * c + r], t = own[sym3(r, c)];
+        o.LL[3 * r + c] += t;
+        nLL[3 * r + c] -= t + x;
+        fin = fin && finite_(val(x));
+        stA(v, YS_SLOT_LL + 9 * s2 + 3 * r + c, n, x);
+      }
+    for (int r = 0; r < 3; ++r) {
+      F[r] = Bf((dir > 0 ? kB_F2 : kB_F1) + r);
+      G[r] = Bf((dir > 0 ? kB_F1 : kB_F2) + r);
+      o.B[r] += h * F[r];
+    }
+    if (N.in) {  // n2 (src/PhysicsCloth.cpp:737-753) or n1 (755-772)
+      const T t = mh2 * Bf(kB_idu);
+      for (int r = 0; r < 3; ++r) {
+        const T x = t * F[r];
+        if (dir > 0) { o.LE[r] += x; o.EL[r] += x; }
+        else { o.LE[r] -= x; o.EL[r] -= x; }
+        if (dir < 0 && inb) nEL[r] += x + t * G[r];  // row n1, column x of n0
+      }
+      o.EE += mh2 * Bf(kB_E1E1);
+      const T fu = h * Bf(kB_Fu2);
+      o.Be += dir > 0 ? fu : -fu;
+    }
+  } else {
+    const int s2 = stencil_index(k == 0 ? 2 * dir : 0, k == 1 ? 2 * dir : 0);
+    for (int i = 0; i < 9; ++i) stA(v, YS_SLOT_LL + 9 * s2 + i, n, T(0.0));
+  }
+  {  // wind on the cell (u - 1 + (m & 1), v - 1 + (m >> 1)) (src/Cloth.cpp:271-287)
+    const int ci = N.u - 1 + (m & 1), cj = N.w - 1 + (m >> 1);
+    if (ci >= 0 && ci < N.W - 1 && cj >= 0 && cj < N.H - 1) {
+      const int tl = n + (ci - N.u) + (cj - N.w) * N.W;
+      const bool right = ci != N.u, below = cj != N.w;  // n is tr / bl / br of that cell
+      const bool even = ((ci + cj) & 1) == 0;
+      const bool inA = !below || right == even, inB = below || right != even;
+      for (int r = 0; r < 3; ++r) {
+        if (inA) o.B[r] += h * ldT<T>(R.face, R.dface, r, nt, tl);
+        if (inB) o.B[r] += h * ldT<T>(R.face, R.dface, 3 + r, nt, tl);
+      }
+    }
+  }
+  // shear segments (src/PhysicsCloth.cpp:2643-3089, 3033-3047). For part
+  // (u, dir): J11 / J13 / F1, and J31 towards the crossing; for part (v, dir)
+  // the same with 1 <-> 3.
+  const int f1 = k == 0 ? kS_J11 : kS_J33, f13 = k == 0 ? kS_J13 : kS_J31, f31 = k == 0 ? kS_J31 : kS_J13;
+  const int fF = k == 0 ? kS_F1 : kS_F3;
+  if (N.in) {  // n is the crossing: its two segments towards nb
+    T t[9];
+    for (int i = 0; i < 9; ++i) t[i] = 0.0;
+    for (int j = 0; j < 2; ++j) {
+      const int seg = k == 0 ? (dir > 0 ? 2 : 0) + j : 2 * j + (dir > 0 ? 0 : 1);
+      for (int i = 0; i < 9; ++i)
+        t[i] += recT<T>(R.shear, R.dshear, f1 + i, 4, seg, nt, n) + recT<T>(R.shear, R.dshear, f31 + i, 4, seg, nt, n);
+      for (int r = 0; r < 3; ++r) o.B[r] -= recT<T>(R.shear, R.dshear, fF + r, 4, seg, nt, n);
+    }
+    for (int i = 0; i < 9; ++i) {  // J01 or J03 = -(J11 + J31), and its share of J00
+      o.LL[i] += t[i];
+      nLL[i] -= t[i];
+    }
+  }
+  if (inb) {  // nb is the crossing, n the end of two of its segments (on its side -dir)
+    for (int j = 0; j < 2; ++j) {
+      const int seg = k == 0 ? (dir > 0 ? 0 : 2) + j : 2 * j + (dir > 0 ? 1 : 0);
+      // the segment's other end lies at offset `side` across the yarn
+      const int side = k == 0 ? shear_dv(seg) : shear_du(seg);
+      const bool mine = k == 0 ? side == dir : side != dir;
+      for (int i = 0; i < 9; ++i) {
+        const T a = recT<T>(R.shear, R.dshear, f1 + i, 4, seg, nt, nb), b = recT<T>(R.shear, R.dshear, f13 + i, 4, seg, nt, nb);
+        o.LL[i] += a;
+        nLL[i] -= a + b;  // J10 or J30
+        share(mine, i, b);
+      }
+      for (int r = 0; r < 3; ++r) o.B[r] += recT<T>(R.shear, R.dshear, fF + r, 4, seg, nt, nb);
+    }
+  } else {
+    for (int i = 0; i < 9; ++i) {
+      share(true, i, T(0.0));
+      share(false, i, T(0.0));
+    }
+  }
+  const int s1 = stencil_index(k == 0 ? dir : 0, k == 1 ? dir : 0);
+  for (int i = 0; i < 9; ++i) {
+    fin = fin && finite_(val(nLL[i]));
+    stA(v, YS_SLOT_LL + 9 * s1 + i, n, nLL[i]);
+  }
+  for (int r = 0; r < 3; ++r) {
+    fin = fin && finite_(val(nLE[r])) && finite_(val(nEL[r]));
+    stA(v, YS_SLOT_LE_NBR + 3 * m + r, n, nLE[r]);
+    stA(v, YS_SLOT_EL_NBR + 3 * m + r, n, nEL[r]);
+  }
+  fin = fin && finite_(val(nEE));
+  stA(v, YS_SLOT_EE_NBR + m, n, nEE);
+}
+
+// Row r of the node's own block from the summed parts: the handle spring
+// (Constraint_F / Constraint_D, src/PhysicsCloth.cpp:232-248), the external
+// force of SimStep(..., ext_force) (src/TrainHelper.cpp:63) and the Jacobi
+// preconditioner (zero diagonal -> 1, as Eigen's DiagonalPreconditioner)
+template <class T>
+YS_HD void row_self_x(const View& v, int n, int r, const T* LL3, T b, double* dinv, bool& fin) {
+  const int nt = v.ntot;
+  const double h = v.h;
+  T dg = LL3[r];
+  if (v.flags[n] & YS_FIXED) {
+    const double kh = v.cp[v.node_cloth[n]].kh;
+    b += h * (-(kh * (ldT<T>(v.X, v.dX, r, nt, n) - ld(v.XF, r, nt, n))));
+    dg += (h * h) * kh;
+  }
+  if (v.ext) b += h * ld(v.ext, r, nt, n);
+  for (int c = 0; c < 3; ++c) {
+    const T x = c == r ? dg : LL3[c];
+    fin = fin && finite_(val(x));
+    stA(v, YS_SLOT_LL + 3 * r + c, n, x);
+  }
+  fin = fin && finite_(val(b));
+  stT(v.B, v.dB, r, nt, n, b);
+  if (dinv) st(dinv, r, nt, n) = val(dg) != 0.0 ? 1.0 / val(dg) : 1.0;
+}
+// the Eulerian row of yarn k (an identity row on the boundary), with the
+// crossing pass's friction
+template <class T>
+YS_HD void row_self_e(const View& v, int n, int k, bool in, const T* LE, const T* EL, T ee, T b, double* dinv, bool& fin) {
+  const int nt = v.ntot;
+  if (in) {
+    ee += ldA<T>(v, YS_SLOT_EE_SELF + k, n);
+    b += ldT<T>(v.B, v.dB, 3 + k, nt, n);
+    if (v.ext) b += v.h * ld(v.ext, 3 + k, nt, n);
+  } else {
+    ee = T(1.0);
+    b = T(0.0);
+  }
+  for (int r = 0; r < 3; ++r) {
+    fin = fin && finite_(val(LE[r])) && finite_(val(EL[r]));
+    stA(v, YS_SLOT_LE_SELF + 2 * r + k, n, LE[r]);
+    stA(v, YS_SLOT_EL_SELF + 3 * k + r, n, EL[r]);
+  }
+  fin = fin && finite_(val(ee)) && finite_(val(b));
+  stA(v, YS_SLOT_EE_SELF + k, n, ee);
+  stT(v.B, v.dB, 3 + k, nt, n, b);
+  if (dinv) st(dinv, 3 + k, nt, n) = val(ee) != 0.0 ? 1.0 / val(ee) : 1.0;
+}
+
+// Row block n whole, after the crossing pass and the shear records: all 159
+// slots and b. Returns false if it holds a non-finite value (SimStep's
+// DetectNaN / DetectInf, src/TrainHelper.cpp:22-37).
 template <class T>
 YS_HD bool gather_shear_finalize(const View& v, const Records& R, int n, double* dinv) {
-  const int nt = v.ntot;
-  const ClothParams& P = v.cp[v.node_cloth[n]];
-  const int W = P.W, H = P.H, u = v.node_u[n], w = v.node_v[n];
-  const uint8_t fl = v.flags[n];
-  const double h = v.h;
-  auto interior = [&](int uu, int vv) { return uu >= 1 && uu <= W - 2 && vv >= 1 && vv <= H - 2; };
-  auto S = [&](int f, int seg, int anc) { return recT<T>(R.shear, R.dshear, f, 4, seg, nt, anc); };
-  bool finf = true;  // every slot value this routine writes is finite
-  auto addLL = [&](int du, int dv, const T* blk) {  // A[x(n)][x(n + (du, dv))] += blk
-    const int s = stencil_index(du, dv);
-    if (s < 0) return;
-    // the block's nine slots are loaded together, then updated: a load per
-    // slot behind the previous slot's store would wait out one memory
-    // latency per slot
-    T a[9];
-#pragma unroll
-    for (int i = 0; i < 9; ++i) a[i] = ldA<T>(v, YS_SLOT_LL + 9 * s + i, n);
-#pragma unroll
-    for (int r = 0; r < 3; ++r)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        T& x = a[3 * r + c];
-        x += blk[3 * r + c];
-        finf = finf && isfinite(val(x));
-      }
-#pragma unroll
-    for (int i = 0; i < 9; ++i) stA(v, YS_SLOT_LL + 9 * s + i, n, a[i]);
-  };
-  auto addB = [&](int c, const T& x) {
-    T b = ldT<T>(v.B, v.dB, c, nt, n);
-    b += x;
-    stT(v.B, v.dB, c, nt, n, b);
-  };
-  T Bx[3] = {0.0, 0.0, 0.0};
-  if constexpr (std::is_same<T, double>::value) {
-    // The contributions below are summed per target block in registers and
-    // each slot of A is then updated once (a global read-modify-write per
-    // contribution would serialise on its own stores). Same terms as the
-    // tangent path in the else branch, summed in another order.
-    const bool in0 = (fl & YS_INTERIOR) != 0;
-    {  // the node's own block and its four yarn neighbours
-      double self[9], xa[2][9], ya[2][9];  // xa: (-1, 0), (1, 0); ya: (0, -1), (0, 1)
-#pragma unroll
-      for (int i = 0; i < 9; ++i) self[i] = xa[0][i] = xa[1][i] = ya[0][i] = ya[1][i] = 0.0;
-#pragma unroll
-      for (int seg = 0; seg < 4; ++seg) {
-        const int du = shear_du(seg), dv = shear_dv(seg);
-        const int ix = du < 0 ? 0 : 1, iy = dv < 0 ? 0 : 1;
-        if (in0) {  // as the crossing n0 (src/PhysicsCloth.cpp:3033-3047)
-#pragma unroll
-          for (int i = 0; i < 9; ++i) {
-            const double a11 = S(kS_J11 + i, seg, n), a13 = S(kS_J13 + i, seg, n);
-            const double a31 = S(kS_J31 + i, seg, n), a33 = S(kS_J33 + i, seg, n);
-            self[i] += -(-(a11 + a13) + -(a31 + a33));  // -(J10 + J30)
-            xa[ix][i] += -(a11 + a31);                   // J01, towards n1 = n + (du, 0)
-            ya[iy][i] += -(a13 + a33);                   // J03, towards n3 = n + (0, dv)
-          }
-          for (int r = 0; r < 3; ++r) Bx[r] -= S(kS_F1 + r, seg, n) + S(kS_F3 + r, seg, n);
-        }
-        if (interior(u - du, w)) {  // as the warp neighbour n1 of the crossing n - (du, 0)
-          const int anc = n - du;
-#pragma unroll
-          for (int i = 0; i < 9; ++i) {
-            const double b11 = S(kS_J11 + i, seg, anc), b13 = S(kS_J13 + i, seg, anc);
-            self[i] += b11;
-            xa[1 - ix][i] += -(b11 + b13);  // J10, towards n0 = n + (-du, 0)
-          }
-          for (int r = 0; r < 3; ++r) Bx[r] += S(kS_F1 + r, seg, anc);
-        }
-        if (interior(u, w - dv)) {  // as the weft neighbour n3 of the crossing n - (0, dv)
-          const int anc = n - dv * W;
-#pragma unroll
-          for (int i = 0; i < 9; ++i) {
-            const double c31 = S(kS_J31 + i, seg, anc), c33 = S(kS_J33 + i, seg, anc);
-            self[i] += c33;
-            ya[1 - iy][i] += -(c31 + c33);  // J30, towards n0 = n + (0, -dv)
-          }
-          for (int r = 0; r < 3; ++r) Bx[r] += S(kS_F3 + r, seg, anc);
-        }
-      }
-      addLL(0, 0, self);
-      addLL(-1, 0, xa[0]);
-      addLL(1, 0, xa[1]);
-      addLL(0, -1, ya[0]);
-      addLL(0, 1, ya[1]);
-    }
-    {  // the diagonal neighbours: J13 of a warp-neighbour role, J31 of a weft-neighbour role
-      double dg[4][9];  // (-1, -1), (1, -1), (-1, 1), (1, 1)
-#pragma unroll
-      for (int i = 0; i < 9; ++i) dg[0][i] = dg[1][i] = dg[2][i] = dg[3][i] = 0.0;
-#pragma unroll
-      for (int seg = 0; seg < 4; ++seg) {
-        const int du = shear_du(seg), dv = shear_dv(seg);
-        if (interior(u - du, w)) {  // towards n3 = n + (-du, dv)
-          const int t = (-du < 0 ? 0 : 1) + (dv < 0 ? 0 : 2);
-#pragma unroll
-          for (int i = 0; i < 9; ++i) dg[t][i] += S(kS_J13 + i, seg, n - du);
-        }
-        if (interior(u, w - dv)) {  // towards n1 = n + (du, -dv)
-          const int t = (du < 0 ? 0 : 1) + (-dv < 0 ? 0 : 2);
-#pragma unroll
-          for (int i = 0; i < 9; ++i) dg[t][i] += S(kS_J31 + i, seg, n - dv * W);
-        }
-      }
-      addLL(-1, -1, dg[0]);
-      addLL(1, -1, dg[1]);
-      addLL(-1, 1, dg[2]);
-      addLL(1, 1, dg[3]);
-    }
-  } else {
-    T J[9];
-    // as the crossing n0 (src/PhysicsCloth.cpp:3033-3047)
-    if (fl & YS_INTERIOR) {
-      for (int seg = 0; seg < 4; ++seg) {
-        for (int i = 0; i < 9; ++i) {
-          const T J10 = -(S(kS_J11 + i, seg, n) + S(kS_J13 + i, seg, n));
-          const T J30 = -(S(kS_J31 + i, seg, n) + S(kS_J33 + i, seg, n));
-          J[i] = -(J10 + J30);
-        }
-        addLL(0, 0, J);
-        for (int i = 0; i < 9; ++i) J[i] = -(S(kS_J11 + i, seg, n) + S(kS_J31 + i, seg, n));  // J01
-        addLL(shear_du(seg), 0, J);
-        for (int i = 0; i < 9; ++i) J[i] = -(S(kS_J13 + i, seg, n) + S(kS_J33 + i, seg, n));  // J03
-        addLL(0, shear_dv(seg), J);
-        for (int r = 0; r < 3; ++r) Bx[r] -= S(kS_F1 + r, seg, n) + S(kS_F3 + r, seg, n);
-      }
-    }
-    // as the warp neighbour n1 = n0 + (du, 0)
-    for (int seg = 0; seg < 4; ++seg) {
-      const int du = shear_du(seg), dv = shear_dv(seg);
-      if (!interior(u - du, w)) continue;
-      const int anc = n - du;
-      for (int i = 0; i < 9; ++i) J[i] = S(kS_J11 + i, seg, anc);
-      addLL(0, 0, J);
-      for (int i = 0; i < 9; ++i) J[i] = -(S(kS_J11 + i, seg, anc) + S(kS_J13 + i, seg, anc));  // J10
-      addLL(-du, 0, J);
-      for (int i = 0; i < 9; ++i) J[i] = S(kS_J13 + i, seg, anc);  // towards n3 = n + (-du, dv)
-      addLL(-du, dv, J);
-      for (int r = 0; r < 3; ++r) Bx[r] += S(kS_F1 + r, seg, anc);
-    }
-    // as the weft neighbour n3 = n0 + (0, dv)
-    for (int seg = 0; seg < 4; ++seg) {
-      const int du = shear_du(seg), dv = shear_dv(seg);
-      if (!interior(u, w - dv)) continue;
-      const int anc = n - dv * W;
-      for (int i = 0; i < 9; ++i) J[i] = S(kS_J33 + i, seg, anc);
-      addLL(0, 0, J);
-      for (int i = 0; i < 9; ++i) J[i] = -(S(kS_J31 + i, seg, anc) + S(kS_J33 + i, seg, anc));  // J30
-      addLL(0, -dv, J);
-      for (int i = 0; i < 9; ++i) J[i] = S(kS_J31 + i, seg, anc);  // towards n1 = n + (du, -dv)
-      addLL(du, -dv, J);
-      for (int r = 0; r < 3; ++r) Bx[r] += S(kS_F3 + r, seg, anc);
-    }
+  const NodeAt N(v, n);
+  bool fin = true;
+  RowPart<T> o[4];
+  T dg[2][4][9];
+  for (int m = 0; m < 4; ++m)
+    row_part(v, R, N, m, o[m], fin, [&](bool mine, int i, const T& x) { dg[mine ? 0 : 1][m][i] = x; });
+  T LL[9];
+  for (int i = 0; i < 9; ++i) LL[i] = (o[0].LL[i] + o[1].LL[i]) + (o[2].LL[i] + o[3].LL[i]);
+  for (int r = 0; r < 3; ++r)
+    row_self_x<T>(v, n, r, LL + 3 * r, (o[0].B[r] + o[1].B[r]) + (o[2].B[r] + o[3].B[r]), dinv, fin);
+  for (int k = 0; k < 2; ++k) {
+    const RowPart<T>&a = o[2 * k], &b = o[2 * k + 1];
+    T LE[3], EL[3];
+    for (int r = 0; r < 3; ++r) { LE[r] = a.LE[r] + b.LE[r]; EL[r] = a.EL[r] + b.EL[r]; }
+    row_self_e<T>(v, n, k, N.in, LE, EL, a.EE + b.EE, a.Be + b.Be, dinv, fin);
   }
-  for (int r = 0; r < 3; ++r) addB(r, Bx[r]);
-  // handles, external force, boundary identity rows
-  if (fl & YS_FIXED) {
-    for (int i = 0; i < 3; ++i) {
-      addB(i, h * (-(P.kh * (ldT<T>(v.X, v.dX, i, nt, n) - ld(v.XF, i, nt, n)))));
-      const int sl = YS_SLOT_LL + i * 3 + i;
-      T a = ldA<T>(v, sl, n);
-      a += -(h * h) * (-P.kh);
-      finf = finf && isfinite(val(a));
-      stA(v, sl, n, a);
+  for (int m = 0; m < 4; ++m)
+    for (int i = 0; i < 9; ++i) {
+      const T x = dg[0][m][i] + dg[1][diag_from(m)][i];
+      fin = fin && finite_(val(x));
+      stA(v, YS_SLOT_LL + 9 * diag_slot(m) + i, n, x);
     }
-  }
-  if (v.ext) {
-    for (int i = 0; i < 3; ++i) addB(i, T(h * ld(v.ext, i, nt, n)));
-    if (fl & YS_INTERIOR)
-      for (int k = 0; k < 2; ++k) addB(3 + k, T(h * ld(v.ext, 3 + k, nt, n)));
-  }
-  if (!(fl & YS_INTERIOR)) {
-    for (int k = 0; k < 2; ++k) {
-      stA(v, YS_SLOT_EE_SELF + k, n, T(1.0));
-      stT(v.B, v.dB, 3 + k, nt, n, T(0.0));
-    }
-  }
-  bool ok = true;
-  if (R.nonfinite) {
-    // the gather checked what it wrote; the slots changed here were checked
-    // as they were written
-    ok = finf && !R.nonfinite[n];
-  } else {
-    for (int s = 0; s < YS_NUM_SLOTS; ++s) ok = ok && isfinite(slot(v, s, n));
-  }
-  for (int c = 0; c < 5; ++c) ok = ok && isfinite(ld(v.B, c, nt, n));
-  if (dinv) {
-    for (int i = 0; i < 3; ++i) {
-      const double dg = slot(v, YS_SLOT_LL + i * 3 + i, n);
-      st(dinv, i, nt, n) = dg != 0.0 ? 1.0 / dg : 1.0;
-    }
-    for (int k = 0; k < 2; ++k) {
-      const double dg = slot(v, YS_SLOT_EE_SELF + k, n);
-      st(dinv, 3 + k, nt, n) = dg != 0.0 ? 1.0 / dg : 1.0;
-    }
-  }
-  return ok;
+  return fin;
 }
 
 // The SpMV rows read their input vector through an accessor: at(j) is a

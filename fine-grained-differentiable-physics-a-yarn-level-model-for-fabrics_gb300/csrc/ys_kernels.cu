@@ -1,11 +1,10 @@
 // ys_kernels.cu -- CUDA kernels of one implicit step of a batch of cloths.
 //
 // Assembly: one thread per element writes that element's record (forces and
-// Jacobian blocks), then one thread per node gathers the records touching its
+// Jacobian blocks), then four threads per node gather the records touching its
 // row block in a fixed order, so every row is accumulated deterministically
-// without atomics. The element and gather kernels are templates over the
-// scalar type: double for the step, Dual<kTangents> for its forward-mode
-// sensitivities.
+// without atomics. The element kernels are templates over the scalar type:
+// double for the step, Dual<kTangents> for its forward-mode sensitivities.
 // Solve: per-cloth Jacobi-PCG (Eigen's ConjugateGradient algorithm, as used by
 // src/Solvers.cpp:3-31) on the structured stencil matrix; thread blocks never
 // straddle cloths, so each cloth's dot products are a fixed-order sum of its
@@ -27,6 +26,90 @@ __global__ void k_geom(View v, const int* __restrict__ nodes, int count) {
   node_normal(v, n, v.cp[v.node_cloth[n]].W);
 }
 
+// ------------------------------------------------------------- the gathers
+// A block takes 32 consecutive nodes, warp m their part m (ys_items.cuh), so
+// a warp's branches are uniform and its loads whole 256-byte runs; the parts
+// meet in shared memory in the order the host code adds them.
+constexpr int kNodesPerBlock = 32;
+
+// crossing pass: compression, slide indicator and friction. FP64-latency bound
+// (an exp and three tanh behind the sums): the two yarns' frictions run in
+// two warps.
+__global__ void __launch_bounds__(4 * kNodesPerBlock) k_cross(View v, Records R) {
+  __shared__ double sc[3][4][kNodesPerBlock], sk[6][4][kNodesPerBlock];
+  const int m = threadIdx.x >> 5, i = threadIdx.x & 31;
+  const int node = blockIdx.x * kNodesPerBlock + i;
+  const bool valid = node < v.ntot;
+  const int n = valid ? node : v.ntot - 1;
+  const NodeAt N(v, n);
+  if (valid && N.in) {
+    CrossPart<double> c;
+    cross_part(v, R, N, m, c);
+    for (int r = 0; r < 3; ++r) { sc[r][m][i] = c.CL[r]; sk[r][m][i] = c.CLE[r]; }
+    sk[3][m][i] = c.FE;
+    sk[4][m][i] = c.KEE;
+    sk[5][m][i] = c.DEE;
+  }
+  __syncthreads();
+  if (m >= 2 || !valid || !N.in) return;
+  double CL[3], s[6];
+  for (int r = 0; r < 3; ++r) CL[r] = (sc[r][0][i] + sc[r][1][i]) + (sc[r][2][i] + sc[r][3][i]);
+  const int k = m;
+  for (int r = 0; r < 6; ++r) s[r] = sk[r][2 * k][i] + sk[r][2 * k + 1][i];
+  const double comp = crossing_comp(v, n, CL);
+  if (k == 0) st(v.COMP, 0, v.ntot, n) = comp;
+  double aEE, bE;
+  friction_node(v, n, k, comp, s[3], s[4], s[5], s, aEE, bE);
+  slot(v, YS_SLOT_EE_SELF + k, n) = aEE;
+  st(v.B, 3 + k, v.ntot, n) = bE;
+}
+
+// row pass: the 159 slots, b and the Jacobi diagonal of every row block, each
+// written once. Latency bound on the record loads: four warps a node hide
+// what one thread a node could not. With k_cross, 0.70 ms on 255,292 nodes for
+// the 0.97 ms of a gather and a finalize that took one thread a node each and
+// passed 81 slots through memory; 34 us for 99 on one 50 x 50 cloth.
+__global__ void __launch_bounds__(4 * kNodesPerBlock) k_rows(View v, Records R, Solver so) {
+  __shared__ double sx[12][4][kNodesPerBlock], se[8][4][kNodesPerBlock], sd[2][9][4][kNodesPerBlock];
+  const int m = threadIdx.x >> 5, i = threadIdx.x & 31;
+  const int node = blockIdx.x * kNodesPerBlock + i;
+  const bool valid = node < v.ntot;
+  const int n = valid ? node : v.ntot - 1;
+  const NodeAt N(v, n);
+  bool fin = true;
+  if (valid) {
+    RowPart<double> o;
+    row_part(v, R, N, m, o, fin, [&](bool mine, int j, double x) { sd[mine ? 0 : 1][j][m][i] = x; });
+    for (int j = 0; j < 9; ++j) sx[j][m][i] = o.LL[j];
+    for (int r = 0; r < 3; ++r) { sx[9 + r][m][i] = o.B[r]; se[r][m][i] = o.LE[r]; se[3 + r][m][i] = o.EL[r]; }
+    se[6][m][i] = o.EE;
+    se[7][m][i] = o.Be;
+  }
+  __syncthreads();
+  if (!valid) return;
+  const int from = diag_from(m), ds = YS_SLOT_LL + 9 * diag_slot(m);
+  for (int j = 0; j < 9; ++j) {
+    const double x = sd[0][j][m][i] + sd[1][j][from][i];
+    fin = fin && finite_(x);
+    slot(v, ds + j, n) = x;
+  }
+  if (m < 3) {
+    double s[4];
+    for (int c = 0; c < 4; ++c) {
+      const int j = c < 3 ? 3 * m + c : 9 + m;
+      s[c] = (sx[j][0][i] + sx[j][1][i]) + (sx[j][2][i] + sx[j][3][i]);
+    }
+    row_self_x<double>(v, n, m, s, s[3], so.dinv, fin);
+  }
+  if (m >= 2) {
+    const int k = m - 2;
+    double s[8];
+    for (int c = 0; c < 8; ++c) s[c] = se[c][2 * k][i] + se[c][2 * k + 1][i];
+    row_self_e<double>(v, n, k, N.in, s, s + 3, s[6], s[7], so.dinv, fin);
+  }
+  if (!fin) atomicOr(&so.pc[v.node_cloth[n]].status, 1);
+}
+
 // ----------------------------------------------------------------- solve
 __device__ __forceinline__ double block_sum(double val, double* sh) {
   for (int o = 16; o > 0; o >>= 1) val += __shfl_down_sync(0xffffffffu, val, o);
@@ -46,17 +129,6 @@ __device__ __forceinline__ double cloth_sum(const Blocks& b, const double* part,
   double s = 0.0;
   for (int i = 0; i < nb; ++i) s += part[which * b.nblk + b0 + i];
   return s;
-}
-
-// shear records into the row blocks, then handles, external force, boundary
-// identity rows, Jacobi diagonal and the finite check of the system
-__global__ void __launch_bounds__(kBlock) k_finalize(View v, Records R, Blocks b, Solver so) {
-  const int blk = blockIdx.x;
-  const int c = b.blk_cloth[blk];
-  const int n = b.blk_node0[blk] + threadIdx.x;
-  bool bad = false;
-  if (threadIdx.x < b.blk_count[blk]) bad = !gather_shear_finalize<double>(v, R, n, so.dinv);
-  if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(&so.pc[c].status, 1);
 }
 
 // x = 0, r = b, p = z = Dinv r; partials |b|^2 (row 0), |r|^2 (row 1) and
@@ -260,14 +332,14 @@ void launch_bend_records(const View& v, const Records& R, cudaStream_t s, int t)
 void launch_face_records(const View& v, const Records& R, cudaStream_t s, int t) {
   k_face_rec<double><<<pblocks(v.ntot, t), t, 0, s>>>(v, R);
 }
-void launch_gather(const View& v, const Records& R, cudaStream_t s, int t) {
-  k_gather<double><<<pblocks(v.ntot, t), t, 0, s>>>(v, R);
+void launch_cross(const View& v, const Records& R, cudaStream_t s) {
+  k_cross<<<pblocks(v.ntot, kNodesPerBlock), 4 * kNodesPerBlock, 0, s>>>(v, R);
 }
 void launch_shear_records(const View& v, const Records& R, cudaStream_t s, int t) {
   k_shear_rec<double><<<pblocks(4LL * v.ntot, t), t, 0, s>>>(v, R);
 }
-void launch_finalize(const View& v, const Records& R, const Blocks& b, const Solver& so, cudaStream_t s) {
-  k_finalize<<<b.nblk, kBlock, 0, s>>>(v, R, b, so);
+void launch_rows(const View& v, const Records& R, const Solver& so, cudaStream_t s) {
+  k_rows<<<pblocks(v.ntot, kNodesPerBlock), 4 * kNodesPerBlock, 0, s>>>(v, R, so);
 }
 void launch_pcg_setup(const View& v, const Blocks& b, const Solver& so, cudaStream_t s) {
   k_pcg_setup<<<b.nblk, kBlock, 0, s>>>(v, b, so);

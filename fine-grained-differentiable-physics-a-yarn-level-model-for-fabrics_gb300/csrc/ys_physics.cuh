@@ -742,42 +742,47 @@ YS_HD void node_normal_dual(const View& v, int n, int W) {
   for (int i = 0; i < 3; ++i) stT(v.NRM, v.dNRM, i, nt, n, nn[i]);
 }
 
-// ConSlideFriction (src/PhysicsCloth.cpp:2579-2641) for interior node n from
-// its gathered no-slide force fe, dF_E/dE diagonals kee / dee and the crimp
-// compression sums cl / cle; returns the A and b contributions of the E rows
-// and stores COMP and SLIDE.
+// The compression of crossing n from the summed crimp forces (src/PhysicsCloth.cpp:97-110)
 template <class T>
-YS_HD void friction_node(const View& v, int n, const T* fe, const T* kee, const T* dee,
-                         const T* cl, const T* cle, T* aEE, T* bE) {
+YS_HD T crossing_comp(const View& v, int n, const T* cl) {
+  T c = 0.0;
+  for (int i = 0; i < 3; ++i) c += ldT<T>(v.NRM, v.dNRM, i, v.ntot, n) * cl[i];
+  c *= 0.5;
+  if (c < 0) c = 0.0;
+  return c;
+}
+
+// ConSlideFriction (src/PhysicsCloth.cpp:2579-2641) for interior node n and
+// yarn k from its gathered no-slide force FEns, its dF_E/dE diagonals EEp /
+// EEv, the crossing's compression and that one's derivative sums cle; returns
+// the A and b contributions of the E row and stores SLIDE.
+template <class T>
+YS_HD void friction_node(const View& v, int n, int k, const T& comp, const T& FEns, const T& EEp, const T& EEv,
+                         const T* cle, T& aEE, T& bE) {
   const int nt = v.ntot;
   const ClothParams& P = v.cp[v.node_cloth[n]];
-  T nrm[3];
-  for (int i = 0; i < 3; ++i) nrm[i] = ldT<T>(v.NRM, v.dNRM, i, nt, n);
-  T comp = 0.5 * dot3(nrm, cl);
-  if (comp < 0) comp = 0.0;
-  const T compEE[2] = {0.5 * dot3(nrm, cle), 0.5 * dot3(nrm, cle + 3)};
-  stT(v.COMP, v.dCOMP, 0, nt, n, comp);
+  T ce = 0.0;
+  for (int i = 0; i < 3; ++i) ce += ldT<T>(v.NRM, v.dNRM, i, nt, n) * cle[i];
+  ce *= 0.5;
   const T mu = cloth_mu<T>(v, v.node_cloth[n]);
   const double kf = P.kf, df = P.df, h = v.h, h2 = v.h * v.h;
-  const T lim = 1.0 * comp * mu;
-  for (int k = 0; k < 2; ++k) {
-    const T uvm = ldT<T>(v.UV, v.dUV, k, nt, n) - ldT<T>(v.UVB, v.dUVB, k, nt, n);
-    const T FEns = fe[k], EEp = kee[k], EEv = dee[k];
-    const T slide = 1.0 / (1.0 + exp(-(1e4 * (fabs(FEns) - lim))));
-    const T t = tanh(10 * uvm), tl = tanh(10 * (lim - FEns));
-    const T uvdot = ldT<T>(v.UVD, v.dUVD, k, nt, n);
-    const T force = (-0.5 * (kf * uvm - t * comp * mu) * tl + 0.5 * (kf * uvm + t * comp * mu)) - df * uvdot;
-    const T pos = (-0.5 * (kf - (1.0 - t * t) * mu * comp - t * mu * compEE[k])) * tl -
-                       (0.5 * (kf * uvm - t * mu * comp)) * (1.0 - tl * tl) * (EEp - mu * compEE[k]) -
-                       (0.5 * (kf + (1.0 - t * t) * mu * comp + t * mu * compEE[k]));
-    // tanh(10 * fric_lim - F) as written at src/PhysicsCloth.cpp:2630-2631
-    const T tq = tanh(10 * lim - FEns);
-    const T vel = (-0.5 * (kf * uvm - t * mu * comp)) * (1.0 - tq * tq) * EEv - df;
-    stT(v.SLIDE, v.dSLIDE, k, nt, n, slide);
-    aEE[k] = -h2 * pos - h * vel;
-    // D enters b without a graph in the reference (src/MatrixMp.cpp:40-99)
-    bE[k] = h * (force - (v.trunc ? detach(vel) : vel) * uvdot);
-  }
+  const T lim = comp * mu;
+  const T uvm = ldT<T>(v.UV, v.dUV, k, nt, n) - ldT<T>(v.UVB, v.dUVB, k, nt, n);
+  const T slide = 1.0 / (1.0 + exp(-(1e4 * (fabs(FEns) - lim))));
+  const T t = tanh(10 * uvm), tl = tanh(10 * (lim - FEns));
+  const T uvdot = ldT<T>(v.UVD, v.dUVD, k, nt, n);
+  const T ku = kf * uvm, tm = t * lim, mce = mu * ce;
+  const T lo = -0.5 * (ku - tm);
+  const T force = lo * tl + 0.5 * (ku + tm) - df * uvdot;
+  const T g = (1.0 - t * t) * lim + t * mce;
+  const T pos = -0.5 * (kf - g) * tl + lo * (1.0 - tl * tl) * (EEp - mce) - 0.5 * (kf + g);
+  // tanh(10 * fric_lim - F) as written at src/PhysicsCloth.cpp:2630-2631
+  const T tq = tanh(10 * lim - FEns);
+  const T vel = lo * (1.0 - tq * tq) * EEv - df;
+  stT(v.SLIDE, v.dSLIDE, k, nt, n, slide);
+  aEE = -h2 * pos - h * vel;
+  // D enters b without a graph in the reference (src/MatrixMp.cpp:40-99)
+  bE = h * (force - (v.trunc ? detach(vel) : vel) * uvdot);
 }
 
 // ------------------------------------------------------------ shear

@@ -23,7 +23,12 @@ __global__ void k_geom_dual(View v, const int* __restrict__ nodes, int count) {
   node_normal_dual<kTangents>(v, n, v.cp[v.node_cloth[n]].W);
 }
 
-__global__ void __launch_bounds__(kBlock) k_finalize_dual(View v, Records R) {
+__global__ void __launch_bounds__(kBlock) k_cross_dual(View v, Records R) {
+  const int n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (n < v.ntot) gather_elements<TD>(v, R, n);
+}
+
+__global__ void __launch_bounds__(kBlock) k_rows_dual(View v, Records R) {
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n < v.ntot) gather_shear_finalize<TD>(v, R, n, nullptr);
 }
@@ -68,9 +73,9 @@ void launch_assembly_dual(const View& v, const Records& R, const int* geom_nodes
   k_edge_rec<TD><<<nblocks_t(2 * v.ntot), kBlock, 0, s>>>(v, R);
   k_bend_rec<TD><<<nblocks_t(2 * v.ntot), kBlock, 0, s>>>(v, R);
   k_face_rec<TD><<<nblocks_t(v.ntot), kBlock, 0, s>>>(v, R);
-  k_gather<TD><<<nblocks_t(v.ntot), kBlock, 0, s>>>(v, R);
+  k_cross_dual<<<nblocks_t(v.ntot), kBlock, 0, s>>>(v, R);
   k_shear_rec<TD><<<nblocks_t(4 * v.ntot), kBlock, 0, s>>>(v, R);
-  k_finalize_dual<<<nblocks_t(v.ntot), kBlock, 0, s>>>(v, R);
+  k_rows_dual<<<nblocks_t(v.ntot), kBlock, 0, s>>>(v, R);
 }
 void launch_tangent_rhs(const View& v, const double* q, double* rt, int kact, cudaStream_t s) {
   k_tangent_rhs<<<nblocks_t(v.ntot), kBlock, 0, s>>>(v, q, rt, kact);
