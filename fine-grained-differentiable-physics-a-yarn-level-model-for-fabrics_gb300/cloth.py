@@ -487,8 +487,8 @@ class Adjoint:
     step) into dL/d(state before it), dL/d(material) and dL/d(external force),
     at a cost independent of how many inputs the gradient is taken for.
     mode: "exact" (the derivative of the discrete step) or "reference" (the
-    gradient the reference's loss.backward() takes). copies: workspace size
-    (128 copies = one pass per step; fewer copies, more passes)."""
+    gradient the reference's loss.backward() takes). copies: 1 to 128,
+    without effect (see ys_adjoint_create)."""
 
     def __init__(self, batch: ClothBatch, mode="exact", copies: int = 128):
         self.batch = batch

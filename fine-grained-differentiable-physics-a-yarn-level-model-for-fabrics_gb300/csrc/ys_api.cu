@@ -143,15 +143,6 @@ struct ys_batch {
   } tan;
   int nlines = 0;
   std::vector<double> line_R;  // yarn radius of each line's cloth
-  // construction parameters of every cloth, kept so that an adjoint can
-  // build copies of the batch (ys_adjoint_create); pointers of `d` are
-  // re-aimed at the vectors where a desc is rebuilt
-  struct DescStore {
-    ys_cloth_desc d;
-    std::vector<double> wr, wY, wB, fr, fY, fB;
-    std::vector<int32_t> handles;
-  };
-  std::vector<DescStore> descs;
   // whole-step CUDA graph (ys_use_graphs): assembly, a conditional while node
   // over the PCG iterations, update; rebuilt when its parameters change
   // `built`: the parameters below are current; each graph is captured on its
@@ -387,16 +378,6 @@ ys_status ys_batch_create(int32_t n_cloths, const ys_cloth_desc* descs, int32_t 
   b->device = device;
   b->stream = static_cast<cudaStream_t>(cuda_stream);
   b->ncloth = n_cloths;
-  for (int c = 0; c < n_cloths; ++c) {
-    const ys_cloth_desc& d = descs[c];
-    ys_batch::DescStore ds;
-    ds.d = d;
-    ds.wr.assign(d.warp_rho, d.warp_rho + d.length); ds.wY.assign(d.warp_Y, d.warp_Y + d.length);
-    ds.wB.assign(d.warp_B, d.warp_B + d.length); ds.fr.assign(d.weft_rho, d.weft_rho + d.width);
-    ds.fY.assign(d.weft_Y, d.weft_Y + d.width); ds.fB.assign(d.weft_B, d.weft_B + d.width);
-    if (d.n_handles > 0) ds.handles.assign(d.handles, d.handles + 2 * d.n_handles);
-    b->descs.push_back(std::move(ds));
-  }
   // ------------------------------------------------------------ topology
   std::vector<int> node_cloth, node_u, node_v;
   std::vector<uint8_t> flags;
@@ -1327,18 +1308,16 @@ ys_status ys_step_tangent_ext(ys_batch* b, double h, const double* ext_force, co
 // ------------------------------------------------------------ reverse mode
 struct ys_adjoint {
   ys_batch* prim = nullptr;  // the caller's batch (not owned)
-  ys_batch* cp = nullptr;    // `copies` copies of prim's cloths, copy-major (owned)
   int mode = YS_TANGENT_EXACT;
-  int copies = 0, passes = 0;
   std::vector<void*> allocs;
-  double *q = nullptr, *qbar = nullptr, *lambda = nullptr, *slide_bar = nullptr, *T = nullptr;
+  double *q = nullptr, *qbar = nullptr, *lambda = nullptr, *slide_bar = nullptr;
+  ys::AdjWork work{};
   double* gin[5] = {nullptr};
   double* gout[5] = {nullptr};
   double* gline[3] = {nullptr};
   double* gcloth[2] = {nullptr};
   double* gext = nullptr;      // [nt][5]
-  double* line_a = nullptr;    // pi R^2 per primal line
-  int* line_kind = nullptr;    // orientation * 3 + position mod 3
+  double* line_a = nullptr;    // pi R^2 per line
   int* line_cloth = nullptr;
   template <class T_>
   ys_status alloc(T_** p, size_t count) {
@@ -1352,21 +1331,13 @@ struct ys_adjoint {
   ~ys_adjoint() {
     if (prim) cudaSetDevice(prim->device);
     for (void* m : allocs) cudaFree(m);
-    if (cp) ys_batch_destroy(cp);
   }
 };
 
 namespace {
 
 constexpr int kStateComps[5] = {3, 3, 2, 2, 2};
-
-__global__ void k_adj_copy_wind(const ys::ClothParams* __restrict__ src, ys::ClothParams* dst, int ncl, int copies) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= ncl * copies) return;
-  const ys::ClothParams& a = src[t % ncl];
-  ys::ClothParams& d = dst[t];
-  for (int k = 0; k < 3; ++k) d.wind[k] = a.wind[k];
-}
+constexpr int kMaxCopies = 128;  // ys_adjoint_create's bound
 
 }  // namespace
 
@@ -1377,47 +1348,32 @@ ys_status ys_adjoint_create(ys_batch* b, int32_t mode, int32_t copies, ys_adjoin
   *out = nullptr;
   if (mode != YS_TANGENT_EXACT && mode != YS_TANGENT_REFERENCE)
     return fail(YS_ERR_ARG, "adjoint mode must be YS_TANGENT_EXACT or YS_TANGENT_REFERENCE");
-  const int ndir = ys::adjoint_direction_count();
-  const int maxc = (ndir + KT - 1) / KT;
-  if (copies < 1 || copies > maxc) return fail(YS_ERR_ARG, "copies must be in [1, 128]");
+  if (copies < 1 || copies > kMaxCopies) return fail(YS_ERR_ARG, "copies must be in [1, 128]");
   YS_CUDA(cudaSetDevice(b->device));
   ys_adjoint* a = new ys_adjoint();
   a->prim = b;
   a->mode = mode;
-  a->copies = copies;
-  a->passes = (maxc + copies - 1) / copies;
-  // the copies' batch: the same cloths, `copies` times, on b's stream
-  std::vector<ys_cloth_desc> d;
-  d.reserve((size_t)copies * b->ncloth);
-  for (int c = 0; c < copies; ++c)
-    for (const ys_batch::DescStore& ds : b->descs) {
-      ys_cloth_desc e = ds.d;
-      e.warp_rho = ds.wr.data(); e.warp_Y = ds.wY.data(); e.warp_B = ds.wB.data();
-      e.weft_rho = ds.fr.data(); e.weft_Y = ds.fY.data(); e.weft_B = ds.fB.data();
-      e.handles = ds.handles.empty() ? nullptr : ds.handles.data();
-      d.push_back(e);
-    }
-  ys_status st = ys_batch_create((int32_t)d.size(), d.data(), b->device, b->stream, &a->cp);
-  if (st == YS_OK) st = ys_tangent_enable(a->cp, mode);
-  const int64_t nt = b->ntot, ntc = a->cp ? a->cp->ntot : 0;
+  const int64_t nt = b->ntot;
+  ys_status st = YS_OK;
   auto A = [&](auto** p, size_t cnt) { if (st == YS_OK) st = a->alloc(p, cnt); };
   A(&a->q, 5 * nt); A(&a->qbar, 5 * nt); A(&a->lambda, 5 * nt); A(&a->slide_bar, 2 * nt);
-  A(&a->T, (size_t)KT * ntc);
+  const ys::AdjSizes z = ys::adjoint_sizes();
+  A(&a->work.edge, z.edge * nt); A(&a->work.bend, z.bend * nt); A(&a->work.face, z.face * nt);
+  A(&a->work.shear, z.shear * nt); A(&a->work.cross, z.cross * nt); A(&a->work.normal, z.normal * nt);
   for (int i = 0; i < 5; ++i) { A(&a->gin[i], kStateComps[i] * nt); A(&a->gout[i], kStateComps[i] * nt); }
   for (int i = 0; i < 3; ++i) A(&a->gline[i], b->nlines);
   for (int i = 0; i < 2; ++i) A(&a->gcloth[i], b->ncloth);
   A(&a->gext, 5 * nt);
-  A(&a->line_a, b->nlines); A(&a->line_kind, b->nlines); A(&a->line_cloth, b->nlines);
+  A(&a->line_a, b->nlines); A(&a->line_cloth, b->nlines);
   if (st != YS_OK) { delete a; return st; }
   std::vector<double> la;
-  std::vector<int> lk, lc;
+  std::vector<int> lc;
   for (int c = 0; c < b->ncloth; ++c) {
     const ys::ClothParams& P = b->cp[c];
-    for (int v = 0; v < P.H; ++v) { lk.push_back(0 * 3 + v % 3); lc.push_back(c); la.push_back(ys::kPi * P.R * P.R); }
-    for (int u = 0; u < P.W; ++u) { lk.push_back(1 * 3 + u % 3); lc.push_back(c); la.push_back(ys::kPi * P.R * P.R); }
+    la.insert(la.end(), P.H + P.W, ys::kPi * P.R * P.R);
+    lc.insert(lc.end(), P.H + P.W, c);
   }
   if (cudaMemcpy(a->line_a, la.data(), sizeof(double) * la.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-      cudaMemcpy(a->line_kind, lk.data(), sizeof(int) * lk.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaMemcpy(a->line_cloth, lc.data(), sizeof(int) * lc.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
     delete a;
     return fail(YS_ERR_CUDA, "cudaMemcpy of the adjoint's line tables failed");
@@ -1433,10 +1389,9 @@ ys_status ys_adjoint_step(ys_adjoint* a, double h, const double* ext_force, cons
                           const ys_solve_opts* opts, ys_cloth_stats* stats) {
   if (!a || !(h > 0)) return fail(YS_ERR_ARG, "bad argument");
   ys_batch* b = a->prim;
-  ys_batch* c = a->cp;
   YS_CUDA(cudaSetDevice(b->device));
   cudaStream_t s = b->stream;
-  const int64_t nt = b->ntot, ntc = c->ntot;
+  const int64_t nt = b->ntot;
   // 1. the forward step's system and solution at the current state
   ys_status st = ys_assemble(b, h, ext_force, flags);
   if (st != YS_OK) return st;
@@ -1470,55 +1425,21 @@ ys_status ys_adjoint_step(ys_adjoint* a, double h, const double* ext_force, cons
     YS_CUDA(cudaMemcpyAsync(a->lambda, b->so.x, sizeof(double) * 5 * nt, cudaMemcpyDeviceToDevice, s));
     YS_CUDA(cudaMemcpyAsync(b->so.x, a->q, sizeof(double) * 5 * nt, cudaMemcpyDeviceToDevice, s));
   }
-  // 4. the copies take the state, wind, step size and external force
+  // 4. the gradient of lambda . (b - A q) + slide_bar . slide, element by element
+  const ys::AdjParamOut gp{{a->gline[0], a->gline[1], a->gline[2]}, {a->gcloth[0], a->gcloth[1]}};
   {
-    ys::View& vc = c->v;
-    const ys::View& vb = b->v;
-    const int cps = a->copies;
-    b->run(YS_PROF_MISC, 7, [&] {
-      ys::launch_adj_broadcast(vb.X, vc.X, (int)nt, 3, cps, s);
-      ys::launch_adj_broadcast(vb.V, vc.V, (int)nt, 3, cps, s);
-      ys::launch_adj_broadcast(vb.XF, vc.XF, (int)nt, 3, cps, s);
-      ys::launch_adj_broadcast(vb.UV, vc.UV, (int)nt, 2, cps, s);
-      ys::launch_adj_broadcast(vb.UVD, vc.UVD, (int)nt, 2, cps, s);
-      ys::launch_adj_broadcast(vb.UVB, vc.UVB, (int)nt, 2, cps, s);
-      k_adj_copy_wind<<<(b->ncloth * cps + 127) / 128, 128, 0, s>>>(vb.cp, const_cast<ys::ClothParams*>(vc.cp),
-                                                                     b->ncloth, cps);
-    });
-    vc.h = h;
-    vc.ext = nullptr;
-    if (ext_force) {
-      b->run(YS_PROF_MISC, 1, [&] { ys::launch_adj_broadcast(b->ext, c->ext, (int)nt, 5, cps, s); });
-      vc.ext = c->ext;
-    }
-    YS_CUDA(cudaGetLastError());
-  }
-  // 5. the residual's vector-Jacobian product, pass by pass
-  for (int i = 0; i < 3; ++i) YS_CUDA(cudaMemsetAsync(a->gline[i], 0, sizeof(double) * b->nlines, s));
-  for (int i = 0; i < 2; ++i) YS_CUDA(cudaMemsetAsync(a->gcloth[i], 0, sizeof(double) * b->ncloth, s));
-  ys::AdjParamOut gp{{a->gline[0], a->gline[1], a->gline[2]}, {a->gcloth[0], a->gcloth[1]}};
-  ys_batch::Tan& t = c->tan;
-  ys::AdjSeeds sd{t.dX, t.dV, t.dUV, t.dUVD, t.dUVB, t.drho, t.dks, t.dkb, t.dS, t.dmu};
-  ys::View dv = dual_view(c);
-  ys::Records dr = c->rec;
-  dr.dedge = t.dedge; dr.dbend = t.dbend; dr.dface = t.dface; dr.dshear = t.dshear;
-  for (int p = 0; p < a->passes; ++p) {
-    const int base = p * a->copies;
-    b->run(YS_PROF_MISC, 2, [&] {
-      ys::launch_adj_seed(c->v, (int)nt, b->nlines, b->ncloth, base, a->line_a, a->line_kind, sd, s);
-    });
-    b->run(YS_PROF_MISC, 7, [&] { ys::launch_assembly_dual(dv, dr, c->anchors, c->geom_n, s); });
-    b->run(YS_PROF_MISC, 2, [&] {
-      ys::launch_adj_broadcast(a->q, t.qsave, (int)nt, 5, a->copies, s);
-      ys::launch_tangent_rhs(dv, t.qsave, t.rt, KT, s);
-    });
-    b->run(YS_PROF_MISC, 3, [&] {
-      ys::launch_adj_contract(dv, (int)nt, a->lambda, a->slide_bar, t.rt, a->T, s);
-      ys::launch_adj_gather(b->v, base, a->copies, a->T, ntc, a->line_cloth, a->line_kind, io, gp, s);
+    ys::View va = b->v;
+    va.trunc = a->mode == YS_TANGENT_REFERENCE ? 1 : 0;
+    ys::AdjWork w = a->work;
+    w.lam = a->lambda;
+    w.q = va.trunc ? nullptr : a->q;
+    w.slide_bar = a->slide_bar;
+    b->run(YS_PROF_MISC, 8, [&] {
+      ys::launch_adj_vjp(va, b->rec, w, b->anchors + b->geom_off, b->geom_n, io, a->line_a, a->line_cloth, gp, s);
     });
     YS_CUDA(cudaGetLastError());
   }
-  // 6. outputs
+  // 5. outputs
   for (int i = 0; i < 5; ++i)
     if (gout && gout[i]) {
       st = download_aos(b, a->gout[i], gout[i], kStateComps[i], flags);

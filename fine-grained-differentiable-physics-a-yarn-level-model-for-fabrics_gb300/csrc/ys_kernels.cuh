@@ -115,27 +115,32 @@ struct AdjIO {
   const double* gin[5];  // dL/d(state after the step)
   double* gout[5];       // dL/d(state before the step)
 };
-// the forward-mode seeds of the copies' batch (its tangent arrays)
-struct AdjSeeds {
-  double *dX, *dV, *dUV, *dUVD, *dUVB;
-  double *drho, *dks, *dkb, *dS, *dmu;
-};
-// material adjoints, accumulated: line[p][l] for p = rho, Y, B of primal
-// line l; cloth[p][c] for p = S, mu
+// material adjoints: line[p][l] for p = rho, Y, B of line l; cloth[p][c] for
+// p = S, mu
 struct AdjParamOut {
   double* line[3];
   double* cloth[2];
 };
-int adjoint_direction_count();
+// scratch of the reverse step, in units of ntot doubles
+struct AdjSizes {
+  int64_t edge, bend, face, shear, cross, normal;
+};
+constexpr int kAdjCrossFields = 23;
+AdjSizes adjoint_sizes();
+struct AdjWork {
+  const double* lam;        // [5][ntot]
+  const double* q;          // [5][ntot], null in the reference mode
+  const double* slide_bar;  // [2][ntot]
+  double *edge, *bend, *face, *shear, *cross, *normal;
+};
 void launch_adj_update(const View& v, const AdjIO& io, const double* q, double* qbar, double* slide_bar,
                        cudaStream_t s);
-void launch_adj_broadcast(const double* src, double* dst, int nt, int ncomp, int copies, cudaStream_t s);
-void launch_adj_seed(const View& vc, int nt, int nl, int ncl, int base, const double* line_a, const int* line_kind,
-                     const AdjSeeds& sd, cudaStream_t s);
-void launch_adj_contract(const View& vc, int nt, const double* lambda, const double* slide_bar, const double* rt,
-                         double* T, cudaStream_t s);
-void launch_adj_gather(const View& v, int base, int copies, const double* T, int64_t ntc, const int* line_cloth,
-                       const int* line_kind, const AdjIO& io, const AdjParamOut& gp, cudaStream_t s);
+// adds d(lambda . (b - A q) + slide_bar . slide) to io.gout and writes gp, from
+// the records R and the normals and compressions of the assembled step (v.trunc
+// selects the reference mode); returns the number of kernels
+int launch_adj_vjp(const View& v, const Records& R, const AdjWork& w, const int* interior, int n_interior,
+                   const AdjIO& io, const double* line_a, const int* line_cloth, const AdjParamOut& gp,
+                   cudaStream_t s);
 void launch_adj_ext(const View& v, const double* lambda, double* gext, cudaStream_t s);
 
 }  // namespace ys

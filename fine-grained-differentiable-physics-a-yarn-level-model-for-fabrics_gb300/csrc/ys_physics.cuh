@@ -186,27 +186,48 @@ struct EdgeOut {
 // the squared r6 of "- rho / 6 r" (2154-2234), ParaColli_D proportional to the
 // overlap itself. Term by term as the reference writes them, an edge took
 // 1,690 FP64 operations; this form takes about 400.
-template <class T, class Put>
-YS_HD void edge_terms(const View& v, int n0, int n1, int k, Put&& put) {
+// One edge's inputs: dx = x1 - x0, gx = G . (x0 + x1), the velocities a and e
+// of its ends, du, and the yarn's density and stretch stiffness.
+template <class T>
+struct EdgeIn {
+  T dx[3], gx, a[2][3], du, e[2], rho, ks;
+  bool in[2];  // interior ends
+  bool over;   // the yarn changes side between them
+};
+template <class T>
+YS_HD EdgeIn<T> edge_load(const View& v, int n0, int n1, int k) {
   const int nt = v.ntot;
   const ClothParams& P = v.cp[v.node_cloth[n0]];
+  EdgeIn<T> s;
   const uint8_t f0 = v.flags[n0], f1 = v.flags[n1];
-  const bool in[2] = {(f0 & YS_INTERIOR) != 0, (f1 & YS_INTERIOR) != 0};
-  const bool both = in[0] && in[1];
+  s.in[0] = (f0 & YS_INTERIOR) != 0;
+  s.in[1] = (f1 & YS_INTERIOR) != 0;
+  s.over = ((f0 & YS_FLIP) != 0) != ((f1 & YS_FLIP) != 0);
   const int line = (k == 0) ? P.warp_line_off + v.node_v[n0] : P.weft_line_off + v.node_u[n0];
-  const T rho = ldpT<T>(v.line_rho, v.dline_rho, line, v.nlines), ks = ldpT<T>(v.line_ks, v.dline_ks, line, v.nlines);
-  const double h = v.h, mh2 = -(v.h * v.h);
-  T a[2][3], e[2], dx[3], gx = 0.0;
+  s.rho = ldpT<T>(v.line_rho, v.dline_rho, line, v.nlines);
+  s.ks = ldpT<T>(v.line_ks, v.dline_ks, line, v.nlines);
+  s.gx = 0.0;
   for (int i = 0; i < 3; ++i) {
     const T x0 = ldT<T>(v.X, v.dX, i, nt, n0), x1 = ldT<T>(v.X, v.dX, i, nt, n1);
-    dx[i] = x1 - x0;
-    gx += P.G[i] * (x0 + x1);
-    a[0][i] = ldT<T>(v.V, v.dV, i, nt, n0);
-    a[1][i] = ldT<T>(v.V, v.dV, i, nt, n1);
+    s.dx[i] = x1 - x0;
+    s.gx += P.G[i] * (x0 + x1);
+    s.a[0][i] = ldT<T>(v.V, v.dV, i, nt, n0);
+    s.a[1][i] = ldT<T>(v.V, v.dV, i, nt, n1);
   }
-  const T du = ldT<T>(v.UV, v.dUV, k, nt, n1) - ldT<T>(v.UV, v.dUV, k, nt, n0);
-  e[0] = ldT<T>(v.UVD, v.dUVD, k, nt, n0);
-  e[1] = ldT<T>(v.UVD, v.dUVD, k, nt, n1);
+  s.du = ldT<T>(v.UV, v.dUV, k, nt, n1) - ldT<T>(v.UV, v.dUV, k, nt, n0);
+  s.e[0] = ldT<T>(v.UVD, v.dUVD, k, nt, n0);
+  s.e[1] = ldT<T>(v.UVD, v.dUVD, k, nt, n1);
+  return s;
+}
+template <class T, class Put>
+YS_HD void edge_terms(const EdgeIn<T>& s, const ClothParams& P, int k, double h, bool trunc, Put&& put) {
+  const bool* in = s.in;
+  const bool both = in[0] && in[1];
+  const T &rho = s.rho, &ks = s.ks, &du = s.du, &gx = s.gx;
+  const T(&dx)[3] = s.dx;
+  const T(&a)[2][3] = s.a;
+  const T(&e)[2] = s.e;
+  const double mh2 = -(h * h);
   const T idu = 1.0 / du, aidu = fabs(idu);
   const T il = rsqrt_(dot3(dx, dx));
   T w[3], d[3];
@@ -245,7 +266,7 @@ YS_HD void edge_terms(const View& v, int n0, int n1, int k, Put&& put) {
     re[b] = r6 * (2.0 * wD * mu[b] - dlww * mu[b] - Dm[b]);
   }
   {
-    T rl = ((((f0 & YS_FLIP) != 0) != ((f1 & YS_FLIP) != 0)) ? 4.0 * P.R : 2.0 * P.R) - du;
+    T rl = (s.over ? 4.0 * P.R : 2.0 * P.R) - du;
     if (rl < 0) rl = 0.0;
     const T crowd = P.kc * P.L * rl;
     const T Saa = dot3(a[0], m[0]) + dot3(a[1], m[1]);
@@ -298,7 +319,7 @@ YS_HD void edge_terms(const View& v, int n0, int n1, int k, Put&& put) {
   // M and D enter b without a graph in the reference (src/MatrixMp.cpp:40-99),
   // so the reference-mode tangents hold their factors constant.
   {
-    auto cst = [&](const T& x) { return v.trunc ? detach(x) : x; };
+    auto cst = [&](const T& x) { return trunc ? detach(x) : x; };
     const T cq = cst(q), ce0 = cst(e[0]), ce1 = cst(e[1]), c2 = cst(-2.0 * h * r6);
     const T cm0 = 2.0 * ce0 + ce1, cm1 = ce0 + 2.0 * ce1, cdl = ce1 - ce0;
     T ca[2][3], cw[3], cD[3];
@@ -372,6 +393,10 @@ YS_HD void edge_terms(const View& v, int n0, int n1, int k, Put&& put) {
     }
   }
 }
+template <class T, class Put>
+YS_HD void edge_terms(const View& v, int n0, int n1, int k, Put&& put) {
+  edge_terms<T>(edge_load<T>(v, n0, n1, k), v.cp[v.node_cloth[n0]], k, v.h, v.trunc != 0, put);
+}
 template <class T>
 YS_HD void edge_element(const View& v, int n0, int n1, int k, EdgeOut<T>& o) {
   edge_terms<T>(v, n0, n1, k, [&](int f, const T& x) { o.f[f] = x; });
@@ -395,8 +420,8 @@ struct BendGeom {
   bool active;
 };
 template <class T>
-YS_HD void bend_geom(const T* x2, const T* x0, const T* x1, BendGeom<T>& g) {
-  for (int i = 0; i < 3; ++i) { g.d1[i] = x1[i] - x0[i]; g.d2[i] = x2[i] - x0[i]; }
+YS_HD void bend_geom(const T* to1, const T* to2, BendGeom<T>& g) {  // x1 - x0, x2 - x0
+  for (int i = 0; i < 3; ++i) { g.d1[i] = to1[i]; g.d2[i] = to2[i]; }
   const T l1 = norm3(g.d1), l2 = norm3(g.d2);
   g.il1 = 1.0 / l1;
   g.il2 = 1.0 / l2;
@@ -446,66 +471,78 @@ YS_HD void bend_diag(const T& k, const T& th, const T& c, const T& kA, const T* 
   }
 }
 
-// Bending_F / Bending_D on the real nodes (src/PhysicsCloth.cpp:579-822) and
-// Crimp_Bending_F / Crimp_Bending_D on the crimp-offset centre lines
-// (src/PhysicsCloth.cpp:824-987) for the segment n2 - n0 - n1 along yarn
-// direction k; put(field, value) receives each field of the record once.
+// Bending_F / Bending_D on the real nodes (src/PhysicsCloth.cpp:579-822) from
+// the segment's arms x1 - x0 and x2 - x0, its Eulerian length and bending
+// stiffness; put(field, value) receives its fields of the record once each.
+template <class T, class Put>
+YS_HD void bend_real(const T* to1, const T* to2, const T& du, const T& kb, double h, Put&& put) {
+  BendGeom<T> g;
+  bend_geom(to1, to2, g);
+  const T idu = 1.0 / du;
+  const T kt = kb * g.th * idu;
+  put(kB_idu, idu);
+  put(kB_Fu2, -kt * idu);
+  put(kB_E1E1, (-2.0 * kt * g.th) * (idu * idu));
+  const T on = g.active ? kb : T(0.0);
+  const T f = -2.0 * (on * g.th) * (idu * g.is), f1 = f * g.il1, f2 = f * g.il2;
+  for (int i = 0; i < 3; ++i) { put(kB_F1 + i, f1 * g.a[i]); put(kB_F2 + i, f2 * g.b[i]); }
+  const T K = (-2.0 * h * h) * on * (idu * g.is);  // 2 kb / (du sin), scaled by -h^2
+  const T k11 = K * (g.il1 * g.il1), k22 = K * (g.il2 * g.il2), k12 = -K * (g.il1 * g.il2);
+  const T tc = g.th * (g.c * (g.is * g.is)) - g.is;
+  bend_diag(k11, g.th, g.c, k11 * tc, g.a, g.d1, kB_L11, put);
+  bend_diag(k22, g.th, g.c, k22 * tc, g.b, g.d2, kB_L22, put);
+  // L12 = k12 (th P1 P2 - tc a b^T), P1 P2 = I - d1 d1^T - a d2^T
+  const T kt12 = k12 * g.th, kab = -k12 * tc;
+  for (int j = 0; j < 3; ++j) {
+    const T pa = kab * g.b[j] - kt12 * g.d2[j], pd = -kt12 * g.d1[j];
+    for (int i = 0; i < 3; ++i) {
+      const T x = pa * g.a[i] + pd * g.d1[i];
+      put(kB_L12 + 3 * i + j, i == j ? x + kt12 : x);
+    }
+  }
+}
+// Crimp_Bending_F / Crimp_Bending_D (src/PhysicsCloth.cpp:824-987) from the
+// arms of the crimp-offset centre line; icu: reciprocal of the Eulerian
+// length of the build, which crimp segments keep (src/Cloth.cpp:107)
+template <class T, class Put>
+YS_HD void bend_crimp(const T* to1, const T* to2, double icu, const T& kb, Put&& put) {
+  BendGeom<T> g;
+  bend_geom(to1, to2, g);
+  const T f = g.active ? T((-2.0 * icu) * (kb * g.th) * g.is) : T(0.0), f1 = f * g.il1, f2 = f * g.il2;
+  put(kB_cidu, T(icu));
+  for (int i = 0; i < 3; ++i) { put(kB_cF1 + i, f1 * g.a[i]); put(kB_cF2 + i, f2 * g.b[i]); }
+}
+// the crimp-offset position of node n: x - R n along the warp, x + R n along the weft
+template <class T>
+YS_HD void crimp_point(const View& v, int n, int k, T* x) {
+  const double R = v.cp[v.node_cloth[n]].R, sg = k == 0 ? -R : R;
+  const bool in = (v.flags[n] & YS_INTERIOR) != 0;
+  for (int i = 0; i < 3; ++i) {
+    x[i] = ldT<T>(v.X, v.dX, i, v.ntot, n);
+    if (in) x[i] += sg * ldT<T>(v.NRM, v.dNRM, i, v.ntot, n);
+  }
+}
+YS_HD double crimp_icu(const View& v, int n2, int n1, int k) {
+  return 1.0 / (ld(v.UV0, k, v.ntot, n1) - ld(v.UV0, k, v.ntot, n2));
+}
+// both for the segment n2 - n0 - n1 along yarn direction k
 template <class T, class Put>
 YS_HD void bend_terms(const View& v, int n2, int n0, int n1, int k, int line, Put&& put) {
   const int nt = v.ntot;
   const T kb = ldpT<T>(v.line_kb, v.dline_kb, line, v.nlines);
-  {
-    T x2[3], x0[3], x1[3];
-    for (int i = 0; i < 3; ++i) {
-      x2[i] = ldT<T>(v.X, v.dX, i, nt, n2);
-      x0[i] = ldT<T>(v.X, v.dX, i, nt, n0);
-      x1[i] = ldT<T>(v.X, v.dX, i, nt, n1);
-    }
-    const T idu = 1.0 / (ldT<T>(v.UV, v.dUV, k, nt, n1) - ldT<T>(v.UV, v.dUV, k, nt, n2));
-    BendGeom<T> g;
-    bend_geom(x2, x0, x1, g);
-    const T kt = kb * g.th * idu;
-    put(kB_idu, idu);
-    put(kB_Fu2, -kt * idu);
-    put(kB_E1E1, (-2.0 * kt * g.th) * (idu * idu));
-    const T on = g.active ? kb : T(0.0);
-    const T f = -2.0 * (on * g.th) * (idu * g.is), f1 = f * g.il1, f2 = f * g.il2;
-    for (int i = 0; i < 3; ++i) { put(kB_F1 + i, f1 * g.a[i]); put(kB_F2 + i, f2 * g.b[i]); }
-    const T K = (-2.0 * v.h * v.h) * on * (idu * g.is);  // 2 kb / (du sin), scaled by -h^2
-    const T k11 = K * (g.il1 * g.il1), k22 = K * (g.il2 * g.il2), k12 = -K * (g.il1 * g.il2);
-    const T tc = g.th * (g.c * (g.is * g.is)) - g.is;
-    bend_diag(k11, g.th, g.c, k11 * tc, g.a, g.d1, kB_L11, put);
-    bend_diag(k22, g.th, g.c, k22 * tc, g.b, g.d2, kB_L22, put);
-    // L12 = k12 (th P1 P2 - tc a b^T), P1 P2 = I - d1 d1^T - a d2^T
-    const T kt12 = k12 * g.th, kab = -k12 * tc;
-    for (int j = 0; j < 3; ++j) {
-      const T pa = kab * g.b[j] - kt12 * g.d2[j], pd = -kt12 * g.d1[j];
-      for (int i = 0; i < 3; ++i) {
-        const T x = pa * g.a[i] + pd * g.d1[i];
-        put(kB_L12 + 3 * i + j, i == j ? x + kt12 : x);
-      }
-    }
+  T to1[3], to2[3];
+  for (int i = 0; i < 3; ++i) {
+    const T x0 = ldT<T>(v.X, v.dX, i, nt, n0);
+    to1[i] = ldT<T>(v.X, v.dX, i, nt, n1) - x0;
+    to2[i] = ldT<T>(v.X, v.dX, i, nt, n2) - x0;
   }
-  {
-    const double R = v.cp[v.node_cloth[n0]].R;
-    const double sg = k == 0 ? -R : R;  // warp: x - R n, weft: x + R n
-    T x[3][3];
-    const int nd[3] = {n2, n0, n1};
-    for (int m = 0; m < 3; ++m) {
-      const bool in = (v.flags[nd[m]] & YS_INTERIOR) != 0;
-      for (int i = 0; i < 3; ++i) {
-        x[m][i] = ldT<T>(v.X, v.dX, i, nt, nd[m]);
-        if (in) x[m][i] += sg * ldT<T>(v.NRM, v.dNRM, i, nt, nd[m]);
-      }
-    }
-    BendGeom<T> g;
-    bend_geom(x[0], x[1], x[2], g);
-    // crimp segments keep the EPos of the build (src/Cloth.cpp:107)
-    const double cidu = 1.0 / (ld(v.UV0, k, nt, n1) - ld(v.UV0, k, nt, n2));
-    const T f = g.active ? T((-2.0 * cidu) * (kb * g.th) * g.is) : T(0.0), f1 = f * g.il1, f2 = f * g.il2;
-    put(kB_cidu, T(cidu));
-    for (int i = 0; i < 3; ++i) { put(kB_cF1 + i, f1 * g.a[i]); put(kB_cF2 + i, f2 * g.b[i]); }
-  }
+  bend_real(to1, to2, ldT<T>(v.UV, v.dUV, k, nt, n1) - ldT<T>(v.UV, v.dUV, k, nt, n2), kb, v.h, put);
+  T x0[3];
+  crimp_point(v, n0, k, x0);
+  crimp_point(v, n1, k, to1);
+  crimp_point(v, n2, k, to2);
+  for (int i = 0; i < 3; ++i) { to1[i] -= x0[i]; to2[i] -= x0[i]; }
+  bend_crimp(to1, to2, crimp_icu(v, n2, n1, k), kb, put);
 }
 // the record in the bend buffer at slot k * ntot + n0
 template <class T>
@@ -514,30 +551,42 @@ YS_HD void bend_element(const View& v, double* buf, double* dbuf, int n2, int n0
 }
 
 // ------------------------------------------------------------ wind (faces)
-// Wind_F (src/PhysicsCloth.cpp:3091-3107), face geometry src/ClothUnit.h:268-273;
-// returns wind_force / 3, the share of each of the face's three nodes.
+// Wind_F (src/PhysicsCloth.cpp:3091-3107), face geometry src/ClothUnit.h:268-273,
+// from the face's edges e1, e2 and the sum of its nodes' velocities; f3 =
+// wind_force / 3, the share of each of its three nodes. area n = cr / 2 and
+// area tang = |cr| rel / 2 - vn cr / 2, so one division serves what nine
+// did (FP64 divisions bound the kernel: 59 us for 203 on 256 cloths of 17 x 17).
+template <class T>
+YS_HD void wind_terms(const ClothParams& P, const T* e1, const T* e2, const T* vs, T* f3) {
+  T cr[3], rel[3];
+  cross3(e1, e2, cr);
+  const T cc = dot3(cr, cr);
+  const T nc = sqrt(cc), inc = cc == 0.0 ? T(0.0) : 1.0 / nc;  // |cr|, 1 / |cr| (0 for a flat face)
+  for (int i = 0; i < 3; ++i) rel[i] = P.wind[i] - vs[i] * (1.0 / 3.0);
+  const T vn = dot3(cr, rel) * inc;
+  const T k = (1.0 / 6.0) * vn * (P.wind_rho * fabs(vn) - P.wind_drag);
+  const T kd = (P.wind_drag / 6.0) * nc;
+  for (int i = 0; i < 3; ++i) f3[i] = k * cr[i] + kd * rel[i];
+}
 template <class T>
 YS_HD void wind_face(const View& v, const ClothParams& P, int n1, int n2, int n3, T* f3) {
   const int nt = v.ntot;
-  T e1[3], e2[3], cr[3], n[3], fv[3], rel[3];
+  T e1[3], e2[3], vs[3];
   for (int i = 0; i < 3; ++i) {
     const T xa = ldT<T>(v.X, v.dX, i, nt, n1);
     e1[i] = ldT<T>(v.X, v.dX, i, nt, n2) - xa;
     e2[i] = ldT<T>(v.X, v.dX, i, nt, n3) - xa;
+    vs[i] = ldT<T>(v.V, v.dV, i, nt, n1) + ldT<T>(v.V, v.dV, i, nt, n2) + ldT<T>(v.V, v.dV, i, nt, n3);
   }
-  cross3(e1, e2, cr);
-  const T nc = norm3(cr), area = 0.5 * nc;
-  for (int i = 0; i < 3; ++i) n[i] = (nc == 0.0) ? cr[i] : cr[i] / nc;
-  for (int i = 0; i < 3; ++i) {
-    fv[i] = (ldT<T>(v.V, v.dV, i, nt, n1) + ldT<T>(v.V, v.dV, i, nt, n2) + ldT<T>(v.V, v.dV, i, nt, n3)) / 3.0;
-    rel[i] = P.wind[i] - fv[i];
-  }
-  const T vn = dot3(n, rel);
-  for (int i = 0; i < 3; ++i) {
-    const T tang = rel[i] - vn * n[i];
-    const T f = P.wind_rho * area * fabs(vn) * vn * n[i] + P.wind_drag * area * tang;
-    f3[i] = f / 3.0;
-  }
+  wind_terms(P, e1, e2, vs, f3);
+}
+// the nodes of face `which` (0, 1) of the cell with top-left node tl
+YS_HD void cell_face(const View& v, int tl, int which, int n[3]) {
+  const int W = v.cp[v.node_cloth[tl]].W, tr = tl + 1, bl = tl + W, br = tl + W + 1;
+  const bool even = ((v.node_u[tl] + v.node_v[tl]) & 1) == 0;
+  n[0] = which == 0 || even ? tl : tr;
+  n[1] = which == 0 ? tr : br;
+  n[2] = which == 0 && even ? br : bl;
 }
 
 // cell with top-left node tl: faces (src/Cloth.cpp:271-287) written to the
@@ -545,15 +594,12 @@ YS_HD void wind_face(const View& v, const ClothParams& P, int n1, int n2, int n3
 template <class T>
 YS_HD void cell_faces(const View& v, double* buf, double* dbuf, int tl) {
   const ClothParams& P = v.cp[v.node_cloth[tl]];
-  const int tr = tl + 1, bl = tl + P.W, br = tl + P.W + 1;
   T fa[3], fb[3];
-  if (((v.node_u[tl] + v.node_v[tl]) & 1) == 0) {
-    wind_face(v, P, tl, tr, br, fa);
-    wind_face(v, P, tl, br, bl, fb);
-  } else {
-    wind_face(v, P, tl, tr, bl, fa);
-    wind_face(v, P, tr, br, bl, fb);
-  }
+  int n[3];
+  cell_face(v, tl, 0, n);
+  wind_face(v, P, n[0], n[1], n[2], fa);
+  cell_face(v, tl, 1, n);
+  wind_face(v, P, n[0], n[1], n[2], fb);
   for (int i = 0; i < 3; ++i) {
     stT(buf, dbuf, i, v.ntot, tl, fa[i]);
     stT(buf, dbuf, 3 + i, v.ntot, tl, fb[i]);
@@ -757,20 +803,13 @@ YS_HD T crossing_comp(const View& v, int n, const T* cl) {
 // EEv, the crossing's compression and that one's derivative sums cle; returns
 // the A and b contributions of the E row and stores SLIDE.
 template <class T>
-YS_HD void friction_node(const View& v, int n, int k, const T& comp, const T& FEns, const T& EEp, const T& EEv,
-                         const T* cle, T& aEE, T& bE) {
-  const int nt = v.ntot;
-  const ClothParams& P = v.cp[v.node_cloth[n]];
-  T ce = 0.0;
-  for (int i = 0; i < 3; ++i) ce += ldT<T>(v.NRM, v.dNRM, i, nt, n) * cle[i];
-  ce *= 0.5;
-  const T mu = cloth_mu<T>(v, v.node_cloth[n]);
-  const double kf = P.kf, df = P.df, h = v.h, h2 = v.h * v.h;
+YS_HD void friction_terms(const ClothParams& P, double h, bool trunc, const T& comp, const T& ce, const T& mu,
+                          const T& uvm, const T& uvdot, const T& FEns, const T& EEp, const T& EEv, T& slide, T& aEE,
+                          T& bE) {
+  const double kf = P.kf, df = P.df, h2 = h * h;
   const T lim = comp * mu;
-  const T uvm = ldT<T>(v.UV, v.dUV, k, nt, n) - ldT<T>(v.UVB, v.dUVB, k, nt, n);
-  const T slide = 1.0 / (1.0 + exp(-(1e4 * (fabs(FEns) - lim))));
+  slide = 1.0 / (1.0 + exp(-(1e4 * (fabs(FEns) - lim))));
   const T t = tanh(10 * uvm), tl = tanh(10 * (lim - FEns));
-  const T uvdot = ldT<T>(v.UVD, v.dUVD, k, nt, n);
   const T ku = kf * uvm, tm = t * lim, mce = mu * ce;
   const T lo = -0.5 * (ku - tm);
   const T force = lo * tl + 0.5 * (ku + tm) - df * uvdot;
@@ -779,10 +818,21 @@ YS_HD void friction_node(const View& v, int n, int k, const T& comp, const T& FE
   // tanh(10 * fric_lim - F) as written at src/PhysicsCloth.cpp:2630-2631
   const T tq = tanh(10 * lim - FEns);
   const T vel = lo * (1.0 - tq * tq) * EEv - df;
-  stT(v.SLIDE, v.dSLIDE, k, nt, n, slide);
   aEE = -h2 * pos - h * vel;
   // D enters b without a graph in the reference (src/MatrixMp.cpp:40-99)
-  bE = h * (force - (v.trunc ? detach(vel) : vel) * uvdot);
+  bE = h * (force - (trunc ? detach(vel) : vel) * uvdot);
+}
+template <class T>
+YS_HD void friction_node(const View& v, int n, int k, const T& comp, const T& FEns, const T& EEp, const T& EEv,
+                         const T* cle, T& aEE, T& bE) {
+  const int nt = v.ntot, c = v.node_cloth[n];
+  T ce = 0.0, slide;
+  for (int i = 0; i < 3; ++i) ce += ldT<T>(v.NRM, v.dNRM, i, nt, n) * cle[i];
+  ce *= 0.5;
+  const T uvm = ldT<T>(v.UV, v.dUV, k, nt, n) - ldT<T>(v.UVB, v.dUVB, k, nt, n);
+  friction_terms(v.cp[c], v.h, v.trunc != 0, comp, ce, cloth_mu<T>(v, c), uvm, ldT<T>(v.UVD, v.dUVD, k, nt, n), FEns,
+                 EEp, EEv, slide, aEE, bE);
+  stT(v.SLIDE, v.dSLIDE, k, nt, n, slide);
 }
 
 // ------------------------------------------------------------ shear
@@ -824,19 +874,33 @@ YS_HD void shear_diag(const T& kA, const T& kS, const T& co, const T* vv, const 
 // FP64-pipe bound: projections as d - (d.d') d', one reciprocal each for the
 // lengths and for the lock's denominator, and the vanishing P3 d3 block left
 // out took the producer from 1.23 to 0.95 ms on 255,292 nodes (0.97 M segments).
-template <class T, class Put>
-YS_HD void shear_terms(const View& v, int n0, int seg, Put&& put) {
+// One segment's inputs: the arms n1 - n0 and n3 - n0, and (compression + 1) S R^2
+template <class T>
+struct ShearIn {
+  T d1[3], d3[3], SR;
+  bool jam;  // the crossing's neighbours lie on its other side
+};
+template <class T>
+YS_HD ShearIn<T> shear_load(const View& v, int n0, int seg) {
   const ClothParams& P = v.cp[v.node_cloth[n0]];
-  const int n1 = n0 + shear_du(seg), n3 = n0 + shear_dv(seg) * P.W;
-  const int nt = v.ntot;
-  const double Lc = P.L, R = P.R, h = v.h, mh2 = -(v.h * v.h);
-  const T SR = (ldT<T>(v.COMP, v.dCOMP, 0, nt, n0) + 1.0) * (cloth_S<T>(v, v.node_cloth[n0]) * (R * R));
-  T d1[3], d3[3], a3[3], a1[3];
+  const int n1 = n0 + shear_du(seg), n3 = n0 + shear_dv(seg) * P.W, nt = v.ntot;
+  ShearIn<T> s;
+  s.SR = (ldT<T>(v.COMP, v.dCOMP, 0, nt, n0) + 1.0) * (cloth_S<T>(v, v.node_cloth[n0]) * (P.R * P.R));
   for (int i = 0; i < 3; ++i) {
     const T x0 = ldT<T>(v.X, v.dX, i, nt, n0);
-    d1[i] = ldT<T>(v.X, v.dX, i, nt, n1) - x0;
-    d3[i] = ldT<T>(v.X, v.dX, i, nt, n3) - x0;
+    s.d1[i] = ldT<T>(v.X, v.dX, i, nt, n1) - x0;
+    s.d3[i] = ldT<T>(v.X, v.dX, i, nt, n3) - x0;
   }
+  const bool f0 = (v.flags[n0] & YS_FLIP) != 0, f1 = (v.flags[n1] & YS_FLIP) != 0, f3 = (v.flags[n3] & YS_FLIP) != 0;
+  s.jam = f0 != f1 && f0 != f3;
+  return s;
+}
+template <class T, class Put>
+YS_HD void shear_terms(const ShearIn<T>& s, const ClothParams& P, double h, bool trunc, Put&& put) {
+  const double Lc = P.L, R = P.R, mh2 = -(h * h);
+  const T& SR = s.SR;
+  T d1[3], d3[3], a3[3], a1[3];
+  for (int i = 0; i < 3; ++i) { d1[i] = s.d1[i]; d3[i] = s.d3[i]; }
   const T il1 = rsqrt_(dot3(d1, d1)), il3 = rsqrt_(dot3(d3, d3));
   for (int i = 0; i < 3; ++i) { d1[i] *= il1; d3[i] *= il3; }
   // the crossing angle phi in [0, pi] and 1 / sin(phi) from its cosine co;
@@ -846,14 +910,12 @@ YS_HD void shear_terms(const View& v, int n0, int seg, Put&& put) {
   const T phi = acos(co);
   const T is = rsqrt_((1.0 - co) * (1.0 + co)), is2 = is * is, cs2 = co * is2;
   const T i11 = il1 * il1, i33 = il3 * il3, i13 = il1 * il3;
-  const uint8_t f0 = v.flags[n0], f1 = v.flags[n1], f3 = v.flags[n3];
-  const bool jam = (((f0 & YS_FLIP) != 0) != ((f1 & YS_FLIP) != 0)) && (((f0 & YS_FLIP) != 0) != ((f3 & YS_FLIP) != 0));
-  if (!jam) {
+  if (!s.jam) {
     const T kL = SR * (kPi * Lc) * is;
     const T ph = phi - kPi / 2;
     // Shear_F takes phi.item() in (phi - PI/2) (src/PhysicsCloth.cpp:2720-2721):
     // that factor carries no derivative along the reference's gradient path
-    const T phf = v.trunc ? detach(phi) - kPi / 2 : ph;
+    const T phf = trunc ? detach(phi) - kPi / 2 : ph;
     const T cf = h * (kL * phf), cf1 = cf * il1, cf3 = cf * il3;
     for (int i = 0; i < 3; ++i) { put(kS_F1 + i, cf1 * a3[i]); put(kS_F3 + i, cf3 * a1[i]); }
     // src/PhysicsCloth.cpp:2715-2751 per block:
@@ -976,7 +1038,9 @@ YS_HD void shear_terms(const View& v, int n0, int seg, Put&& put) {
 // the record in the shear buffer at slot seg * ntot + n0
 template <class T>
 YS_HD void shear_element(const View& v, double* buf, double* dbuf, int n0, int seg) {
-  shear_terms<T>(v, n0, seg, [&](int f, const T& x) { stT(buf, dbuf, 4 * f + seg, v.ntot, n0, x); });
+  shear_terms<T>(shear_load<T>(v, n0, seg), v.cp[v.node_cloth[n0]], v.h, v.trunc != 0, [&](int f, const T& x) {
+    stT(buf, dbuf, 4 * f + seg, v.ntot, n0, x);
+  });
 }
 
 }  // namespace ys

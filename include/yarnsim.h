@@ -273,13 +273,13 @@ ys_status ys_step_tangent_ext(ys_batch *b, double h, const double *ext_force, co
  *   the derivative of the discrete step) or A^-1 q_bar
  *   (YS_TANGENT_REFERENCE: what the reference's autograd computes, A, M and
  *   dF/dv held constant); then -lambda^T d(A q - b) / d(state, materials)
- *   by forward-mode directional derivatives of the residual on copies of the
- *   cloths (512 directions per step, 4 per copy), compressed by a colouring
- *   of the nodes (row blocks depend on nodes within grid distance 4).
- * The adjoint owns a workspace batch of `copies` copies of b's cloths
- * (about 25 KB per copied node); 512 / (4 copies) passes per step. */
+ *   by vector-Jacobian products of the edge, bend, face, shear and friction
+ *   terms, summed per node in a fixed order.
+ * The adjoint owns about 1.5 KB of workspace per node of b. */
 typedef struct ys_adjoint ys_adjoint;
-/* copies: 1..128 (128: one pass per step). b must outlive the adjoint. */
+/* copies: 1..128; any value gives the same results in the same time (it sized a
+ * workspace of cloth copies, which the step no longer needs). b must outlive the
+ * adjoint. */
 ys_status ys_adjoint_create(ys_batch *b, int32_t mode, int32_t copies, ys_adjoint **out);
 void ys_adjoint_destroy(ys_adjoint *a);
 /* One step backwards from the state b holds now (the state at the start of
