@@ -136,8 +136,8 @@ struct ys_batch {
     double *dX = nullptr, *dV = nullptr, *dUV = nullptr, *dUVD = nullptr, *dUVB = nullptr;
     double *dNRM = nullptr, *dCOMP = nullptr, *dSLIDE = nullptr;
     double *drho = nullptr, *dks = nullptr, *dkb = nullptr, *dS = nullptr, *dmu = nullptr;
-    double *dA = nullptr, *dB = nullptr, *As = nullptr, *Bs = nullptr, *qsave = nullptr, *rt = nullptr, *dq = nullptr;
-    double *dedge = nullptr, *dbend = nullptr, *dface = nullptr, *dshear = nullptr;
+    double *qsave = nullptr, *rt = nullptr, *dq = nullptr;
+    double* scratch = nullptr;  // [kTangents][kTangentScratch][ntot]
     double* io = nullptr;  // [kTangents][ntot][3] staging of host tangents
     double* dext = nullptr;  // [kTangents][ntot][5] external-force tangents
   } tan;
@@ -1113,18 +1113,15 @@ ys_status tan_download(ys_batch* b, const double* src, double* dst, int c, int32
   return YS_OK;
 }
 
-// the view of the dual assembly: values of A and b into shadows, tangents alongside
+// the step's view with the tangent arrays
 ys::View dual_view(ys_batch* b) {
   ys::View dv = b->v;
   const ys_batch::Tan& t = b->tan;
-  dv.A = t.As;
-  dv.B = t.Bs;
   dv.K = KT;
   dv.trunc = t.mode == YS_TANGENT_REFERENCE ? 1 : 0;
   dv.dX = t.dX; dv.dV = t.dV; dv.dUV = t.dUV; dv.dUVD = t.dUVD; dv.dUVB = t.dUVB;
   dv.dNRM = t.dNRM; dv.dCOMP = t.dCOMP; dv.dSLIDE = t.dSLIDE;
   dv.dline_rho = t.drho; dv.dline_ks = t.dks; dv.dline_kb = t.dkb; dv.dS = t.dS; dv.dmu = t.dmu;
-  dv.dA = t.dA; dv.dB = t.dB;
   return dv;
 }
 
@@ -1147,11 +1144,8 @@ ys_status ys_tangent_enable(ys_batch* b, int32_t mode) {
     A(&t.dX, 3 * KT * nt); A(&t.dV, 3 * KT * nt); A(&t.dUV, 2 * KT * nt); A(&t.dUVD, 2 * KT * nt);
     A(&t.dUVB, 2 * KT * nt); A(&t.dNRM, 3 * KT * nt); A(&t.dCOMP, KT * nt); A(&t.dSLIDE, 2 * KT * nt);
     A(&t.drho, KT * nl); A(&t.dks, KT * nl); A(&t.dkb, KT * nl); A(&t.dS, KT * nc); A(&t.dmu, KT * nc);
-    A(&t.dA, (size_t)ys::YS_NUM_SLOTS * KT * nt); A(&t.dB, 5 * KT * nt);
-    A(&t.As, (size_t)ys::YS_NUM_SLOTS * nt); A(&t.Bs, 5 * nt); A(&t.qsave, 5 * nt); A(&t.rt, 5 * KT * nt);
-    A(&t.dq, 5 * KT * nt);
-    A(&t.dedge, (size_t)ys::kEdgeFields * 2 * KT * nt); A(&t.dbend, (size_t)ys::kBendFields * 2 * KT * nt);
-    A(&t.dface, 6 * KT * nt); A(&t.dshear, (size_t)ys::kShearFields * 4 * KT * nt);
+    A(&t.qsave, 5 * nt); A(&t.rt, 5 * KT * nt); A(&t.dq, 5 * KT * nt);
+    A(&t.scratch, (size_t)ys::kTangentScratch * KT * nt);
     A(&t.io, 3 * KT * nt);
     if (st != YS_OK) return st;
     t.on = true;
@@ -1261,18 +1255,12 @@ ys_status ys_step_tangent_ext(ys_batch* b, double h, const double* ext_force, co
   const int64_t nt = b->ntot;
   ys_batch::Tan& t = b->tan;
   YS_CUDA(cudaMemcpyAsync(t.qsave, b->so.x, sizeof(double) * 5 * nt, cudaMemcpyDeviceToDevice, cs));
-  // dual assembly: tangents of A and b
+  // tangents of the residual b - A q at the step's q
   ys::View dv = dual_view(b);
-  ys::Records dr = b->rec;
-  dr.dedge = t.dedge; dr.dbend = t.dbend; dr.dface = t.dface; dr.dshear = t.dshear;
-  b->run(YS_PROF_MISC, 7, [&] { ys::launch_assembly_dual(dv, dr, b->anchors, b->geom_n, cs); });
+  b->run(YS_PROF_MISC, 7, [&] {
+    ys::launch_tangent_residual(dv, b->rec, b->anchors + b->geom_off, b->geom_n, t.qsave, t.scratch, d_dext, kact, t.rt, cs);
+  });
   YS_CUDA(cudaGetLastError());
-  b->run(YS_PROF_MISC, 1, [&] { ys::launch_tangent_rhs(dv, t.qsave, t.rt, kact, cs); });
-  YS_CUDA(cudaGetLastError());
-  if (d_dext) {
-    b->run(YS_PROF_MISC, 1, [&] { ys::launch_tangent_ext(dv, d_dext, t.rt, h, kact, cs); });
-    YS_CUDA(cudaGetLastError());
-  }
   // tangent solves with the step's A and Jacobi diagonal: A dq_k = db_k - dA_k q
   // (exact), or A^T dq_k = db_k with M, D held constant -- the transpose of
   // the reference's backward b_bar = A^-1 q_bar (src/Solvers.cpp:33-58)

@@ -3,15 +3,13 @@
 // Assembly: one thread per element writes that element's record (forces and
 // Jacobian blocks), then four threads per node gather the records touching its
 // row block in a fixed order, so every row is accumulated deterministically
-// without atomics. The element kernels are templates over the scalar type:
-// double for the step, Dual<kTangents> for its forward-mode sensitivities.
+// without atomics.
 // Solve: per-cloth Jacobi-PCG (Eigen's ConjugateGradient algorithm, as used by
 // src/Solvers.cpp:3-31) on the structured stencil matrix; thread blocks never
 // straddle cloths, so each cloth's dot products are a fixed-order sum of its
 // blocks' partials, recomputed redundantly by every block that needs them.
 #include <cfloat>
 
-#include "ys_elem_kernels.cuh"
 #include "ys_items.cuh"
 #include "ys_kernels.cuh"
 
@@ -24,6 +22,58 @@ __global__ void k_geom(View v, const int* __restrict__ nodes, int count) {
   if (t >= count) return;
   const int n = nodes[t];
   node_normal(v, n, v.cp[v.node_cloth[n]].W);
+}
+
+// The record producers: one thread per element, nothing shared between
+// threads, so any block size gives the same bits; the
+// block size is a schedule choice (up to kMaxProducerBlock threads; up to
+// kBlock for the edges, whose 254 registers spill when compiled for 256-thread
+// blocks).
+
+// one thread per (yarn direction, node): the edge starting at that node
+__global__ void __launch_bounds__(kBlock) k_edge_rec(View v, Records R) {
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= 2LL * v.ntot) return;
+  const int k = t >= v.ntot ? 1 : 0;
+  const int n0 = (int)(t - (int64_t)k * v.ntot);
+  const ClothParams& P = v.cp[v.node_cloth[n0]];
+  if (k == 0 ? v.node_u[n0] >= P.W - 1 : v.node_v[n0] >= P.H - 1) return;
+  // each field goes to memory as soon as it is known, so none is held
+  edge_terms<double>(v, n0, n0 + (k == 0 ? 1 : P.W), k,
+                [&](int f, double x) { stT(R.edge, R.dedge, 2 * f + k, v.ntot, n0, x); });
+}
+
+// one thread per (yarn direction, middle node) of a bend segment
+__global__ void __launch_bounds__(kMaxProducerBlock) k_bend_rec(View v, Records R) {
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= 2LL * v.ntot) return;
+  const int k = t >= v.ntot ? 1 : 0;
+  const int n0 = (int)(t - (int64_t)k * v.ntot);
+  const ClothParams& P = v.cp[v.node_cloth[n0]];
+  const int pos = k == 0 ? v.node_u[n0] : v.node_v[n0], len = k == 0 ? P.W : P.H;
+  if (pos < 1 || pos > len - 2) return;
+  const int step = k == 0 ? 1 : P.W;
+  const int line = k == 0 ? P.warp_line_off + v.node_v[n0] : P.weft_line_off + v.node_u[n0];
+  bend_element<double>(v, R.bend, R.dbend, n0 - step, n0, n0 + step, k, line);
+}
+
+// one thread per grid cell (top-left node): its two faces
+__global__ void __launch_bounds__(kMaxProducerBlock) k_face_rec(View v, Records R) {
+  const int n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (n >= v.ntot) return;
+  const ClothParams& P = v.cp[v.node_cloth[n]];
+  if (v.node_u[n] >= P.W - 1 || v.node_v[n] >= P.H - 1) return;
+  cell_faces<double>(v, R.face, R.dface, n);
+}
+
+// one thread per (segment type, crossing)
+__global__ void __launch_bounds__(kMaxProducerBlock) k_shear_rec(View v, Records R) {
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= 4LL * v.ntot) return;
+  const int seg = (int)(t / v.ntot);
+  const int n0 = (int)(t - (int64_t)seg * v.ntot);
+  if (!(v.flags[n0] & YS_INTERIOR)) return;
+  shear_element<double>(v, R.shear, R.dshear, n0, seg);
 }
 
 // ------------------------------------------------------------- the gathers
@@ -324,19 +374,19 @@ void launch_geom(const View& v, const int* nodes, int n, cudaStream_t s) {
 static inline unsigned pblocks(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
 void launch_edge_records(const View& v, const Records& R, cudaStream_t s, int t) {
   t = t < kBlock ? t : kBlock;  // k_edge_rec is compiled for at most kBlock threads
-  k_edge_rec<double><<<pblocks(2LL * v.ntot, t), t, 0, s>>>(v, R);
+  k_edge_rec<<<pblocks(2LL * v.ntot, t), t, 0, s>>>(v, R);
 }
 void launch_bend_records(const View& v, const Records& R, cudaStream_t s, int t) {
-  k_bend_rec<double><<<pblocks(2LL * v.ntot, t), t, 0, s>>>(v, R);
+  k_bend_rec<<<pblocks(2LL * v.ntot, t), t, 0, s>>>(v, R);
 }
 void launch_face_records(const View& v, const Records& R, cudaStream_t s, int t) {
-  k_face_rec<double><<<pblocks(v.ntot, t), t, 0, s>>>(v, R);
+  k_face_rec<<<pblocks(v.ntot, t), t, 0, s>>>(v, R);
 }
 void launch_cross(const View& v, const Records& R, cudaStream_t s) {
   k_cross<<<pblocks(v.ntot, kNodesPerBlock), 4 * kNodesPerBlock, 0, s>>>(v, R);
 }
 void launch_shear_records(const View& v, const Records& R, cudaStream_t s, int t) {
-  k_shear_rec<double><<<pblocks(4LL * v.ntot, t), t, 0, s>>>(v, R);
+  k_shear_rec<<<pblocks(4LL * v.ntot, t), t, 0, s>>>(v, R);
 }
 void launch_rows(const View& v, const Records& R, const Solver& so, cudaStream_t s) {
   k_rows<<<pblocks(v.ntot, kNodesPerBlock), 4 * kNodesPerBlock, 0, s>>>(v, R, so);

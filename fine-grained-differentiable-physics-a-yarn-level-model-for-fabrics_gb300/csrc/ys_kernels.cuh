@@ -97,12 +97,14 @@ struct TangentState {
   double* dUVD;
   double* dUVB;
 };
-// the element / gather / finalize kernels over Dual<kTangents>
-void launch_assembly_dual(const View& v, const Records& R, const int* geom_nodes, int geom_n, cudaStream_t s);
-// rt[k][c][ntot] = db_k - dA_k q (or db_k when v.trunc) for k < kact
-void launch_tangent_rhs(const View& v, const double* q, double* rt, int kact, cudaStream_t s);
-// rt_k += h dext_k for the external force's tangents dext [kact][ntot][5]
-void launch_tangent_ext(const View& v, const double* dext, double* rt, double h, int kact, cudaStream_t s);
+// scratch of the tangent step, in units of kTangents * ntot doubles
+constexpr int kTangentScratch = 2 * 20 + 2 * 20 + 6 + 4 * 6 + 2;
+// after the step's own assembly (records R, values in v): the tangents of the
+// normals, compressions and slide indicators, and rt[k][c][ntot] =
+// db_k - dA_k q + h dext_k (without dA_k q when v.trunc; dext [kact][ntot][5]
+// may be null) for k < kact; returns the number of kernels
+int launch_tangent_residual(const View& v, const Records& R, const int* interior, int n_interior, const double* q,
+                            double* scratch, const double* dext, int kact, double* rt, cudaStream_t s);
 // solution check, then Cloth::update of the state (solution so.x) and its
 // tangents (dq, [5][kTangents][ntot])
 void launch_update_dual(const View& v, const Blocks& b, const Solver& so, const double* dq, const TangentState& ts,

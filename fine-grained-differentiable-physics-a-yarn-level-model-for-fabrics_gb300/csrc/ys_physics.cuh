@@ -3,7 +3,7 @@
 // Each routine handles one element (edge, bend segment, crossing, shear
 // segment, face) and returns its contribution to the step's system
 //     A = M - h^2 dF/dx - h dF/dv,   b = h (F - (dF/dv)^T v) + M v
-// (src/TrainHelper.cpp:19-20). The record producers (ys_elem_kernels.cuh)
+// (src/TrainHelper.cpp:19-20). The record producers (ys_kernels.cu)
 // write each element's contribution to its own record, and the per-node
 // gathers (ys_items.cuh) sum a node's records in a fixed order into the
 // structured stencil layout of ys_common.cuh, so the accumulation is
@@ -90,9 +90,9 @@ YS_HD double& st(double* p, int comp, int ntot, int node) { return p[(int64_t)co
 
 // Scalar-generic loads and stores. A per-node array p holds comp c of node i
 // at p[c * ntot + i]; its tangent array dp (forward-mode runs only) holds
-// tangent k at dp[(c * K + k) * ntot + i]. Record buffers use the same rule
-// with c = field * nslot + slot. With T = double the tangent arrays are
-// never touched.
+// tangent k at dp[(c * kTangents + k) * ntot + i]; a Dual of fewer directions
+// reads those from dp on. Record buffers use the same rule with c = field *
+// nslot + slot. With T = double the tangent arrays are never touched.
 YS_HD void lds(const double* p, const double* dp, int c, int ntot, int i, double& x) {
   (void)dp;
   x = p[(int64_t)c * ntot + i];
@@ -100,7 +100,7 @@ YS_HD void lds(const double* p, const double* dp, int c, int ntot, int i, double
 template <int K>
 YS_HD void lds(const double* p, const double* dp, int c, int ntot, int i, Dual<K>& x) {
   x.v = p[(int64_t)c * ntot + i];
-  for (int k = 0; k < K; ++k) x.d[k] = dp ? dp[((int64_t)c * K + k) * ntot + i] : 0.0;
+  for (int k = 0; k < K; ++k) x.d[k] = dp ? dp[((int64_t)c * kTangents + k) * ntot + i] : 0.0;
 }
 template <class T>
 YS_HD T ldT(const double* p, const double* dp, int c, int ntot, int i) {
@@ -116,7 +116,7 @@ template <int K>
 YS_HD void stT(double* p, double* dp, int c, int ntot, int i, const Dual<K>& x) {
   p[(int64_t)c * ntot + i] = x.v;
   if (dp)
-    for (int k = 0; k < K; ++k) dp[((int64_t)c * K + k) * ntot + i] = x.d[k];
+    for (int k = 0; k < K; ++k) dp[((int64_t)c * kTangents + k) * ntot + i] = x.d[k];
 }
 // a parameter of index i in a table of n entries (tangent k at dp[k * n + i])
 YS_HD void ldp(const double* p, const double* dp, int i, int n, double& x) {
