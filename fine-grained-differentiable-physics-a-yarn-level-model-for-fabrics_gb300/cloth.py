@@ -316,10 +316,10 @@ class ClothBatch:
         N.check(N.load().ys_set_producer_threads(self._h, int(threads)), "ys_set_producer_threads")
 
     def set_pcg_schedule(self, persistent: bool, threads: int = 0, cluster: int = 0):
-        """Phase PCG (three launches per iteration, the default) or the
-        persistent per-cloth PCG (one launch per solve, `cluster` CTAs of
-        `threads` threads per cloth; threads * cluster >= the largest cloth's
-        nodes). Both give the same bits (see ys_set_pcg_schedule)."""
+        """Phase PCG (three launches per iteration) or the persistent per-cloth
+        PCG (one launch per solve; threads * cluster >= the largest cloth's
+        nodes). Both give the same bits; a batch starts with the one expected
+        to be faster (see ys_set_pcg_schedule)."""
         N.check(N.load().ys_set_pcg_schedule(self._h, 1 if persistent else 0, int(threads), int(cluster)),
                 "ys_set_pcg_schedule")
 

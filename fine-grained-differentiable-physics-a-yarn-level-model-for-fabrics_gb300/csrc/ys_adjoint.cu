@@ -71,12 +71,6 @@ __device__ __forceinline__ void keep(double* buf, int nvar, int pair, int64_t st
     if (2 * pair + k < nvar) buf[(int64_t)(2 * pair + k) * stride + at] = phi.d[k];
 }
 
-// sum over a warp, the same bits in every lane
-__device__ __forceinline__ double warp_total(double s) {
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  return s;
-}
-
 // lambda and q at a node
 struct Weights {
   const double* lam;
@@ -575,7 +569,7 @@ __global__ void __launch_bounds__(128) k_adj_params(View v, AdjWork w, const dou
       if (i >= 1 && i <= len - 2) s[2] += w.bend[7 * st2 + o] + w.bend[14 * st2 + o];
     }
     for (int p = 0; p < 3; ++p) {
-      const double x = warp_total(s[p]);
+      const double x = cloth_tree(s[p]);
       if (lane == 0) gp.line[p][id] = p == 0 ? x : x * line_a[id];
     }
   } else if (id < nl + v.ncloth) {
@@ -590,8 +584,8 @@ __global__ void __launch_bounds__(128) k_adj_params(View v, AdjWork w, const dou
       for (int seg = 0; seg < 4; ++seg) a += w.shear[(int64_t)6 * 4 * nt + (int64_t)seg * nt + n];
       sS += (v.COMP[n] + 1.0) * (P.R * P.R) * a;
     }
-    sS = warp_total(sS);
-    sm = warp_total(sm);
+    sS = cloth_tree(sS);
+    sm = cloth_tree(sm);
     if (lane == 0) { gp.cloth[0][c] = sS; gp.cloth[1][c] = sm; }
   }
 }

@@ -182,12 +182,13 @@ struct ys_batch {
   } graph;
   int check_every = 16;  // PCG iterations between convergence checks when the call gives none
   // PCG schedule (ys_set_pcg_schedule): phases, or the persistent per-cloth
-  // kernel with `threads` x `csize` nodes per cloth; `order` lists the cloths
-  // largest first, so the biggest clusters start first
+  // kernel; `order` lists the cloths largest first, so the biggest clusters
+  // start first
   struct PcgPlan {
     int kind = YS_PCG_PHASES;
-    int threads = 0, csize = 0;
-    int* order = nullptr;  // device [ncloth]
+    int threads = 0, csize = 0;  // as the caller gave them
+    ys::ClusterShape shape{};  // what runs
+    int* order = nullptr;      // device [ncloth]
     int max_nodes = 0;
   } plan;
   std::vector<ys_schedule> tuned;  // every schedule the last ys_autotune timed
@@ -343,6 +344,26 @@ int weave_flip(int weave, int i, int j) {
   return ru == 0;
 }
 
+// (threads, cluster) as ys_set_pcg_schedule takes them
+bool pcg_shape_ok(int threads, int csize) {
+  if (threads != 128 && threads != 256 && threads != 512 && threads != 1024) return false;
+  return csize == 1 || csize == 2 || csize == 4 || csize == 8 || csize == 16;
+}
+
+// the order of the cloths, the persistent PCG's shape and the default schedule
+ys_status plan_pcg(ys_batch* b) {
+  ys_batch::PcgPlan& P = b->plan;
+  std::vector<int> ord(b->ncloth);
+  for (int c = 0; c < b->ncloth; ++c) ord[c] = c;
+  std::stable_sort(ord.begin(), ord.end(),
+                   [&](int x, int y) { return b->cp[x].W * b->cp[x].H > b->cp[y].W * b->cp[y].H; });
+  YS_CUDA(cudaMemcpy(P.order, ord.data(), sizeof(int) * b->ncloth, cudaMemcpyHostToDevice));
+  P.max_nodes = b->cp[ord[0]].W * b->cp[ord[0]].H;
+  YS_CUDA(ys::pcg_cluster_shape(b->cp.data(), b->ncloth, b->device, &P.shape));
+  if (P.shape.faster) P.kind = YS_PCG_PERSISTENT;
+  return YS_OK;
+}
+
 }  // namespace
 
 // error reporting for the other translation units of the library (not exported)
@@ -484,7 +505,7 @@ ys_status ys_batch_create(int32_t n_cloths, const ys_cloth_desc* descs, int32_t 
     b->so.q = b->vecs + 15 * nt; b->so.dinv = b->vecs + 20 * nt;
   }
   A(&b->so.part, 4 * blk_cloth.size()); A(&b->so.pc, n_cloths); A(&b->so.nactive, 1);
-  A(&b->stage, 15 * nt); A(&b->ext, 5 * nt);
+  A(&b->stage, 15 * nt); A(&b->ext, 5 * nt); A(&b->plan.order, n_cloths);
   if (st != YS_OK) { delete b; return st; }
   if (cudaMallocHost(&b->h_nactive, sizeof(int)) != cudaSuccess ||
       cudaMallocHost(&b->h_wind, sizeof(double) * 3 * n_cloths) != cudaSuccess ||
@@ -543,6 +564,8 @@ ys_status ys_batch_create(int32_t n_cloths, const ys_cloth_desc* descs, int32_t 
   b->blk.blk_cloth = d_bc; b->blk.blk_node0 = d_bn; b->blk.blk_count = d_bk;
   b->blk.cloth_blk0 = d_cb; b->blk.cloth_nblk = d_cn;
   b->so.tol = DBL_EPSILON;
+  const ys_status sp = plan_pcg(b);
+  if (sp != YS_OK) { delete b; return sp; }
   *out = b;
   return YS_OK;
 }
@@ -769,7 +792,7 @@ ys_status solve_impl(ys_batch* b, const ys::View& v, const ys_solve_opts* opts, 
   if (b->plan.kind == YS_PCG_PERSISTENT) {
     cudaError_t e = cudaSuccess;
     b->run(YS_PROF_PCG_PERSIST, 1, [&] {
-      e = ys::launch_pcg_cluster(v, b->so, b->plan.order, b->ncloth, b->plan.threads, b->plan.csize, cap, s);
+      e = ys::launch_pcg_cluster(v, b->so, b->plan.order, b->ncloth, b->plan.shape, cap, s);
     });
     if (e != cudaSuccess) return fail(YS_ERR_CUDA, std::string("persistent PCG: ") + cudaGetErrorString(e));
   }
@@ -1588,7 +1611,7 @@ ys_status graph_build(ys_batch* b, int m, int cap, int override_max) {
     YS_CUDA(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
     capture_assembly(b, cs, override_max);
     const cudaError_t e =
-        ys::launch_pcg_cluster(v, so, b->plan.order, b->ncloth, b->plan.threads, b->plan.csize, cap, cs);
+        ys::launch_pcg_cluster(v, so, b->plan.order, b->ncloth, b->plan.shape, cap, cs);
     ys::launch_update(v, b->blk, b->so, cs);
     cudaGraph_t one = nullptr;
     YS_CUDA(cudaStreamEndCapture(cs, &one));
@@ -1733,30 +1756,14 @@ ys_status ys_set_pcg_schedule(ys_batch* b, int32_t pcg, int32_t threads, int32_t
     return YS_OK;
   }
   if (pcg != YS_PCG_PERSISTENT) return fail(YS_ERR_ARG, "ys_set_pcg_schedule: unknown schedule");
-  if (!ys::pcg_cluster_shape_ok(threads, cluster))
+  if (!pcg_shape_ok(threads, cluster))
     return fail(YS_ERR_ARG, "ys_set_pcg_schedule: threads must be 128, 256, 512 or 1024 and cluster 1, 2, 4, 8 "
                             "or 16, at most 16384 nodes");
-  if (!P.order) {
-    // cloths largest first
-    std::vector<int> ord(b->ncloth);
-    for (int c = 0; c < b->ncloth; ++c) ord[c] = c;
-    std::stable_sort(ord.begin(), ord.end(),
-                     [&](int x, int y) { return b->cp[x].W * b->cp[x].H > b->cp[y].W * b->cp[y].H; });
-    const ys_status s = b->alloc(&P.order, b->ncloth);
-    if (s != YS_OK) return s;
-    YS_CUDA(cudaMemcpy(P.order, ord.data(), sizeof(int) * b->ncloth, cudaMemcpyHostToDevice));
-    P.max_nodes = b->cp[ord[0]].W * b->cp[ord[0]].H;
-  }
   if (P.max_nodes > threads * cluster)
     return fail(YS_ERR_ARG, "ys_set_pcg_schedule: the largest cloth has " + std::to_string(P.max_nodes) +
                                 " nodes, more than threads x cluster");
-  int fit = 0;
-  const cudaError_t e = ys::pcg_cluster_occupancy(threads, cluster, &fit);
-  if (e != cudaSuccess || fit < 1) {
-    cudaGetLastError();
-    return fail(YS_ERR_ARG, "ys_set_pcg_schedule: this GPU cannot run a cluster of that shape");
-  }
-  P.kind = YS_PCG_PERSISTENT;
+  // where no cluster holds the largest cloth: the phases, the same bits
+  P.kind = P.shape.groups ? YS_PCG_PERSISTENT : YS_PCG_PHASES;
   P.threads = threads;
   P.csize = cluster;
   b->graph.built = false;
@@ -1849,8 +1856,6 @@ ys_status ys_autotune(ys_batch* b, double h, const ys_solve_opts* opts, int32_t 
   b->profiling = false;
   // the candidates
   std::vector<ys_schedule> cand;
-  int max_nodes = 0;
-  for (int c = 0; c < b->ncloth; ++c) max_nodes = std::max(max_nodes, b->cp[c].W * b->cp[c].H);
   for (int g = 0; g < 2; ++g) {
     for (int every : {2, 4, 8, 16, 32}) {
       ys_schedule k{};
@@ -1859,19 +1864,19 @@ ys_status ys_autotune(ys_batch* b, double h, const ys_solve_opts* opts, int32_t 
       k.pcg = YS_PCG_PHASES;
       cand.push_back(k);
     }
-    for (int t : {128, 256, 512, 1024})
-      for (int cl : {1, 2, 4, 8, 16}) {
-        const int cap_nodes = t * cl;
-        if (!ys::pcg_cluster_shape_ok(t, cl) || cap_nodes < max_nodes || cap_nodes >= 4 * std::max(max_nodes, 128))
-          continue;
-        ys_schedule k{};
-        k.graphs = g;
-        k.check_every = b->check_every;
-        k.pcg = YS_PCG_PERSISTENT;
-        k.pcg_threads = t;
-        k.pcg_cluster = cl;
-        cand.push_back(k);
+    if (b->plan.shape.groups) {  // in the smallest shape that holds the largest cloth
+      ys_schedule k{};
+      k.graphs = g;
+      k.check_every = b->check_every;
+      k.pcg = YS_PCG_PERSISTENT;
+      k.pcg_threads = 128;
+      k.pcg_cluster = 1;
+      while (k.pcg_threads * k.pcg_cluster < b->plan.max_nodes) {
+        if (k.pcg_cluster < 16) k.pcg_cluster *= 2;
+        else k.pcg_threads *= 2;
       }
+      cand.push_back(k);
+    }
   }
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   ys_status st = YS_OK;

@@ -173,12 +173,15 @@ __device__ __forceinline__ double block_sum(double val, double* sh) {
   return s;  // valid in thread 0
 }
 
-// fixed-order sum of cloth c's block partials in row `which`
+// fixed-order sum of cloth c's block partials in row `which`, by a whole warp:
+// lane l adds blocks l, l + 32, ... in order, then the lanes as a tree. (One
+// thread adding them all waited out an FP64 addition per block, up to 79 of
+// them on a 100 x 100 cloth, in every block of every launch.)
 __device__ __forceinline__ double cloth_sum(const Blocks& b, const double* part, int which, int c) {
   const int b0 = b.cloth_blk0[c], nb = b.cloth_nblk[c];
   double s = 0.0;
-  for (int i = 0; i < nb; ++i) s += part[which * b.nblk + b0 + i];
-  return s;
+  for (int i = threadIdx.x & 31; i < nb; i += 32) s += part[which * b.nblk + b0 + i];
+  return cloth_tree(s);
 }
 
 // x = 0, r = b, p = z = Dinv r; partials |b|^2 (row 0), |r|^2 (row 1) and
@@ -192,12 +195,9 @@ __global__ void __launch_bounds__(kBlock) k_pcg_setup(View v, Blocks b, Solver s
   if (threadIdx.x < b.blk_count[blk]) {
     for (int k = 0; k < 5; ++k) {
       const double r = ld(v.B, k, nt, n);
-      const double z = ld(so.dinv, k, nt, n) * r;
       st(so.x, k, nt, n) = 0.0;
       st(so.r, k, nt, n) = r;
-      st(so.p, k, nt, n) = z;
-      rr += r * r;
-      rz += r * z;
+      st(so.p, k, nt, n) = pcg_norms(r, ld(so.dinv, k, nt, n), rr, rz);
     }
   }
   double s1 = block_sum(rr, sh);
@@ -209,16 +209,17 @@ __global__ void __launch_bounds__(kBlock) k_pcg_setup(View v, Blocks b, Solver s
   if (threadIdx.x == 0) so.part[2 * b.nblk + blk] = s2;
 }
 
+// one warp per cloth
 __global__ void k_pcg_start(Blocks b, Solver so, int ncloth) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (c >= ncloth) return;
   PcgCloth& pc = so.pc[c];
   const double bb = cloth_sum(b, so.part, 0, c);
   const double rr = cloth_sum(b, so.part, 1, c);
   const double rz = cloth_sum(b, so.part, 2, c);
+  if (threadIdx.x & 31) return;
   pc.bb = bb;
-  double thr = so.tol * so.tol * bb;
-  if (thr < DBL_MIN) thr = DBL_MIN;
+  const double thr = pcg_threshold(so.tol, bb);
   pc.thr = thr;
   pc.rr = rr;
   pc.rz[0] = rz;
@@ -242,7 +243,7 @@ __global__ void __launch_bounds__(kBlock) k_pcg_spmv(View v, Blocks b, Solver so
     else spmv_row(v, so.p, n, y);
     for (int k = 0; k < 5; ++k) {
       st(so.q, k, nt, n) = y[k];
-      pq += ld(so.p, k, nt, n) * y[k];
+      pq = fma(ld(so.p, k, nt, n), y[k], pq);
     }
   }
   const double s = block_sum(pq, sh);
@@ -256,7 +257,10 @@ __global__ void __launch_bounds__(kBlock) k_pcg_axpy(View v, Blocks b, Solver so
   const int blk = blockIdx.x;
   const int c = b.blk_cloth[blk];
   if (!so.pc[c].active) return;
-  if (threadIdx.x == 0) alpha_sh = so.pc[c].rz[parity] / cloth_sum(b, so.part, 0, c);
+  if (threadIdx.x < 32) {
+    const double pq = cloth_sum(b, so.part, 0, c);
+    if (threadIdx.x == 0) alpha_sh = so.pc[c].rz[parity] / pq;
+  }
   __syncthreads();
   const double alpha = alpha_sh;
   const int n = b.blk_node0[blk] + threadIdx.x;
@@ -264,11 +268,11 @@ __global__ void __launch_bounds__(kBlock) k_pcg_axpy(View v, Blocks b, Solver so
   double rr = 0.0, rz = 0.0;
   if (threadIdx.x < b.blk_count[blk]) {
     for (int k = 0; k < 5; ++k) {
-      st(so.x, k, nt, n) += alpha * ld(so.p, k, nt, n);
-      const double r = ld(so.r, k, nt, n) - alpha * ld(so.q, k, nt, n);
+      double x = ld(so.x, k, nt, n), r = ld(so.r, k, nt, n);
+      pcg_advance(alpha, ld(so.p, k, nt, n), ld(so.q, k, nt, n), x, r);
+      st(so.x, k, nt, n) = x;
       st(so.r, k, nt, n) = r;
-      rr += r * r;
-      rz += r * (ld(so.dinv, k, nt, n) * r);
+      pcg_norms(r, ld(so.dinv, k, nt, n), rr, rz);
     }
   }
   double s1 = block_sum(rr, sh);
@@ -288,21 +292,23 @@ __global__ void __launch_bounds__(kBlock) k_pcg_dir(View v, Blocks b, Solver so,
   const int c = b.blk_cloth[blk];
   PcgCloth& pc = so.pc[c];
   if (!pc.active) return;
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < 32) {
     const double rr = cloth_sum(b, so.part, 1, c);
     const double rzn = cloth_sum(b, so.part, 2, c);
-    const bool lead = blk == b.cloth_blk0[c];
-    const bool conv = rr < pc.thr;
-    // every active cloth has completed exactly `it` iterations before this one
-    const bool cap = !conv && it + 1 >= pc.maxiter;
-    go_sh = !(conv || cap);
-    beta_sh = rzn / pc.rz[parity];
-    if (lead) {
-      pc.rr = rr;
-      pc.rz[parity ^ 1] = rzn;
-      pc.iters = conv ? it : it + 1;
-      if (conv || cap) pc.active = 0;
-      if (cap) pc.status |= 4;
+    if (threadIdx.x == 0) {
+      const bool lead = blk == b.cloth_blk0[c];
+      const bool conv = rr < pc.thr;
+      // every active cloth has completed exactly `it` iterations before this one
+      const bool cap = !conv && it + 1 >= pc.maxiter;
+      go_sh = !(conv || cap);
+      beta_sh = rzn / pc.rz[parity];
+      if (lead) {
+        pc.rr = rr;
+        pc.rz[parity ^ 1] = rzn;
+        pc.iters = conv ? it : it + 1;
+        if (conv || cap) pc.active = 0;
+        if (cap) pc.status |= 4;
+      }
     }
   }
   __syncthreads();
@@ -312,7 +318,7 @@ __global__ void __launch_bounds__(kBlock) k_pcg_dir(View v, Blocks b, Solver so,
   const int nt = v.ntot;
   if (threadIdx.x < b.blk_count[blk])
     for (int k = 0; k < 5; ++k)
-      st(so.p, k, nt, n) = ld(so.dinv, k, nt, n) * ld(so.r, k, nt, n) + beta * ld(so.p, k, nt, n);
+      st(so.p, k, nt, n) = fma(beta, ld(so.p, k, nt, n), ld(so.dinv, k, nt, n) * ld(so.r, k, nt, n));
 }
 
 __global__ void k_count_active(Solver so, int ncloth) {
@@ -393,7 +399,7 @@ void launch_rows(const View& v, const Records& R, const Solver& so, cudaStream_t
 }
 void launch_pcg_setup(const View& v, const Blocks& b, const Solver& so, cudaStream_t s) {
   k_pcg_setup<<<b.nblk, kBlock, 0, s>>>(v, b, so);
-  k_pcg_start<<<(v.ncloth + 127) / 128, 128, 0, s>>>(b, so, v.ncloth);
+  k_pcg_start<<<(v.ncloth + 3) / 4, 128, 0, s>>>(b, so, v.ncloth);
 }
 void launch_pcg_spmv(const View& v, const Blocks& b, const Solver& so, cudaStream_t s) {
   if (so.trans) k_pcg_spmv<true><<<b.nblk, kBlock, 0, s>>>(v, b, so);

@@ -19,6 +19,30 @@ struct PcgCloth {
   int status;       // bit 0: non-finite system, bit 1: non-finite solution, bit 2: iteration cap
 };
 
+// The PCG's arithmetic, written once for every schedule (the contraction is
+// spelled out, so the bits do not depend on what the compiler fuses).
+// z = D^-1 r of one component, and its terms of |r|^2 and r.z
+__device__ __forceinline__ double pcg_norms(double r, double dinv, double& rr, double& rz) {
+  const double z = dinv * r;
+  rr = fma(r, r, rr);
+  rz = fma(r, z, rz);
+  return z;
+}
+// the step along p
+__device__ __forceinline__ void pcg_advance(double alpha, double p, double q, double& x, double& r) {
+  x = fma(alpha, p, x);
+  r = fma(-alpha, q, r);
+}
+__device__ __forceinline__ double pcg_threshold(double tol, double bb) {
+  const double thr = tol * tol * bb;
+  return thr < 2.2250738585072014e-308 ? 2.2250738585072014e-308 : thr;
+}
+// sum over a warp, the same bits in every lane
+__device__ __forceinline__ double cloth_tree(double s) {
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
+}
+
 // thread-block partition of the nodes: blocks never straddle two cloths, so
 // per-cloth reductions are a fixed-order sum over a contiguous block range
 struct Blocks {
@@ -79,14 +103,21 @@ void launch_learned_verdict(const Solver& so, int ncloth, const int* err, int ca
                             cudaStream_t s);
 void launch_spmv(const View& v, const double* x, double* y, cudaStream_t s);
 
-// ---- persistent per-cloth PCG (ys_pcg_cluster.cu): one cluster of csize
-// CTAs of `threads` threads per listed cloth runs that cloth's whole solve
-// (set-up included) with at most `cap` iterations; a cloth needs
-// width * length <= threads * csize. Same results as the phase kernels above.
-bool pcg_cluster_shape_ok(int threads, int csize);
-// clusters of this shape that fit on the GPU at once (0: the shape cannot run)
-cudaError_t pcg_cluster_occupancy(int threads, int csize, int* clusters);
-cudaError_t launch_pcg_cluster(const View& v, const Solver& so, const int* cloths, int ncl, int threads, int csize,
+// ---- persistent per-cloth PCG (ys_pcg_cluster.cu): one cluster per listed
+// cloth runs that cloth's whole solve (set-up included) with at most `cap`
+// iterations. Same results as the phase kernels above.
+constexpr int kClusterMaxNodes = 4096;  // of a cloth
+constexpr int kClusterShared = (5 * kClusterMaxNodes + 10 * 256) * (int)sizeof(double);
+struct ClusterShape {
+  int groups;   // of 32 nodes in a CTA (0: a cloth of the batch does not fit, or the GPU cannot run any shape)
+  int csize;    // CTAs of a cluster
+  int shared;   // dynamic shared memory of a CTA
+  double cost;  // of an iteration, in units of a group's product
+  bool faster;  // than the phases
+};
+// the shape for these cloths (host array); enables its kernels, so outside any capture
+cudaError_t pcg_cluster_shape(const ClothParams* cp, int ncloth, int device, ClusterShape* out);
+cudaError_t launch_pcg_cluster(const View& v, const Solver& so, const int* cloths, int ncl, const ClusterShape& sh,
                                int cap, cudaStream_t s);
 
 // state tangents updated by the tangent step (layout [c][kTangents][ntot])

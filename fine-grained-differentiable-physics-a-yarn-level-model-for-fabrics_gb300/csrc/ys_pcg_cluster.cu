@@ -2,25 +2,34 @@
 // cluster runs one cloth's whole solve (set-up, every iteration, the stop
 // test) in a single launch.
 //
-// Each thread owns one node of its cloth (cloth-local index rank * T + tid):
-// its solution, residual and inverse diagonal stay in registers for the whole
-// solve, and its search direction sits in the CTA's shared memory, where the
-// other CTAs of the cluster read it through distributed shared memory when
-// their stencil reaches it. The system matrix is the only array streamed from
-// HBM per iteration. An iteration has three cluster barriers: after the p.q
-// partials, after the |r|^2 and r.z partials, and after the new direction.
+// A CTA owns `groups` groups of 32 consecutive nodes, a group has four warps:
+// warp m < 3 computes row m of the node's x rows, 45 of the row block's 159
+// coefficients, warp 3 the two Eulerian rows, 24. An SM issues one warp's
+// FP64 instruction over 64 cycles of one of its four pipes, so with a thread
+// per node a group's product took 159 x 64 cycles of one pipe while the other
+// three waited; split by rows the sums keep their order, so the bits are those
+// of a thread per node. Each warp keeps its rows' solution, residual and
+// inverse diagonal in registers for the whole solve (and, one group a CTA, its
+// coefficients).
+//
+// The direction sits in each CTA's shared memory for the CTA's own nodes and
+// the two cloth rows on either side that their stencils reach. z = D^-1 r is
+// what the CTAs exchange: it is published with the |r|^2 and r.z partials, and
+// after the sums every CTA forms p = z + beta p on its whole window, the same
+// bits for a node in every window it lies in. So an iteration has two cluster
+// barriers, after the p.q partials and after the others.
 //
 // The arithmetic is the batched PCG's (k_pcg_setup, k_pcg_spmv, k_pcg_axpy,
 // k_pcg_dir in ys_kernels.cu) term for term, and the dot products are summed
-// in its order: a warp shuffle tree per 32 nodes, the four warp sums of each
-// 128-node block in warp order, then the cloth's blocks in node order. So the
-// two schedules give the same bits, and both restate Eigen's
-// ConjugateGradient with its diagonal preconditioner (src/Solvers.cpp:3-31).
+// in its order: the components of a node chained, a warp shuffle tree per 32
+// nodes, the four group sums of each 128-node block in order, then the cloth's
+// blocks (cloth_tree). So the two schedules give the same bits, and both
+// restate Eigen's ConjugateGradient with its diagonal preconditioner
+// (src/Solvers.cpp:3-31).
 #include <cooperative_groups.h>
 
 #include <cfloat>
 #include <cstdint>
-#include <type_traits>
 
 #include "ys_items.cuh"
 #include "ys_kernels.cuh"
@@ -31,193 +40,252 @@ namespace ys {
 
 namespace {
 
-constexpr int kMaxClusterBlocks = 128;  // 128-node blocks per cloth (16 CTAs x 1024 threads)
+constexpr int kGroup = 32;         // nodes of a group
+constexpr int kMaxGroups = 8;      // groups of a CTA
+constexpr int kMaxCluster = 16;    // CTAs of a cluster
+constexpr int kRowCoefs = 45;      // coefficients of an x row; the Eulerian rows have 24
+constexpr int kMaxBlocks = kMaxCluster * kMaxGroups / 4;  // 128-node blocks of a cloth: one per lane
+static_assert(kMaxBlocks <= 32, "one block partial per lane");
+static_assert(kMaxCluster * kMaxGroups * kGroup == kClusterMaxNodes, "nodes of a cluster");
 
-// The cluster's direction vector: node li of the cloth at rank li / T, slot
-// li % T of that CTA's [5][T] slice. Handles are 32-bit shared::cluster
-// addresses (mapa), read with ld.shared::cluster; without a cluster, plain
-// shared-memory pointers.
-template <int T, bool CLUSTER>
-struct ClusterVec {
-  double* base;    // this CTA's [5][T] slice
-  uint32_t base32; // its shared::cta address
-  int off;         // the cloth's first node
-  typedef typename std::conditional<CLUSTER, uint32_t, const double*>::type Ptr;
-  __device__ __forceinline__ Ptr at(int j) const {
-    const int lj = j - off;
-    if constexpr (!CLUSTER) {
-      return base + lj;
-    } else {
-      const int rk = lj / T;
-      const uint32_t a = base32 + 8u * (uint32_t)(lj - rk * T);
-      uint32_t r;
-      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rk));
-      return r;
-    }
+// the window of a CTA: the nodes [lo, hi) of the cloth that the stencils of its
+// own nodes reach
+struct Window {
+  int lo, hi;
+  __host__ __device__ Window(int first, int nodes, int W, int N) {
+    lo = first - 2 * W > 0 ? first - 2 * W : 0;
+    hi = first + nodes + 2 * W < N ? first + nodes + 2 * W : N;
+    if (first >= N) lo = hi = N;  // a CTA without nodes
   }
-  __device__ __forceinline__ double get(Ptr p, int c) const {
-    if constexpr (!CLUSTER) {
-      return p[c * T];
-    } else {
-      double x;
-      asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(x) : "r"(p + 8u * (uint32_t)(c * T)));
-      return x;
-    }
-  }
+  __host__ __device__ int size() const { return hi - lo; }
 };
 
-// Sums NQ per-thread values over the cloth in the batched solver's order and
-// returns them in every thread. wp is this CTA's [NQ][T/32] warp-partial
-// buffer for this reduction (double-buffered by the caller); out is a shared
-// [NQ] broadcast slot.
-template <int T, bool CLUSTER, int NQ>
-__device__ __forceinline__ void cloth_reduce(double (&val)[NQ], double* wp, double* out, int nblk) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-  for (int q = 0; q < NQ; ++q) {
-    double s = val[q];
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if (lane == 0) wp[q * (T / 32) + wid] = s;
+// Coefficient j of row part m of row block n of A, or of A^T (TRANS: read from
+// the rows of the neighbours, 0 where there is none), in the order of
+// spmv_row_sv and spmv_row_tv. i(du, dv): the row to read for the neighbour
+// there, negative outside the cloth.
+template <bool TRANS, class Row>
+__device__ __forceinline__ double row_coef(const double* __restrict__ A, int64_t nt, int n, int m, int j,
+                                           const Row& i) {
+  auto at = [&](int slot, int row) { return row < 0 ? 0.0 : __ldg(A + (int64_t)slot * nt + row); };
+  auto nbr = [&](int mm) { return TRANS ? i(mm == 0 ? -1 : mm == 1 ? 1 : 0, mm == 2 ? -1 : mm == 3 ? 1 : 0) : n; };
+  if (m < 3) {
+    if (j < 39) {
+      const int s = j / 3, c = j - 3 * s;
+      return at(YS_SLOT_LL + 9 * s + (TRANS ? 3 * c + m : 3 * m + c), TRANS ? i(stencil_du(s), stencil_dv(s)) : n);
+    }
+    if (j < 41) return at(TRANS ? YS_SLOT_EL_SELF + 3 * (j - 39) + m : YS_SLOT_LE_SELF + 2 * m + (j - 39), n);
+    return at((TRANS ? YS_SLOT_EL_NBR : YS_SLOT_LE_NBR) + 3 * (j - 41) + m, nbr(j - 41));
   }
-  if (CLUSTER) cg::this_cluster().sync();
-  else __syncthreads();
-  if (wid == 0) {
-    // lane l forms the partials of blocks l, l + 32, ...: each the four warp
-    // sums of the block added to 0 in warp order (block_sum)
-    double bp[NQ][kMaxClusterBlocks / 32];
-#pragma unroll
-    for (int m = 0; m < kMaxClusterBlocks / 32; ++m) {
-      const int blk = lane + 32 * m;
-#pragma unroll
-      for (int q = 0; q < NQ; ++q) bp[q][m] = 0.0;
-      if (blk < nblk) {
-        const int g0 = 4 * blk;  // the block's first warp in the cloth
-        const int rk = g0 / (T / 32), lw = g0 - rk * (T / 32);
-        const double* src = CLUSTER ? cg::this_cluster().map_shared_rank(wp, rk) : wp;
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) {
-          double s = 0.0;
-#pragma unroll
-          for (int i = 0; i < 4; ++i) s += src[q * (T / 32) + lw + i];
-          bp[q][m] = s;
-        }
-      }
-    }
-    // the cloth sum: the block partials added to 0 in block order (cloth_sum)
-    double tot[NQ];
-#pragma unroll
-    for (int q = 0; q < NQ; ++q) tot[q] = 0.0;
-#pragma unroll
-    for (int m = 0; m < kMaxClusterBlocks / 32; ++m) {
-      const int cnt = min(32, nblk - 32 * m);  // <= 0 past the last block
-      for (int l = 0; l < cnt; ++l) {
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) tot[q] += __shfl_sync(0xffffffffu, bp[q][m], l);
-      }
-    }
-    if (lane == 0) {
-#pragma unroll
-      for (int q = 0; q < NQ; ++q) out[q] = tot[q];
-    }
-  }
-  __syncthreads();
-#pragma unroll
-  for (int q = 0; q < NQ; ++q) val[q] = out[q];
+  const int k = j / 12, e = j - 12 * k;
+  if (e < 3) return at(TRANS ? YS_SLOT_LE_SELF + 2 * e + k : YS_SLOT_EL_SELF + 3 * k + e, n);
+  if (e == 3) return at(YS_SLOT_EE_SELF + k, n);
+  const int mm = 2 * k + (e >= 8), c = (e - 4) & 3;
+  if (c < 3) return at((TRANS ? YS_SLOT_LE_NBR : YS_SLOT_EL_NBR) + 3 * mm + c, nbr(mm));
+  return at(YS_SLOT_EE_NBR + mm, nbr(mm));
 }
 
-template <int T, bool CLUSTER, bool TRANS>
-__global__ void __launch_bounds__(T, 1) k_pcg_cluster(View v, Solver so, const int* __restrict__ cloths, int cap) {
-  __shared__ double psm[5 * T];
-  __shared__ double wp[2][3 * (T / 32)];
-  __shared__ double bc[3];
+// y = the rows of part m times x: y[0] of x row m, y[0..1] of the two Eulerian
+// rows. coef(j): row_coef's; x(c, du, dv): component c of the neighbour there,
+// any finite number outside the cloth (the coefficient is 0).
+template <bool TRANS, class Coef, class Vec>
+__device__ __forceinline__ void row_product(int m, const Coef& coef, const Vec& x, double y[2]) {
+  constexpr int sg = TRANS ? -1 : 1;
+  if (m < 3) {
+    double s = 0.0;
+#pragma unroll
+    for (int t = 0; t < kNumStencil; ++t) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) s = fma(coef(3 * t + c), x(c, sg * stencil_du(t), sg * stencil_dv(t)), s);
+    }
+    s = fma(coef(39), x(3, 0, 0), s);
+    s = fma(coef(40), x(4, 0, 0), s);
+    s = fma(coef(41), x(3, -sg, 0), s);
+    s = fma(coef(42), x(3, sg, 0), s);
+    s = fma(coef(43), x(4, 0, -sg), s);
+    s = fma(coef(44), x(4, 0, sg), s);
+    y[0] = s;
+    y[1] = 0.0;
+  } else {
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int du = k == 0 ? sg : 0, dv = k == 0 ? 0 : sg, b = 12 * k;
+      double e = 0.0;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) e = fma(coef(b + c), x(c, 0, 0), e);
+      e = fma(coef(b + 3), x(3 + k, 0, 0), e);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) e = fma(coef(b + 4 + c), x(c, -du, -dv), e);
+      e = fma(coef(b + 7), x(3 + k, -du, -dv), e);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) e = fma(coef(b + 8 + c), x(c, du, dv), e);
+      e = fma(coef(b + 11), x(3 + k, du, dv), e);
+      y[k] = e;
+    }
+  }
+}
+
+// T: most threads a CTA (128 per group); HOLD: coefficients in registers
+template <int T, bool CLUSTER, bool TRANS, bool HOLD>
+__global__ void __launch_bounds__(T, T <= 256 ? 2 : 1) k_pcg_cluster(View v, Solver so, const int* __restrict__ cloths, int cap) {
+  extern __shared__ double dyn[];
+  __shared__ double gp[2][2][kMaxGroups];  // group partials of two dot products, alternating
+  __shared__ double out[2];
+  const int groups = blockDim.x / (4 * kGroup), own_nodes = groups * kGroup;
+  double* zs = dyn;                    // [5][own_nodes] z, read by the other CTAs
+  double* rs = dyn + 5 * own_nodes;    // [5][own_nodes] q, then r, for the dot products
+  double* sp = dyn + 10 * own_nodes;   // [5][window] direction
   const int csize = CLUSTER ? (int)cg::this_cluster().num_blocks() : 1;
   const int rank = CLUSTER ? (int)cg::this_cluster().block_rank() : 0;
   const int c = cloths[blockIdx.x / csize];
   PcgCloth& pc = so.pc[c];
   const ClothParams& P = v.cp[c];
-  const int N = P.W * P.H, off = P.node_off;
+  const int W = P.W, H = P.H, N = W * H, off = P.node_off, nt = v.ntot;
   const int nblk = (N + kBlock - 1) / kBlock;
-  const int li = rank * T + threadIdx.x;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, grp = wid >> 2;
+  const int m = (wid + grp) & 3;  // a group's light warp 3 on another pipe than the next group's
+  const int nc = m == 3 ? 2 : 1;
+  const int at = grp * kGroup + lane, li = rank * own_nodes + at;
   const bool own = li < N;
   const int n = off + (own ? li : 0);
-  const int nt = v.ntot;
-  const ClusterVec<T, CLUSTER> pv{psm, (uint32_t)__cvta_generic_to_shared(psm), off};
+  const int u = v.node_u[n], w = v.node_v[n];
+  const Window win(rank * own_nodes, own_nodes, W, N);
+  const int WN = win.size(), pos = own ? li - win.lo : 0;
   const int maxiter = pc.maxiter;
   const bool ok_sys = pc.status == 0;  // read before any CTA of the cluster can write it
-  int red = 0;  // reductions so far: selects the warp-partial buffer
-
-  // set-up (k_pcg_setup, k_pcg_start): x = 0, r = b, p = z = Dinv r. The
-  // solution and residual stay in registers; p lives in shared memory and the
-  // inverse diagonal is re-read (L1) where it is needed, which keeps the
-  // 1024-thread form within its 64 registers.
-  double x[5], r[5];
-  double rr = 0.0, rz = 0.0;
+  const double* __restrict__ A = v.A;
+  auto sync_all = [&] {
+    if (CLUSTER) cg::this_cluster().sync();
+    else __syncthreads();
+  };
+  auto has = [&](int du, int dv) { return u + du >= 0 && u + du < W && w + dv >= 0 && w + dv < H; };
+  // A^T: the row that refers to this node through (du, dv) lies opposite
+  auto row = [&](int du, int dv) { return has(-du, -dv) ? n - du - dv * W : -1; };
+  auto coef = [&](int j) { return row_coef<TRANS>(A, nt, n, m, j, row); };
+  auto x_at = [&](int k, int du, int dv) { return sp[k * WN + (has(du, dv) ? pos + du + dv * W : pos)]; };
+  // the chain over a node's components and the tree over the group's nodes;
+  // lane 0 keeps the group's partial
+  auto dot = [&](double (*slot)[kMaxGroups], int q, const double* a, int as, const double* b, int bs) {
+    double t = 0.0;
 #pragma unroll
-  for (int k = 0; k < 5; ++k) {
-    x[k] = 0.0;
-    r[k] = own ? ld(v.B, k, nt, n) : 0.0;
-    const double z = (own ? __ldg(so.dinv + (int64_t)k * nt + n) : 0.0) * r[k];
-    psm[k * T + threadIdx.x] = z;
-    rr += r[k] * r[k];
-    rz += r[k] * z;
+    for (int k = 0; k < 5; ++k) t = fma(a[k * as], b[k * bs], t);
+    if (!own) t = 0.0;
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+    if (lane == 0) slot[q][grp] = t;
+  };
+  // the cloth's sums of NQ partials in `slot`, to out: a block is four groups
+  auto total = [&](double (*slot)[kMaxGroups], int nq) {
+    if (wid == 0)
+      for (int q = 0; q < nq; ++q) {
+        double s = 0.0;
+        if (lane < nblk) {
+          double part[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int g = 4 * lane + i, rk = g / groups, lg = g - rk * groups;
+            const double* src = slot[q];
+            if (CLUSTER) src = cg::this_cluster().map_shared_rank(src, rk < csize ? rk : 0);
+            part[i] = rk < csize ? src[lg] : 0.0;
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i) s += part[i];
+        }
+        s = cloth_tree(s);
+        if (lane == 0) out[q] = s;
+      }
+    __syncthreads();
+  };
+
+  double held[HOLD ? kRowCoefs : 1];
+  if (HOLD && own) {
+#pragma unroll
+    for (int j = 0; j < kRowCoefs; ++j) held[j] = m < 3 || j < 24 ? coef(j) : 0.0;
   }
-  double s0[2] = {rr, rz};
-  cloth_reduce<T, CLUSTER, 2>(s0, wp[red++ & 1], bc, nblk);
-  const double bb = s0[0];
-  double thr = so.tol * so.tol * bb;
-  if (thr < DBL_MIN) thr = DBL_MIN;
-  double rzc = s0[1], rrc = bb;
+  // set-up (k_pcg_setup, k_pcg_start): x = 0, r = b, p = z = D^-1 r
+  double x[2] = {0.0, 0.0}, r[2] = {0.0, 0.0}, dinv[2] = {0.0, 0.0};
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    if (i >= nc) break;
+    if (own) {
+      r[i] = ld(v.B, m + i, nt, n);
+      dinv[i] = ld(so.dinv, m + i, nt, n);
+    }
+    rs[(m + i) * own_nodes + at] = r[i];
+    zs[(m + i) * own_nodes + at] = dinv[i] * r[i];
+  }
+  for (int e = threadIdx.x; e < WN; e += blockDim.x)
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+      const int64_t g = (int64_t)k * nt + off + win.lo + e;
+      sp[k * WN + e] = so.dinv[g] * v.B[g];
+    }
+  __syncthreads();
+  int red = 0;  // reductions so far: selects the partials' buffer
+  if (m == 0) dot(gp[0], 0, rs + at, own_nodes, rs + at, own_nodes);
+  if (m == 1) dot(gp[0], 1, rs + at, own_nodes, zs + at, own_nodes);
+  sync_all();
+  total(gp[red++ & 1], 2);
+  const double bb = out[0];
+  const double thr = pcg_threshold(so.tol, bb);
+  double rzc = out[1], rrc = bb;
   bool active = ok_sys && bb != 0.0 && bb >= thr;
   int iters = 0, capped = 0;
-  int it = 0;
-  for (; it < cap && active; ++it) {
+  for (int it = 0; it < cap && active; ++it) {
     // q = A p and p.q (k_pcg_spmv)
-    double q[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    double pq[1] = {0.0};
+    double q[2] = {0.0, 0.0};
     if (own) {
-      if (TRANS) spmv_row_tv(v, pv, n, q);
-      else spmv_row_sv(v, v.A, v.ntot, pv, n, q);
-#pragma unroll
-      for (int k = 0; k < 5; ++k) pq[0] += psm[k * T + threadIdx.x] * q[k];
+      if (HOLD) row_product<TRANS>(m, [&](int j) { return held[HOLD ? j : 0]; }, x_at, q);
+      else row_product<TRANS>(m, coef, x_at, q);
     }
-    cloth_reduce<T, CLUSTER, 1>(pq, wp[red++ & 1], bc, nblk);
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+      if (i < nc) rs[(m + i) * own_nodes + at] = q[i];
+    __syncthreads();
+    if (m == 3) dot(gp[red & 1], 0, sp + pos, WN, rs + at, own_nodes);
+    sync_all();
+    total(gp[red++ & 1], 1);
     // alpha, x += alpha p, r -= alpha q, |r|^2 and r.z (k_pcg_axpy)
-    const double alpha = rzc / pq[0];
-    double s1[2] = {0.0, 0.0};
-    if (own) {
+    const double alpha = rzc / out[0];
 #pragma unroll
-      for (int k = 0; k < 5; ++k) {
-        x[k] += alpha * psm[k * T + threadIdx.x];
-        const double rk = r[k] - alpha * q[k];
-        r[k] = rk;
-        s1[0] += rk * rk;
-        s1[1] += rk * (__ldg(so.dinv + (int64_t)k * nt + n) * rk);
-      }
+    for (int i = 0; i < 2; ++i) {
+      if (i >= nc) break;
+      if (own) pcg_advance(alpha, sp[(m + i) * WN + pos], q[i], x[i], r[i]);
+      rs[(m + i) * own_nodes + at] = r[i];
+      zs[(m + i) * own_nodes + at] = dinv[i] * r[i];
     }
-    cloth_reduce<T, CLUSTER, 2>(s1, wp[red++ & 1], bc, nblk);
+    __syncthreads();
+    if (m == 0) dot(gp[red & 1], 0, rs + at, own_nodes, rs + at, own_nodes);
+    if (m == 1) dot(gp[red & 1], 1, rs + at, own_nodes, zs + at, own_nodes);
+    sync_all();
+    total(gp[red++ & 1], 2);
     // the stop test, then beta and p = z + beta p (k_pcg_dir)
-    const bool conv = s1[0] < thr;
+    const double rrn = out[0], rzn = out[1];
+    const bool conv = rrn < thr;
     const bool cp = !conv && it + 1 >= maxiter;
-    const double beta = s1[1] / rzc;
-    rrc = s1[0];
-    rzc = s1[1];
+    const double beta = rzn / rzc;
+    rrc = rrn;
+    rzc = rzn;
     iters = conv ? it : it + 1;
     if (conv || cp) {
       active = false;
       capped = cp;
       break;
     }
-    if (own) {
+    for (int e = threadIdx.x; e < WN; e += blockDim.x) {
+      const int j = win.lo + e, rk = j / own_nodes;
+      const double* z = zs + (j - rk * own_nodes);
+      if (CLUSTER) z = cg::this_cluster().map_shared_rank(z, rk);
+      double zw[5];
 #pragma unroll
-      for (int k = 0; k < 5; ++k)
-        psm[k * T + threadIdx.x] = __ldg(so.dinv + (int64_t)k * nt + n) * r[k] + beta * psm[k * T + threadIdx.x];
+      for (int k = 0; k < 5; ++k) zw[k] = z[k * own_nodes];
+#pragma unroll
+      for (int k = 0; k < 5; ++k) sp[k * WN + e] = fma(beta, sp[k * WN + e], zw[k]);
     }
-    if (CLUSTER) cg::this_cluster().sync();
-    else __syncthreads();
+    __syncthreads();
   }
-  if (own)
 #pragma unroll
-    for (int k = 0; k < 5; ++k) st(so.x, k, nt, n) = x[k];
+  for (int i = 0; i < 2; ++i)
+    if (own && i < nc) st(so.x, m + i, nt, n) = x[i];
   if (rank == 0 && threadIdx.x == 0) {
     pc.bb = bb;
     pc.thr = thr;
@@ -232,87 +300,122 @@ __global__ void __launch_bounds__(T, 1) k_pcg_cluster(View v, Solver so, const i
   if (CLUSTER) cg::this_cluster().sync();
 }
 
-template <int T, bool CLUSTER, bool TRANS>
-cudaError_t launch_t(const View& v, const Solver& so, const int* cloths, int ncl, int csize, int cap, cudaStream_t s) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(ncl * csize));
-  cfg.blockDim = dim3(T);
-  cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = (unsigned)csize;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = CLUSTER ? 1 : 0;
-  // clusters above 8 CTAs were enabled by occupancy_t (ys_set_pcg_schedule)
-  return cudaLaunchKernelEx(&cfg, k_pcg_cluster<T, CLUSTER, TRANS>, v, so, cloths, cap);
+// calls f with the kernel that runs CTAs of up to `groups` groups
+template <class F>
+cudaError_t with_kernel(int groups, bool cluster, bool trans, F&& f) {
+#define YS_PCGC(TT, HOLD)                                                                                     \
+  if (groups * 4 * kGroup <= TT) {                                                                            \
+    if (cluster) return trans ? f(k_pcg_cluster<TT, true, true, HOLD>) : f(k_pcg_cluster<TT, true, false, HOLD>); \
+    return trans ? f(k_pcg_cluster<TT, false, true, HOLD>) : f(k_pcg_cluster<TT, false, false, HOLD>);        \
+  }
+  YS_PCGC(128, true)
+  YS_PCGC(256, false)
+  YS_PCGC(512, false)
+  YS_PCGC(1024, false)
+#undef YS_PCGC
+  return cudaErrorInvalidValue;
 }
 
-template <int T, bool CLUSTER>
-cudaError_t occupancy_t(int csize, int* clusters) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)csize);
-  cfg.blockDim = dim3(T);
-  cudaLaunchAttribute at[1];
+void config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at, const ClusterShape& sh, int ncl) {
+  cfg.gridDim = dim3((unsigned)(ncl * sh.csize));
+  cfg.blockDim = dim3((unsigned)(sh.groups * 4 * kGroup));
+  cfg.dynamicSmemBytes = sh.shared;
   at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = (unsigned)csize;
+  at[0].val.clusterDim.x = (unsigned)sh.csize;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
-  if (csize > 8) {
-    // both forms, before any launch (and outside any stream capture)
-    cudaError_t e = cudaFuncSetAttribute(k_pcg_cluster<T, CLUSTER, false>,
-                                         cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_pcg_cluster<T, CLUSTER, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e != cudaSuccess) return e;
-  }
-  return cudaOccupancyMaxActiveClusters(clusters, k_pcg_cluster<T, CLUSTER, false>, &cfg);
+  cfg.numAttrs = sh.csize > 1 ? 1 : 0;
 }
 
 }  // namespace
 
-bool pcg_cluster_shape_ok(int threads, int csize) {
-  if (threads != 128 && threads != 256 && threads != 512 && threads != 1024) return false;
-  if (csize != 1 && csize != 2 && csize != 4 && csize != 8 && csize != 16) return false;
-  return threads * csize <= kMaxClusterBlocks * kBlock;
-}
-
-cudaError_t pcg_cluster_occupancy(int threads, int csize, int* clusters) {
+// clusters of the shape that fit on the GPU at once; enables its kernels
+static cudaError_t cluster_fit(const ClusterShape& sh, int sms, int* clusters) {
   *clusters = 0;
-  if (!pcg_cluster_shape_ok(threads, csize)) return cudaErrorInvalidValue;
-  if (csize == 1) {
-    *clusters = 1;  // plain CTAs: one always fits
-    return cudaSuccess;
-  }
-  switch (threads) {
-    case 128: return occupancy_t<128, true>(csize, clusters);
-    case 256: return occupancy_t<256, true>(csize, clusters);
-    case 512: return occupancy_t<512, true>(csize, clusters);
-    default: return occupancy_t<1024, true>(csize, clusters);
-  }
+  cudaError_t e = cudaSuccess;
+  for (int trans = 0; trans < 2 && e == cudaSuccess; ++trans)
+    e = with_kernel(sh.groups, sh.csize > 1, trans != 0, [&](auto* k) {
+      cudaError_t r = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kClusterShared);
+      if (r == cudaSuccess && sh.csize > 8) r = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+      if (r != cudaSuccess) return r;
+      cudaLaunchConfig_t cfg = {};
+      cudaLaunchAttribute at[1] = {};
+      config(cfg, at, sh, 1);
+      int fit = 0;
+      if (sh.csize > 1) {
+        r = cudaOccupancyMaxActiveClusters(&fit, k, &cfg);
+      } else {
+        r = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, k, sh.groups * 4 * kGroup, sh.shared);
+        fit *= sms;
+      }
+      if (r == cudaSuccess) *clusters = trans == 0 || fit < *clusters ? fit : *clusters;
+      return r;
+    });
+  return e;
 }
 
-cudaError_t launch_pcg_cluster(const View& v, const Solver& so, const int* cloths, int ncl, int threads, int csize,
-                               int cap, cudaStream_t s) {
-  if (!pcg_cluster_shape_ok(threads, csize) || ncl <= 0) return cudaErrorInvalidValue;
-  const bool cl = csize > 1, tr = so.trans != 0;
-#define YS_PCGC(TT)                                                                              \
-  case TT:                                                                                       \
-    if (cl) return tr ? launch_t<TT, true, true>(v, so, cloths, ncl, csize, cap, s)              \
-                      : launch_t<TT, true, false>(v, so, cloths, ncl, csize, cap, s);            \
-    return tr ? launch_t<TT, false, true>(v, so, cloths, ncl, 1, cap, s)                         \
-              : launch_t<TT, false, false>(v, so, cloths, ncl, 1, cap, s);
-  switch (threads) {
-    YS_PCGC(128)
-    YS_PCGC(256)
-    YS_PCGC(512)
-    YS_PCGC(1024)
+// The groups of a CTA: more of them put a cloth on fewer SMs, which one cloth
+// wants least and a batch that fills the GPU most. An iteration takes about
+// groups + 2.5 times a group's product (two cluster barriers and the sums), and
+// the batch as many rounds of it as it has CTAs per SM, or as its clusters take
+// turns. Steps of 17 x 17 cloths with 1, 2, 3, 5, 8 groups, us (cost): one
+// cloth 352, 394, 447, 566, 738 (3.5 to 10.5); 24 cloths 587, 531, 473, 593, 766
+// (10.5, 9, 5.5, 7.5, 10.5); 64 cloths 1247, 950, 840, 705, 870 (24, 18, 11,
+// 7.5, 10.5); 256 cloths 4428, 3244, 3001, 2442, 3107 (94, 63, 38, 30, 42).
+//
+// And the schedule: 1.8 us a unit of cost, 2.4 where CTAs take turns, against
+// the phases' 20 us an iteration and 0.65 ns a node. Steps in a graph, us,
+// persistent / phases: 1 x 17 x 17 281 / 800, 24 of them 407 / 850, 64 654 /
+// 1033, 256 2409 / 2310, 1,024 8471 / 7379; 1 x 64 x 64 737 / 810; 8 x 50 x 50
+// 1143 / 1061, 64 of them 5872 / 3989.
+cudaError_t pcg_cluster_shape(const ClothParams* cp, int ncloth, int device, ClusterShape* out) {
+  ClusterShape best{};
+  *out = best;
+  int most = 0, sms = 0;
+  int64_t nodes = 0;
+  for (int c = 0; c < ncloth; ++c) {
+    const int n = cp[c].W * cp[c].H;
+    most = n > most ? n : most;
+    nodes += n;
   }
-#undef YS_PCGC
-  return cudaErrorInvalidValue;
+  if (most > kClusterMaxNodes) return cudaSuccess;
+  cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  if (e != cudaSuccess) return e;
+  const int all = (most + kGroup - 1) / kGroup;
+  for (int g = (all + kMaxCluster - 1) / kMaxCluster; g <= kMaxGroups; ++g) {
+    ClusterShape sh{g, 1, 0, 0.0, false};
+    while (sh.csize * g < all) sh.csize *= 2;
+    int win = 0, fit = 0;
+    for (int c = 0; c < ncloth; ++c)
+      for (int r = 0; r < sh.csize; ++r) {
+        const int z = Window(r * g * kGroup, g * kGroup, cp[c].W, cp[c].W * cp[c].H).size();
+        win = z > win ? z : win;
+      }
+    sh.shared = (10 * g * kGroup + 5 * win) * (int)sizeof(double);
+    if (cluster_fit(sh, sms, &fit) != cudaSuccess || fit < 1) {
+      cudaGetLastError();  // this GPU cannot run the shape
+      continue;
+    }
+    const int64_t ctas = (int64_t)ncloth * sh.csize, turns = (ctas + sms - 1) / sms, waves = (ncloth + fit - 1) / fit;
+    const int64_t rounds = turns > waves ? turns : waves;
+    sh.cost = (double)rounds * (g + 2.5);
+    sh.faster = (rounds > 1 ? 2.4 : 1.8) * sh.cost < 20.0 + 0.65e-3 * (double)nodes;
+    if (!best.groups || sh.cost < best.cost) best = sh;
+  }
+  *out = best;
+  return cudaSuccess;
+}
+
+cudaError_t launch_pcg_cluster(const View& v, const Solver& so, const int* cloths, int ncl, const ClusterShape& sh,
+                               int cap, cudaStream_t s) {
+  return with_kernel(sh.groups, sh.csize > 1, so.trans != 0, [&](auto* k) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1] = {};
+    config(cfg, at, sh, ncl);
+    cfg.stream = s;
+    return cudaLaunchKernelEx(&cfg, k, v, so, cloths, cap);
+  });
 }
 
 }  // namespace ys

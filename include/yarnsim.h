@@ -177,10 +177,13 @@ typedef struct ys_schedule {
  * same summation order, so they give bit-identical solutions:
  *  - phases: three launches per iteration over every 128-node block of the
  *    batch (SpMV, axpy, direction), convergence checked every check_every
- *    iterations (the default);
- *  - persistent: one launch for the whole solve, a cluster of pcg_cluster CTAs
- *    of pcg_threads threads per cloth, each thread owning one node; needs
- *    width * length <= pcg_threads * pcg_cluster for every cloth. */
+ *    iterations;
+ *  - persistent: one launch for the whole solve, a cluster of up to 16 CTAs
+ *    per cloth, four warps per 32 nodes; needs width * length <= pcg_threads *
+ *    pcg_cluster for every cloth. The split over CTAs follows from the cloths'
+ *    sizes and number, whatever shape is given; with a cloth of more than 4,096
+ *    nodes the phases run (and are faster).
+ * A batch starts with the one expected to be faster for its cloths. */
 enum { YS_PCG_PHASES = 0, YS_PCG_PERSISTENT = 1 };
 /* Selects the PCG schedule for every later solve of the batch (steps, tangent
  * and adjoint solves). YS_ERR_ARG if a cloth does not fit the persistent shape

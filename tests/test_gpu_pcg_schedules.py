@@ -1,0 +1,58 @@
+"""The persistent PCG and the default choice between it and the phases, at
+sizes where the cluster kernel's split can go wrong: one and several groups of
+32 nodes a CTA, one CTA and sixteen, windows cut by the cloth's ends (cloths
+3 crossings wide or high), the largest cloth a cluster holds and one more row,
+and batches whose small cloths leave CTAs without nodes. Every schedule sums
+in the same order, so the results are the same bits.
+"""
+import numpy as np
+import pytest
+
+from pkg import gpu_available, ys
+from test_gpu_pcg_persistent import _specs
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _need_gpu():
+    if not gpu_available():
+        pytest.skip("no CUDA device")
+
+
+def _run(sides, schedule, graphed, mode):
+    b = ys.ClothBatch(_specs(sides, 3))
+    if schedule == "phases":
+        b.set_pcg_schedule(False)
+    elif schedule == "persistent":
+        b.set_pcg_schedule(True, 1024, 16)
+    b.use_graphs(graphed)
+    N = b.total_nodes
+    ext = 1e-4 * np.random.default_rng(4).standard_normal((N, 5))
+    out, stats = [], []
+    for k in range(2):
+        st = b.step(1e-3, ext if k else None, tol=1e-10)
+        assert all(s["ok"] for s in st)
+        stats += [(s["cg_iterations"], s["cg_error"]) for s in st]
+        out += list(b.get_state().values())
+    if mode:  # a solve with A^T as well
+        rng = np.random.default_rng(5)
+        g = {k: rng.standard_normal((N, c)) for k, c in dict(LPos=3, LVel=3, EPos=2, EVel=2, EPosBar=2).items()}
+        adj = ys.Adjoint(b, "exact")
+        gs, gp, _ = adj.step_back(1e-3, g, None, tol=1e-10)
+        adj.close()
+        out += list(gs.values()) + list(gp.values())
+    b.close()
+    return out, stats
+
+
+@pytest.mark.parametrize("sides", [[(3, 3)], [(3, 11), (4, 8)], [(3, 171)], [(170, 3)], [(23, 22)], [(33, 31), (3, 3)],
+                                   [(64, 64)], [(64, 65)], [(17, 17)] * 24, [(41, 41)] + [(7, 9)] * 20])
+@pytest.mark.parametrize("graphed", [False, True])
+def test_schedules_give_the_same_bits(sides, graphed):
+    ref, it = _run(sides, "phases", False, not graphed)
+    for schedule in ("persistent", "default"):
+        got, n = _run(sides, schedule, graphed, not graphed)
+        assert n == it, schedule
+        for a, c in zip(ref, got):
+            assert np.array_equal(a, c), schedule
