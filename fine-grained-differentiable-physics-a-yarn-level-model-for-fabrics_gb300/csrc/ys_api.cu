@@ -359,6 +359,9 @@ ys_status plan_pcg(ys_batch* b) {
                    [&](int x, int y) { return b->cp[x].W * b->cp[x].H > b->cp[y].W * b->cp[y].H; });
   YS_CUDA(cudaMemcpy(P.order, ord.data(), sizeof(int) * b->ncloth, cudaMemcpyHostToDevice));
   P.max_nodes = b->cp[ord[0]].W * b->cp[ord[0]].H;
+  int sms = 0;
+  YS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device));
+  b->blk.by_rows = b->blk.nblk <= 2 * sms;
   YS_CUDA(ys::pcg_cluster_shape(b->cp.data(), b->ncloth, b->device, &P.shape));
   if (P.shape.faster) P.kind = YS_PCG_PERSISTENT;
   return YS_OK;
@@ -504,7 +507,7 @@ ys_status ys_batch_create(int32_t n_cloths, const ys_cloth_desc* descs, int32_t 
     b->so.x = b->vecs; b->so.r = b->vecs + 5 * nt; b->so.p = b->vecs + 10 * nt;
     b->so.q = b->vecs + 15 * nt; b->so.dinv = b->vecs + 20 * nt;
   }
-  A(&b->so.part, 4 * blk_cloth.size()); A(&b->so.pc, n_cloths); A(&b->so.nactive, 1);
+  A(&b->so.part, 8 * blk_cloth.size()); A(&b->so.pc, n_cloths); A(&b->so.nactive, 1);
   A(&b->stage, 15 * nt); A(&b->ext, 5 * nt); A(&b->plan.order, n_cloths);
   if (st != YS_OK) { delete b; return st; }
   if (cudaMallocHost(&b->h_nactive, sizeof(int)) != cudaSuccess ||

@@ -7,7 +7,7 @@
 #include <cmath>
 
 #include "ys_gnn.cuh"
-#include "ys_items.cuh"
+#include "ys_pcg.cuh"
 #include "ys_tc.cuh"
 
 namespace ys {
@@ -681,16 +681,8 @@ __device__ __forceinline__ double blk_sum(double val, double* sh) {
     for (int i = 0; i < (int)(blockDim.x >> 5); ++i) s += sh[i];
   return s;
 }
-__device__ __forceinline__ double cl_sum(const Blocks& b, const double* part, int which, int c) {
-  const int b0 = b.cloth_blk0[c], nb = b.cloth_nblk[c];
-  double s = 0.0;
-  for (int i = 0; i < nb; ++i) s += part[which * b.nblk + b0 + i];
-  return s;
-}
-
 // alpha = r.z / p.q; x += alpha p; r -= alpha q (setup: x = 0, r = b); the
-// FP32 copy of r the preconditioner reads; partial |r|^2 (row 1; setup also
-// |b|^2, row 0)
+// FP32 copy of r the preconditioner reads; partial |r|^2 (row 1)
 __global__ void __launch_bounds__(kBlock) k_lp_axpy(View v, Blocks b, Solver so, LpcgExtra lx, int parity,
                                                      int setup) {
   __shared__ double sh[kBlock / 32];
@@ -710,7 +702,10 @@ __global__ void __launch_bounds__(kBlock) k_lp_axpy(View v, Blocks b, Solver so,
       q[k] = setup ? 0.0 : ld(so.q, k, nt, n);
       p[k] = setup ? 0.0 : ld(so.p, k, nt, n);
     }
-  if (threadIdx.x == 0) alpha_sh = setup ? 0.0 : so.pc[c].rz[parity] / cl_sum(b, so.part, 0, c);
+  if (threadIdx.x < 32) {
+    const double pq = setup ? 0.0 : cloth_sum_pq(b, so.part, c);
+    if (threadIdx.x == 0) alpha_sh = setup ? 0.0 : so.pc[c].rz[parity] / pq;
+  }
   __syncthreads();
   const double alpha = alpha_sh;
   double rr = 0.0;
@@ -725,10 +720,7 @@ __global__ void __launch_bounds__(kBlock) k_lp_axpy(View v, Blocks b, Solver so,
       rr += rn * rn;
     }
   const double s1 = blk_sum(rr, sh);
-  if (threadIdx.x == 0) {
-    so.part[1 * b.nblk + blk] = s1;
-    if (setup) so.part[0 * b.nblk + blk] = s1;
-  }
+  if (threadIdx.x == 0) so.part[1 * b.nblk + blk] = s1;
 }
 
 // z = G^T G r (FP32 r, BF16 G, FP32 sums). Block b of row i couples node
@@ -822,13 +814,14 @@ __global__ void __launch_bounds__(kBlock, 6) k_lp_prec(View v, Blocks b, Solver 
   }
 }
 
+// one warp per cloth
 __global__ void k_lp_start(Blocks b, Solver so, int ncloth) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (c >= ncloth) return;
   PcgCloth& pc = so.pc[c];
-  const double bb = cl_sum(b, so.part, 0, c);
-  const double rr = cl_sum(b, so.part, 1, c);
-  const double rz = cl_sum(b, so.part, 2, c);
+  const double rr = cloth_sum(b, so.part, 1, c), bb = rr;  // r = b
+  const double rz = cloth_sum(b, so.part, 2, c);
+  if (threadIdx.x & 31) return;
   pc.bb = bb;
   double thr = so.tol * so.tol * bb;
   if (thr < DBL_MIN) thr = DBL_MIN;
@@ -852,8 +845,8 @@ __global__ void __launch_bounds__(kBlock) k_lp_dir(View v, Blocks b, Solver so, 
   const int c = b.blk_cloth[blk];
   PcgCloth& pc = so.pc[c];
   if (!pc.active) return;
-  // the four cloth sums (p.q, |r|^2, r.z, z.q), each in block order, in four
-  // lanes at once; the direction's operands load meanwhile
+  // the four cloth sums (p.q, |r|^2, r.z, z.q) in four warps at once; the
+  // direction's operands load meanwhile
   const int n = b.blk_node0[blk] + threadIdx.x;
   const int nt = v.ntot;
   const bool own = threadIdx.x < b.blk_count[blk];
@@ -864,7 +857,10 @@ __global__ void __launch_bounds__(kBlock) k_lp_dir(View v, Blocks b, Solver so, 
       zk[k] = lx.z[(int64_t)k * nt + n];
       pk[k] = ld(so.p, k, nt, n);
     }
-  if (threadIdx.x < 4) sums_sh[threadIdx.x] = cl_sum(b, so.part, threadIdx.x, c);
+  static_assert(kBlock == 128, "a warp per sum");
+  const int wid = threadIdx.x >> 5;
+  const double sum = wid == 0 ? cloth_sum_pq(b, so.part, c) : cloth_sum(b, so.part, wid, c);
+  if ((threadIdx.x & 31) == 0) sums_sh[wid] = sum;
   __syncthreads();
   if (threadIdx.x == 0) {
     const int it = so.it_base ? *so.it_base + it_local : it_local;
@@ -1453,7 +1449,7 @@ void gnn_adam(const GnnNet& net, const GnnBufs& g, float* m, float* vv, float lr
 void lpcg_setup(const View& v, const Blocks& b, const Solver& so, const LpcgExtra& lx, cudaStream_t s) {
   k_lp_axpy<<<b.nblk, kBlock, 0, s>>>(v, b, so, lx, 0, 1);
   k_lp_prec<<<b.nblk, kBlock, 0, s>>>(v, b, so, lx, 1);
-  k_lp_start<<<(v.ncloth + 127) / 128, 128, 0, s>>>(b, so, v.ncloth);
+  k_lp_start<<<(v.ncloth + 3) / 4, 128, 0, s>>>(b, so, v.ncloth);
 }
 
 void lpcg_axpy(const View& v, const Blocks& b, const Solver& so, const LpcgExtra& lx, int parity, cudaStream_t s) {

@@ -10,8 +10,7 @@
 // blocks' partials, recomputed redundantly by every block that needs them.
 #include <cfloat>
 
-#include "ys_items.cuh"
-#include "ys_kernels.cuh"
+#include "ys_pcg.cuh"
 
 namespace ys {
 
@@ -161,6 +160,7 @@ __global__ void __launch_bounds__(4 * kNodesPerBlock) k_rows(View v, Records R, 
 }
 
 // ----------------------------------------------------------------- solve
+// sum over the block in thread 0: a tree per warp, the warps in order
 __device__ __forceinline__ double block_sum(double val, double* sh) {
   for (int o = 16; o > 0; o >>= 1) val += __shfl_down_sync(0xffffffffu, val, o);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -173,19 +173,17 @@ __device__ __forceinline__ double block_sum(double val, double* sh) {
   return s;  // valid in thread 0
 }
 
-// fixed-order sum of cloth c's block partials in row `which`, by a whole warp:
-// lane l adds blocks l, l + 32, ... in order, then the lanes as a tree. (One
-// thread adding them all waited out an FP64 addition per block, up to 79 of
-// them on a 100 x 100 cloth, in every block of every launch.)
-__device__ __forceinline__ double cloth_sum(const Blocks& b, const double* part, int which, int c) {
-  const int b0 = b.cloth_blk0[c], nb = b.cloth_nblk[c];
-  double s = 0.0;
-  for (int i = threadIdx.x & 31; i < nb; i += 32) s += part[which * b.nblk + b0 + i];
-  return cloth_tree(s);
+// In a batch that leaves SMs idle (by_rows) a thread's vectors are loaded
+// together, before the cloth sum: the loads of one component cannot pass the
+// stores of the one before. In one that fills them the registers this takes
+// cost more warps than it hides: k_pcg_axpy 28 us for 23 on 255,292 nodes.
+__device__ __forceinline__ void load5(const double* p, int64_t nt, int n, bool own, double (&x)[5]) {
+#pragma unroll
+  for (int k = 0; k < 5; ++k) x[k] = own ? p[k * nt + n] : 0.0;
 }
 
-// x = 0, r = b, p = z = Dinv r; partials |b|^2 (row 0), |r|^2 (row 1) and
-// r.z (row 2)
+// x = 0, r = b, p = z = Dinv r; partials |r|^2 (row 1, and |b|^2)
+// and r.z (row 2)
 __global__ void __launch_bounds__(kBlock) k_pcg_setup(View v, Blocks b, Solver so) {
   __shared__ double sh[kBlock / 32];
   const int blk = blockIdx.x;
@@ -201,10 +199,7 @@ __global__ void __launch_bounds__(kBlock) k_pcg_setup(View v, Blocks b, Solver s
     }
   }
   double s1 = block_sum(rr, sh);
-  if (threadIdx.x == 0) {
-    so.part[0 * b.nblk + blk] = s1;  // r = b here
-    so.part[1 * b.nblk + blk] = s1;
-  }
+  if (threadIdx.x == 0) so.part[1 * b.nblk + blk] = s1;
   double s2 = block_sum(rz, sh);
   if (threadIdx.x == 0) so.part[2 * b.nblk + blk] = s2;
 }
@@ -214,8 +209,7 @@ __global__ void k_pcg_start(Blocks b, Solver so, int ncloth) {
   const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (c >= ncloth) return;
   PcgCloth& pc = so.pc[c];
-  const double bb = cloth_sum(b, so.part, 0, c);
-  const double rr = cloth_sum(b, so.part, 1, c);
+  const double rr = cloth_sum(b, so.part, 1, c), bb = rr;  // r = b
   const double rz = cloth_sum(b, so.part, 2, c);
   if (threadIdx.x & 31) return;
   pc.bb = bb;
@@ -227,7 +221,7 @@ __global__ void k_pcg_start(Blocks b, Solver so, int ncloth) {
   pc.active = (pc.status == 0 && bb != 0.0 && rr >= thr) ? 1 : 0;
 }
 
-// q = A p and partial p.q (row 0)
+// q = A p and partial p.q (row 0), a thread per node
 template <bool TRANS>
 __global__ void __launch_bounds__(kBlock) k_pcg_spmv(View v, Blocks b, Solver so) {
   __shared__ double sh[kBlock / 32];
@@ -248,6 +242,47 @@ __global__ void __launch_bounds__(kBlock) k_pcg_spmv(View v, Blocks b, Solver so
   }
   const double s = block_sum(pq, sh);
   if (threadIdx.x == 0) so.part[0 * b.nblk + blk] = s;
+}
+
+// The same for batches that leave SMs idle with a thread per node (b.by_rows):
+// a group of 32 nodes a block, a warp per part of their rows, the groups'
+// partials of p.q. The light part 3 takes turns over the SM's four FP64 pipes.
+// Measured, us for 32 products (events): one 17 x 17 cloth 361 for 468, one
+// 100 x 100 384 for 502, four 592 for 674 (316 blocks of 128 nodes), 96 of 17 x
+// 17 512 for 514 (288), 64 of 40 x 40 1596 for 1151 (832): three warps read
+// each x where one did. Hence the line at two blocks an SM.
+template <bool TRANS>
+__global__ void __launch_bounds__(4 * kGroup) k_pcg_spmv_rows(View v, Blocks b, Solver so) {
+  __shared__ double sq[5][kGroup];
+  const int blk = blockIdx.x >> 2, first = kGroup * (blockIdx.x & 3);
+  if (!so.pc[b.blk_cloth[blk]].active) return;
+  const int lane = threadIdx.x & 31, m = ((threadIdx.x >> 5) + blockIdx.x) & 3;
+  const bool own = first + lane < b.blk_count[blk];
+  const int nt = v.ntot, n = own ? b.blk_node0[blk] + first + lane : b.blk_node0[blk];
+  const ClothParams& P = v.cp[v.node_cloth[n]];
+  const int W = P.W, H = P.H, u = v.node_u[n], w = v.node_v[n];
+  auto has = [&](int du, int dv) { return u + du >= 0 && u + du < W && w + dv >= 0 && w + dv < H; };
+  auto row = [&](int du, int dv) { return has(-du, -dv) ? n - du - dv * W : -1; };
+  const double* __restrict__ A = v.A;
+  const double* __restrict__ x = so.p;
+  double q[2] = {0.0, 0.0};
+  if (own) {
+    row_product<TRANS>(
+        m, [&](int j) { return row_coef<TRANS>(A, nt, n, m, j, row); },
+        [&](int k, int du, int dv) { return __ldg(x + (int64_t)k * nt + (has(du, dv) ? n + du + dv * W : n)); }, q);
+    st(so.q, m, nt, n) = q[0];
+    if (m == 3) st(so.q, 4, nt, n) = q[1];
+  }
+  sq[m][lane] = q[0];
+  if (m == 3) sq[4][lane] = q[1];
+  __syncthreads();
+  if (m != 3) return;
+  double t = 0.0;
+  if (own)
+#pragma unroll
+    for (int k = 0; k < 5; ++k) t = fma(__ldg(x + (int64_t)k * nt + n), sq[k][lane], t);
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+  if (lane == 0) so.part[pq_row(b) + blockIdx.x] = t;
 }
 
 // alpha = rz / pq; x += alpha p; r -= alpha q; partials |r|^2 (row 1), r.z (row 2)
@@ -281,9 +316,44 @@ __global__ void __launch_bounds__(kBlock) k_pcg_axpy(View v, Blocks b, Solver so
   if (threadIdx.x == 0) so.part[2 * b.nblk + blk] = s2;
 }
 
+// The same where batches leave SMs idle (by_rows)
+__global__ void __launch_bounds__(kBlock) k_pcg_axpy_early(View v, Blocks b, Solver so, int parity) {
+  __shared__ double sh[kBlock / 32];
+  __shared__ double alpha_sh;
+  const int blk = blockIdx.x, c = b.blk_cloth[blk], nt = v.ntot;
+  if (!so.pc[c].active) return;
+  const bool own = threadIdx.x < b.blk_count[blk];
+  const int n = b.blk_node0[blk] + threadIdx.x;
+  double x[5], r[5], p[5], q[5], dinv[5], dot[2] = {0.0, 0.0};
+  load5(so.q, nt, n, own, q);
+  load5(so.r, nt, n, own, r);
+  load5(so.dinv, nt, n, own, dinv);
+  load5(so.p, nt, n, own, p);
+  load5(so.x, nt, n, own, x);
+  if (threadIdx.x < 32) {
+    const double pq = cloth_sum_pq(b, so.part, c);
+    if (threadIdx.x == 0) alpha_sh = so.pc[c].rz[parity] / pq;
+  }
+  __syncthreads();
+  const double alpha = alpha_sh;
+  if (own)
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+      pcg_advance(alpha, p[k], q[k], x[k], r[k]);
+      st(so.x, k, nt, n) = x[k];
+      st(so.r, k, nt, n) = r[k];
+      pcg_norms(r[k], dinv[k], dot[0], dot[1]);
+    }
+  const double s1 = block_sum(dot[0], sh);
+  if (threadIdx.x == 0) so.part[1 * b.nblk + blk] = s1;
+  const double s2 = block_sum(dot[1], sh);
+  if (threadIdx.x == 0) so.part[2 * b.nblk + blk] = s2;
+}
+
 // stop test |r|^2 < thr, else beta = rz_new / rz and p = z + beta p. Every
 // block of a cloth reaches the same decision from the same fixed-order sums;
 // only the cloth's first block writes the cloth's bookkeeping.
+template <bool EARLY>
 __global__ void __launch_bounds__(kBlock) k_pcg_dir(View v, Blocks b, Solver so, int parity, int it_local) {
   __shared__ int go_sh;
   const int it = so.it_base ? *so.it_base + it_local : it_local;
@@ -292,6 +362,15 @@ __global__ void __launch_bounds__(kBlock) k_pcg_dir(View v, Blocks b, Solver so,
   const int c = b.blk_cloth[blk];
   PcgCloth& pc = so.pc[c];
   if (!pc.active) return;
+  const bool own = threadIdx.x < b.blk_count[blk];
+  const int n = b.blk_node0[blk] + threadIdx.x, nt = v.ntot;
+  double r[5], dinv[5], p[5];
+  auto load = [&] {
+    load5(so.r, nt, n, own, r);
+    load5(so.dinv, nt, n, own, dinv);
+    load5(so.p, nt, n, own, p);
+  };
+  if (EARLY) load();
   if (threadIdx.x < 32) {
     const double rr = cloth_sum(b, so.part, 1, c);
     const double rzn = cloth_sum(b, so.part, 2, c);
@@ -313,12 +392,11 @@ __global__ void __launch_bounds__(kBlock) k_pcg_dir(View v, Blocks b, Solver so,
   }
   __syncthreads();
   if (!go_sh) return;
+  if (!EARLY) load();
   const double beta = beta_sh;
-  const int n = b.blk_node0[blk] + threadIdx.x;
-  const int nt = v.ntot;
-  if (threadIdx.x < b.blk_count[blk])
-    for (int k = 0; k < 5; ++k)
-      st(so.p, k, nt, n) = fma(beta, ld(so.p, k, nt, n), ld(so.dinv, k, nt, n) * ld(so.r, k, nt, n));
+  if (own)
+#pragma unroll
+    for (int k = 0; k < 5; ++k) st(so.p, k, nt, n) = fma(beta, p[k], dinv[k] * r[k]);
 }
 
 __global__ void k_count_active(Solver so, int ncloth) {
@@ -402,14 +480,21 @@ void launch_pcg_setup(const View& v, const Blocks& b, const Solver& so, cudaStre
   k_pcg_start<<<(v.ncloth + 3) / 4, 128, 0, s>>>(b, so, v.ncloth);
 }
 void launch_pcg_spmv(const View& v, const Blocks& b, const Solver& so, cudaStream_t s) {
-  if (so.trans) k_pcg_spmv<true><<<b.nblk, kBlock, 0, s>>>(v, b, so);
-  else k_pcg_spmv<false><<<b.nblk, kBlock, 0, s>>>(v, b, so);
+  if (b.by_rows) {
+    if (so.trans) k_pcg_spmv_rows<true><<<4 * b.nblk, 4 * kGroup, 0, s>>>(v, b, so);
+    else k_pcg_spmv_rows<false><<<4 * b.nblk, 4 * kGroup, 0, s>>>(v, b, so);
+  } else {
+    if (so.trans) k_pcg_spmv<true><<<b.nblk, kBlock, 0, s>>>(v, b, so);
+    else k_pcg_spmv<false><<<b.nblk, kBlock, 0, s>>>(v, b, so);
+  }
 }
 void launch_pcg_axpy(const View& v, const Blocks& b, const Solver& so, int it, cudaStream_t s) {
-  k_pcg_axpy<<<b.nblk, kBlock, 0, s>>>(v, b, so, it & 1);
+  if (b.by_rows) k_pcg_axpy_early<<<b.nblk, kBlock, 0, s>>>(v, b, so, it & 1);
+  else k_pcg_axpy<<<b.nblk, kBlock, 0, s>>>(v, b, so, it & 1);
 }
 void launch_pcg_dir(const View& v, const Blocks& b, const Solver& so, int it, cudaStream_t s) {
-  k_pcg_dir<<<b.nblk, kBlock, 0, s>>>(v, b, so, it & 1, it);
+  if (b.by_rows) k_pcg_dir<true><<<b.nblk, kBlock, 0, s>>>(v, b, so, it & 1, it);
+  else k_pcg_dir<false><<<b.nblk, kBlock, 0, s>>>(v, b, so, it & 1, it);
 }
 void launch_count_active(const View& v, const Solver& so, cudaStream_t s) {
   k_count_active<<<1, 256, 0, s>>>(so, v.ncloth);

@@ -19,24 +19,6 @@ struct PcgCloth {
   int status;       // bit 0: non-finite system, bit 1: non-finite solution, bit 2: iteration cap
 };
 
-// The PCG's arithmetic, written once for every schedule (the contraction is
-// spelled out, so the bits do not depend on what the compiler fuses).
-// z = D^-1 r of one component, and its terms of |r|^2 and r.z
-__device__ __forceinline__ double pcg_norms(double r, double dinv, double& rr, double& rz) {
-  const double z = dinv * r;
-  rr = fma(r, r, rr);
-  rz = fma(r, z, rz);
-  return z;
-}
-// the step along p
-__device__ __forceinline__ void pcg_advance(double alpha, double p, double q, double& x, double& r) {
-  x = fma(alpha, p, x);
-  r = fma(-alpha, q, r);
-}
-__device__ __forceinline__ double pcg_threshold(double tol, double bb) {
-  const double thr = tol * tol * bb;
-  return thr < 2.2250738585072014e-308 ? 2.2250738585072014e-308 : thr;
-}
 // sum over a warp, the same bits in every lane
 __device__ __forceinline__ double cloth_tree(double s) {
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
@@ -52,6 +34,7 @@ struct Blocks {
   const int* blk_count;   // [nblk] nodes in the block
   const int* cloth_blk0;  // [ncloth] first block
   const int* cloth_nblk;  // [ncloth]
+  bool by_rows;           // products by four warps per 32 nodes (k_pcg_spmv_rows)
 };
 
 struct Solver {
@@ -60,7 +43,7 @@ struct Solver {
   double* p;      // [5][ntot]
   double* q;      // [5][ntot]
   double* dinv;   // [5][ntot]
-  double* part;   // [3][nblk] block partial sums
+  double* part;   // [4][nblk] block partial sums, then [nblk][4] group partials of p.q
   PcgCloth* pc;   // [ncloth]
   int* nactive;   // device counter
   double tol;

@@ -31,8 +31,7 @@
 #include <cfloat>
 #include <cstdint>
 
-#include "ys_items.cuh"
-#include "ys_kernels.cuh"
+#include "ys_pcg.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -40,10 +39,8 @@ namespace ys {
 
 namespace {
 
-constexpr int kGroup = 32;         // nodes of a group
 constexpr int kMaxGroups = 8;      // groups of a CTA
 constexpr int kMaxCluster = 16;    // CTAs of a cluster
-constexpr int kRowCoefs = 45;      // coefficients of an x row; the Eulerian rows have 24
 constexpr int kMaxBlocks = kMaxCluster * kMaxGroups / 4;  // 128-node blocks of a cloth: one per lane
 static_assert(kMaxBlocks <= 32, "one block partial per lane");
 static_assert(kMaxCluster * kMaxGroups * kGroup == kClusterMaxNodes, "nodes of a cluster");
@@ -59,71 +56,6 @@ struct Window {
   }
   __host__ __device__ int size() const { return hi - lo; }
 };
-
-// Coefficient j of row part m of row block n of A, or of A^T (TRANS: read from
-// the rows of the neighbours, 0 where there is none), in the order of
-// spmv_row_sv and spmv_row_tv. i(du, dv): the row to read for the neighbour
-// there, negative outside the cloth.
-template <bool TRANS, class Row>
-__device__ __forceinline__ double row_coef(const double* __restrict__ A, int64_t nt, int n, int m, int j,
-                                           const Row& i) {
-  auto at = [&](int slot, int row) { return row < 0 ? 0.0 : __ldg(A + (int64_t)slot * nt + row); };
-  auto nbr = [&](int mm) { return TRANS ? i(mm == 0 ? -1 : mm == 1 ? 1 : 0, mm == 2 ? -1 : mm == 3 ? 1 : 0) : n; };
-  if (m < 3) {
-    if (j < 39) {
-      const int s = j / 3, c = j - 3 * s;
-      return at(YS_SLOT_LL + 9 * s + (TRANS ? 3 * c + m : 3 * m + c), TRANS ? i(stencil_du(s), stencil_dv(s)) : n);
-    }
-    if (j < 41) return at(TRANS ? YS_SLOT_EL_SELF + 3 * (j - 39) + m : YS_SLOT_LE_SELF + 2 * m + (j - 39), n);
-    return at((TRANS ? YS_SLOT_EL_NBR : YS_SLOT_LE_NBR) + 3 * (j - 41) + m, nbr(j - 41));
-  }
-  const int k = j / 12, e = j - 12 * k;
-  if (e < 3) return at(TRANS ? YS_SLOT_LE_SELF + 2 * e + k : YS_SLOT_EL_SELF + 3 * k + e, n);
-  if (e == 3) return at(YS_SLOT_EE_SELF + k, n);
-  const int mm = 2 * k + (e >= 8), c = (e - 4) & 3;
-  if (c < 3) return at((TRANS ? YS_SLOT_LE_NBR : YS_SLOT_EL_NBR) + 3 * mm + c, nbr(mm));
-  return at(YS_SLOT_EE_NBR + mm, nbr(mm));
-}
-
-// y = the rows of part m times x: y[0] of x row m, y[0..1] of the two Eulerian
-// rows. coef(j): row_coef's; x(c, du, dv): component c of the neighbour there,
-// any finite number outside the cloth (the coefficient is 0).
-template <bool TRANS, class Coef, class Vec>
-__device__ __forceinline__ void row_product(int m, const Coef& coef, const Vec& x, double y[2]) {
-  constexpr int sg = TRANS ? -1 : 1;
-  if (m < 3) {
-    double s = 0.0;
-#pragma unroll
-    for (int t = 0; t < kNumStencil; ++t) {
-#pragma unroll
-      for (int c = 0; c < 3; ++c) s = fma(coef(3 * t + c), x(c, sg * stencil_du(t), sg * stencil_dv(t)), s);
-    }
-    s = fma(coef(39), x(3, 0, 0), s);
-    s = fma(coef(40), x(4, 0, 0), s);
-    s = fma(coef(41), x(3, -sg, 0), s);
-    s = fma(coef(42), x(3, sg, 0), s);
-    s = fma(coef(43), x(4, 0, -sg), s);
-    s = fma(coef(44), x(4, 0, sg), s);
-    y[0] = s;
-    y[1] = 0.0;
-  } else {
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const int du = k == 0 ? sg : 0, dv = k == 0 ? 0 : sg, b = 12 * k;
-      double e = 0.0;
-#pragma unroll
-      for (int c = 0; c < 3; ++c) e = fma(coef(b + c), x(c, 0, 0), e);
-      e = fma(coef(b + 3), x(3 + k, 0, 0), e);
-#pragma unroll
-      for (int c = 0; c < 3; ++c) e = fma(coef(b + 4 + c), x(c, -du, -dv), e);
-      e = fma(coef(b + 7), x(3 + k, -du, -dv), e);
-#pragma unroll
-      for (int c = 0; c < 3; ++c) e = fma(coef(b + 8 + c), x(c, du, dv), e);
-      e = fma(coef(b + 11), x(3 + k, du, dv), e);
-      y[k] = e;
-    }
-  }
-}
 
 // T: most threads a CTA (128 per group); HOLD: coefficients in registers
 template <int T, bool CLUSTER, bool TRANS, bool HOLD>

@@ -2,7 +2,8 @@
 sizes where the cluster kernel's split can go wrong: one and several groups of
 32 nodes a CTA, one CTA and sixteen, windows cut by the cloth's ends (cloths
 3 crossings wide or high), the largest cloth a cluster holds and one more row,
-and batches whose small cloths leave CTAs without nodes. Every schedule sums
+batches whose small cloths leave CTAs without nodes, and one of more 128-node
+blocks than two an SM, whose phases run a thread per node. Every schedule sums
 in the same order, so the results are the same bits.
 """
 import numpy as np
@@ -47,7 +48,8 @@ def _run(sides, schedule, graphed, mode):
 
 
 @pytest.mark.parametrize("sides", [[(3, 3)], [(3, 11), (4, 8)], [(3, 171)], [(170, 3)], [(23, 22)], [(33, 31), (3, 3)],
-                                   [(64, 64)], [(64, 65)], [(17, 17)] * 24, [(41, 41)] + [(7, 9)] * 20])
+                                   [(64, 64)], [(64, 65)], [(17, 17)] * 24, [(41, 41)] + [(7, 9)] * 20,
+                                   [(3, 5), (12, 11)] * 160])
 @pytest.mark.parametrize("graphed", [False, True])
 def test_schedules_give_the_same_bits(sides, graphed):
     ref, it = _run(sides, "phases", False, not graphed)
