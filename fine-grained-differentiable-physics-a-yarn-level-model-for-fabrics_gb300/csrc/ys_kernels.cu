@@ -160,17 +160,15 @@ __global__ void __launch_bounds__(4 * kNodesPerBlock) k_rows(View v, Records R, 
 }
 
 // ----------------------------------------------------------------- solve
-// sum over the block in thread 0: a tree per warp, the warps in order
+// sum over the block in thread 0: a tree per warp, then the warps
 __device__ __forceinline__ double block_sum(double val, double* sh) {
   for (int o = 16; o > 0; o >>= 1) val += __shfl_down_sync(0xffffffffu, val, o);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   __syncthreads();
   if (lane == 0) sh[wid] = val;
   __syncthreads();
-  double s = 0.0;
-  if (threadIdx.x == 0)
-    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) s += sh[i];
-  return s;  // valid in thread 0
+  static_assert(kBlock == 128, "four warps");
+  return threadIdx.x == 0 ? four_sum(sh[0], sh[1], sh[2], sh[3]) : 0.0;
 }
 
 // In a batch that leaves SMs idle (by_rows) a thread's vectors are loaded
@@ -380,7 +378,7 @@ __global__ void __launch_bounds__(kBlock) k_pcg_dir(View v, Blocks b, Solver so,
       // every active cloth has completed exactly `it` iterations before this one
       const bool cap = !conv && it + 1 >= pc.maxiter;
       go_sh = !(conv || cap);
-      beta_sh = rzn / pc.rz[parity];
+      beta_sh = rzn * (1.0 / pc.rz[parity]);  // (the persistent solve has the reciprocal early)
       if (lead) {
         pc.rr = rr;
         pc.rz[parity ^ 1] = rzn;

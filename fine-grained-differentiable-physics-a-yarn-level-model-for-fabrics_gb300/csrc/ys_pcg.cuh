@@ -100,6 +100,16 @@ __device__ __forceinline__ void row_product(int m, const Coef& coef, const Vec& 
   }
 }
 
+// four group sums of a block; n lanes' sums (zero elsewhere): the levels of the
+// tree that would add zeros are left out
+__device__ __forceinline__ double four_sum(double a, double b, double c, double d) { return (a + b) + (c + d); }
+__device__ __forceinline__ double lanes_sum(double s, int n) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+    if (o < n) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
+}
+
 // fixed-order sum of cloth c's block partials in row `which`, by a whole warp:
 // lane l adds blocks l, l + 32, ... in order, then the lanes as a tree. (One
 // thread adding them all waited out an FP64 addition per block, up to 79 of
@@ -108,7 +118,7 @@ __device__ __forceinline__ double cloth_sum(const Blocks& b, const double* part,
   const int b0 = b.cloth_blk0[c], nb = b.cloth_nblk[c];
   double s = 0.0;
   for (int i = threadIdx.x & 31; i < nb; i += 32) s += part[which * b.nblk + b0 + i];
-  return cloth_tree(s);
+  return lanes_sum(s, nb);
 }
 
 // where the groups' p.q partials start in Solver::part
@@ -121,11 +131,9 @@ __device__ __forceinline__ double cloth_sum_pq(const Blocks& b, const double* pa
   double s = 0.0;
   for (int i = threadIdx.x & 31; i < nb; i += 32) {
     const double* g = part + pq_row(b) + 4LL * (b0 + i);
-    double t = 0.0;
-    for (int k = 0; k < 4; ++k) t += g[k];
-    s += t;
+    s += four_sum(g[0], g[1], g[2], g[3]);
   }
-  return cloth_tree(s);
+  return lanes_sum(s, nb);
 }
 
 }  // namespace ys

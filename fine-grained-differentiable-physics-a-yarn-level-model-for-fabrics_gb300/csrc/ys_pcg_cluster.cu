@@ -22,8 +22,8 @@
 // The arithmetic is the batched PCG's (k_pcg_setup, k_pcg_spmv, k_pcg_axpy,
 // k_pcg_dir in ys_kernels.cu) term for term, and the dot products are summed
 // in its order: the components of a node chained, a warp shuffle tree per 32
-// nodes, the four group sums of each 128-node block in order, then the cloth's
-// blocks (cloth_tree). So the two schedules give the same bits, and both
+// nodes, the four group sums of each 128-node block (four_sum), then the
+// cloth's blocks (lanes_sum). So the two schedules give the same bits, and both
 // restate Eigen's ConjugateGradient with its diagonal preconditioner
 // (src/Solvers.cpp:3-31).
 #include <cooperative_groups.h>
@@ -62,7 +62,7 @@ template <int T, bool CLUSTER, bool TRANS, bool HOLD>
 __global__ void __launch_bounds__(T, T <= 256 ? 2 : 1) k_pcg_cluster(View v, Solver so, const int* __restrict__ cloths, int cap) {
   extern __shared__ double dyn[];
   __shared__ double gp[2][2][kMaxGroups];  // group partials of two dot products, alternating
-  __shared__ double out[2];
+  __shared__ double out[2], irz;
   const int groups = blockDim.x / (4 * kGroup), own_nodes = groups * kGroup;
   double* zs = dyn;                    // [5][own_nodes] z, read by the other CTAs
   double* rs = dyn + 5 * own_nodes;    // [5][own_nodes] q, then r, for the dot products
@@ -119,10 +119,9 @@ __global__ void __launch_bounds__(T, T <= 256 ? 2 : 1) k_pcg_cluster(View v, Sol
             if (CLUSTER) src = cg::this_cluster().map_shared_rank(src, rk < csize ? rk : 0);
             part[i] = rk < csize ? src[lg] : 0.0;
           }
-#pragma unroll
-          for (int i = 0; i < 4; ++i) s += part[i];
+          s = four_sum(part[0], part[1], part[2], part[3]);
         }
-        s = cloth_tree(s);
+        s = lanes_sum(s, nblk);
         if (lane == 0) out[q] = s;
       }
     __syncthreads();
@@ -172,6 +171,7 @@ __global__ void __launch_bounds__(T, T <= 256 ? 2 : 1) k_pcg_cluster(View v, Sol
 #pragma unroll
     for (int i = 0; i < 2; ++i)
       if (i < nc) rs[(m + i) * own_nodes + at] = q[i];
+    if (m == 3 && grp == 0 && lane == 0) irz = 1.0 / rzc;  // by the warp that finishes first
     __syncthreads();
     if (m == 3) dot(gp[red & 1], 0, sp + pos, WN, rs + at, own_nodes);
     sync_all();
@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(T, T <= 256 ? 2 : 1) k_pcg_cluster(View v, Sol
     const double rrn = out[0], rzn = out[1];
     const bool conv = rrn < thr;
     const bool cp = !conv && it + 1 >= maxiter;
-    const double beta = rzn / rzc;
+    const double beta = rzn * irz;
     rrc = rrn;
     rzc = rzn;
     iters = conv ? it : it + 1;
