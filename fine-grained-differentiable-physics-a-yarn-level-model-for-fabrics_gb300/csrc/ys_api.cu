@@ -91,6 +91,17 @@ __global__ void k_reset_pc(ys::PcgCloth* pc, const int* maxiter, int ncloth, int
   pc[c].iters = 0;
   pc[c].maxiter = maxiter_override >= 0 ? maxiter_override : maxiter[c];
 }
+// the bookkeeping of nrhs further solves with the system of `from`
+__global__ void k_reset_pc_rhs(ys::PcgCloth* pc, const ys::PcgCloth* from, const int* maxiter, int ncloth, int nrhs,
+                               int maxiter_override) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= ncloth * nrhs) return;
+  const int c = t % ncloth;
+  ys::PcgCloth r{};
+  r.status = from[c].status & 1;
+  r.maxiter = maxiter_override >= 0 ? maxiter_override : maxiter[c];
+  pc[t] = r;
+}
 __global__ void k_reset_status(ys::PcgCloth* pc, int ncloth) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c < ncloth) pc[c].status = 0;
@@ -137,6 +148,7 @@ struct ys_batch {
     double *dNRM = nullptr, *dCOMP = nullptr, *dSLIDE = nullptr;
     double *drho = nullptr, *dks = nullptr, *dkb = nullptr, *dS = nullptr, *dmu = nullptr;
     double *qsave = nullptr, *rt = nullptr, *dq = nullptr;
+    ys::PcgCloth* pc = nullptr;  // [kTangents][ncloth]
     double* scratch = nullptr;  // [kTangents][kTangentScratch][ntot]
     double* io = nullptr;  // [kTangents][ntot][3] staging of host tangents
     double* dext = nullptr;  // [kTangents][ntot][5] external-force tangents
@@ -782,6 +794,11 @@ ys_status ys_assemble(ys_batch* b, double h, const double* ext_force, int32_t fl
 namespace {
 // Jacobi-PCG on the assembled A with the right-hand side v.B (the step's b,
 // or the right-hand side of a tangent solve); the solution lands in so.x.
+// one right-hand side: the view's b, the solver's x
+ys::ClusterRhs cluster_rhs(const ys_batch* b, const ys::View& v) {
+  return ys::ClusterRhs{v.B, b->so.x, b->so.pc, 0, 0, b->ntot};
+}
+
 ys_status solve_impl(ys_batch* b, const ys::View& v, const ys_solve_opts* opts, ys_cloth_stats* stats) {
   cudaStream_t s = b->stream;
   b->so.tol = (opts && opts->tol > 0) ? opts->tol : DBL_EPSILON;
@@ -795,7 +812,7 @@ ys_status solve_impl(ys_batch* b, const ys::View& v, const ys_solve_opts* opts, 
   if (b->plan.kind == YS_PCG_PERSISTENT) {
     cudaError_t e = cudaSuccess;
     b->run(YS_PROF_PCG_PERSIST, 1, [&] {
-      e = ys::launch_pcg_cluster(v, b->so, b->plan.order, b->ncloth, b->plan.shape, cap, s);
+      e = ys::launch_pcg_cluster(v, b->so, cluster_rhs(b, v), 1, b->plan.order, b->ncloth, b->plan.shape, cap, s);
     });
     if (e != cudaSuccess) return fail(YS_ERR_CUDA, std::string("persistent PCG: ") + cudaGetErrorString(e));
   }
@@ -1151,6 +1168,45 @@ ys::View dual_view(ys_batch* b) {
   return dv;
 }
 
+// A dq_k = rt_k (A^T with so.trans) for k < kact, by the default schedule; so.x
+// keeps the step's solution
+ys_status solve_tangents(ys_batch* b, int kact, const ys_solve_opts* opts) {
+  ys_batch::Tan& t = b->tan;
+  const int64_t nt = b->ntot;
+  cudaStream_t cs = b->stream;
+  if (b->plan.kind == YS_PCG_PERSISTENT) {
+    // every direction's clusters in one launch: a 17 x 17 cloth's ten CTAs leave
+    // most of the GPU to the other directions (two cloths, four directions: one
+    // solve's 0.16 ms for four, and no wait of the host between them)
+    const int override_max = (opts && opts->maxiter >= 0) ? opts->maxiter : -1;
+    b->so.tol = (opts && opts->tol > 0) ? opts->tol : DBL_EPSILON;
+    cudaError_t e = cudaSuccess;
+    b->run(YS_PROF_MISC, 1, [&] {
+      k_reset_pc_rhs<<<(b->ncloth * kact + 127) / 128, 128, 0, cs>>>(t.pc, b->so.pc, b->maxiter_dev, b->ncloth, kact,
+                                                                     override_max);
+    });
+    b->run(YS_PROF_PCG_PERSIST, 1, [&] {
+      const ys::ClusterRhs io{t.rt, t.dq, t.pc, 5 * nt, nt, KT * nt};
+      e = ys::launch_pcg_cluster(b->v, b->so, io, kact, b->plan.order, b->ncloth, b->plan.shape,
+                                 override_max >= 0 ? override_max : b->max_maxiter, cs);
+    });
+    if (e != cudaSuccess) return fail(YS_ERR_CUDA, std::string("persistent PCG: ") + cudaGetErrorString(e));
+    YS_CUDA(cudaGetLastError());
+    return YS_OK;
+  }
+  YS_CUDA(cudaMemcpyAsync(t.qsave, b->so.x, sizeof(double) * 5 * nt, cudaMemcpyDeviceToDevice, cs));
+  for (int k = 0; k < kact; ++k) {
+    ys::View vk = b->v;
+    vk.B = t.rt + (int64_t)k * 5 * nt;
+    const ys_status sk = solve_impl(b, vk, opts, nullptr);
+    if (sk == YS_ERR_ARG || sk == YS_ERR_CUDA) return sk;
+    YS_CUDA(cudaMemcpy2DAsync(t.dq + (int64_t)k * nt, sizeof(double) * KT * nt, b->so.x, sizeof(double) * nt,
+                              sizeof(double) * nt, 5, cudaMemcpyDeviceToDevice, cs));
+  }
+  YS_CUDA(cudaMemcpyAsync(b->so.x, t.qsave, sizeof(double) * 5 * nt, cudaMemcpyDeviceToDevice, cs));
+  return YS_OK;
+}
+
 }  // namespace
 
 extern "C" {
@@ -1173,6 +1229,7 @@ ys_status ys_tangent_enable(ys_batch* b, int32_t mode) {
     A(&t.qsave, 5 * nt); A(&t.rt, 5 * KT * nt); A(&t.dq, 5 * KT * nt);
     A(&t.scratch, (size_t)ys::kTangentScratch * KT * nt);
     A(&t.io, 3 * KT * nt);
+    if (st == YS_OK) st = b->alloc(&t.pc, KT * nc);
     if (st != YS_OK) return st;
     t.on = true;
   }
@@ -1280,27 +1337,20 @@ ys_status ys_step_tangent_ext(ys_batch* b, double h, const double* ext_force, co
   cudaStream_t cs = b->stream;
   const int64_t nt = b->ntot;
   ys_batch::Tan& t = b->tan;
-  YS_CUDA(cudaMemcpyAsync(t.qsave, b->so.x, sizeof(double) * 5 * nt, cudaMemcpyDeviceToDevice, cs));
   // tangents of the residual b - A q at the step's q
   ys::View dv = dual_view(b);
   b->run(YS_PROF_MISC, 7, [&] {
-    ys::launch_tangent_residual(dv, b->rec, b->anchors + b->geom_off, b->geom_n, t.qsave, t.scratch, d_dext, kact, t.rt, cs);
+    ys::launch_tangent_residual(dv, b->rec, b->anchors + b->geom_off, b->geom_n, b->so.x, t.scratch, d_dext, kact, t.rt,
+                                cs);
   });
   YS_CUDA(cudaGetLastError());
   // tangent solves with the step's A and Jacobi diagonal: A dq_k = db_k - dA_k q
   // (exact), or A^T dq_k = db_k with M, D held constant -- the transpose of
   // the reference's backward b_bar = A^-1 q_bar (src/Solvers.cpp:33-58)
-  for (int k = 0; k < kact; ++k) {
-    ys::View vk = b->v;
-    vk.B = t.rt + (int64_t)k * 5 * nt;
-    b->so.trans = t.mode == YS_TANGENT_REFERENCE ? 1 : 0;
-    const ys_status sk = solve_impl(b, vk, opts, nullptr);
-    b->so.trans = 0;
-    if (sk == YS_ERR_ARG || sk == YS_ERR_CUDA) return sk;
-    YS_CUDA(cudaMemcpy2DAsync(t.dq + (int64_t)k * nt, sizeof(double) * KT * nt, b->so.x, sizeof(double) * nt,
-                              sizeof(double) * nt, 5, cudaMemcpyDeviceToDevice, cs));
-  }
-  YS_CUDA(cudaMemcpyAsync(b->so.x, t.qsave, sizeof(double) * 5 * nt, cudaMemcpyDeviceToDevice, cs));
+  b->so.trans = t.mode == YS_TANGENT_REFERENCE ? 1 : 0;
+  const ys_status sk = kact == 0 ? YS_OK : solve_tangents(b, kact, opts);
+  b->so.trans = 0;
+  if (sk == YS_ERR_ARG || sk == YS_ERR_CUDA) return sk;
   ys::TangentState ts{t.dX, t.dV, t.dUV, t.dUVD, t.dUVB};
   b->run(YS_PROF_UPDATE, 2, [&] { ys::launch_update_dual(dv, b->blk, b->so, t.dq, ts, cs); });
   YS_CUDA(cudaGetLastError());
@@ -1614,7 +1664,7 @@ ys_status graph_build(ys_batch* b, int m, int cap, int override_max) {
     YS_CUDA(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
     capture_assembly(b, cs, override_max);
     const cudaError_t e =
-        ys::launch_pcg_cluster(v, so, b->plan.order, b->ncloth, b->plan.shape, cap, cs);
+        ys::launch_pcg_cluster(v, so, cluster_rhs(b, v), 1, b->plan.order, b->ncloth, b->plan.shape, cap, cs);
     ys::launch_update(v, b->blk, b->so, cs);
     cudaGraph_t one = nullptr;
     YS_CUDA(cudaStreamEndCapture(cs, &one));

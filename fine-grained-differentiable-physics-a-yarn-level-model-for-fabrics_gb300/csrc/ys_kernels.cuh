@@ -100,8 +100,16 @@ struct ClusterShape {
 };
 // the shape for these cloths (host array); enables its kernels, so outside any capture
 cudaError_t pcg_cluster_shape(const ClothParams* cp, int ncloth, int device, ClusterShape* out);
-cudaError_t launch_pcg_cluster(const View& v, const Solver& so, const int* cloths, int ncl, const ClusterShape& sh,
-                               int cap, cudaStream_t s);
+// right-hand sides of one launch: rhs k at b + k b_rhs ([5][ntot]), its solution
+// at x + k x_rhs with components x_comp apart, its bookkeeping at pc + k ncloth
+struct ClusterRhs {
+  const double* b;
+  double* x;
+  PcgCloth* pc;
+  int64_t b_rhs, x_rhs, x_comp;
+};
+cudaError_t launch_pcg_cluster(const View& v, const Solver& so, const ClusterRhs& io, int nrhs, const int* cloths,
+                               int ncl, const ClusterShape& sh, int cap, cudaStream_t s);
 
 // state tangents updated by the tangent step (layout [c][kTangents][ntot])
 struct TangentState {

@@ -59,7 +59,7 @@ struct Window {
 
 // T: most threads a CTA (128 per group); HOLD: coefficients in registers
 template <int T, bool CLUSTER, bool TRANS, bool HOLD>
-__global__ void __launch_bounds__(T, T <= 256 ? 2 : 1) k_pcg_cluster(View v, Solver so, const int* __restrict__ cloths, int cap) {
+__global__ void __launch_bounds__(T, T <= 256 ? 2 : 1) k_pcg_cluster(View v, Solver so, ClusterRhs io, const int* __restrict__ cloths, int cap) {
   extern __shared__ double dyn[];
   __shared__ double gp[2][2][kMaxGroups];  // group partials of two dot products, alternating
   __shared__ double out[2], irz;
@@ -70,7 +70,9 @@ __global__ void __launch_bounds__(T, T <= 256 ? 2 : 1) k_pcg_cluster(View v, Sol
   const int csize = CLUSTER ? (int)cg::this_cluster().num_blocks() : 1;
   const int rank = CLUSTER ? (int)cg::this_cluster().block_rank() : 0;
   const int c = cloths[blockIdx.x / csize];
-  PcgCloth& pc = so.pc[c];
+  const int rhs = blockIdx.y;
+  PcgCloth& pc = io.pc[(int64_t)rhs * v.ncloth + c];
+  const double* __restrict__ b = io.b + rhs * io.b_rhs;
   const ClothParams& P = v.cp[c];
   const int W = P.W, H = P.H, N = W * H, off = P.node_off, nt = v.ntot;
   const int nblk = (N + kBlock - 1) / kBlock;
@@ -138,7 +140,7 @@ __global__ void __launch_bounds__(T, T <= 256 ? 2 : 1) k_pcg_cluster(View v, Sol
   for (int i = 0; i < 2; ++i) {
     if (i >= nc) break;
     if (own) {
-      r[i] = ld(v.B, m + i, nt, n);
+      r[i] = ld(b, m + i, nt, n);
       dinv[i] = ld(so.dinv, m + i, nt, n);
     }
     rs[(m + i) * own_nodes + at] = r[i];
@@ -148,7 +150,7 @@ __global__ void __launch_bounds__(T, T <= 256 ? 2 : 1) k_pcg_cluster(View v, Sol
 #pragma unroll
     for (int k = 0; k < 5; ++k) {
       const int64_t g = (int64_t)k * nt + off + win.lo + e;
-      sp[k * WN + e] = so.dinv[g] * v.B[g];
+      sp[k * WN + e] = so.dinv[g] * b[g];
     }
   __syncthreads();
   int red = 0;  // reductions so far: selects the partials' buffer
@@ -217,7 +219,7 @@ __global__ void __launch_bounds__(T, T <= 256 ? 2 : 1) k_pcg_cluster(View v, Sol
   }
 #pragma unroll
   for (int i = 0; i < 2; ++i)
-    if (own && i < nc) st(so.x, m + i, nt, n) = x[i];
+    if (own && i < nc) io.x[rhs * io.x_rhs + (m + i) * io.x_comp + n] = x[i];
   if (rank == 0 && threadIdx.x == 0) {
     pc.bb = bb;
     pc.thr = thr;
@@ -248,8 +250,8 @@ cudaError_t with_kernel(int groups, bool cluster, bool trans, F&& f) {
   return cudaErrorInvalidValue;
 }
 
-void config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at, const ClusterShape& sh, int ncl) {
-  cfg.gridDim = dim3((unsigned)(ncl * sh.csize));
+void config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at, const ClusterShape& sh, int ncl, int nrhs) {
+  cfg.gridDim = dim3((unsigned)(ncl * sh.csize), (unsigned)nrhs);
   cfg.blockDim = dim3((unsigned)(sh.groups * 4 * kGroup));
   cfg.dynamicSmemBytes = sh.shared;
   at[0].id = cudaLaunchAttributeClusterDimension;
@@ -273,7 +275,7 @@ static cudaError_t cluster_fit(const ClusterShape& sh, int sms, int* clusters) {
       if (r != cudaSuccess) return r;
       cudaLaunchConfig_t cfg = {};
       cudaLaunchAttribute at[1] = {};
-      config(cfg, at, sh, 1);
+      config(cfg, at, sh, 1, 1);
       int fit = 0;
       if (sh.csize > 1) {
         r = cudaOccupancyMaxActiveClusters(&fit, k, &cfg);
@@ -339,14 +341,14 @@ cudaError_t pcg_cluster_shape(const ClothParams* cp, int ncloth, int device, Clu
   return cudaSuccess;
 }
 
-cudaError_t launch_pcg_cluster(const View& v, const Solver& so, const int* cloths, int ncl, const ClusterShape& sh,
-                               int cap, cudaStream_t s) {
+cudaError_t launch_pcg_cluster(const View& v, const Solver& so, const ClusterRhs& io, int nrhs, const int* cloths,
+                               int ncl, const ClusterShape& sh, int cap, cudaStream_t s) {
   return with_kernel(sh.groups, sh.csize > 1, so.trans != 0, [&](auto* k) {
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute at[1] = {};
-    config(cfg, at, sh, ncl);
+    config(cfg, at, sh, ncl, nrhs);
     cfg.stream = s;
-    return cudaLaunchKernelEx(&cfg, k, v, so, cloths, cap);
+    return cudaLaunchKernelEx(&cfg, k, v, so, io, cloths, cap);
   });
 }
 

@@ -58,3 +58,27 @@ def test_schedules_give_the_same_bits(sides, graphed):
         assert n == it, schedule
         for a, c in zip(ref, got):
             assert np.array_equal(a, c), schedule
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("sides", [[(3, 3)], [(23, 22), (5, 9)]])
+@pytest.mark.parametrize("kact", [1, 3, 4])
+def test_directions_solved_together(sides, mode, kact):
+    """The directions' solves of a tangent step in one launch, and one by one in phases."""
+    outs = []
+    for persistent in (False, True):
+        b = ys.ClothBatch(_specs(sides, 5))
+        b.set_pcg_schedule(persistent, 1024, 16)
+        b.tangent_enable(mode)
+        K, nl, nc = b.n_tangents, sum(w + h for w, h in sides), len(sides)
+        rng = np.random.default_rng(2)
+        b.tangent_seed(rng.standard_normal((K, nl)) * 1e-4, rng.standard_normal((K, nl)) * 1e2,
+                       rng.standard_normal((K, nl)) * 1e-6, rng.standard_normal((K, nc)) * 1e-5,
+                       rng.standard_normal((K, nc)) * 1e-2)
+        for _ in range(2):
+            assert all(s["ok"] for s in b.step_tangent(1e-3, tol=1e-12, kact=kact))
+        outs.append((b.get_state(), b.tangent_get_state()))
+        b.close()
+    for a, c in zip(*outs):
+        for k in a:
+            assert np.array_equal(a[k], c[k]), k
