@@ -36,6 +36,10 @@ using ys::Kdop;
 constexpr int kStack = 64;  // traversal stack; deeper trees report an error
 constexpr int kBroadBlock = 64;
 constexpr int kSliceDepth = 4;  // broad-phase slices: up to 16 subtrees per tree
+constexpr int kTestBlocks = 8 * 152;  // of the narrow tests, which walk the lists
+// the thickness and sqrt(2) times it, widened, for the FP32 prune
+inline float prune1(double d) { return (float)(d * (1.0 + 1e-6)); }
+inline float prune2(double d) { return (float)(std::sqrt(2.0) * d * (1.0 + 1e-6)); }
 
 #define YC_CUDA(call)                                                                   \
   do {                                                                                  \
@@ -49,19 +53,64 @@ struct DevTree {
   const int* face;
   Kdop* box;
   int nnodes;
-  float* fbox;  // [nnodes][18] the boxes widened to float (lower bounds down, upper up)
+  float4* fbox;  // [nnodes][5]: FBox of each node
 };
 
-// inner-node prune in FP32 on the widened boxes: wider again by a relative
-// 1e-6 of the magnitudes, far above float rounding, it keeps every subtree
-// holding a pair the exact FP64 leaf test accepts
-__device__ __forceinline__ bool kdop_overlap_f(const float* a, const float* b, float d1, float d2) {
+// A box widened to float, lower bounds down, upper up: pairs (lower, upper) of
+// the nine axes, then for a tree node its children, (face, -1) at a leaf. Five
+// 16-byte loads, of which a box that fails on the first two axes costs one,
+// where 18 floats and three links took 21 scattered loads.
+constexpr int kFBox = 5;
+__device__ __forceinline__ void fbox_store(float4* q, const Kdop& b, int l, int r) {
+  float x[20];
 #pragma unroll
-  for (int i = 0; i < 9; ++i) {
-    const float dd = i < 3 ? d1 : d2;
-    const float slack = 1e-6f * (fabsf(a[i]) + fabsf(a[i + 9]) + fabsf(b[i]) + fabsf(b[i + 9])) + 1e-30f;
-    if (a[i] > b[i + 9] + dd + slack) return false;
-    if (a[i + 9] < b[i] - dd - slack) return false;
+  for (int k = 0; k < 9; ++k) {
+    x[2 * k] = __double2float_rd(b.d[k]);
+    x[2 * k + 1] = __double2float_ru(b.d[k + 9]);
+  }
+  x[18] = __int_as_float(l);
+  x[19] = __int_as_float(r);
+#pragma unroll
+  for (int k = 0; k < kFBox; ++k) q[k] = make_float4(x[4 * k], x[4 * k + 1], x[4 * k + 2], x[4 * k + 3]);
+}
+__device__ __forceinline__ void fbox_load(float (&x)[18], const float4* q) {
+#pragma unroll
+  for (int k = 0; k < kFBox; ++k) {
+    const float4 f = q[k];
+    x[4 * k] = f.x;
+    x[4 * k + 1] = f.y;
+    if (k < 4) {
+      x[4 * k + 2] = f.z;
+      x[4 * k + 3] = f.w;
+    }
+  }
+}
+
+// a prune in FP32 on the widened boxes: wider again by a relative 1e-6 of the
+// magnitudes, far above float rounding, it keeps every pair the exact FP64 test
+// accepts. One axis of it:
+__device__ __forceinline__ bool axis_apart(float alo, float ahi, float blo, float bhi, float dd) {
+  const float slack = 1e-6f * (fabsf(alo) + fabsf(ahi) + fabsf(blo) + fabsf(bhi)) + 1e-30f;
+  return alo > bhi + dd + slack || ahi < blo - dd - slack;
+}
+__device__ __forceinline__ bool fbox_overlap(const float (&a)[18], const float (&b)[18], float d1, float d2) {
+  bool apart = false;
+#pragma unroll
+  for (int i = 0; i < 9; ++i) apart = apart || axis_apart(a[2 * i], a[2 * i + 1], b[2 * i], b[2 * i + 1], i < 3 ? d1 : d2);
+  return !apart;
+}
+// the same against a stored box, read as far as it takes; its links
+__device__ __forceinline__ bool fbox_overlap(const float (&a)[18], const float4* q, float d1, float d2, int& l, int& r) {
+#pragma unroll
+  for (int k = 0; k < kFBox; ++k) {
+    const float4 f = q[k];
+    if (axis_apart(a[4 * k], a[4 * k + 1], f.x, f.y, 2 * k < 3 ? d1 : d2)) return false;
+    if (k < 4) {
+      if (axis_apart(a[4 * k + 2], a[4 * k + 3], f.z, f.w, 2 * k + 1 < 3 ? d1 : d2)) return false;
+    } else {
+      l = __float_as_int(f.z);
+      r = __float_as_int(f.w);
+    }
   }
   return true;
 }
@@ -75,45 +124,51 @@ __device__ __forceinline__ bool kdop_overlap_f(const float* a, const float* b, f
 // bit for bit. No thread waits for another: every climb ends at the root or
 // at a first arrival.
 __device__ __forceinline__ void kdop_load_l2(Kdop& b, const Kdop* src) {
-  const double* p = reinterpret_cast<const double*>(src);
+  const double2* p = reinterpret_cast<const double2*>(src);  // 144 bytes a box, 16-byte aligned
 #pragma unroll
-  for (int k = 0; k < 18; ++k) b.d[k] = __ldcg(p + k);
-}
-__device__ __forceinline__ void refit_store(const DevTree& t, int n, const Kdop& b) {
-  t.box[n] = b;
   for (int k = 0; k < 9; ++k) {
-    t.fbox[18 * (int64_t)n + k] = __double2float_rd(b.d[k]);
-    t.fbox[18 * (int64_t)n + 9 + k] = __double2float_ru(b.d[k + 9]);
+    const double2 x = __ldcg(p + k);
+    b.d[2 * k] = x.x;
+    b.d[2 * k + 1] = x.y;
   }
+}
+__device__ __forceinline__ void refit_store(const DevTree& t, int n, const Kdop& b, int l, int r) {
+  t.box[n] = b;
+  fbox_store(t.fbox + kFBox * (int64_t)n, b, l, r);
 }
 __global__ void k_refit_up(DevTree t, const int* __restrict__ leaves, int nleaves, const int* __restrict__ parent,
                            int* arrive, const CFace* __restrict__ faces, CMesh m, int ccd) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nleaves) return;
   int n = leaves[i];
+  Kdop b;
   {
     const CFace& fc = faces[t.face[n]];
-    Kdop b;
     ys::kdop_node(b, ys::cc_pos(m, fc.v[0], false), ys::cc_pos(m, fc.v[0], true), ccd != 0);
     for (int k = 1; k < 3; ++k) {
       Kdop nb;
       ys::kdop_node(nb, ys::cc_pos(m, fc.v[k], false), ys::cc_pos(m, fc.v[k], true), ccd != 0);
       ys::kdop_add(b, nb);
     }
-    refit_store(t, n, b);
+    refit_store(t, n, b, t.face[n], -1);
   }
   for (;;) {
     const int p = parent[n];
     if (p < 0) return;
+    const int l = t.left[p], r = t.right[p];
     // release: this node's box is visible before the count says so; acquire:
-    // the second arrival sees its sibling's box
+    // the second arrival sees its sibling's box (its own is still here)
     cuda::atomic_ref<int, cuda::thread_scope_device> cnt(arrive[p]);
     if (cnt.fetch_add(1, cuda::memory_order_acq_rel) == 0) return;  // the sibling's thread goes on
-    Kdop b, rb;
-    kdop_load_l2(b, t.box + t.left[p]);
-    kdop_load_l2(rb, t.box + t.right[p]);
-    ys::kdop_add(b, rb);
-    refit_store(t, p, b);
+    Kdop sib;
+    kdop_load_l2(sib, t.box + (n == l ? r : l));
+    if (n == l) {
+      ys::kdop_add(b, sib);
+    } else {
+      ys::kdop_add(sib, b);
+      b = sib;
+    }
+    refit_store(t, p, b, l, r);
     n = p;
   }
 }
@@ -182,7 +237,7 @@ __global__ void k_broad(BroadArgs a) {
     const int leaf = a.leaf_of_face[f];
     const Kdop bf = a.cloth.box[leaf];
     float bfl[18];  // the face's widened box, as refit left it for its leaf
-    for (int k = 0; k < 18; ++k) bfl[k] = a.cloth.fbox[18 * (int64_t)leaf + k];
+    fbox_load(bfl, a.cloth.fbox + kFBox * (int64_t)leaf);
     const int uf = a.upper[f], rf = a.rank[f];
     const int64_t o = WRITE ? a.offset[idx] : 0;
     int stack[kStack];
@@ -191,111 +246,188 @@ __global__ void k_broad(BroadArgs a) {
     while (sp > 0) {
       const int n = stack[--sp];
       if (!fa && a.node_active[n] == 0) continue;  // pass 0 only: no active face below
-      const int g = t.face[n];
-      if (g >= 0) {
-        if (pass == 0) {
-          if (g == f || !ys::bvh_first(uf, rf, a.upper[g], a.rank[g])) continue;
-        }
-        // the FP32 test first: it rejects only boxes the exact test rejects
-        if (!kdop_overlap_f(bfl, t.fbox + 18 * (int64_t)n, a.thick1, a.thick2)) continue;
-        if (!ys::kdop_overlap(bf, t.box[n], a.thickness)) continue;
-        if (WRITE) {
-          if (o + c < a.cap) {
-            a.out[3 * (o + c)] = f;
-            a.out[3 * (o + c) + 1] = g;
-            a.out[3 * (o + c) + 2] = pass;
-          } else {
-            atomicOr(a.overflow, 2);
-          }
-        } else if (c < kBroadKeep) {
-          a.keep[idx * kBroadKeep + c] = g;
-        }
-        ++c;
-      } else {
-        if (!kdop_overlap_f(bfl, t.fbox + 18 * (int64_t)n, a.thick1, a.thick2)) continue;
+      // the FP32 test first: it rejects only boxes the exact test rejects
+      int l, r;
+      if (!fbox_overlap(bfl, t.fbox + kFBox * (int64_t)n, a.thick1, a.thick2, l, r)) continue;
+      if (r >= 0) {
         if (sp + 2 > kStack) {
           atomicOr(a.overflow, 1);
           continue;
         }
-        stack[sp++] = t.right[n];
-        stack[sp++] = t.left[n];
+        stack[sp++] = r;
+        stack[sp++] = l;
+        continue;
       }
+      const int g = l;
+      if (pass == 0 && (g == f || !ys::bvh_first(uf, rf, a.upper[g], a.rank[g]))) continue;
+      if (!ys::kdop_overlap(bf, t.box[n], a.thickness)) continue;
+      if (WRITE) {
+        if (o + c < a.cap) {
+          a.out[3 * (o + c)] = f;
+          a.out[3 * (o + c) + 1] = g;
+          a.out[3 * (o + c) + 2] = pass;
+        } else {
+          atomicOr(a.overflow, 2);
+        }
+      } else if (c < kBroadKeep) {
+        a.keep[idx * kBroadKeep + c] = g;
+      }
+      ++c;
     }
   }
   if (!WRITE) a.count[idx] = c;
 }
 
-// Narrow phase in two kernels. k_narrow_mask: one thread per pair forms the
-// k-DOPs of its six nodes and decides which of the 15 tests run (cc_face_pair's
-// overlap and shared-node rules). k_narrow_test: one thread per (test, pair),
-// test-major, so a warp runs one kind of test on 32 pairs; test t of pair p
-// writes slot 15 p + t (type -1: no impact) and counts its impact for the
-// pair. The compaction then takes each pair's slots in test order: the
-// impacts, and their order, are cc_face_pair's.
+// Narrow phase in two kernels. k_narrow_mask: one thread per pair decides from
+// the k-DOPs of its six nodes which of the 15 tests run (cc_face_pair's overlap
+// and shared-node rules) and lists them. k_narrow_test: one thread per listed
+// test; test t of pair p writes slot 15 p + t (type -1: no impact) and counts
+// its impact for the pair. The compaction then takes each pair's slots in test
+// order: the impacts, and their order, are cc_face_pair's.
 // k-DOP of every node's motion (kdop_node of its two positions): cloth node
 // i at [i], obstacle node j at [n_nodes + j]
-__global__ void k_node_kdop(CMesh m, int n_nodes, int n_obs, int ccd, Kdop* __restrict__ out) {
+// (and its widened form; zeroes the lists' lengths for k_narrow_mask)
+__global__ void k_node_kdop(CMesh m, int n_nodes, int n_obs, int ccd, Kdop* __restrict__ out, float4* __restrict__ fout,
+                            int64_t* list_n) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < 2) list_n[i] = 0;
   if (i >= n_nodes + n_obs) return;
   const int id = i < n_nodes ? i : -1 - (i - n_nodes);  // obstacle ids as -1 - id
   Kdop b;
   ys::kdop_node(b, ys::cc_pos(m, id, false), ys::cc_pos(m, id, true), ccd != 0);
   out[i] = b;
+  fbox_store(fout + kFBox * (int64_t)i, b, 0, 0);
 }
 struct NodeKdops {
   const Kdop* k;
+  const float4* f;
   int n_nodes;
-  __device__ __forceinline__ Kdop operator()(int id) const { return k[id >= 0 ? id : n_nodes + (-1 - id)]; }
+  __device__ __forceinline__ int at(int id) const { return id >= 0 ? id : n_nodes + (-1 - id); }
+  __device__ __forceinline__ Kdop operator()(int id) const { return k[at(id)]; }
 };
-// (np_dev: the pair count on the device, the launch covering npairs >= it
-// entries, or null: npairs pairs)
-__global__ void k_narrow_mask(const int* __restrict__ pairs, int64_t npairs, const CFace* __restrict__ faces,
-                              const CFace* __restrict__ ofaces, NodeKdops nk, double thickness,
-                              int* __restrict__ mask, int64_t* __restrict__ count, const int64_t* np_dev) {
-  const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= npairs) return;
-  if (np_dev && p >= *np_dev) {
-    count[p] = 0;  // the scan of the impact counts covers the launch's npairs entries
-    mask[p] = 0;
-    return;
+// the tests that the FP32 prune leaves of cc_face_pair_mask's 15 (a box of a
+// face or an edge widened to float is the union of its nodes' widened boxes)
+__device__ __forceinline__ int pair_candidates(const NodeKdops& nk, const CFace& f0, const CFace& f1, float d1, float d2) {
+  float b0[3][18], b1[3][18], u[18];
+  for (int k = 0; k < 3; ++k) {
+    fbox_load(b0[k], nk.f + kFBox * (int64_t)nk.at(f0.v[k]));
+    fbox_load(b1[k], nk.f + kFBox * (int64_t)nk.at(f1.v[k]));
   }
-  const CFace& f0 = faces[pairs[3 * p]];
-  const CFace& f1 = pairs[3 * p + 2] ? ofaces[pairs[3 * p + 1]] : faces[pairs[3 * p + 1]];
-  mask[p] = ys::cc_face_pair_mask(nk, f0, f1, thickness);
-  count[p] = 0;
+  auto join = [&](const float (&x)[18], const float (&y)[18]) {
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+      u[2 * k] = y[2 * k] < x[2 * k] ? y[2 * k] : x[2 * k];
+      u[2 * k + 1] = y[2 * k + 1] > x[2 * k + 1] ? y[2 * k + 1] : x[2 * k + 1];
+    }
+  };
+  auto in = [](int nd, const CFace& f) { return nd == f.v[0] || nd == f.v[1] || nd == f.v[2]; };
+  int mask = 0;
+  join(b1[0], b1[1]);
+  join(u, b1[2]);
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+    if (!in(f0.v[k], f1) && fbox_overlap(b0[k], u, d1, d2)) mask |= 1 << k;
+  join(b0[0], b0[1]);
+  join(u, b0[2]);
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+    if (!in(f1.v[k], f0) && fbox_overlap(b1[k], u, d1, d2)) mask |= 1 << (3 + k);
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    float ea[18];
+    join(b0[a], b0[a != 2 ? a + 1 : 0]);
+#pragma unroll
+    for (int k = 0; k < 18; ++k) ea[k] = u[k];
+#pragma unroll
+    for (int b = 0; b < 3; ++b) {
+      const int *e0 = f0.e[a], *e1 = f1.e[b];
+      if (e0[0] == e1[0] || e0[0] == e1[1] || e0[1] == e1[0] || e0[1] == e1[1]) continue;
+      join(b1[b], b1[b != 2 ? b + 1 : 0]);
+      if (fbox_overlap(ea, u, d1, d2)) mask |= 1 << (6 + 3 * a + b);
+    }
+  }
+  return mask;
 }
-__global__ void k_narrow_test(const int* __restrict__ pairs, int64_t npairs, const CFace* __restrict__ faces,
-                              const CFace* __restrict__ ofaces, CMesh m, const int* __restrict__ mask, Impact* slots,
-                              unsigned long long* count) {
-  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= 15 * npairs) return;
-  const int t = (int)(idx / npairs);
-  const int64_t p = idx - (int64_t)t * npairs;
-  // (pairs past a device count have mask 0: k_narrow_mask)
-  Impact& out = slots[15 * p + t];
-  out.type = -1;
-  if (!((mask[p] >> t) & 1)) return;
-  const CFace& f0 = faces[pairs[3 * p]];
-  const CFace& f1 = pairs[3 * p + 2] ? ofaces[pairs[3 * p + 1]] : faces[pairs[3 * p + 1]];
-  int type, ids[4];
-  ys::cc_pair_test_nodes(f0, f1, t, type, ids);
-  const double* xs[4];
-  const double* xps[4];
-  for (int k = 0; k < 4; ++k) {
-    xs[k] = ys::cc_pos(m, ids[k], false);
-    xps[k] = ys::cc_pos(m, ids[k], true);
+// (np_dev: the pair count on the device, the launch covering npairs >= it
+// entries, or null: npairs pairs). The tests that run go to two lists, list[0]
+// of vertex-face (t < 6, 6 npairs entries) and edge-edge tests, as 16 p + t.
+// Bound by the FP64 pipe when every pair took its 15 box tests of 18 compares
+// and unions there: few pairs keep a test after the FP32 prune.
+__global__ void __launch_bounds__(128) k_narrow_mask(const int* __restrict__ pairs, int64_t npairs,
+                                                     const CFace* __restrict__ faces, const CFace* __restrict__ ofaces,
+                                                     NodeKdops nk, double thickness, float d1, float d2,
+                                                     int* __restrict__ mask, int64_t* __restrict__ count,
+                                                     int64_t* __restrict__ list, unsigned long long* list_n,
+                                                     const int64_t* np_dev) {
+  const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  int mk = 0;
+  if (p < npairs && (!np_dev || p < *np_dev)) {
+    const CFace& f0 = faces[pairs[3 * p]];
+    const CFace& f1 = pairs[3 * p + 2] ? ofaces[pairs[3 * p + 1]] : faces[pairs[3 * p + 1]];
+    mk = pair_candidates(nk, f0, f1, d1, d2);
+    if (mk) mk &= ys::cc_face_pair_mask(nk, f0, f1, thickness);
   }
-  Impact im;
-  if (ys::cc_test(type, xs, xps, im)) {
-    for (int k = 0; k < 4; ++k) im.node[k] = ids[k];
-    out = im;
-    atomicAdd(count + p, 1ull);
+  if (p < npairs) {
+    mask[p] = mk;
+    count[p] = 0;  // the scan of the impact counts covers the launch's npairs entries
+  }
+  for (int kind = 0; kind < 2; ++kind) {
+    const int t0 = kind ? 6 : 0, t1 = kind ? 15 : 6;
+    const int bits = kind ? mk >> 6 : mk & 63;
+    const unsigned any = __ballot_sync(0xffffffffu, bits != 0);
+    if (!any) continue;
+    int n = 0;
+    for (int t = t0; t < t1; ++t) n += __popc(__ballot_sync(0xffffffffu, (mk >> t) & 1));
+    unsigned long long base = 0;
+    if (lane == 0) base = atomicAdd(list_n + kind, (unsigned long long)n);
+    base = __shfl_sync(0xffffffffu, base, 0);
+    int64_t* out = list + (kind ? 6 * npairs : 0) + base;
+    for (int t = t0; t < t1; ++t) {
+      const unsigned b = __ballot_sync(0xffffffffu, (mk >> t) & 1);
+      if ((mk >> t) & 1) out[__popc(b & ((1u << lane) - 1u))] = 16 * p + t;
+      out += __popc(b);
+    }
+  }
+}
+// one thread per listed test, so that a warp's lanes all run one: with a thread
+// per (test, pair) most lanes had none and the FP64 pipe waited for the few.
+// Results go to the pair's slots, whatever the lists' order.
+__global__ void __launch_bounds__(128) k_narrow_test(const int* __restrict__ pairs, int64_t npairs,
+                                                     const CFace* __restrict__ faces, const CFace* __restrict__ ofaces,
+                                                     CMesh m, const int64_t* __restrict__ list,
+                                                     const int64_t* __restrict__ list_n, Impact* slots,
+                                                     unsigned long long* count) {
+  const int64_t nv = list_n[0], ne = list_n[1], nv32 = (nv + 31) / 32 * 32;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nv32 + ne; i += (int64_t)gridDim.x * blockDim.x) {
+    if (i >= nv && i < nv32) continue;
+    const int64_t e = i < nv ? list[i] : list[6 * npairs + i - nv32], p = e >> 4;
+    const int t = (int)(e & 15);
+    Impact& out = slots[15 * p + t];
+    out.type = -1;
+    const CFace& f0 = faces[pairs[3 * p]];
+    const CFace& f1 = pairs[3 * p + 2] ? ofaces[pairs[3 * p + 1]] : faces[pairs[3 * p + 1]];
+    int type, ids[4];
+    ys::cc_pair_test_nodes(f0, f1, t, type, ids);
+    const double* xs[4];
+    const double* xps[4];
+    for (int k = 0; k < 4; ++k) {
+      xs[k] = ys::cc_pos(m, ids[k], false);
+      xps[k] = ys::cc_pos(m, ids[k], true);
+    }
+    Impact im;
+    if (ys::cc_test(type, xs, xps, im)) {
+      for (int k = 0; k < 4; ++k) im.node[k] = ids[k];
+      out = im;
+      atomicAdd(count + p, 1ull);
+    }
   }
 }
 
 // (np_dev as for k_narrow_mask; impacts at or past cap are not written and
 // set bit 2 of *overflow)
-__global__ void k_compact(const Impact* __restrict__ slots, const int64_t* __restrict__ count,
+__global__ void k_compact(const Impact* __restrict__ slots, const int* __restrict__ mask,
+                          const int64_t* __restrict__ count,
                           const int64_t* __restrict__ offset, int64_t npairs, ys_impact* out,
                           const int64_t* np_dev, int64_t cap, int* overflow) {
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -304,7 +436,7 @@ __global__ void k_compact(const Impact* __restrict__ slots, const int64_t* __res
   int64_t k = 0;
   for (int t = 0; t < 15 && k < count[p]; ++t) {
     const Impact& s = slots[15 * p + t];
-    if (s.type < 0) continue;
+    if (!((mask[p] >> t) & 1) || s.type < 0) continue;  // (a test that did not run left its slot alone)
     if (offset[p] + k >= cap) {
       atomicOr(overflow, 4);
       return;
@@ -429,7 +561,7 @@ struct ys_collider {
   // the arrival counters of the inner nodes
   DVec<int> c_parent, c_leaves, c_arrive, o_parent, o_leaves, o_arrive;
   DVec<Kdop> c_box, o_box;
-  DVec<float> c_fbox, o_fbox;
+  DVec<float4> c_fbox, o_fbox;
   // outputs
   DVec<int64_t> counts, offsets, sums, total;
   DVec<int> keep;  // the broad phase's kept partners ([work][kBroadKeep])
@@ -438,6 +570,8 @@ struct ys_collider {
   DVec<Impact> slots;
   DVec<int64_t> icount, ioffset;
   DVec<int> tmask;  // narrow phase: the tests each pair runs (bit t)
+  DVec<int64_t> tlist, tlist_n;  // and their lists, vertex-face, edge-edge, with the lengths
+  DVec<float4> nfbox;
   DVec<Kdop> nkdop;  // narrow phase: every node's motion k-DOP (cloth, then obstacle)
   DVec<ys_impact> impacts;
   int64_t nimpacts = 0;
@@ -505,8 +639,8 @@ ys_status upload_tree(ys_collider* c, const ys::BvhTree& t, DVec<int>& l, DVec<i
 ys_status refit(ys_collider* c, bool obstacle) {
   const ys::BvhTree& t = obstacle ? c->ot : c->ct;
   if (t.face.empty()) return YS_OK;
-  DVec<float>& fb = obstacle ? c->o_fbox : c->c_fbox;
-  YC_CUDA(fb.reserve(18 * t.face.size()));
+  DVec<float4>& fb = obstacle ? c->o_fbox : c->c_fbox;
+  YC_CUDA(fb.reserve(kFBox * t.face.size()));
   DevTree dt{obstacle ? c->o_left.p : c->c_left.p, obstacle ? c->o_right.p : c->c_right.p,
              obstacle ? c->o_face.p : c->c_face.p, obstacle ? c->o_box.p : c->c_box.p, (int)t.face.size(), fb.p};
   CMesh m{c->x.p, c->xp.p, c->ox.p, c->oxp.p};
@@ -609,8 +743,8 @@ ys_status broad_args(ys_collider* c, bool masked, BroadArgs& a, int64_t& work) {
   a = BroadArgs{};
   a.cloth = DevTree{c->c_left.p, c->c_right.p, c->c_face.p, c->c_box.p, (int)c->ct.face.size(), c->c_fbox.p};
   a.obs = DevTree{c->o_left.p, c->o_right.p, c->o_face.p, c->o_box.p, (int)c->ot.face.size(), c->o_fbox.p};
-  a.thick1 = (float)(c->thickness * (1.0 + 1e-6));
-  a.thick2 = (float)(std::sqrt(2.0) * c->thickness * (1.0 + 1e-6));
+  a.thick1 = prune1(c->thickness);
+  a.thick2 = prune2(c->thickness);
   a.leaf_of_face = c->c_lof.p;
   a.rank = c->c_rank.p;
   a.upper = c->c_upper.p;
@@ -657,30 +791,48 @@ ys_status broad_phase(ys_collider* c, bool masked) {
   return YS_OK;
 }
 
+// the narrow phase's buffers for n pairs
+ys_status narrow_reserve(ys_collider* c, int64_t n) {
+  const int nn = std::max(c->n_nodes + c->n_obs_nodes, 1);
+  YC_CUDA(c->slots.reserve(15 * (size_t)n));
+  YC_CUDA(c->icount.reserve(n));
+  YC_CUDA(c->ioffset.reserve(n));
+  YC_CUDA(c->tmask.reserve(n));
+  YC_CUDA(c->tlist.reserve(15 * (size_t)n));
+  YC_CUDA(c->tlist_n.reserve(2));
+  YC_CUDA(c->nkdop.reserve(nn));
+  YC_CUDA(c->nfbox.reserve(kFBox * (size_t)nn));
+  return YS_OK;
+}
+// the tests of n pairs (np_dev: their number on the device, at most n)
+void narrow_kernels(ys_collider* c, int64_t n, const int64_t* np_dev) {
+  CMesh m{c->x.p, c->xp.p, c->ox.p, c->oxp.p};
+  const int nn = c->n_nodes + c->n_obs_nodes;
+  k_node_kdop<<<(nn + 127) / 128, 128, 0, c->stream>>>(m, c->n_nodes, c->n_obs_nodes, c->ccd, c->nkdop.p, c->nfbox.p,
+                                                       c->tlist_n.p);
+  k_narrow_mask<<<(unsigned)((n + 127) / 128), 128, 0, c->stream>>>(
+      c->pairs.p, n, c->faces.p, c->ofaces.p, NodeKdops{c->nkdop.p, c->nfbox.p, c->n_nodes}, c->thickness,
+      prune1(c->thickness), prune2(c->thickness), c->tmask.p, c->icount.p, c->tlist.p,
+      reinterpret_cast<unsigned long long*>(c->tlist_n.p), np_dev);
+  const int64_t blocks = std::min<int64_t>((15 * n + 127) / 128, kTestBlocks);
+  k_narrow_test<<<(unsigned)blocks, 128, 0, c->stream>>>(c->pairs.p, n, c->faces.p, c->ofaces.p, m, c->tlist.p,
+                                                         c->tlist_n.p, c->slots.p,
+                                                         reinterpret_cast<unsigned long long*>(c->icount.p));
+}
+
 ys_status narrow_phase(ys_collider* c) {
   const int64_t P = c->npairs;
-  YC_CUDA(c->slots.reserve(15 * (size_t)std::max<int64_t>(P, 1)));
-  YC_CUDA(c->icount.reserve(std::max<int64_t>(P, 1)));
-  YC_CUDA(c->ioffset.reserve(std::max<int64_t>(P, 1)));
-  YC_CUDA(c->tmask.reserve(std::max<int64_t>(P, 1)));
-  YC_CUDA(c->nkdop.reserve(std::max(c->n_nodes + c->n_obs_nodes, 1)));
-  CMesh m{c->x.p, c->xp.p, c->ox.p, c->oxp.p};
+  const ys_status sr = narrow_reserve(c, std::max<int64_t>(P, 1));
+  if (sr != YS_OK) return sr;
   if (P) {
-    const int nn = c->n_nodes + c->n_obs_nodes;
-    k_node_kdop<<<(nn + 127) / 128, 128, 0, c->stream>>>(m, c->n_nodes, c->n_obs_nodes, c->ccd, c->nkdop.p);
-    k_narrow_mask<<<(unsigned)((P + 127) / 128), 128, 0, c->stream>>>(c->pairs.p, P, c->faces.p, c->ofaces.p,
-                                                                       NodeKdops{c->nkdop.p, c->n_nodes},
-                                                                       c->thickness, c->tmask.p, c->icount.p, nullptr);
-    k_narrow_test<<<(unsigned)((15 * P + 127) / 128), 128, 0, c->stream>>>(
-        c->pairs.p, P, c->faces.p, c->ofaces.p, m, c->tmask.p, c->slots.p,
-        reinterpret_cast<unsigned long long*>(c->icount.p));
+    narrow_kernels(c, P, nullptr);
     YC_CUDA(cudaGetLastError());
   }
   ys_status s = scan(c, c->icount.p, P, c->ioffset.p, &c->nimpacts);
   if (s != YS_OK) return s;
   YC_CUDA(c->impacts.reserve(std::max<int64_t>(c->nimpacts, 1)));
   if (P) {
-    k_compact<<<(unsigned)((P + 127) / 128), 128, 0, c->stream>>>(c->slots.p, c->icount.p, c->ioffset.p, P,
+    k_compact<<<(unsigned)((P + 127) / 128), 128, 0, c->stream>>>(c->slots.p, c->tmask.p, c->icount.p, c->ioffset.p, P,
                                                                    c->impacts.p, nullptr, c->nimpacts,
                                                                    c->overflow.p);
     YC_CUDA(cudaGetLastError());
@@ -710,11 +862,8 @@ ys_status detect_one_wait(ys_collider* c, bool masked, std::vector<ys_impact>& g
     YC_CUDA(c->sums.reserve(std::max<int64_t>(nb, 1)));
     YC_CUDA(c->total.reserve(2));
     YC_CUDA(c->pairs.reserve(3 * (size_t)cp));
-    YC_CUDA(c->slots.reserve(15 * (size_t)cp));
-    YC_CUDA(c->icount.reserve(cp));
-    YC_CUDA(c->ioffset.reserve(cp));
-    YC_CUDA(c->tmask.reserve(cp));
-    YC_CUDA(c->nkdop.reserve(std::max(c->n_nodes + c->n_obs_nodes, 1)));
+    s = narrow_reserve(c, cp);
+    if (s != YS_OK) return s;
     YC_CUDA(c->impacts.reserve(ci));
     if (c->pin_imp_cap < ci) {
       if (c->pin_imp) cudaFreeHost(c->pin_imp);
@@ -733,18 +882,9 @@ ys_status detect_one_wait(ys_collider* c, bool masked, std::vector<ys_impact>& g
     a.out = c->pairs.p;
     a.cap = cp;
     if (work) k_broad<true><<<g, kBroadBlock, 0, c->stream>>>(a);
-    CMesh m{c->x.p, c->xp.p, c->ox.p, c->oxp.p};
-    const int nn = c->n_nodes + c->n_obs_nodes;
-    k_node_kdop<<<(nn + 127) / 128, 128, 0, c->stream>>>(m, c->n_nodes, c->n_obs_nodes, c->ccd, c->nkdop.p);
-    k_narrow_mask<<<(unsigned)((cp + 127) / 128), 128, 0, c->stream>>>(c->pairs.p, cp, c->faces.p, c->ofaces.p,
-                                                                        NodeKdops{c->nkdop.p, c->n_nodes},
-                                                                        c->thickness, c->tmask.p, c->icount.p,
-                                                                        np_dev);
-    k_narrow_test<<<(unsigned)((15 * cp + 127) / 128), 128, 0, c->stream>>>(
-        c->pairs.p, cp, c->faces.p, c->ofaces.p, m, c->tmask.p, c->slots.p,
-        reinterpret_cast<unsigned long long*>(c->icount.p));
+    narrow_kernels(c, cp, np_dev);
     scan_kernels(c, c->icount.p, cp, c->ioffset.p, ni_dev);
-    k_compact<<<(unsigned)((cp + 127) / 128), 128, 0, c->stream>>>(c->slots.p, c->icount.p, c->ioffset.p, cp,
+    k_compact<<<(unsigned)((cp + 127) / 128), 128, 0, c->stream>>>(c->slots.p, c->tmask.p, c->icount.p, c->ioffset.p, cp,
                                                                     c->impacts.p, np_dev, ci, c->overflow.p);
     YC_CUDA(cudaGetLastError());
     YC_CUDA(cudaMemcpyAsync(c->pin, c->total.p, 2 * sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream));
