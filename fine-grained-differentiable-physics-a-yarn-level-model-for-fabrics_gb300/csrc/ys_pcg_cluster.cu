@@ -245,6 +245,7 @@ cudaError_t with_kernel(int groups, bool cluster, bool trans, F&& f) {
   YS_PCGC(128, true)
   YS_PCGC(256, false)
   YS_PCGC(512, false)
+  YS_PCGC(640, false)
   YS_PCGC(1024, false)
 #undef YS_PCGC
   return cudaErrorInvalidValue;
