@@ -40,9 +40,9 @@ __device__ __forceinline__ double pcg_threshold(double tol, double bb) {
 // spmv_row_sv and spmv_row_tv. i(du, dv): the row to read for the neighbour
 // there, negative outside the cloth.
 template <bool TRANS, class Row>
-__device__ __forceinline__ double row_coef(const double* __restrict__ A, int64_t nt, int n, int m, int j,
+__device__ __forceinline__ double row_coef(const double* A, int64_t nt, int n, int m, int j,
                                            const Row& i) {
-  auto at = [&](int slot, int row) { return row < 0 ? 0.0 : __ldg(A + (int64_t)slot * nt + row); };
+  auto at = [&](int slot, int row) { return row < 0 ? 0.0 : A[(int64_t)slot * nt + row]; };
   auto nbr = [&](int mm) { return TRANS ? i(mm == 0 ? -1 : mm == 1 ? 1 : 0, mm == 2 ? -1 : mm == 3 ? 1 : 0) : n; };
   if (m < 3) {
     if (j < 39) {
