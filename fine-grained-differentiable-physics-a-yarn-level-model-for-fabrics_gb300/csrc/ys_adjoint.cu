@@ -86,8 +86,9 @@ struct Weights {
 // EPos [2][nt], EVel [2][nt], EPosBar [2][nt] (component-major). Writes
 // qbar [5][nt], the pass-through part of g (gout, same layout) and
 // slide_bar [2][nt].
-__global__ void k_adj_update(View v, AdjIO io, const double* __restrict__ q, double* __restrict__ qbar,
-                             double* __restrict__ slide_bar) {
+__global__ void k_adj_update(View v, AdjIO io, const double* q, double* qbar,
+                             double* slide_bar) {
+  chained();
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= v.ntot) return;
   const int nt = v.ntot;
@@ -119,6 +120,7 @@ __global__ void k_adj_update(View v, AdjIO io, const double* __restrict__ q, dou
 
 // one thread per (pair, segment type, crossing)
 __global__ void __launch_bounds__(64) k_adj_shear(View v, AdjWork w) {
+  chained();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int nt = v.ntot;
   if (t >= (int64_t)kShearPairs * 4 * nt) return;
@@ -157,6 +159,7 @@ __global__ void __launch_bounds__(64) k_adj_shear(View v, AdjWork w) {
 // (as k_cross), then each of two yarns' derivatives in two warps of two pairs
 // each. comp and ce are the only inputs that lead to other elements.
 __global__ void __launch_bounds__(128) k_adj_cross(View v, Records R, AdjWork w) {
+  chained();
   __shared__ double sc[3][4][32], sk[6][4][32], sg[2][kCrossVars][32];
   const int m = threadIdx.x >> 5, i = threadIdx.x & 31;
   const int node = blockIdx.x * 32 + i;
@@ -234,6 +237,7 @@ __global__ void __launch_bounds__(128) k_adj_cross(View v, Records R, AdjWork w)
 
 // one thread per (pair, yarn direction, node): the edge starting at that node
 __global__ void __launch_bounds__(64) k_adj_edge(View v, AdjWork w) {
+  chained();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int nt = v.ntot;
   if (t >= (int64_t)kEdgePairs * 2 * nt) return;
@@ -312,6 +316,7 @@ __global__ void __launch_bounds__(64) k_adj_edge(View v, AdjWork w) {
 
 // one thread per (pair, yarn direction, middle node)
 __global__ void __launch_bounds__(64) k_adj_bend(View v, AdjWork w) {
+  chained();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int nt = v.ntot;
   if (t >= (int64_t)kBendPairs * 2 * nt) return;
@@ -397,6 +402,7 @@ __global__ void __launch_bounds__(64) k_adj_bend(View v, AdjWork w) {
 
 // one thread per (pair, face of a cell, cell)
 __global__ void __launch_bounds__(64) k_adj_face(View v, AdjWork w) {
+  chained();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int nt = v.ntot;
   if (t >= (int64_t)kFacePairs * 2 * nt) return;
@@ -422,11 +428,12 @@ __global__ void __launch_bounds__(64) k_adj_face(View v, AdjWork w) {
 
 // The normal's adjoint at an interior crossing (friction's, and the crimp
 // offsets' of the up to six bend segments it is part of) carried to the
-// scatter matrix: with eigenpairs (l_j, v_j) and the normal v_m, phi changes by
-// g^T dS v_m, g = sum_{j != m} (n_bar . v_j) / (l_m - l_j) v_j
-// (node_normal_dual's perturbation, transposed). Writes g, v_m and the
-// crossing's mean; k_adj_gather forms the five positions' shares.
+// scatter matrix: with eigenpairs (l_j, v_j) and the normal n = +-v_m, phi changes
+// by g^T dS n, g = sum_{j != m} (n_bar . v_j) / (l_m - l_j) v_j
+// (node_normal_dual's perturbation, transposed). Writes g, n and the crossing's
+// mean; k_adj_gather forms the five positions' shares.
 __global__ void __launch_bounds__(128) k_adj_normal(View v, const int* __restrict__ nodes, int count, AdjWork w) {
+  chained();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= count) return;
   const int n = nodes[t], nt = v.ntot;
@@ -448,27 +455,18 @@ __global__ void __launch_bounds__(128) k_adj_normal(View v, const int* __restric
     }
   }
   const int ids[5] = {n, n - 1, n + 1, n - N.W, n + N.W};
-  double p[5][3], mean[3] = {0, 0, 0}, S[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}}, a[3][3], V[3][3];
+  double p[5][3], mean[3] = {0, 0, 0}, S[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}}, nn[3], g[3];
   for (int m = 0; m < 5; ++m)
     for (int i = 0; i < 3; ++i) { p[m][i] = ld(v.X, i, nt, ids[m]); mean[i] += p[m][i]; }
   for (int i = 0; i < 3; ++i) mean[i] /= 5.0;
   for (int m = 0; m < 5; ++m)
     for (int i = 0; i < 3; ++i)
       for (int j = 0; j < 3; ++j) S[i][j] += (p[m][i] - mean[i]) * (p[m][j] - mean[j]);
-  sym3_jacobi(S, a, V);
-  const int mm = sym3_argmin(a);
-  // the step's normal is +-v_m: the sign cancels in (n_bar . v_j) (v_j . dS n)
-  double sgn = 0.0, g[3] = {0, 0, 0};
-  for (int i = 0; i < 3; ++i) sgn += V[i][mm] * ld(v.NRM, i, nt, n);
-  sgn = sgn < 0.0 ? -1.0 : 1.0;
-  for (int j = 0; j < 3; ++j) {
-    if (j == mm) continue;
-    const double c = (nb[0] * V[0][j] + nb[1] * V[1][j] + nb[2] * V[2][j]) / (a[mm][mm] - a[j][j]);
-    for (int i = 0; i < 3; ++i) g[i] += c * V[i][j];
-  }
+  for (int i = 0; i < 3; ++i) nn[i] = ld(v.NRM, i, nt, n);
+  NormalResponse(S, nn).respond(nb, g);
   for (int i = 0; i < 3; ++i) {
     w.normal[(int64_t)i * nt + n] = g[i];
-    w.normal[(int64_t)(3 + i) * nt + n] = sgn * V[i][mm];
+    w.normal[(int64_t)(3 + i) * nt + n] = nn[i];
     w.normal[(int64_t)(6 + i) * nt + n] = mean[i];
   }
 }
@@ -476,6 +474,7 @@ __global__ void __launch_bounds__(128) k_adj_normal(View v, const int* __restric
 // adds every element's share to node n's state adjoints, in a fixed order;
 // one thread per (component, node): x, y, z and the two yarns
 __global__ void __launch_bounds__(128) k_adj_gather(View v, AdjWork w, AdjIO io) {
+  chained();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int nt = v.ntot;
   if (t >= 5LL * nt) return;
@@ -550,14 +549,19 @@ __global__ void __launch_bounds__(128) k_adj_gather(View v, AdjWork w, AdjIO io)
   io.gout[1][(int64_t)r * nt + n] += gv;
 }
 
-// material adjoints, one warp each: rho, Y, B of every line over the line's
+constexpr int kParamThreads = 256;
+// material adjoints: rho, Y, B of every line, one warp each, over the line's
 // edges and bend segments (ks, kb = (Y, B) a, a = pi R^2), S and mu of every
-// cloth over its crossings
-__global__ void __launch_bounds__(128) k_adj_params(View v, AdjWork w, const double* __restrict__ line_a,
+// cloth, one block each (one warp took 97 us over a 50 x 50 cloth's crossings)
+__global__ void __launch_bounds__(kParamThreads) k_adj_params(View v, AdjWork w, const double* __restrict__ line_a,
                                                     const int* __restrict__ line_cloth, AdjParamOut gp) {
-  const int id = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  chained();
+  __shared__ double sh[2][kParamThreads / 32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int nl = v.nlines, nt = v.ntot;
-  if (id < nl) {
+  if ((int)blockIdx.x >= v.ncloth) {
+    const int id = (blockIdx.x - v.ncloth) * (kParamThreads / 32) + wid;
+    if (id >= nl) return;
     const ClothParams& P = v.cp[line_cloth[id]];
     const bool weft = id >= P.weft_line_off;
     const int k = weft ? 1 : 0, at = weft ? id - P.weft_line_off : id - P.warp_line_off;
@@ -572,11 +576,11 @@ __global__ void __launch_bounds__(128) k_adj_params(View v, AdjWork w, const dou
       const double x = cloth_tree(s[p]);
       if (lane == 0) gp.line[p][id] = p == 0 ? x : x * line_a[id];
     }
-  } else if (id < nl + v.ncloth) {
-    const int c = id - nl;
+  } else {
+    const int c = blockIdx.x;
     const ClothParams& P = v.cp[c];
     double sS = 0.0, sm = 0.0;
-    for (int i = lane; i < P.W * P.H; i += 32) {
+    for (int i = threadIdx.x; i < P.W * P.H; i += kParamThreads) {
       const int n = P.node_off + i;
       sm += w.cross[(int64_t)kC_MU * nt + n];
       if (!(v.flags[n] & YS_INTERIOR)) continue;
@@ -586,13 +590,20 @@ __global__ void __launch_bounds__(128) k_adj_params(View v, AdjWork w, const dou
     }
     sS = cloth_tree(sS);
     sm = cloth_tree(sm);
-    if (lane == 0) { gp.cloth[0][c] = sS; gp.cloth[1][c] = sm; }
+    if (lane == 0) { sh[0][wid] = sS; sh[1][wid] = sm; }
+    __syncthreads();
+    if (threadIdx.x < 2) {
+      double x = 0.0;
+      for (int i = 0; i < kParamThreads / 32; ++i) x += sh[threadIdx.x][i];
+      gp.cloth[threadIdx.x][c] = x;
+    }
   }
 }
 
 // dL/d ext = h lambda on the components the gather adds ext to (x, y, z of
 // every node, u, v of interior crossings); node layout [nt][5]
-__global__ void k_adj_ext(View v, const double* __restrict__ lambda, double* __restrict__ gext) {
+__global__ void k_adj_ext(View v, const double* lambda, double* gext) {
+  chained();
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= v.ntot) return;
   const bool in = (v.flags[n] & YS_INTERIOR) != 0;
@@ -608,24 +619,24 @@ AdjSizes adjoint_sizes() {
 
 void launch_adj_update(const View& v, const AdjIO& io, const double* q, double* qbar, double* slide_bar,
                        cudaStream_t s) {
-  k_adj_update<<<nbl(v.ntot, 256), 256, 0, s>>>(v, io, q, qbar, slide_bar);
+  chain(k_adj_update, nbl(v.ntot, 256), 256, s, v, io, q, qbar, slide_bar);
 }
 int launch_adj_vjp(const View& v, const Records& R, const AdjWork& w, const int* interior, int n_interior,
                    const AdjIO& io, const double* line_a, const int* line_cloth, const AdjParamOut& gp,
                    cudaStream_t s) {
   const int64_t nt = v.ntot;
-  k_adj_shear<<<nbl(kShearPairs * 4 * nt, 64), 64, 0, s>>>(v, w);
-  k_adj_cross<<<nbl(nt, 32), 128, 0, s>>>(v, R, w);
-  k_adj_edge<<<nbl(kEdgePairs * 2 * nt, 64), 64, 0, s>>>(v, w);
-  k_adj_bend<<<nbl(kBendPairs * 2 * nt, 64), 64, 0, s>>>(v, w);
-  k_adj_face<<<nbl(kFacePairs * 2 * nt, 64), 64, 0, s>>>(v, w);
-  k_adj_normal<<<nbl(n_interior, 128), 128, 0, s>>>(v, interior, n_interior, w);
-  k_adj_gather<<<nbl(5 * nt, 128), 128, 0, s>>>(v, w, io);
-  k_adj_params<<<nbl(32LL * (v.nlines + v.ncloth), 128), 128, 0, s>>>(v, w, line_a, line_cloth, gp);
+  chain(k_adj_shear, nbl(kShearPairs * 4 * nt, 64), 64, s, v, w);
+  chain(k_adj_cross, nbl(nt, 32), 128, s, v, R, w);
+  chain(k_adj_edge, nbl(kEdgePairs * 2 * nt, 64), 64, s, v, w);
+  chain(k_adj_bend, nbl(kBendPairs * 2 * nt, 64), 64, s, v, w);
+  chain(k_adj_face, nbl(kFacePairs * 2 * nt, 64), 64, s, v, w);
+  chain(k_adj_normal, nbl(n_interior, 128), 128, s, v, interior, n_interior, w);
+  chain(k_adj_gather, nbl(5 * nt, 128), 128, s, v, w, io);
+  chain(k_adj_params, v.ncloth + nbl(v.nlines, kParamThreads / 32), kParamThreads, s, v, w, line_a, line_cloth, gp);
   return 8;
 }
 void launch_adj_ext(const View& v, const double* lambda, double* gext, cudaStream_t s) {
-  k_adj_ext<<<nbl(v.ntot, 256), 256, 0, s>>>(v, lambda, gext);
+  chain(k_adj_ext, nbl(v.ntot, 256), 256, s, v, lambda, gext);
 }
 
 }  // namespace ys

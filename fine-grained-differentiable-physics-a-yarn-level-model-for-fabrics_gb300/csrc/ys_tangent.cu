@@ -59,15 +59,14 @@ struct Scratch {
 
 }  // namespace
 
-// Tangents of the normal n = +-v_m, the eigenvector of the smallest eigenvalue
-// l_m of the stencil's scatter matrix S: dn = sum_{j != m} (v_j . dS n) /
-// (l_m - l_j) v_j. One eigensystem a node serves every direction.
+// Tangents of the normals: the stencil's scatter matrix S changes by dS
 __global__ void __launch_bounds__(64) k_tan_geom(View v, const int* __restrict__ nodes, int count) {
+  chained();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= count) return;
   const int n = nodes[t], nt = v.ntot, W = v.cp[v.node_cloth[n]].W;
   const int ids[5] = {n, n - 1, n + 1, n - W, n + W};
-  double p[5][3], mean[3] = {0, 0, 0}, S[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}}, a[3][3], V[3][3], nn[3];
+  double p[5][3], mean[3] = {0, 0, 0}, S[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}}, nn[3];
   for (int m = 0; m < 5; ++m)
     for (int i = 0; i < 3; ++i) { p[m][i] = ld(v.X, i, nt, ids[m]); mean[i] += p[m][i]; }
   for (int m = 0; m < 5; ++m)
@@ -75,11 +74,10 @@ __global__ void __launch_bounds__(64) k_tan_geom(View v, const int* __restrict__
   for (int m = 0; m < 5; ++m)
     for (int i = 0; i < 3; ++i)
       for (int j = 0; j < 3; ++j) S[i][j] += p[m][i] * p[m][j];
-  sym3_jacobi(S, a, V);
-  const int mm = sym3_argmin(a);
   for (int i = 0; i < 3; ++i) nn[i] = ld(v.NRM, i, nt, n);
+  const NormalResponse N(S, nn);
   for (int k = 0; k < K; ++k) {
-    double g[3] = {0, 0, 0}, dn[3] = {0, 0, 0};  // dS n (the mean's share sums to 0)
+    double g[3] = {0, 0, 0}, dn[3];  // dS n (the mean's share sums to 0)
     for (int m = 0; m < 5; ++m) {
       double x[3], rn = 0.0, xn = 0.0;
       for (int i = 0; i < 3; ++i) {
@@ -89,17 +87,14 @@ __global__ void __launch_bounds__(64) k_tan_geom(View v, const int* __restrict__
       }
       for (int i = 0; i < 3; ++i) g[i] += x[i] * rn + p[m][i] * xn;
     }
-    for (int j = 0; j < 3; ++j) {
-      if (j == mm) continue;
-      const double c = (V[0][j] * g[0] + V[1][j] * g[1] + V[2][j] * g[2]) / (a[mm][mm] - a[j][j]);
-      for (int i = 0; i < 3; ++i) dn[i] += c * V[i][j];
-    }
+    N.respond(g, dn);
     for (int i = 0; i < 3; ++i) v.dNRM[((int64_t)i * K + k) * nt + n] = dn[i];
   }
 }
 
 // q: the solution, null in the reference mode (no dA q)
-__global__ void __launch_bounds__(64) k_tan_edge(View v, const double* __restrict__ q, double* scratch) {
+__global__ void __launch_bounds__(64) k_tan_edge(View v, const double* q, double* scratch) {
+  chained();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int nt = v.ntot;
   if (t >= 2 * nt) return;
@@ -157,7 +152,8 @@ __global__ void __launch_bounds__(64) k_tan_edge(View v, const double* __restric
   for (int i = 0; i < 8; ++i) put(kTE_r + i, r[i]);
 }
 
-__global__ void __launch_bounds__(64) k_tan_bend(View v, const double* __restrict__ q, double* scratch) {
+__global__ void __launch_bounds__(64) k_tan_bend(View v, const double* q, double* scratch) {
+  chained();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int nt = v.ntot;
   if (t >= 2 * nt) return;
@@ -240,6 +236,7 @@ __global__ void __launch_bounds__(64) k_tan_bend(View v, const double* __restric
 }
 
 __global__ void __launch_bounds__(64) k_tan_face(View v, double* scratch) {
+  chained();
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   const int nt = v.ntot;
   if (n >= 2 * nt) return;
@@ -257,7 +254,8 @@ __global__ void __launch_bounds__(64) k_tan_face(View v, double* scratch) {
 // Compression and friction at the crossings (k_cross): values from the step's
 // records R, tangents from the scratch; writes dCOMP, dSLIDE and the tangent
 // of bE - aEE q
-__global__ void __launch_bounds__(128) k_tan_cross(View v, Records R, const double* __restrict__ q, double* scratch) {
+__global__ void __launch_bounds__(128) k_tan_cross(View v, Records R, const double* q, double* scratch) {
+  chained();
   __shared__ double sc[3][4][32], sk[6][4][32], tc[3][4][32], tk[6][4][32];
   const int m = threadIdx.x >> 5, i = threadIdx.x & 31;
   const int node = blockIdx.x * 32 + i;
@@ -337,7 +335,8 @@ __global__ void __launch_bounds__(128) k_tan_cross(View v, Records R, const doub
   S.cross[(int64_t)k * nt + n] = bE.d[0] - (q ? aEE.d[0] * q[(int64_t)(3 + k) * nt + n] : 0.0);
 }
 
-__global__ void __launch_bounds__(64) k_tan_shear(View v, const double* __restrict__ q, double* scratch) {
+__global__ void __launch_bounds__(64) k_tan_shear(View v, const double* q, double* scratch) {
+  chained();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int nt = v.ntot;
   if (t >= 4LL * nt) return;
@@ -369,8 +368,9 @@ __global__ void __launch_bounds__(64) k_tan_shear(View v, const double* __restri
 // rt[k][c][ntot]: every element's residual at node n, one thread per
 // (component, node); dext (or null) [kact][ntot][5]: the external force's
 // tangents, which add h dext where the rows add h ext
-__global__ void __launch_bounds__(128) k_tan_gather(View v, double* scratch, const double* __restrict__ dext,
-                                                    double* __restrict__ rt) {
+__global__ void __launch_bounds__(128) k_tan_gather(View v, double* scratch, const double* dext,
+                                                    double* rt) {
+  chained();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int nt = v.ntot, dirn = blockIdx.y;
   if (t >= 5LL * nt) return;
@@ -419,8 +419,9 @@ __global__ void __launch_bounds__(128) k_tan_gather(View v, double* scratch, con
 }
 
 // Cloth::update of state and tangents for every cloth whose step succeeded
-__global__ void __launch_bounds__(kBlock) k_update_dual(View v, Blocks b, Solver so, const double* __restrict__ dq,
+__global__ void __launch_bounds__(kBlock) k_update_dual(View v, Blocks b, Solver so, const double* dq,
                                                         TangentState ts) {
+  chained();
   const int blk = blockIdx.x;
   const int c = b.blk_cloth[blk];
   const int n = b.blk_node0[blk] + threadIdx.x;
@@ -434,19 +435,19 @@ int launch_tangent_residual(const View& v, const Records& R, const int* interior
   const int64_t nt = v.ntot;
   const double* x = v.trunc ? nullptr : q;
   auto grid = [](int64_t n, int t, int k) { return dim3((unsigned)((n + t - 1) / t), (unsigned)k); };
-  k_tan_geom<<<grid(n_interior, 64, 1), 64, 0, s>>>(v, interior, n_interior);
-  k_tan_edge<<<grid(2 * nt, 64, K), 64, 0, s>>>(v, x, scratch);
-  k_tan_bend<<<grid(2 * nt, 64, K), 64, 0, s>>>(v, x, scratch);
-  k_tan_face<<<grid(2 * nt, 64, K), 64, 0, s>>>(v, scratch);
-  k_tan_cross<<<grid(nt, 32, K), 128, 0, s>>>(v, R, x, scratch);
-  k_tan_shear<<<grid(4 * nt, 64, K), 64, 0, s>>>(v, x, scratch);
-  if (kact > 0) k_tan_gather<<<grid(5 * nt, 128, kact), 128, 0, s>>>(v, scratch, dext, rt);
+  chain(k_tan_geom, grid(n_interior, 64, 1), 64, s, v, interior, n_interior);
+  chain(k_tan_edge, grid(2 * nt, 64, K), 64, s, v, x, scratch);
+  chain(k_tan_bend, grid(2 * nt, 64, K), 64, s, v, x, scratch);
+  chain(k_tan_face, grid(2 * nt, 64, K), 64, s, v, scratch);
+  chain(k_tan_cross, grid(nt, 32, K), 128, s, v, R, x, scratch);
+  chain(k_tan_shear, grid(4 * nt, 64, K), 64, s, v, x, scratch);
+  if (kact > 0) chain(k_tan_gather, grid(5 * nt, 128, kact), 128, s, v, scratch, dext, rt);
   return 7;
 }
 void launch_update_dual(const View& v, const Blocks& b, const Solver& so, const double* dq, const TangentState& ts,
                         cudaStream_t s) {
   launch_check_solution(v, b, so, s);
-  k_update_dual<<<b.nblk, kBlock, 0, s>>>(v, b, so, dq, ts);
+  chain(k_update_dual, b.nblk, kBlock, s, v, b, so, dq, ts);
 }
 
 }  // namespace ys
