@@ -769,15 +769,22 @@ ys_status ys_assemble(ys_batch* b, double h, const double* ext_force, int32_t fl
   }
   cudaStream_t s = b->stream;
   const ys::View& v = b->v;
-  b->run(YS_PROF_MISC, 1, [&] { k_reset_status<<<(b->ncloth + 127) / 128, 128, 0, s>>>(b->so.pc, b->ncloth); });
-  // UpdateClothUnits normals for the current positions (src/Cloth.cpp:307-327)
-  if (b->geom_n) b->run(YS_PROF_GEOM, 1, [&] { ys::launch_geom(v, b->anchors + b->geom_off, b->geom_n, s); });
+  // UpdateClothUnits normals for the current positions (src/Cloth.cpp:307-327),
   // element records (FillMV's element loops, src/PhysicsCloth.cpp:64-95)
   const ys::Records& R = b->rec;
   const int pt = b->producer_threads;
-  b->run(YS_PROF_EDGES, 1, [&] { ys::launch_edge_records(v, R, s, pt); });
-  b->run(YS_PROF_BENDS, 1, [&] { ys::launch_bend_records(v, R, s, pt); });
-  b->run(YS_PROF_FACES, 1, [&] { ys::launch_face_records(v, R, s, pt); });
+  if (b->blk.by_rows && !b->profiling) {
+    b->run(YS_PROF_MISC, 1, [&] {
+      ys::launch_state_records(v, R, b->anchors + b->geom_off, b->geom_n, b->so.pc, s);
+    });
+    b->run(YS_PROF_BENDS, 1, [&] { ys::launch_bend_records(v, R, s, pt); });
+  } else {
+    b->run(YS_PROF_MISC, 1, [&] { k_reset_status<<<(b->ncloth + 127) / 128, 128, 0, s>>>(b->so.pc, b->ncloth); });
+    if (b->geom_n) b->run(YS_PROF_GEOM, 1, [&] { ys::launch_geom(v, b->anchors + b->geom_off, b->geom_n, s); });
+    b->run(YS_PROF_EDGES, 1, [&] { ys::launch_edge_records(v, R, s, pt); });
+    b->run(YS_PROF_BENDS, 1, [&] { ys::launch_bend_records(v, R, s, pt); });
+    b->run(YS_PROF_FACES, 1, [&] { ys::launch_face_records(v, R, s, pt); });
+  }
   // ConSlideFriction (needs every edge and bend term; shear needs its
   // compression, src/PhysicsCloth.cpp:97-131), then the row blocks
   b->run(YS_PROF_GATHER, 1, [&] { ys::launch_cross(v, R, s); });

@@ -16,12 +16,14 @@ namespace ys {
 
 static inline int nblocks(int n) { return (n + kBlock - 1) / kBlock; }
 
-__global__ void k_geom(View v, const int* __restrict__ nodes, int count) {
-  chained();
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void geom_item(const View& v, const int* nodes, int count, int t) {
   if (t >= count) return;
   const int n = nodes[t];
   node_normal(v, n, v.cp[v.node_cloth[n]].W);
+}
+__global__ void k_geom(View v, const int* __restrict__ nodes, int count) {
+  chained();
+  geom_item(v, nodes, count, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 // The record producers: one thread per element, nothing shared between
@@ -31,9 +33,7 @@ __global__ void k_geom(View v, const int* __restrict__ nodes, int count) {
 // blocks).
 
 // one thread per (yarn direction, node): the edge starting at that node
-__global__ void __launch_bounds__(kBlock) k_edge_rec(View v, Records R) {
-  chained();
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void edge_item(const View& v, const Records& R, int64_t t) {
   if (t >= 2LL * v.ntot) return;
   const int k = t >= v.ntot ? 1 : 0;
   const int n0 = (int)(t - (int64_t)k * v.ntot);
@@ -41,7 +41,11 @@ __global__ void __launch_bounds__(kBlock) k_edge_rec(View v, Records R) {
   if (k == 0 ? v.node_u[n0] >= P.W - 1 : v.node_v[n0] >= P.H - 1) return;
   // each field goes to memory as soon as it is known, so none is held
   edge_terms<double>(v, n0, n0 + (k == 0 ? 1 : P.W), k,
-                [&](int f, double x) { stT(R.edge, R.dedge, 2 * f + k, v.ntot, n0, x); });
+                     [&](int f, double x) { stT(R.edge, R.dedge, 2 * f + k, v.ntot, n0, x); });
+}
+__global__ void __launch_bounds__(kBlock) k_edge_rec(View v, Records R) {
+  chained();
+  edge_item(v, R, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 // one thread per (yarn direction, middle node) of a bend segment
@@ -60,13 +64,30 @@ __global__ void __launch_bounds__(kMaxProducerBlock) k_bend_rec(View v, Records 
 }
 
 // one thread per grid cell (top-left node): its two faces
-__global__ void __launch_bounds__(kMaxProducerBlock) k_face_rec(View v, Records R) {
-  chained();
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void face_item(const View& v, const Records& R, int n) {
   if (n >= v.ntot) return;
   const ClothParams& P = v.cp[v.node_cloth[n]];
   if (v.node_u[n] >= P.W - 1 || v.node_v[n] >= P.H - 1) return;
   cell_faces<double>(v, R.face, R.dface, n);
+}
+__global__ void __launch_bounds__(kMaxProducerBlock) k_face_rec(View v, Records R) {
+  chained();
+  face_item(v, R, blockIdx.x * blockDim.x + threadIdx.x);
+}
+
+// What depends on the state alone in one launch, for batches that leave SMs idle
+// (Blocks::by_rows) launch by launch: normals, edges, faces, the cloths' status
+// cleared. Each of the three is 8 to 20 us of one thread's latency on a small
+// cloth. Blocks [0, ng) take the normals, the next ne the edges, the rest faces.
+__global__ void __launch_bounds__(kBlock) k_state_rec(View v, Records R, const int* __restrict__ nodes, int count,
+                                                      PcgCloth* pc, int ng, int ne) {
+  chained();
+  const int blk = blockIdx.x;
+  if (blk == 0)
+    for (int c = threadIdx.x; c < v.ncloth; c += kBlock) pc[c].status = 0;
+  if (blk < ng) geom_item(v, nodes, count, blk * kBlock + threadIdx.x);
+  else if (blk < ng + ne) edge_item(v, R, (int64_t)(blk - ng) * kBlock + threadIdx.x);
+  else face_item(v, R, (blk - ng - ne) * kBlock + threadIdx.x);
 }
 
 // one thread per (segment type, crossing)
@@ -478,6 +499,10 @@ void launch_bend_records(const View& v, const Records& R, cudaStream_t s, int t)
 }
 void launch_face_records(const View& v, const Records& R, cudaStream_t s, int t) {
   chain(k_face_rec, pblocks(v.ntot, t), t, s, v, R);
+}
+void launch_state_records(const View& v, const Records& R, const int* nodes, int n, PcgCloth* pc, cudaStream_t s) {
+  const unsigned ng = pblocks(n, kBlock), ne = pblocks(2LL * v.ntot, kBlock), nf = pblocks(v.ntot, kBlock);
+  chain(k_state_rec, ng + ne + nf, kBlock, s, v, R, nodes, n, pc, (int)ng, (int)ne);
 }
 void launch_cross(const View& v, const Records& R, cudaStream_t s) {
   chain(k_cross, pblocks(v.ntot, kNodesPerBlock), 4 * kNodesPerBlock, s, v, R);

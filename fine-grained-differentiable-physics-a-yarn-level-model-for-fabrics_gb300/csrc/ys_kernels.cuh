@@ -92,6 +92,8 @@ void launch_bend_records(const View& v, const Records& R, cudaStream_t s, int th
 void launch_face_records(const View& v, const Records& R, cudaStream_t s, int threads = kBlock);
 // compression, friction (needs every edge and bend record); then, after the
 // shear records, the row blocks, b and so.dinv
+// the normals, edge and face records, and pc[].status = 0, in one launch
+void launch_state_records(const View& v, const Records& R, const int* nodes, int n, PcgCloth* pc, cudaStream_t s);
 void launch_cross(const View& v, const Records& R, cudaStream_t s);
 void launch_shear_records(const View& v, const Records& R, cudaStream_t s, int threads = kBlock);
 void launch_rows(const View& v, const Records& R, const Solver& so, cudaStream_t s);
