@@ -107,25 +107,28 @@ __global__ void __launch_bounds__(T, T <= 256 ? 2 : 1) k_pcg_cluster(View v, Sol
     for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
     if (lane == 0) slot[q][grp] = t;
   };
-  // the cloth's sums of NQ partials in `slot`, to out: a block is four groups
-  auto total = [&](double (*slot)[kMaxGroups], int nq) {
-    if (wid == 0)
-      for (int q = 0; q < nq; ++q) {
-        double s = 0.0;
-        if (lane < nblk) {
-          double part[4];
+  // the cloth's sum of partials q in `slot`, valid in lane 0: a block is four groups
+  auto sum = [&](double (*slot)[kMaxGroups], int q) {
+    double s = 0.0;
+    if (lane < nblk) {
+      double part[4];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int g = 4 * lane + i, rk = g / groups, lg = g - rk * groups;
-            const double* src = slot[q];
-            if (CLUSTER) src = cg::this_cluster().map_shared_rank(src, rk < csize ? rk : 0);
-            part[i] = rk < csize ? src[lg] : 0.0;
-          }
-          s = four_sum(part[0], part[1], part[2], part[3]);
-        }
-        s = lanes_sum(s, nblk);
-        if (lane == 0) out[q] = s;
+      for (int i = 0; i < 4; ++i) {
+        const int g = 4 * lane + i, rk = g / groups, lg = g - rk * groups;
+        const double* src = slot[q];
+        if (CLUSTER) src = cg::this_cluster().map_shared_rank(src, rk < csize ? rk : 0);
+        part[i] = rk < csize ? src[lg] : 0.0;
       }
+      s = four_sum(part[0], part[1], part[2], part[3]);
+    }
+    return lanes_sum(s, nblk);
+  };
+  // two sums to out, a warp each
+  auto totals = [&](double (*slot)[kMaxGroups]) {
+    if (wid < 2) {
+      const double s = sum(slot, wid);
+      if (lane == 0) out[wid] = s;
+    }
     __syncthreads();
   };
 
@@ -157,7 +160,7 @@ __global__ void __launch_bounds__(T, T <= 256 ? 2 : 1) k_pcg_cluster(View v, Sol
   if (m == 0) dot(gp[0], 0, rs + at, own_nodes, rs + at, own_nodes);
   if (m == 1) dot(gp[0], 1, rs + at, own_nodes, zs + at, own_nodes);
   sync_all();
-  total(gp[red++ & 1], 2);
+  totals(gp[red++ & 1]);
   const double bb = out[0];
   const double thr = pcg_threshold(so.tol, bb);
   double rzc = out[1], rrc = bb;
@@ -177,9 +180,16 @@ __global__ void __launch_bounds__(T, T <= 256 ? 2 : 1) k_pcg_cluster(View v, Sol
     __syncthreads();
     if (m == 3) dot(gp[red & 1], 0, sp + pos, WN, rs + at, own_nodes);
     sync_all();
-    total(gp[red++ & 1], 1);
-    // alpha, x += alpha p, r -= alpha q, |r|^2 and r.z (k_pcg_axpy)
-    const double alpha = rzc / out[0];
+    // alpha, by one warp (a division is some ten FP64 instructions, and every
+    // warp of the CTA would issue them); x += alpha p, r -= alpha q, |r|^2 and
+    // r.z (k_pcg_axpy)
+    if (wid == 0) {
+      const double pq = sum(gp[red & 1], 0);
+      if (lane == 0) out[0] = rzc / pq;
+    }
+    ++red;
+    __syncthreads();
+    const double alpha = out[0];
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       if (i >= nc) break;
@@ -191,7 +201,7 @@ __global__ void __launch_bounds__(T, T <= 256 ? 2 : 1) k_pcg_cluster(View v, Sol
     if (m == 0) dot(gp[red & 1], 0, rs + at, own_nodes, rs + at, own_nodes);
     if (m == 1) dot(gp[red & 1], 1, rs + at, own_nodes, zs + at, own_nodes);
     sync_all();
-    total(gp[red++ & 1], 2);
+    totals(gp[red++ & 1]);
     // the stop test, then beta and p = z + beta p (k_pcg_dir)
     const double rrn = out[0], rzn = out[1];
     const bool conv = rrn < thr;
