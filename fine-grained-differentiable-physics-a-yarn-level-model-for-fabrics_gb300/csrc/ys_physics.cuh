@@ -659,45 +659,77 @@ YS_HD void sym3_min_eigvec(const double S[3][3], double* out) {
   for (int k = 0; k < 3; ++k) out[k] = V[k][m];
 }
 
+// One step of Rayleigh-quotient iteration on a symmetric 3x3 S: x <- adj(S - mu
+// I) x / |.|, mu = x^T S x (the adjugate solves the shifted system up to scale
+// without a division and stays exact when mu hits the eigenvalue); false where
+// x is already exact. Converges cubically.
+template <class F>
+YS_HD bool rqi_step(const F S[3][3], F x[3]) {
+  F Sx[3];
+  for (int i = 0; i < 3; ++i) Sx[i] = S[i][0] * x[0] + S[i][1] * x[1] + S[i][2] * x[2];
+  const F mu = x[0] * Sx[0] + x[1] * Sx[1] + x[2] * Sx[2];
+  const F m00 = S[0][0] - mu, m11 = S[1][1] - mu, m22 = S[2][2] - mu;
+  const F m01 = S[0][1], m02 = S[0][2], m12 = S[1][2];
+  // adjugate of the symmetric M = S - mu I
+  const F c00 = m11 * m22 - m12 * m12, c01 = m02 * m12 - m01 * m22, c02 = m01 * m12 - m02 * m11;
+  const F c11 = m00 * m22 - m02 * m02, c12 = m01 * m02 - m00 * m12, c22 = m00 * m11 - m01 * m01;
+  const F y[3] = {c00 * x[0] + c01 * x[1] + c02 * x[2], c01 * x[0] + c11 * x[1] + c12 * x[2],
+                  c02 * x[0] + c12 * x[1] + c22 * x[2]};
+  const F ny = sqrt(y[0] * y[0] + y[1] * y[1] + y[2] * y[2]);
+  if (!(ny > F(0)) || !isfinite(ny)) return false;
+  const F iy = F(1) / ny;
+  for (int i = 0; i < 3; ++i) x[i] = y[i] * iy;
+  return true;
+}
+
 // Eigenvector of the smallest eigenvalue of a symmetric 3x3 S by Rayleigh-
-// quotient iteration from a guess close to it: x <- adj(S - mu I) x / |.|,
-// mu = x^T S x (the adjugate solves the shifted system up to scale without a
-// division and stays exact when mu hits the eigenvalue). Converges cubically;
-// returns false (out untouched) unless the result is an eigenvector of the
-// smallest eigenvalue to 1e-12 relative, for the caller to fall back on the
-// Jacobi solver.
+// quotient iteration from a guess close to it. Returns false (out untouched)
+// unless the result is an eigenvector of the smallest eigenvalue to 1e-12
+// relative, for the caller to fall back on the Jacobi solver. Bound by the FP64
+// pipe: three steps in FP32 (on S scaled to trace 1) bring the guess to 1e-6,
+// from where one step in FP64 is exact to rounding; up to three more follow
+// where the test asks for them. 255,292 normals take 109 us, 191 with four steps
+// in FP64 (the pipe 89 % busy); one 50 x 50 cloth 16 for 22.
 YS_HD bool sym3_min_eigvec_rqi(const double S[3][3], const double* guess, double* out) {
-  double x[3] = {guess[0], guess[1], guess[2]};
-  double nx = norm3(x);
-  if (!(nx > 0.0)) return false;
-  for (int i = 0; i < 3; ++i) x[i] /= nx;
-  double mu = 0.0;
+  const double tr = S[0][0] + S[1][1] + S[2][2];
+  double x[3];
+  {
+    const float gs = (float)fmax(fabs(guess[0]), fmax(fabs(guess[1]), fabs(guess[2])));
+    float Sf[3][3], xf[3];
+    const float ts = 1.0f / (float)tr, g1 = 1.0f / gs;
+    bool ok = gs > 0.0f && isfinite(g1) && isfinite(ts) && ts > 0.0f;
+    for (int i = 0; i < 3; ++i) {
+      xf[i] = (float)guess[i] * g1;
+      for (int j = 0; j < 3; ++j) Sf[i][j] = (float)S[i][j] * ts;
+    }
+    const float in = 1.0f / sqrt(xf[0] * xf[0] + xf[1] * xf[1] + xf[2] * xf[2]);
+    for (int i = 0; i < 3; ++i) xf[i] *= in;
+    for (int it = 0; it < 3 && ok; ++it)
+      if (!rqi_step(Sf, xf)) break;
+    const float n2 = xf[0] * xf[0] + xf[1] * xf[1] + xf[2] * xf[2];
+    ok = ok && n2 > 0.5f && n2 < 2.0f;
+    if (ok) {
+      for (int i = 0; i < 3; ++i) x[i] = xf[i];
+    } else {  // out of FP32's range
+      const double nx = norm3(guess);
+      if (!(nx > 0.0)) return false;
+      for (int i = 0; i < 3; ++i) x[i] = guess[i] / nx;
+    }
+  }
+  const double sc = fabs(S[0][0]) + fabs(S[1][1]) + fabs(S[2][2]) + 1e-300;
+  double mu = 0.0, r2 = 0.0;
   for (int it = 0; it < 4; ++it) {
+    const bool more = rqi_step(S, x);
     double Sx[3];
     for (int i = 0; i < 3; ++i) Sx[i] = S[i][0] * x[0] + S[i][1] * x[1] + S[i][2] * x[2];
     mu = dot3(x, Sx);
-    const double m00 = S[0][0] - mu, m11 = S[1][1] - mu, m22 = S[2][2] - mu;
-    const double m01 = S[0][1], m02 = S[0][2], m12 = S[1][2];
-    // adjugate of the symmetric M = S - mu I
-    const double c00 = m11 * m22 - m12 * m12, c01 = m02 * m12 - m01 * m22, c02 = m01 * m12 - m02 * m11;
-    const double c11 = m00 * m22 - m02 * m02, c12 = m01 * m02 - m00 * m12, c22 = m00 * m11 - m01 * m01;
-    double y[3] = {c00 * x[0] + c01 * x[1] + c02 * x[2], c01 * x[0] + c11 * x[1] + c12 * x[2],
-                   c02 * x[0] + c12 * x[1] + c22 * x[2]};
-    const double ny = norm3(y);
-    if (!(ny > 0.0) || !isfinite(ny)) break;  // x is already exact
-    const double iy = 1.0 / ny;
-    for (int i = 0; i < 3; ++i) x[i] = y[i] * iy;
+    r2 = 0.0;
+    for (int i = 0; i < 3; ++i) r2 += (Sx[i] - mu * x[i]) * (Sx[i] - mu * x[i]);
+    if (!more || r2 <= 1e-30 * sc * sc) break;
   }
-  double Sx[3];
-  for (int i = 0; i < 3; ++i) Sx[i] = S[i][0] * x[0] + S[i][1] * x[1] + S[i][2] * x[2];
-  mu = dot3(x, Sx);
-  const double sc = fabs(S[0][0]) + fabs(S[1][1]) + fabs(S[2][2]) + 1e-300;
-  double r2 = 0.0;
-  for (int i = 0; i < 3; ++i) r2 += (Sx[i] - mu * x[i]) * (Sx[i] - mu * x[i]);
   if (!(r2 <= 1e-24 * sc * sc)) return false;
   // mu is the smallest eigenvalue iff the other two, l2 + l3 = tr - mu and
   // l2 l3 = e2 - mu (tr - mu), are both >= mu
-  const double tr = S[0][0] + S[1][1] + S[2][2];
   const double e2 = S[0][0] * S[1][1] + S[0][0] * S[2][2] + S[1][1] * S[2][2] - S[0][1] * S[0][1] -
                     S[0][2] * S[0][2] - S[1][2] * S[1][2];
   const double sum = tr - mu, prod = e2 - mu * sum;
@@ -726,13 +758,10 @@ YS_HD void node_normal(const View& v, int n, int W) {
   // eigenvector of their scatter S; warp x weft is a close starting guess
   double nn[3];
   if (!sym3_min_eigvec_rqi(S, cr, nn)) sym3_min_eigvec(S, nn);
-  const double len = norm3(nn);
-  for (int i = 0; i < 3; ++i) nn[i] /= len;
-  if (dot3(cr, nn) / (norm3(cr) * norm3(nn)) < 0)
-    for (int i = 0; i < 3; ++i) nn[i] = -nn[i];
-  if (v.flags[n] & YS_FLIP)
-    for (int i = 0; i < 3; ++i) nn[i] = -nn[i];
-  for (int i = 0; i < 3; ++i) st(v.NRM, i, nt, n) = nn[i];
+  const double len = norm3(nn), il = 1.0 / len;
+  for (int i = 0; i < 3; ++i) nn[i] = quot(nn[i], len, il);
+  const bool flip = (dot3(cr, nn) < 0) != ((v.flags[n] & YS_FLIP) != 0);
+  for (int i = 0; i < 3; ++i) st(v.NRM, i, nt, n) = flip ? -nn[i] : nn[i];
 }
 
 // How the unit eigenvector n of a scatter matrix's smallest eigenvalue l_m moves:
