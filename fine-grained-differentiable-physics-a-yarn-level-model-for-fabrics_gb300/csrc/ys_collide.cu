@@ -570,8 +570,6 @@ struct ys_collider {
   DVec<Impact> slots;
   DVec<int64_t> icount, ioffset;
   DVec<int> tmask;  // narrow phase: the tests each pair runs (bit t)
-  DVec<int64_t> tlist, tlist_n;  // and their lists, vertex-face, edge-edge, with the lengths
-  DVec<float4> nfbox;
   DVec<Kdop> nkdop;  // narrow phase: every node's motion k-DOP (cloth, then obstacle)
   DVec<ys_impact> impacts;
   int64_t nimpacts = 0;
@@ -676,7 +674,7 @@ ys_status scan(ys_collider* c, const int64_t* counts, int64_t n, int64_t* off, i
                const int* flag = nullptr, int* flag_host = nullptr) {
   const int64_t nb = (n + kScanTile - 1) / kScanTile;
   YC_CUDA(c->sums.reserve(std::max<int64_t>(nb, 1)));
-  YC_CUDA(c->total.reserve(1));
+  YC_CUDA(c->total.reserve(4));
   c->pin[0] = 0;
   c->pin[1] = 0;
   if (n > 0) {
@@ -794,29 +792,33 @@ ys_status broad_phase(ys_collider* c, bool masked) {
 // the narrow phase's buffers for n pairs
 ys_status narrow_reserve(ys_collider* c, int64_t n) {
   const int nn = std::max(c->n_nodes + c->n_obs_nodes, 1);
-  YC_CUDA(c->slots.reserve(15 * (size_t)n));
+  // (the lists of tests follow the slots, the widened boxes the k-DOPs, the
+  // lists' lengths the totals: no allocation of their own)
+  YC_CUDA(c->slots.reserve(15 * (size_t)n + (15 * sizeof(int64_t) * (size_t)n + sizeof(Impact) - 1) / sizeof(Impact)));
   YC_CUDA(c->icount.reserve(n));
   YC_CUDA(c->ioffset.reserve(n));
   YC_CUDA(c->tmask.reserve(n));
-  YC_CUDA(c->tlist.reserve(15 * (size_t)n));
-  YC_CUDA(c->tlist_n.reserve(2));
-  YC_CUDA(c->nkdop.reserve(nn));
-  YC_CUDA(c->nfbox.reserve(kFBox * (size_t)nn));
+  YC_CUDA(c->total.reserve(4));
+  YC_CUDA(c->nkdop.reserve(nn + (kFBox * sizeof(float4) * nn + sizeof(Kdop) - 1) / sizeof(Kdop)));
   return YS_OK;
 }
 // the tests of n pairs (np_dev: their number on the device, at most n)
 void narrow_kernels(ys_collider* c, int64_t n, const int64_t* np_dev) {
   CMesh m{c->x.p, c->xp.p, c->ox.p, c->oxp.p};
   const int nn = c->n_nodes + c->n_obs_nodes;
-  k_node_kdop<<<(nn + 127) / 128, 128, 0, c->stream>>>(m, c->n_nodes, c->n_obs_nodes, c->ccd, c->nkdop.p, c->nfbox.p,
-                                                       c->tlist_n.p);
+  static_assert(alignof(Impact) >= alignof(int64_t) && sizeof(Kdop) % sizeof(float4) == 0, "lists behind slots and boxes");
+  int64_t* list = reinterpret_cast<int64_t*>(c->slots.p + 15 * n);
+  int64_t* list_n = c->total.p + 2;
+  float4* fbox = reinterpret_cast<float4*>(c->nkdop.p + nn);
+  k_node_kdop<<<(nn + 127) / 128, 128, 0, c->stream>>>(m, c->n_nodes, c->n_obs_nodes, c->ccd, c->nkdop.p, fbox,
+                                                       list_n);
   k_narrow_mask<<<(unsigned)((n + 127) / 128), 128, 0, c->stream>>>(
-      c->pairs.p, n, c->faces.p, c->ofaces.p, NodeKdops{c->nkdop.p, c->nfbox.p, c->n_nodes}, c->thickness,
-      prune1(c->thickness), prune2(c->thickness), c->tmask.p, c->icount.p, c->tlist.p,
-      reinterpret_cast<unsigned long long*>(c->tlist_n.p), np_dev);
+      c->pairs.p, n, c->faces.p, c->ofaces.p, NodeKdops{c->nkdop.p, fbox, c->n_nodes}, c->thickness,
+      prune1(c->thickness), prune2(c->thickness), c->tmask.p, c->icount.p, list,
+      reinterpret_cast<unsigned long long*>(list_n), np_dev);
   const int64_t blocks = std::min<int64_t>((15 * n + 127) / 128, kTestBlocks);
-  k_narrow_test<<<(unsigned)blocks, 128, 0, c->stream>>>(c->pairs.p, n, c->faces.p, c->ofaces.p, m, c->tlist.p,
-                                                         c->tlist_n.p, c->slots.p,
+  k_narrow_test<<<(unsigned)blocks, 128, 0, c->stream>>>(c->pairs.p, n, c->faces.p, c->ofaces.p, m, list, list_n,
+                                                         c->slots.p,
                                                          reinterpret_cast<unsigned long long*>(c->icount.p));
 }
 
@@ -860,7 +862,7 @@ ys_status detect_one_wait(ys_collider* c, bool masked, std::vector<ys_impact>& g
     const int64_t cp = c->cap_pairs[kind], ci = c->cap_imp[kind];
     const int64_t nb = (std::max<int64_t>(work, cp) + kScanTile - 1) / kScanTile;
     YC_CUDA(c->sums.reserve(std::max<int64_t>(nb, 1)));
-    YC_CUDA(c->total.reserve(2));
+    YC_CUDA(c->total.reserve(4));
     YC_CUDA(c->pairs.reserve(3 * (size_t)cp));
     s = narrow_reserve(c, cp);
     if (s != YS_OK) return s;
