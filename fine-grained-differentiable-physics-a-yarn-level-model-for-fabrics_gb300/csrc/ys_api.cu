@@ -1822,6 +1822,8 @@ ys_status ys_set_pcg_schedule(ys_batch* b, int32_t pcg, int32_t threads, int32_t
   if (P.max_nodes > threads * cluster)
     return fail(YS_ERR_ARG, "ys_set_pcg_schedule: the largest cloth has " + std::to_string(P.max_nodes) +
                                 " nodes, more than threads x cluster");
+  if (!P.shape.groups && P.max_nodes <= ys::kClusterMaxNodes)
+    return fail(YS_ERR_ARG, "ys_set_pcg_schedule: this GPU cannot run a cluster of that shape");
   // where no cluster holds the largest cloth: the phases, the same bits
   P.kind = P.shape.groups ? YS_PCG_PERSISTENT : YS_PCG_PHASES;
   P.threads = threads;

@@ -55,11 +55,10 @@ YS_HD bool finite_(double x) {
 // towards that neighbour give to the node's own block, and owns the blocks
 // towards the neighbour, towards the next crossing beyond it and towards one
 // diagonal neighbour. No record is read by two parts except a bend segment's
-// L12 and forces (by the two parts along its yarn). On the device four lanes
-// of a warp (lanes i, i + 8, i + 16, i + 24 for node i of eight) run the parts
-// of a node and combine the sums by shuffles, so a small cloth has four times
-// the threads and a quarter of the chain; combined in the same order on the
-// host and for the tangents.
+// L12 and forces (by the two parts along its yarn). On the device four warps
+// run the parts of 32 nodes and combine the sums through shared memory, so a
+// small cloth has four times the threads and a quarter of the chain; combined
+// in the same order on the host.
 YS_HD int part_k(int m) { return m >> 1; }
 YS_HD int part_dir(int m) { return (m & 1) ? 1 : -1; }
 

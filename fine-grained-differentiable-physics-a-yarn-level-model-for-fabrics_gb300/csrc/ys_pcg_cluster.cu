@@ -307,13 +307,14 @@ static cudaError_t cluster_fit(const ClusterShape& sh, int sms, int* clusters) {
 // turns. Steps of 17 x 17 cloths with 1, 2, 3, 5, 8 groups, us (cost): one
 // cloth 352, 394, 447, 566, 738 (3.5 to 10.5); 24 cloths 587, 531, 473, 593, 766
 // (10.5, 9, 5.5, 7.5, 10.5); 64 cloths 1247, 950, 840, 705, 870 (24, 18, 11,
-// 7.5, 10.5); 256 cloths 4428, 3244, 3001, 2442, 3107 (94, 63, 38, 30, 42).
+// 7.5, 10.5); 256 cloths 4428, 3244, 3001, 2442, 3107 (94, 63, 38, 30, 42)
+// (measured before the window and the sums took their present form).
 //
-// And the schedule: 1.8 us a unit of cost, 2.4 where CTAs take turns, against
-// the phases' 20 us an iteration and 0.65 ns a node. Steps in a graph, us,
-// persistent / phases: 1 x 17 x 17 281 / 800, 24 of them 407 / 850, 64 654 /
-// 1033, 256 2409 / 2310, 1,024 8471 / 7379; 1 x 64 x 64 737 / 810; 8 x 50 x 50
-// 1143 / 1061, 64 of them 5872 / 3989.
+// And the schedule: 1.6 us a unit of cost, 2.05 where CTAs take turns, against
+// the phases' 16 us an iteration and 0.62 ns a node. Steps in a graph, us,
+// persistent / phases: 1 x 5 x 5 202 / 520, 1 x 17 x 17 245 / 591, 24 of them 369
+// / 664, 64 568 / 878, 256 2047 / 2233; 1 x 50 x 50 449 / 628, 8 of them 981 /
+// 901, 64 5010 / 3915; 1 x 64 x 64 640 / 637 (launch by launch 706 / 732).
 cudaError_t pcg_cluster_shape(const ClothParams* cp, int ncloth, int device, ClusterShape* out) {
   ClusterShape best{};
   *out = best;
@@ -345,7 +346,7 @@ cudaError_t pcg_cluster_shape(const ClothParams* cp, int ncloth, int device, Clu
     const int64_t ctas = (int64_t)ncloth * sh.csize, turns = (ctas + sms - 1) / sms, waves = (ncloth + fit - 1) / fit;
     const int64_t rounds = turns > waves ? turns : waves;
     sh.cost = (double)rounds * (g + 2.5);
-    sh.faster = (rounds > 1 ? 2.4 : 1.8) * sh.cost < 20.0 + 0.65e-3 * (double)nodes;
+    sh.faster = (rounds > 1 ? 2.05 : 1.6) * sh.cost < 16.0 + 0.62e-3 * (double)nodes;
     if (!best.groups || sh.cost < best.cost) best = sh;
   }
   *out = best;
