@@ -160,7 +160,7 @@ constexpr int kE_fe = 44;   // [2]     F_E before friction
 constexpr int kE_kee = 46;  // [2]     dF_E/dE, position
 constexpr int kE_dee = 48;  // [2]     dF_E/dE, velocity
 constexpr int kE_cl = 50;   //         crimp compression: +cl d at n0, -cl d at n1
-constexpr int kE_cle = 51;  //         its Eulerian derivative: cle d at the interior ends
+constexpr int kE_cle = 51;  //         its Eulerian derivative: cle d at the interior ends, of the sign of du
 constexpr int kEdgeFields = 52;
 
 template <class T>
@@ -241,7 +241,7 @@ YS_HD void edge_terms(const EdgeIn<T>& s, const ClothParams& P, int k, double h,
   {
     const double sgn = (k == 0) ? 1.0 : -1.0;
     put(kE_cl, sgn * strf);
-    put(kE_cle, sgn * (ksw * nw));
+    put(kE_cle, sgn * (ksi * nw));
     put(kE_lP, mh2 * (ks * il));
     for (int i = 0; i < 3; ++i) put(kE_d + i, d[i]);
   }
