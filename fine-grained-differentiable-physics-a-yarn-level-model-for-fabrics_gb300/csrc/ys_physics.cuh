@@ -85,6 +85,15 @@ YS_HD Dual<K> quot(const Dual<K>& x, const Dual<K>& l, const Dual<K>& il) {
   for (int k = 0; k < K; ++k) r.d[k] = (x.d[k] - r.v * l.d[k]) * il.v;
   return r;
 }
+// sqrt(x) from x and ix = 1 / sqrt(x), correctly rounded but for rare ties
+YS_HD double root(double x, double ix) {
+  const double l = x * ix;
+  return fma(fma(-l, l, x), 0.5 * ix, l);
+}
+template <int K>
+YS_HD Dual<K> root(const Dual<K>& x, const Dual<K>& ix) {
+  return chain(x, root(x.v, ix.v), 0.5 * ix.v);
+}
 YS_HD double ld(const double* p, int comp, int ntot, int node) { return p[(int64_t)comp * ntot + node]; }
 YS_HD double& st(double* p, int comp, int ntot, int node) { return p[(int64_t)comp * ntot + node]; }
 
@@ -229,11 +238,13 @@ YS_HD void edge_terms(const EdgeIn<T>& s, const ClothParams& P, int k, double h,
   const T(&e)[2] = s.e;
   const double mh2 = -(h * h);
   const T idu = 1.0 / du, aidu = fabs(idu);
-  const T il = rsqrt_(dot3(dx, dx));
+  const T d2 = dot3(dx, dx), il = rsqrt_(d2);
   T w[3], d[3];
   for (int i = 0; i < 3; ++i) { w[i] = dx[i] * idu; d[i] = dx[i] * il; }
-  const T ww = dot3(w, w);
-  const T nw = (dot3(dx, dx) * il) * aidu;  // |w|
+  // |w|, rounded as a square root and a division: exactly 1 at rest, whatever
+  // the spacing, so that a resting yarn has no stretch force
+  const T nw = quot(root(d2, il), T(fabs(du)), aidu);
+  const T ww = nw * nw;
   const T r6 = (1.0 / 6.0) * rho, q = r6 * du;
   const T zero = T(0.0);
   // ---- stretch scalars; the crimp accumulators
