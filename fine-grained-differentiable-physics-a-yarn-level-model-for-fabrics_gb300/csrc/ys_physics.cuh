@@ -695,7 +695,7 @@ YS_HD bool rqi_step(const F S[3][3], F x[3]) {
 
 // Eigenvector of the smallest eigenvalue of a symmetric 3x3 S by Rayleigh-
 // quotient iteration from a guess close to it. Returns false (out untouched)
-// unless the result is an eigenvector of the smallest eigenvalue to 1e-12
+// unless the result is an eigenvector of the smallest eigenvalue to 1e-15
 // relative, for the caller to fall back on the Jacobi solver. Bound by the FP64
 // pipe: three steps in FP32 (on S scaled to trace 1) bring the guess to 1e-6,
 // from where FP64 steps go on: a second one unless the first left a residual
@@ -744,7 +744,7 @@ YS_HD bool sym3_min_eigvec_rqi(const double S[3][3], const double* guess, double
     for (int i = 0; i < 3; ++i) r2 += (Sx[i] - mu * x[i]) * (Sx[i] - mu * x[i]);
     if (!more || r2 <= (it == 0 ? 3e-34 : 1e-30) * sc * sc) break;
   }
-  if (!(r2 <= 1e-24 * sc * sc)) return false;
+  if (!(r2 <= 1e-30 * sc * sc)) return false;
   // mu is the smallest eigenvalue iff the other two, l2 + l3 = tr - mu and
   // l2 l3 = e2 - mu (tr - mu), are both >= mu
   const double e2 = S[0][0] * S[1][1] + S[0][0] * S[2][2] + S[1][1] * S[2][2] - S[0][1] * S[0][1] -
