@@ -38,25 +38,6 @@ YS_HD void cross3(const T* a, const T* b, T* o) {
   o[1] = a[2] * b[0] - a[0] * b[2];
   o[2] = a[0] * b[1] - a[1] * b[0];
 }
-template <class T>
-YS_HD void proj3(const T* d, T P[3][3]) {
-  for (int i = 0; i < 3; ++i)
-    for (int j = 0; j < 3; ++j) P[i][j] = (i == j ? 1.0 : 0.0) - d[i] * d[j];
-}
-template <class T>
-YS_HD void matvec3(const T P[3][3], const T* a, T* o) {
-  for (int i = 0; i < 3; ++i) o[i] = P[i][0] * a[0] + P[i][1] * a[1] + P[i][2] * a[2];
-}
-template <class T>
-YS_HD void outer3(const T* a, const T* b, T O[3][3]) {
-  for (int i = 0; i < 3; ++i)
-    for (int j = 0; j < 3; ++j) O[i][j] = a[i] * b[j];
-}
-template <class T>
-YS_HD void matmul3(const T A[3][3], const T B[3][3], T O[3][3]) {
-  for (int i = 0; i < 3; ++i)
-    for (int j = 0; j < 3; ++j) O[i][j] = A[i][0] * B[0][j] + A[i][1] * B[1][j] + A[i][2] * B[2][j];
-}
 // 1 / sqrt(x): one device instruction sequence instead of a square root and a
 // division (1 ulp)
 YS_HD double rsqrt_(double x) {
