@@ -3,6 +3,8 @@
 
 #include <cuda_runtime.h>
 
+#include <utility>
+
 #include "ys_items.cuh"
 
 namespace ys {
@@ -25,8 +27,10 @@ struct PcgCloth {
 // then lets the next be set up. Some 2 us a launch of a kernel of 4 to 8 us:
 // steps of 24 ragged cloths 1.15 -> 0.97 ms, a 61 x 83 system 1.11 -> 0.87. In a
 // capture they are plain nodes: a graph's own edges were faster (100 x 100 0.68
-// ms for 0.71 with programmatic edges), and kernels of batches that fill the GPU
-// are not chained.
+// ms for 0.71 with programmatic edges). The PCG's product, axpy and direction of
+// batches that fill the GPU are not chained (256 cloths 4.93 ms for 4.96); the
+// assembly, the PCG's set-up, the update and the sensitivities' kernels are,
+// whatever the batch (4.93 ms either way).
 __device__ __forceinline__ void chained() {
 #if defined(__CUDA_ARCH__)
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -45,7 +49,9 @@ inline void chain(void (*k)(P...), dim3 grid, unsigned block, cudaStream_t s, A&
   cfg.attrs = at;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   cfg.numAttrs = cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone ? 1 : 0;
-  cudaLaunchKernelEx(&cfg, k, P(a)...);
+  // (arguments convert as in a call; an error stays the runtime's last error, which
+  // every entry point reads after its launches)
+  cudaLaunchKernelEx(&cfg, k, std::forward<A>(a)...);
 }
 
 // sum over a warp, the same bits in every lane
