@@ -249,10 +249,10 @@ PERSIST_DRAM_BYTES_PER_ROW_PASS = None
 
 
 def schedule_name(c):
-    """'graph|launch/phases-every-E/producers-P' or 'graph|launch/persistent-TxC/producers-P'."""
+    """'graph|launch/phases-every-E/producers-P' or 'graph|launch/persistent/producers-P'."""
     g = "graph" if c["graphs"] else "launch"
     if c["pcg"] == "persistent":
-        return "%s/persistent-%dx%d/producers-%d" % (g, c["pcg_threads"], c["pcg_cluster"], c["producer_threads"])
+        return "%s/persistent/producers-%d" % (g, c["producer_threads"])
     return "%s/phases-every-%d/producers-%d" % (g, c["check_every"], c["producer_threads"])
 
 
@@ -503,8 +503,7 @@ def main():
     ap.add_argument("--schedule", default="auto", choices=["auto", "graph", "launch", "persistent"],
                     help="auto: ys_autotune picks graph or launch-by-launch steps and the PCG schedule; "
                          "graph: one CUDA graph launch per step (conditional PCG loop); launch: kernel by kernel; "
-                         "persistent: kernel by kernel with the persistent PCG (512-thread CTAs, the smallest "
-                         "cluster that holds the largest cloth)")
+                         "persistent: kernel by kernel with the persistent PCG")
     args = ap.parse_args()
 
     world = int(os.environ.get("WORLD_SIZE", "1"))
@@ -555,10 +554,8 @@ def main():
         batch.set_winds(wind_at(wind, 0))
         sched = batch.autotune(H, tol=TOL, steps=3)
         config["schedule"] = {"chosen_by": "ys_autotune", "graph": sched["graphs"],
-                              "check_every": sched["check_every"], "pcg": sched["pcg"]}
+                              "check_every": sched["check_every"]}
         config["schedule"]["producer_threads"] = sched["producer_threads"]
-        if sched["pcg"] == "persistent":
-            config["schedule"].update(pcg_threads=sched["pcg_threads"], pcg_cluster=sched["pcg_cluster"])
         config["schedule"]["timed_ms_per_step"] = {schedule_name(c): round(c["ms_per_step"], 4)
                                                    for c in sched["candidates"]}
     elif args.schedule == "persistent":
@@ -567,12 +564,15 @@ def main():
         while 512 * cl < big:
             cl *= 2
         batch.set_pcg_schedule(True, 512, cl)
-        config["schedule"] = {"chosen_by": "flag", "graph": False, "pcg": "persistent", "pcg_threads": 512,
-                              "pcg_cluster": cl}
+        config["schedule"] = {"chosen_by": "flag", "graph": False}
     else:
         batch.use_graphs(args.schedule == "graph")
-        config["schedule"] = {"chosen_by": "flag", "graph": args.schedule == "graph", "check_every": 16,
-                              "pcg": "phases"}
+        batch.set_pcg_schedule(False)
+        config["schedule"] = {"chosen_by": "flag", "graph": args.schedule == "graph", "check_every": 16}
+    runs = batch.pcg_schedule()
+    config["schedule"]["pcg"] = runs["pcg"]
+    if runs["pcg"] == "persistent":
+        config["schedule"].update(pcg_threads=runs["threads"], pcg_cluster=runs["cluster"])
 
     def barrier():
         if dist is not None:
@@ -721,7 +721,7 @@ def main():
         # launch over every node of a 64-cloth batch, divided by its row passes
         tr = PERSIST_DRAM_BYTES_PER_ROW_PASS
         roofline = {"kernel": "k_pcg_cluster (persistent per-cloth Jacobi-PCG, %d x %d threads per cloth)" %
-                              (config["schedule"].get("pcg_cluster", 0), config["schedule"].get("pcg_threads", 0)),
+                              (runs["cluster"], runs["threads"]),
                     "bound": "hbm", "achieved": persist["gbs"], "peak": hbm_peak, "unit": "GB/s",
                     "frac": persist["gbs"] / hbm_peak, "peak_source": peak_kind,
                     "traffic": tr * n if tr else None,

@@ -311,8 +311,8 @@ class ClothBatch:
         N.check(N.load().ys_use_graphs(self._h, int(bool(enable))), "ys_use_graphs")
 
     def set_producer_threads(self, threads: int):
-        """Block size of the element-record producers and the gather (64..256;
-        results do not depend on it; see ys_set_producer_threads)."""
+        """Block size of the element-record producers (64..256; results do not
+        depend on it; see ys_set_producer_threads)."""
         N.check(N.load().ys_set_producer_threads(self._h, int(threads)), "ys_set_producer_threads")
 
     def set_pcg_schedule(self, persistent: bool, threads: int = 0, cluster: int = 0):
@@ -322,6 +322,13 @@ class ClothBatch:
         to be faster (see ys_set_pcg_schedule)."""
         N.check(N.load().ys_set_pcg_schedule(self._h, 1 if persistent else 0, int(threads), int(cluster)),
                 "ys_set_pcg_schedule")
+
+    def pcg_schedule(self) -> dict:
+        """What the solves run: pcg ("phases" or "persistent") and, persistent,
+        the threads of a CTA and the CTAs of a cloth (see ys_get_pcg_schedule)."""
+        v = [ctypes.c_int32() for _ in range(3)]
+        N.check(N.load().ys_get_pcg_schedule(self._h, *[ctypes.byref(x) for x in v]), "ys_get_pcg_schedule")
+        return dict(pcg="persistent" if v[0].value == 1 else "phases", threads=v[1].value, cluster=v[2].value)
 
     def normals(self) -> np.ndarray:
         """Node normals [total_nodes, 3] of the current positions (zero on boundary nodes)."""

@@ -198,9 +198,8 @@ struct ys_batch {
   // start first
   struct PcgPlan {
     int kind = YS_PCG_PHASES;
-    int threads = 0, csize = 0;  // as the caller gave them
-    ys::ClusterShape shape{};  // what runs
-    int* order = nullptr;      // device [ncloth]
+    ys::ClusterShape shape{};
+    int* order = nullptr;  // device [ncloth]
     int max_nodes = 0;
   } plan;
   std::vector<ys_schedule> tuned;  // every schedule the last ys_autotune timed
@@ -1826,9 +1825,16 @@ ys_status ys_set_pcg_schedule(ys_batch* b, int32_t pcg, int32_t threads, int32_t
     return fail(YS_ERR_ARG, "ys_set_pcg_schedule: this GPU cannot run a cluster of that shape");
   // where no cluster holds the largest cloth: the phases, the same bits
   P.kind = P.shape.groups ? YS_PCG_PERSISTENT : YS_PCG_PHASES;
-  P.threads = threads;
-  P.csize = cluster;
   b->graph.built = false;
+  return YS_OK;
+}
+
+ys_status ys_get_pcg_schedule(const ys_batch* b, int32_t* pcg, int32_t* threads, int32_t* cluster) {
+  if (!b) return fail(YS_ERR_ARG, "null handle");
+  const bool on = b->plan.kind == YS_PCG_PERSISTENT;
+  if (pcg) *pcg = b->plan.kind;
+  if (threads) *threads = on ? ys::cluster_threads(b->plan.shape) : 0;
+  if (cluster) *cluster = on ? b->plan.shape.csize : 0;
   return YS_OK;
 }
 
@@ -1889,7 +1895,7 @@ ys_status ys_step_graphed(ys_batch* b, double h, const double* ext_force, int32_
 
 // The schedule tuner: every candidate (whole-step graph or launch by launch;
 // phase PCG with its iterations between convergence checks, or the persistent
-// per-cloth PCG in one cluster shape) runs the same steps from the same state
+// per-cloth PCG) runs the same steps from the same state
 // and gives bit-identical results -- the choices only move launches, host
 // synchronisations and which threads do the same arithmetic -- so the tuner
 // times each on a snapshot of the state, restores it, and keeps the fastest.
@@ -1913,7 +1919,7 @@ ys_status ys_autotune(ys_batch* b, double h, const ys_solve_opts* opts, int32_t 
     return cudaSuccess;
   };
   const bool was_graph = b->graph.enabled, was_prof = b->profiling;
-  const ys_batch::PcgPlan was_plan = b->plan;
+  const int was_kind = b->plan.kind;
   const int was_pt = b->producer_threads;
   b->profiling = false;
   // the candidates
@@ -2005,9 +2011,7 @@ ys_status ys_autotune(ys_batch* b, double h, const ys_solve_opts* opts, int32_t 
   b->assembled = false;
   if (ce != cudaSuccess || st != YS_OK || top.ms_per_step < 0) {
     b->graph.enabled = was_graph;
-    b->plan.kind = was_plan.kind;
-    b->plan.threads = was_plan.threads;
-    b->plan.csize = was_plan.csize;
+    b->plan.kind = was_kind;
     b->producer_threads = was_pt;
     b->graph.built = false;
     if (ce != cudaSuccess) return fail(YS_ERR_CUDA, std::string("ys_autotune: ") + cudaGetErrorString(ce));

@@ -135,6 +135,7 @@ struct ClusterShape {
   double cost;  // of an iteration, in units of a group's product
   bool faster;  // than the phases
 };
+inline int cluster_threads(const ClusterShape& sh) { return 4 * 32 * sh.groups; }  // of a CTA
 // the shape for these cloths (host array); enables its kernels, so outside any capture
 cudaError_t pcg_cluster_shape(const ClothParams* cp, int ncloth, int device, ClusterShape* out);
 // right-hand sides of one launch: rhs k at b + k b_rhs ([5][ntot]), its solution

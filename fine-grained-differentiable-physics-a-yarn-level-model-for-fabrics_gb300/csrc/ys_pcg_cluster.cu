@@ -42,7 +42,7 @@ namespace {
 constexpr int kMaxGroups = 8;      // groups of a CTA
 constexpr int kMaxCluster = 16;    // CTAs of a cluster
 constexpr int kMaxBlocks = kMaxCluster * kMaxGroups / 4;  // 128-node blocks of a cloth: one per lane
-static_assert(kMaxBlocks <= 32, "one block partial per lane");
+static_assert(kMaxBlocks <= 32 && kGroup == 32, "one block partial per lane");
 static_assert(kMaxCluster * kMaxGroups * kGroup == kClusterMaxNodes, "nodes of a cluster");
 
 // the window of a CTA: the nodes [lo, hi) of the cloth that the stencils of its
@@ -263,7 +263,7 @@ cudaError_t with_kernel(int groups, bool cluster, bool trans, F&& f) {
 
 void config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at, const ClusterShape& sh, int ncl, int nrhs) {
   cfg.gridDim = dim3((unsigned)(ncl * sh.csize), (unsigned)nrhs);
-  cfg.blockDim = dim3((unsigned)(sh.groups * 4 * kGroup));
+  cfg.blockDim = dim3((unsigned)cluster_threads(sh));
   cfg.dynamicSmemBytes = sh.shared;
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = (unsigned)sh.csize;
@@ -291,7 +291,7 @@ static cudaError_t cluster_fit(const ClusterShape& sh, int sms, int* clusters) {
       if (sh.csize > 1) {
         r = cudaOccupancyMaxActiveClusters(&fit, k, &cfg);
       } else {
-        r = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, k, sh.groups * 4 * kGroup, sh.shared);
+        r = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, k, cluster_threads(sh), sh.shared);
         fit *= sms;
       }
       if (r == cudaSuccess) *clusters = trans == 0 || fit < *clusters ? fit : *clusters;
