@@ -241,7 +241,7 @@ def measure_fp64_peak(torch):
 # divided by the batch's nodes. The counts depend on the state only through
 # branch outcomes and on the sizes through the share of boundary nodes, so
 # they carry over to the 256-cloth batch to within a few per cent.
-ASSEMBLY_FP64_FLOPS_PER_NODE = {"geom": 304.3, "edges": 1483.3, "bends": 1032.7, "faces": 155.5,
+ASSEMBLY_FP64_FLOPS_PER_NODE = {"geom": 304.3, "edges": 1522.1, "bends": 1032.7, "faces": 155.5,
                                 "gather": 482.5, "shear": 2467.2, "finalize": 1108.0}
 # DRAM bytes (read + write) of the persistent solve per pass over the rows
 # (not captured: the tuner does not pick the persistent PCG for this batch)

@@ -33,8 +33,9 @@
 // Bound by the FP64 pipe on large cloths and by latency on small ones: about
 // 90,000 FP64 operations a node. Two inputs a thread: the values are evaluated
 // once per pair, and Dual<4> spills (1.8 to 2.7 KB a thread in the edge and
-// shear terms). The whole call, its two solves included, takes 2.57 ms at
-// 17 x 17 and 3.39 ms at 50 x 50; with forward-mode directions compressed by a
+// shear terms). The whole call, its two solves included, takes 0.97 ms at
+// 17 x 17 and 1.98 ms at 50 x 50 (2.57 and 3.39 when these kernels came, before
+// the solves' present form); with forward-mode directions compressed by a
 // 41-colouring over 128 copies of the cloths (512 directions of every element,
 // 3.2 MB of workspace a node) it took 8.5 and 53.6 ms.
 #include "ys_items.cuh"

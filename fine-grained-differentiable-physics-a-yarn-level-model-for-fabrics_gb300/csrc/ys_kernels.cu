@@ -27,10 +27,9 @@ __global__ void k_geom(View v, const int* __restrict__ nodes, int count) {
 }
 
 // The record producers: one thread per element, nothing shared between
-// threads, so any block size gives the same bits; the
-// block size is a schedule choice (up to kMaxProducerBlock threads; up to
-// kBlock for the edges, whose 254 registers spill when compiled for 256-thread
-// blocks).
+// threads, so any block size gives the same bits; the block size is a schedule
+// choice (up to kMaxProducerBlock threads; the edges are compiled for kBlock,
+// 128 registers a thread).
 
 // one thread per (yarn direction, node): the edge starting at that node
 __device__ __forceinline__ void edge_item(const View& v, const Records& R, int64_t t) {

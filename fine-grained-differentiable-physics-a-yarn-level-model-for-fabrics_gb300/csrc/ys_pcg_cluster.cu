@@ -304,17 +304,20 @@ static cudaError_t cluster_fit(const ClusterShape& sh, int sms, int* clusters) {
 // wants least and a batch that fills the GPU most. An iteration takes about
 // groups + 2.5 times a group's product (two cluster barriers and the sums), and
 // the batch as many rounds of it as it has CTAs per SM, or as its clusters take
-// turns. Steps of 17 x 17 cloths with 1, 2, 3, 5, 8 groups, us (cost): one
-// cloth 352, 394, 447, 566, 738 (3.5 to 10.5); 24 cloths 587, 531, 473, 593, 766
-// (10.5, 9, 5.5, 7.5, 10.5); 64 cloths 1247, 950, 840, 705, 870 (24, 18, 11,
-// 7.5, 10.5); 256 cloths 4428, 3244, 3001, 2442, 3107 (94, 63, 38, 30, 42)
-// (measured before the window and the sums took their present form).
+// turns. Steps of 17 x 17 cloths in a graph with 1, 2, 3, 5, 8 groups, us (cost):
+// one cloth 205, 224, 251, 308, 419 (3.5 to 10.5); 24 cloths 371, 324, 302, 358,
+// 467 (10.5, 9, 5.5, 7.5, 10.5); 64 cloths 805, 609, 558, 474, 584 (24, 18, 11,
+// 7.5, 10.5); 256 cloths 2880, 2161, 2023, 1682, 2122 (94, 63, 38, 30, 42).
 //
 // And the schedule: 1.6 us a unit of cost, 2.05 where CTAs take turns, against
 // the phases' 16 us an iteration and 0.62 ns a node. Steps in a graph, us,
-// persistent / phases: 1 x 5 x 5 202 / 520, 1 x 17 x 17 245 / 591, 24 of them 369
-// / 664, 64 568 / 878, 256 2047 / 2233; 1 x 50 x 50 449 / 628, 8 of them 981 /
-// 901, 64 5010 / 3915; 1 x 64 x 64 640 / 637 (launch by launch 706 / 732).
+// persistent / phases: 1 x 5 x 5 173 / 375, 1 x 17 x 17 202 / 473, 24 of them 307
+// / 546, 256 1665 / 1855; 1 x 50 x 50 334 / 507, 7 of them 485 / 681, 64 3742 /
+// 3215; 1 x 64 x 64 435 / 482, 7 of them 706 / 842, 8 1028 / 939. Over sides of 10
+// to 64 and 1 to 256 cloths the persistent PCG was the faster one wherever the
+// rule takes it, in graphs and launch by launch; it leaves the phases to some
+// batches that it would step up to 8 % faster in a graph (8 x 50 x 50 694 / 747)
+// and up to 21 % launch by launch (16 x 50 x 50 1188 / 1443).
 cudaError_t pcg_cluster_shape(const ClothParams* cp, int ncloth, int device, ClusterShape* out) {
   ClusterShape best{};
   *out = best;

@@ -175,7 +175,8 @@ struct EdgeOut {
 // Inertia_D_Pos (1357-1361; the +1 / -3 below), MDotVDot_D_Pos added and with
 // the squared r6 of "- rho / 6 r" (2154-2234), ParaColli_D proportional to the
 // overlap itself. Term by term as the reference writes them, an edge took
-// 1,690 FP64 operations; this form takes about 400.
+// 1,690 FP64 operations; this form takes about 500 (on 255,292 nodes 453 us for
+// 1,044; 443 with |w| rounded once less, see nw).
 // One edge's inputs: dx = x1 - x0, gx = G . (x0 + x1), the velocities a and e
 // of its ends, du, and the yarn's density and stretch stiffness.
 template <class T>
@@ -547,7 +548,7 @@ YS_HD void bend_element(const View& v, double* buf, double* dbuf, int n2, int n0
 // from the face's edges e1, e2 and the sum of its nodes' velocities; f3 =
 // wind_force / 3, the share of each of its three nodes. area n = cr / 2 and
 // area tang = |cr| rel / 2 - vn cr / 2, so one division serves what nine
-// did (FP64 divisions bound the kernel: 59 us for 203 on 256 cloths of 17 x 17).
+// did (FP64 divisions bound the kernel: 59 us for 203 on 255,292 nodes).
 template <class T>
 YS_HD void wind_terms(const ClothParams& P, const T* e1, const T* e2, const T* vs, T* f3) {
   T cr[3], rel[3];

@@ -9,9 +9,10 @@
 // is the element's residual (8 to 12 numbers) and, for friction, the tangents
 // of the gathered forces. Bound by FP64 latency on small cloths (the shear
 // terms' chains at 250 registers). Two 17 x 17 copies with four directions:
-// 5.59 ms a step, five solves included, for 7.26 ms with records and rows over
-// Dual<4>, which spilled 2 to 8 KB a thread and wrote 159 tangents a node and
-// direction; 4.5 KB of buffers a node for 21.
+// 0.96 ms a step (5.59 with the five solves one after another, as when these
+// kernels came), for 7.26 ms with records and rows over Dual<4>, which spilled 2
+// to 8 KB a thread and wrote 159 tangents a node and direction; 4.5 KB of
+// buffers a node for 21.
 #include "ys_items.cuh"
 #include "ys_kernels.cuh"
 
